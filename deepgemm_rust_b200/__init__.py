@@ -37,7 +37,19 @@ def _load():
     return C.CDLL(_LIB_PATH)
 
 
+def _load_binding():
+    """The compiled binding of the operators (csrc/dg_binding.cpp), pointed at the loaded library."""
+    try:
+        from . import _dg_binding
+    except ImportError as e:
+        raise ImportError(f"{os.path.join(_HERE, '_dg_binding.so')} does not load ({e}): build it with "
+                          "`python deepgemm_rust_b200/build.py`. There is no fallback implementation.") from e
+    _dg_binding.bind(_lib._handle, DgError)
+    return _dg_binding
+
+
 _lib = _load()
+_native = _load_binding()
 
 
 class _LpOperand(C.Structure):
@@ -82,30 +94,12 @@ _ctx_num_sms = _proto("dg_ctx_num_sms", C.c_int, _vp, C.POINTER(C.c_int))
 _ctx_stream = _proto("dg_ctx_stream", _vp, _vp)
 _ctx_set_stream = _proto("dg_ctx_set_stream", C.c_int, _vp, _vp)
 _ctx_check_status = _proto("dg_ctx_check_status", C.c_int, _vp)
-_gemm = _proto("dg_fp8_fp4_gemm", C.c_int, _vp, C.POINTER(_LpOperand), C.POINTER(_LpOperand), C.POINTER(_Out), C.POINTER(_Epilogue))
-_gemm_contig = _proto("dg_m_grouped_fp8_fp4_gemm_contiguous", C.c_int, _vp, C.POINTER(_LpOperand), _vp, C.POINTER(_LpOperand),
-                      C.POINTER(_Out), _u32, C.POINTER(_Epilogue))
-_gemm_contig_ends = _proto("dg_m_grouped_fp8_fp4_gemm_contiguous_ends", C.c_int, _vp, C.POINTER(_LpOperand), _vp,
-                           C.POINTER(_LpOperand), C.POINTER(_Out), _u32, C.POINTER(_Epilogue))
 _gemm_contig_static = _proto("dg_m_grouped_fp8_fp4_gemm_contiguous_static", C.c_int, C.c_int, _vp, C.POINTER(_LpOperand), _vp,
                              C.POINTER(_LpOperand), C.POINTER(_Out), _u32, C.POINTER(_Epilogue))
 _static_check_status = _proto("dg_static_check_status", C.c_int, C.c_int, _vp)
-_bf16_gemm = _proto("dg_bf16_gemm", C.c_int, _vp, _vp, _u32, _u32, _vp, _u32, _u32, _u32, C.POINTER(_Out), C.POINTER(_Epilogue))
-_gemm_masked = _proto("dg_m_grouped_fp8_fp4_gemm_masked", C.c_int, _vp, C.POINTER(_LpOperand), _vp, C.POINTER(_LpOperand),
-                      C.POINTER(_Out), _u32, _u32, C.POINTER(_Epilogue))
-_bmm = _proto("dg_fp8_fp4_bmm", C.c_int, _vp, C.POINTER(_LpOperand), C.POINTER(_LpOperand), C.POINTER(_Out), _u32, C.POINTER(_Epilogue))
-_f32 = (_vp, _vp, _u32, _vp, _vp, _u32, _vp, _u32, _u32, _u32, _vp, _u32)
-_gemm_nt = _proto("dg_fp8_gemm_nt", C.c_int, *_f32)
-_gemm_nt_contig = _proto("dg_m_grouped_fp8_gemm_nt_contiguous", C.c_int, *_f32, _vp, _u32)
-_gemm_nt_masked = _proto("dg_m_grouped_fp8_gemm_nt_masked", C.c_int, *_f32, _vp, _u32, _u32)
-_bmm_nt = _proto("dg_fp8_bmm_nt", C.c_int, *_f32, _u32)
 _sf_packed_cols = _proto("dg_sf_packed_cols", _u32, _u32, _u32)
 _sf_aligned_rows = _proto("dg_sf_aligned_rows", _u32, _u32)
 _sf_words = _proto("dg_sf_words", _sz, _u32, _u32, _u32, _u32)
-_cast_fp8 = _proto("dg_cast_bf16_to_fp8_sf", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp)
-_silu_cast = _proto("dg_silu_mul_cast_fp8_sf", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp, _vp)
-_cast_fp4 = _proto("dg_cast_bf16_to_fp4_packed_sf", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, C.c_int, _vp, _vp)
-_transform_sf = _proto("dg_transform_sf", C.c_int, _vp, _vp, _u32, _u32, _u32, _vp)
 _tsf1d = _proto("dg_transform_sf1d_packed_ue8m0", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp)
 _tsf2d = _proto("dg_transform_sf2d_packed_ue8m0", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _vp)
 _tsft = _proto("dg_transform_sf_t_packed_ue8m0", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _vp)
@@ -120,11 +114,6 @@ _peer_open = _proto("dg_peer_open", C.c_int, _vp, C.c_char_p, C.POINTER(_vp))
 _peer_close = _proto("dg_peer_close", C.c_int, _vp, _vp)
 _peer_free = _proto("dg_peer_free", C.c_int, _vp, _vp)
 _ep_hist_words = _proto("dg_ep_block_hist_words", _sz, _u32, _u32)
-_ep_count = _proto("dg_ep_count", C.c_int, _vp, _vp, _u32, _u32, _vp, _vp, _vp)
-_ep_layout = _proto("dg_ep_layout", C.c_int, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _u32, _vp, _vp, _vp)
-_ep_dispatch = _proto("dg_ep_dispatch", C.c_int, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _vp, _u32, _vp, _u32, _u32, _vp, _vp, _u32,
-                      _u32, _u32, _vp, _u32)
-_ep_combine = _proto("dg_ep_combine", C.c_int, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _vp, _sz, _u32, _vp, _sz, _u32)
 _expire_wait = _proto("dg_debug_expire_wait", C.c_int, _vp, _u32)
 _set_mk = _proto("dg_set_mk_alignment_for_contiguous_layout", C.c_int, _u32)
 _get_mk = _proto("dg_get_mk_alignment_for_contiguous_layout", _u32)
@@ -154,6 +143,7 @@ class DgContext:
 
     def __init__(self, ordinal: int = 0, stream: Optional[int] = None, own_stream: bool = False):
         self._h = _vp()
+        self._addr = 0          # the handle as an integer, what the compiled binding reads
         self.ordinal = ordinal
         if own_stream:
             _check(_ctx_create(ordinal, C.byref(self._h)))
@@ -163,6 +153,7 @@ class DgContext:
                     raise DgError(1, "no CUDA device available; this library has no CPU path")
                 stream = torch.cuda.current_stream(ordinal).cuda_stream
             _check(_ctx_create_on_stream(ordinal, _vp(stream), C.byref(self._h)))
+        self._addr = self._h.value
 
     @classmethod
     def new(cls, ordinal: int = 0) -> "DgContext":
@@ -188,6 +179,7 @@ class DgContext:
         if self._h:
             _ctx_destroy(self._h)
             self._h = _vp()
+            self._addr = 0
 
     def __del__(self):
         try:
@@ -263,8 +255,7 @@ def _epi(epi):
 
 def fp8_fp4_gemm_dev(ctx: DgContext, a: LpOperand, b: LpOperand, out: Sm100Out, epi: Optional[Sm100Epilogue] = None):
     """ops_sm100.rs:719"""
-    ca, cb, co, ce = a._c(), b._c(), out._c(), _epi(epi)
-    _check(_gemm(ctx._h, C.byref(ca), C.byref(cb), C.byref(co), C.byref(ce)))
+    _native.gemm(ctx, a, b, out, epi)
 
 
 def fp4_gemm_packed_dev(ctx, a_data: torch.Tensor, a_sf: torch.Tensor, b_data: torch.Tensor, b_sf: torch.Tensor, out: torch.Tensor,
@@ -289,8 +280,7 @@ def fp4_gemm_nt_native(ctx, a_bf16: torch.Tensor, b_bf16: torch.Tensor, m: int, 
 
 def bf16_gemm_dev(ctx, a: torch.Tensor, a_ld: int, m: int, b: torch.Tensor, b_ld: int, n: int, k: int, out, epi=None):
     """ops_sm100.rs:893: D[m,n] = A[m,k] . B[n,k]^T, bf16 K-major operands, f32 accumulation."""
-    co, ce = out._c(), _epi(epi)
-    _check(_bf16_gemm(ctx._h, _vp(a.data_ptr()), a_ld, m, _vp(b.data_ptr()), b_ld, n, k, C.byref(co), C.byref(ce)))
+    _native.bf16_gemm(ctx, a, a_ld, m, b, b_ld, n, k, out, epi)
 
 
 @dataclass
@@ -313,14 +303,12 @@ def bf16_gemm_nt_dev(ctx, a: "Bf16Tensor", b: "Bf16Tensor", out: torch.Tensor, o
 
 def m_grouped_fp8_fp4_gemm_contiguous_dev(ctx, a, m_indices: torch.Tensor, b, out, num_groups: int, epi=None):
     """ops_sm100.rs:759; b.rows = num_groups * n."""
-    ca, cb, co, ce = a._c(), b._c(), out._c(), _epi(epi)
-    _check(_gemm_contig(ctx._h, C.byref(ca), _vp(m_indices.data_ptr()), C.byref(cb), C.byref(co), num_groups, C.byref(ce)))
+    _native.gemm_contiguous(ctx, a, m_indices, b, out, num_groups, epi)
 
 
 def m_grouped_fp8_fp4_gemm_contiguous_ends_dev(ctx, a, group_ends: torch.Tensor, b, out, num_groups: int, epi=None):
     """Same GEMM from a prebuilt group-end table (see psum_from_m_indices_dev)."""
-    ca, cb, co, ce = a._c(), b._c(), out._c(), _epi(epi)
-    _check(_gemm_contig_ends(ctx._h, C.byref(ca), _vp(group_ends.data_ptr()), C.byref(cb), C.byref(co), num_groups, C.byref(ce)))
+    _native.gemm_contiguous_ends(ctx, a, group_ends, b, out, num_groups, epi)
 
 
 STATIC_MAX_GROUPS = 4096
@@ -346,14 +334,12 @@ def static_check_status(device: int, cuda_stream: int):
 
 def m_grouped_fp8_fp4_gemm_masked_dev(ctx, a, masked_m: torch.Tensor, b, out, num_groups: int, expected_m: int, epi=None):
     """ops_sm100.rs:815; a.rows = m_max, b.rows = num_groups * n."""
-    ca, cb, co, ce = a._c(), b._c(), out._c(), _epi(epi)
-    _check(_gemm_masked(ctx._h, C.byref(ca), _vp(masked_m.data_ptr()), C.byref(cb), C.byref(co), num_groups, expected_m, C.byref(ce)))
+    _native.gemm_masked(ctx, a, masked_m, b, out, num_groups, expected_m, epi)
 
 
 def fp8_fp4_bmm_dev(ctx, a, b, out, num_groups: int, epi=None):
     """ops_sm100.rs:864; a.rows = m and b.rows = n per group."""
-    ca, cb, co, ce = a._c(), b._c(), out._c(), _epi(epi)
-    _check(_bmm(ctx._h, C.byref(ca), C.byref(cb), C.byref(co), num_groups, C.byref(ce)))
+    _native.bmm(ctx, a, b, out, num_groups, epi)
 
 
 @dataclass
@@ -365,31 +351,24 @@ class Fp8Tensor:
     ld: int
 
 
-def _f32_args(ctx, a, a_sf_t, b, sfb, m, n, out, out_ld):
-    return (ctx._h, _vp(a.data.data_ptr()), a.ld, _vp(a_sf_t.data_ptr()), _vp(b.data.data_ptr()), b.ld, _vp(sfb.data_ptr()), m, n, a.k,
-            _vp(out.data_ptr()), out_ld)
-
-
 def fp8_gemm_nt_dev(ctx, a: Fp8Tensor, a_sf_t: torch.Tensor, b: Fp8Tensor, sfb: torch.Tensor, out: torch.Tensor, out_ld: int):
     """deepgemm/src/ops.rs:328: f32 scales (a_sf_t from transform_sf_dev, sfb per 128x128 tile), bf16 out."""
-    _check(_gemm_nt(*_f32_args(ctx, a, a_sf_t, b, sfb, a.rows, b.rows, out, out_ld)))
+    _native.f32_gemm(ctx, a, a_sf_t, b, sfb, a.rows, b.rows, out, out_ld)
 
 
 def m_grouped_fp8_gemm_nt_contiguous_dev(ctx, a, a_sf_t, b, sfb, out, out_ld, m_indices, num_groups: int):
     """deepgemm/src/ops.rs:422; b.rows = num_groups * n."""
-    _check(_gemm_nt_contig(*_f32_args(ctx, a, a_sf_t, b, sfb, a.rows, b.rows // max(num_groups, 1), out, out_ld), _vp(m_indices.data_ptr()),
-                           num_groups))
+    _native.f32_gemm_contiguous(ctx, a, a_sf_t, b, sfb, a.rows, b.rows // max(num_groups, 1), out, out_ld, m_indices, num_groups)
 
 
 def m_grouped_fp8_gemm_nt_masked_dev(ctx, a, a_sf_t, b, sfb, out, out_ld, masked_m, num_groups: int, m_max: int, expected_m: int):
     """deepgemm/src/ops.rs:535; a is (num_groups, m_max, k), b.rows = num_groups * n."""
-    _check(_gemm_nt_masked(*_f32_args(ctx, a, a_sf_t, b, sfb, m_max, b.rows // max(num_groups, 1), out, out_ld), _vp(masked_m.data_ptr()),
-                           num_groups, expected_m))
+    _native.f32_gemm_masked(ctx, a, a_sf_t, b, sfb, m_max, b.rows // max(num_groups, 1), out, out_ld, masked_m, num_groups, expected_m)
 
 
 def fp8_bmm_nt_dev(ctx, a, a_sf_t, b, sfb, out, out_ld, num_groups: int, m: int, n: int):
     """deepgemm/src/ops.rs:635; a is (num_groups, m, k), b is (num_groups, n, k)."""
-    _check(_bmm_nt(*_f32_args(ctx, a, a_sf_t, b, sfb, m, n, out, out_ld), num_groups))
+    _native.f32_bmm(ctx, a, a_sf_t, b, sfb, m, n, out, out_ld, num_groups)
 
 
 def sf_packed_cols(k: int, gran_k: int) -> int:
@@ -410,10 +389,7 @@ def alloc_sf(ctx: DgContext, rows: int, k: int, gran_k: int, num_groups: int = 1
 def cast_bf16_to_fp8_sf_dev(ctx, src: torch.Tensor, src_ld: int, rows: int, k: int, gran_k: int, num_groups: int = 1
                             ) -> Tuple[torch.Tensor, torch.Tensor]:
     """ops_sm100.rs:1186: bf16 -> (e4m3 bytes (rows, k), packed UE8M0 words)."""
-    dst = torch.empty((rows, k), dtype=torch.uint8, device=src.device)
-    sf = alloc_sf(ctx, rows, k, gran_k, num_groups)
-    _check(_cast_fp8(ctx._h, _vp(src.data_ptr()), src_ld, rows, k, gran_k, num_groups, _vp(dst.data_ptr()), _vp(sf.data_ptr())))
-    return dst, sf
+    return _native.cast_fp8(ctx, src, src_ld, rows, k, gran_k, num_groups)
 
 
 def silu_mul_cast_fp8_sf_dev(ctx, gate_up: torch.Tensor, src_ld: int, rows: int, n: int, gran_k: int = 128, num_groups: int = 1,
@@ -427,25 +403,19 @@ def silu_mul_cast_fp8_sf_dev(ctx, gate_up: torch.Tensor, src_ld: int, rows: int,
     else:
         dst = torch.empty((rows, n), dtype=torch.uint8, device=gate_up.device)
         sf = alloc_sf(ctx, rows, n, gran_k, num_groups)
-    _check(_silu_cast(ctx._h, _vp(gate_up.data_ptr()), src_ld, rows, n, gran_k, num_groups, _vp(dst.data_ptr()), _vp(sf.data_ptr()),
-                      _vp(live_rows.data_ptr()) if live_rows is not None else _vp()))
+    _native.silu_cast(ctx, gate_up, src_ld, rows, n, gran_k, num_groups, live_rows, dst, sf)
     return dst, sf
 
 
 def cast_bf16_to_fp4_packed_sf_dev(ctx, src: torch.Tensor, src_ld: int, rows: int, k: int, num_groups: int = 1,
                                    sf_rule: int = SF_RULE_REFERENCE_CPU) -> Tuple[torch.Tensor, torch.Tensor]:
     """ops_sm100.rs:1135: bf16 -> (packed e2m1 (rows, k/2), packed per-32 UE8M0 words)."""
-    dst = torch.empty((rows, k // 2), dtype=torch.uint8, device=src.device)
-    sf = alloc_sf(ctx, rows, k, 32, num_groups)
-    _check(_cast_fp4(ctx._h, _vp(src.data_ptr()), src_ld, rows, k, num_groups, sf_rule, _vp(dst.data_ptr()), _vp(sf.data_ptr())))
-    return dst, sf
+    return _native.cast_fp4(ctx, src, src_ld, rows, k, num_groups, sf_rule)
 
 
 def transform_sf_dev(ctx, sf: torch.Tensor, mn: int, sf_k: int, num_batches: int = 1) -> torch.Tensor:
     """deepgemm/src/ops.rs:52: (batches, mn, sf_k) f32 -> (batches*sf_k, align4(mn)) f32."""
-    dst = torch.empty((num_batches * sf_k, sf_aligned_rows(mn)), dtype=torch.float32, device=sf.device)
-    _check(_transform_sf(ctx._h, _vp(sf.data_ptr()), mn, sf_k, num_batches, _vp(dst.data_ptr())))
-    return dst
+    return _native.transform_sf(ctx, sf, mn, sf_k, num_batches)
 
 
 def transform_sf1d_packed_ue8m0_dev(ctx, src, src_ld, rows, k, gran_k, num_groups=1) -> torch.Tensor:
@@ -565,27 +535,22 @@ def ep_block_hist_words(pairs: int, num_experts: int) -> int:
 
 
 def ep_count_dev(ctx, expert_of_pair, pairs, num_experts, local_rank, block_hist, counts):
-    _check(_ep_count(ctx._h, _vp(expert_of_pair.data_ptr()), pairs, num_experts, _vp(local_rank.data_ptr()), _vp(block_hist.data_ptr()),
-                     _vp(counts.data_ptr())))
+    _native.ep_count(ctx, expert_of_pair, pairs, num_experts, local_rank, block_hist, counts)
 
 
 def ep_layout_dev(ctx, all_counts, world, rank, num_experts, alignment, capacity, pair_base, group_ends, totals, slot_rows=0):
-    _check(_ep_layout(ctx._h, _vp(all_counts.data_ptr()), world, rank, num_experts, alignment, capacity, slot_rows, _vp(pair_base.data_ptr()),
-                      _vp(group_ends.data_ptr()), _vp(totals.data_ptr())))
+    _native.ep_layout(ctx, all_counts, world, rank, num_experts, alignment, capacity, slot_rows, pair_base, group_ends, totals)
 
 
 def ep_dispatch_dev(ctx, expert_of_pair, local_rank, block_base, pair_base, pairs, topk, num_experts, world, data, k, sf, sf_stride, sf_cols,
                     peer_data, peer_sf, peer_sf_stride, capacity, pos_of_pair, max_blocks=0, slot_rows=0):
-    _check(_ep_dispatch(ctx._h, _vp(expert_of_pair.data_ptr()), _vp(local_rank.data_ptr()), _vp(block_base.data_ptr()),
-                        _vp(pair_base.data_ptr()), pairs, topk, num_experts, world, _vp(data.data_ptr()), k, _vp(sf.data_ptr()), sf_stride,
-                        sf_cols, _vp(peer_data.data_ptr()), _vp(peer_sf.data_ptr()), peer_sf_stride, capacity, slot_rows,
-                        _vp(pos_of_pair.data_ptr()), max_blocks))
+    _native.ep_dispatch(ctx, expert_of_pair, local_rank, block_base, pair_base, pairs, topk, num_experts, world, data, k, sf, sf_stride, sf_cols,
+                        peer_data, peer_sf, peer_sf_stride, capacity, slot_rows, pos_of_pair, max_blocks)
 
 
 def ep_combine_dev(ctx, expert_of_pair, pos_of_pair, weights, tokens, topk, num_experts, world, peer_rows, pitch, n, out, out_pitch,
                    max_blocks=0):
-    _check(_ep_combine(ctx._h, _vp(expert_of_pair.data_ptr()), _vp(pos_of_pair.data_ptr()), _vp(weights.data_ptr()), tokens, topk,
-                       num_experts, world, _vp(peer_rows.data_ptr()), pitch, n, _vp(out.data_ptr()), out_pitch, max_blocks))
+    _native.ep_combine(ctx, expert_of_pair, pos_of_pair, weights, tokens, topk, num_experts, world, peer_rows, pitch, n, out, out_pitch, max_blocks)
 
 
 def debug_expire_wait(ctx, limit_us: int = 1000):

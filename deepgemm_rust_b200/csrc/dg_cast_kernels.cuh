@@ -47,6 +47,8 @@ struct CastParams {
 // activation quantiser), read from a (rows, 2k) gate|up matrix; the bf16 activation never reaches memory.
 template <uint32_t kGran, bool kFp4, bool kSiluMul = false>
 __global__ void __launch_bounds__(256) dg_cast_kernel(const CastParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
     constexpr uint32_t kLoads = 4, kSeg = 256 * kLoads;
     // a block takes 8 consecutive rows (one per warp) of one segment, so that the scale words of a word column,
     // which are contiguous over rows, leave the block as whole 32-byte sectors
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(256) dg_cast_kernel(const CastParams p) {
     const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
     const uint32_t segs_per_row = (p.k + kSeg - 1) / kSeg;
     const uint32_t seg = blockIdx.x % segs_per_row, row0 = (blockIdx.x / segs_per_row) * 8;
-    if (p.live_rows != nullptr && row0 >= __ldg(p.live_rows)) return;   // the same for the whole block
+    if (p.live_rows != nullptr && row0 >= ld_ro(p.live_rows)) return;   // the same for the whole block
     const uint32_t row = row0 + warp;
     const bool live = row < p.rows;
     const uint16_t* src_row = p.src + static_cast<size_t>(live ? row : 0) * p.src_ld;
@@ -65,9 +67,9 @@ __global__ void __launch_bounds__(256) dg_cast_kernel(const CastParams p) {
     #pragma unroll
     for (uint32_t h = 0; h < kLoads; ++h) {
         k0[h] = seg * kSeg + h * 256 + lane * 8;
-        raw[h] = (live && k0[h] < p.k) ? __ldg(reinterpret_cast<const uint4*>(src_row + k0[h])) : make_uint4(0, 0, 0, 0);
+        raw[h] = (live && k0[h] < p.k) ? ld_ro(reinterpret_cast<const uint4*>(src_row + k0[h])) : make_uint4(0, 0, 0, 0);
         if constexpr (kSiluMul)
-            raw_up[h] = (live && k0[h] < p.k) ? __ldg(reinterpret_cast<const uint4*>(src_row + p.k + k0[h])) : make_uint4(0, 0, 0, 0);
+            raw_up[h] = (live && k0[h] < p.k) ? ld_ro(reinterpret_cast<const uint4*>(src_row + p.k + k0[h])) : make_uint4(0, 0, 0, 0);
     }
     uint32_t exps[kLoads];
     #pragma unroll
@@ -148,7 +150,11 @@ __global__ void __launch_bounds__(256) dg_cast_kernel(const CastParams p) {
         const uint32_t col = seg * kWordsPerWarp + c;
         if (r < p.rows && col < p.sf_cols) {
             const uint32_t g = r / p.group_rows, lr = r - g * p.group_rows;
-            p.sf[(static_cast<size_t>(g) * p.sf_cols + col) * p.sf_stride + lr] = words[c][threadIdx.x % 8];
+            uint32_t* dst = p.sf + (static_cast<size_t>(g) * p.sf_cols + col) * p.sf_stride + lr;
+            *dst = words[c][threadIdx.x % 8];
+            // the group's last row also clears the alignment padding behind it, so nobody has to clear the buffer first
+            if (lr + 1 == p.group_rows)
+                for (uint32_t pad = lr + 1; pad < p.sf_stride; ++pad) *++dst = 0;
         }
     }
 }
@@ -163,6 +169,8 @@ struct SfPackParams {
     uint32_t src_ld, rows, group_rows, k_blocks, cols, dst_stride, mode;
 };
 __global__ void __launch_bounds__(256) dg_sf_pack_kernel(const SfPackParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
     // consecutive threads take consecutive rows of one word column: the writes coalesce
     const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<uint64_t>(p.rows) * p.cols) return;
@@ -174,9 +182,9 @@ __global__ void __launch_bounds__(256) dg_sf_pack_kernel(const SfPackParams p) {
         const uint32_t kc = col * 4 + j;
         uint32_t bits = 0x3F800000u;
         if (kc < p.k_blocks) {
-            if (p.mode == 0) bits = __float_as_uint(__ldg(p.src + static_cast<size_t>(row) * p.src_ld + kc));
-            else if (p.mode == 1) bits = __float_as_uint(__ldg(p.src + static_cast<size_t>(row / 128) * p.src_ld + kc));
-            else bits = __float_as_uint(__ldg(p.src + (static_cast<size_t>(group) * p.k_blocks + kc) * p.src_ld + local_row));
+            if (p.mode == 0) bits = __float_as_uint(ld_ro(p.src + static_cast<size_t>(row) * p.src_ld + kc));
+            else if (p.mode == 1) bits = __float_as_uint(ld_ro(p.src + static_cast<size_t>(row / 128) * p.src_ld + kc));
+            else bits = __float_as_uint(ld_ro(p.src + (static_cast<size_t>(group) * p.k_blocks + kc) * p.src_ld + local_row));
         }
         w |= ((bits >> 23) & 0xFFu) << (8 * j);
     }
@@ -187,6 +195,8 @@ __global__ void __launch_bounds__(256) dg_sf_pack_kernel(const SfPackParams p) {
 // 32x32 tiles through shared memory so both the reads and the writes coalesce.
 __global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* __restrict__ src, float* __restrict__ dst, uint32_t mn,
                                                               uint32_t sf_k, uint32_t aligned_mn) {
+    griddep_wait();
+    griddep_launch_dependents();
     __shared__ float tile[32][33];
     const uint32_t b = blockIdx.z, r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     const uint32_t tx = threadIdx.x % 32, ty = threadIdx.x / 32;
@@ -206,15 +216,19 @@ __global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* __res
 // rows inherits the previous end and the scheduler's prefix walk stays monotone.
 __global__ void __launch_bounds__(256) dg_group_ends_kernel(const int32_t* __restrict__ m_indices, uint32_t* ends, uint32_t groups,
                                                             uint32_t m) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const int32_t g = __ldg(m_indices + i);
+    const int32_t g = ld_ro(m_indices + i);
     if (g < 0 || static_cast<uint32_t>(g) >= groups) return;
     // only the last row of a run needs to publish
-    if (i + 1 < m && __ldg(m_indices + i + 1) == g) return;
+    if (i + 1 < m && ld_ro(m_indices + i + 1) == g) return;
     atomicMax(ends + g, static_cast<uint32_t>(i) + 1);
 }
 __global__ void __launch_bounds__(1024) dg_group_ends_scan_kernel(uint32_t* ends, uint32_t groups) {
+    griddep_wait();
+    griddep_launch_dependents();
     // inclusive running maximum over `groups` entries, 1024 threads, any length
     __shared__ uint32_t warp_max[32];
     __shared__ uint32_t carry;
@@ -260,7 +274,7 @@ __global__ void __launch_bounds__(256) dg_splitk_reduce_kernel(const float* __re
         float4 v[4];
         #pragma unroll
         for (uint32_t u = 0; u < 4; ++u)
-            v[u] = s + u < splits ? __ldg(reinterpret_cast<const float4*>(first + (s + u) * plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = s + u < splits ? ld_ro(reinterpret_cast<const float4*>(first + (s + u) * plane)) : make_float4(0.f, 0.f, 0.f, 0.f);
         #pragma unroll
         for (uint32_t u = 0; u < 4; ++u) {
             if (s + u < splits) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
@@ -298,6 +312,8 @@ __global__ void dg_expire_wait_kernel(Status* status, uint64_t limit_ns) {
 
 // Packed e2m1 -> one code per byte (low nibble), 16 bytes in, 32 bytes out per thread.
 __global__ void __launch_bounds__(256) dg_unpack_fp4_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint64_t packed_len) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
     if (i + 16 <= packed_len) {
         const uint4 v = *reinterpret_cast<const uint4*>(src + i);

@@ -155,8 +155,8 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
             for (uint32_t i = 0; i < kF32ColsPerWarp; ++i) acc[i] = 0.0f;
             for (uint32_t kb = 0; kb < total_kb; ++kb, ++block) {
                 const uint32_t e = block & 1, buf_phase = (block >> 1) & 1;
-                const float sa = row_ok ? __ldg(sfa_row + static_cast<size_t>(kb) * q.sfa_stride) : 0.0f;
-                const float sb = __ldg(sfb_tile + kb);
+                const float sa = row_ok ? ld_ro(sfa_row + static_cast<size_t>(kb) * q.sfa_stride) : 0.0f;
+                const float sb = ld_ro(sfb_tile + kb);
                 if (!mbar_wait(bar_tmem_full + e, buf_phase, abort_flag, p.status, 0x600 + e)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * kF32BlockN + col_half * kF32ColsPerWarp;

@@ -149,14 +149,14 @@ struct Scheduler {
         if (cur_group >= p.num_groups) return;
         const uint32_t limit = swap ? p.n : p.m, block = swap ? p.block_n : tile_m;
         if (p.gemm_type == kGemmContiguous) {
-            const uint32_t prev_end = cur_group == 0 ? 0u : __ldg(p.grouped_layout + cur_group - 1);
-            const uint32_t end = __ldg(p.grouped_layout + cur_group);
+            const uint32_t prev_end = cur_group == 0 ? 0u : ld_ro(p.grouped_layout + cur_group - 1);
+            const uint32_t end = ld_ro(p.grouped_layout + cur_group);
             cur_row_start = (prev_end + p.mk_alignment - 1) / p.mk_alignment * p.mk_alignment;
             const uint32_t rows = end > cur_row_start ? end - cur_row_start : 0u;
             cur_row_end = end < limit ? end : limit;
             cur_m_blocks = (rows + block - 1) / block;
         } else {
-            const int32_t valid = static_cast<int32_t>(__ldg(p.grouped_layout + cur_group));
+            const int32_t valid = static_cast<int32_t>(ld_ro(p.grouped_layout + cur_group));
             const uint32_t rows = valid <= 0 ? 0u : (static_cast<uint32_t>(valid) < limit ? static_cast<uint32_t>(valid) : limit);
             cur_row_start = 0;
             cur_row_end = rows;      // nothing is stored (and a pair's second CTA loads nothing) past the group's valid rows

@@ -10,17 +10,19 @@ namespace dg {
 // dst row i = src row idx[i] (row_bytes, a multiple of 16); idx[i] < 0 writes zeros.
 __global__ void __launch_bounds__(256) dg_gather_rows_kernel(const uint8_t* __restrict__ src, size_t src_pitch, const int32_t* __restrict__ idx,
                                                              uint32_t n_dst, uint32_t row_bytes, uint8_t* __restrict__ dst, size_t dst_pitch) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint64_t row = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
     if (row >= n_dst) return;
-    const int32_t s = __ldg(idx + row);
+    const int32_t s = ld_ro(idx + row);
     uint4* d = reinterpret_cast<uint4*>(dst + row * dst_pitch);
     if (s < 0) {
         for (uint32_t c = lane; c < row_bytes / 16; c += 32) d[c] = make_uint4(0, 0, 0, 0);
         return;
     }
     const uint4* p = reinterpret_cast<const uint4*>(src + static_cast<size_t>(s) * src_pitch);
-    for (uint32_t c = lane; c < row_bytes / 16; c += 32) d[c] = __ldg(p + c);
+    for (uint32_t c = lane; c < row_bytes / 16; c += 32) d[c] = ld_ro(p + c);
 }
 
 // Send row i = [k data bytes of token idx[i] | its sf_cols scale words | zero padding up to out_pitch].
@@ -28,16 +30,18 @@ __global__ void __launch_bounds__(256) dg_gather_rows_kernel(const uint8_t* __re
 __global__ void __launch_bounds__(256) dg_moe_pack_rows_kernel(const uint8_t* __restrict__ data, uint32_t k, const uint32_t* __restrict__ sf,
                                                                uint32_t sf_stride, uint32_t sf_cols, const int32_t* __restrict__ idx, uint32_t n,
                                                                uint8_t* __restrict__ out, size_t out_pitch) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint64_t row = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
     if (row >= n) return;
-    const uint32_t tok = static_cast<uint32_t>(__ldg(idx + row));
+    const uint32_t tok = static_cast<uint32_t>(ld_ro(idx + row));
     const uint4* p = reinterpret_cast<const uint4*>(data + static_cast<size_t>(tok) * k);
     uint4* d = reinterpret_cast<uint4*>(out + row * out_pitch);
-    for (uint32_t c = lane; c < k / 16; c += 32) d[c] = __ldg(p + c);
+    for (uint32_t c = lane; c < k / 16; c += 32) d[c] = ld_ro(p + c);
     uint32_t* tail = reinterpret_cast<uint32_t*>(out + row * out_pitch + k);
     const uint32_t tail_words = static_cast<uint32_t>((out_pitch - k) / 4);
-    for (uint32_t c = lane; c < tail_words; c += 32) tail[c] = c < sf_cols ? __ldg(sf + static_cast<size_t>(c) * sf_stride + tok) : 0u;
+    for (uint32_t c = lane; c < tail_words; c += 32) tail[c] = c < sf_cols ? ld_ro(sf + static_cast<size_t>(c) * sf_stride + tok) : 0u;
 }
 
 // Arena row i takes received row idx[i]: data bytes to dst_data, scale words to the packed layout
@@ -45,10 +49,12 @@ __global__ void __launch_bounds__(256) dg_moe_pack_rows_kernel(const uint8_t* __
 __global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* __restrict__ in, size_t in_pitch, uint32_t k, uint32_t sf_cols,
                                                                  const int32_t* __restrict__ idx, uint32_t n_dst, uint8_t* __restrict__ dst_data,
                                                                  uint32_t* __restrict__ dst_sf, uint32_t dst_sf_stride) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint64_t row = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
     if (row >= n_dst) return;
-    const int32_t s = __ldg(idx + row);
+    const int32_t s = ld_ro(idx + row);
     uint4* d = reinterpret_cast<uint4*>(dst_data + row * k);
     if (s < 0) {
         for (uint32_t c = lane; c < k / 16; c += 32) d[c] = make_uint4(0, 0, 0, 0);
@@ -57,9 +63,9 @@ __global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* 
     }
     const uint8_t* src = in + static_cast<size_t>(s) * in_pitch;
     const uint4* p = reinterpret_cast<const uint4*>(src);
-    for (uint32_t c = lane; c < k / 16; c += 32) d[c] = __ldg(p + c);
+    for (uint32_t c = lane; c < k / 16; c += 32) d[c] = ld_ro(p + c);
     const uint32_t* tail = reinterpret_cast<const uint32_t*>(src + k);
-    for (uint32_t c = lane; c < sf_cols; c += 32) dst_sf[static_cast<size_t>(c) * dst_sf_stride + row] = __ldg(tail + c);
+    for (uint32_t c = lane; c < sf_cols; c += 32) dst_sf[static_cast<size_t>(c) * dst_sf_stride + row] = ld_ro(tail + c);
 }
 
 // out[t, :] = bf16( sum_j w[t, j] * rows[pos[t, j], :] ), f32 accumulation in order j = 0..topk-1
@@ -67,16 +73,18 @@ __global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* 
 __global__ void __launch_bounds__(256) dg_moe_combine_kernel(const uint16_t* __restrict__ rows, size_t pitch, const int32_t* __restrict__ pos,
                                                              const float* __restrict__ w, uint32_t tokens, uint32_t topk, uint32_t n,
                                                              uint16_t* __restrict__ out, size_t out_pitch) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t chunks = n / 8;
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= static_cast<uint64_t>(tokens) * chunks) return;
     const uint32_t t = static_cast<uint32_t>(i / chunks), c = static_cast<uint32_t>(i % chunks);
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (uint32_t j = 0; j < topk; ++j) {
-        const int32_t p = __ldg(pos + static_cast<size_t>(t) * topk + j);
+        const int32_t p = ld_ro(pos + static_cast<size_t>(t) * topk + j);
         if (p < 0) continue;
-        const float wj = __ldg(w + static_cast<size_t>(t) * topk + j);
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(rows + static_cast<size_t>(p) * pitch) + c);
+        const float wj = ld_ro(w + static_cast<size_t>(t) * topk + j);
+        const uint4 v = ld_ro(reinterpret_cast<const uint4*>(rows + static_cast<size_t>(p) * pitch) + c);
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
         #pragma unroll
         for (uint32_t q = 0; q < 4; ++q) {
@@ -115,10 +123,12 @@ constexpr uint32_t kEpChunk = 256;   // pairs per block of the ranking kernel
 // [0, num_experts) are dropped (rank -1): such a pair is neither sent nor reduced.
 __global__ void __launch_bounds__(kEpChunk) dg_ep_rank_pairs_kernel(const int32_t* __restrict__ expert_of_pair, uint32_t pairs, uint32_t num_experts,
                                                                     int32_t* __restrict__ local_rank, uint32_t* __restrict__ block_hist) {
+    griddep_wait();
+    griddep_launch_dependents();
     extern __shared__ uint32_t ep_hist[];
     __shared__ int32_t ids[kEpChunk];
     const uint32_t tid = threadIdx.x, p = blockIdx.x * kEpChunk + tid;
-    int32_t e = p < pairs ? __ldg(expert_of_pair + p) : -1;
+    int32_t e = p < pairs ? ld_ro(expert_of_pair + p) : -1;
     if (e < 0 || static_cast<uint32_t>(e) >= num_experts) e = -1;
     ids[tid] = e;
     for (uint32_t i = tid; i < num_experts; i += kEpChunk) ep_hist[i] = 0;
@@ -136,6 +146,8 @@ __global__ void __launch_bounds__(kEpChunk) dg_ep_rank_pairs_kernel(const int32_
 // round trips instead of one per chunk.
 __global__ void __launch_bounds__(256) dg_ep_block_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t num_blocks, uint32_t num_experts,
                                                                uint32_t* __restrict__ counts) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint32_t e = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (e >= num_experts) return;
@@ -168,6 +180,8 @@ __global__ void __launch_bounds__(256) dg_ep_block_scan_kernel(uint32_t* __restr
 __global__ void __launch_bounds__(1024) dg_ep_layout_kernel(const uint32_t* __restrict__ all_counts, uint32_t world, uint32_t rank, uint32_t num_experts,
                                                             uint32_t alignment, uint32_t capacity, uint32_t slot_rows, uint32_t* __restrict__ pair_base,
                                                             uint32_t* __restrict__ group_ends, uint32_t* __restrict__ totals) {
+    griddep_wait();
+    griddep_launch_dependents();
     extern __shared__ uint32_t ep_smem[];
     uint32_t* rows_of = ep_smem;                  // [num_experts] rows of the expert over all source ranks
     uint32_t* before_me = ep_smem + num_experts;  // [num_experts] rows from lower source ranks
@@ -177,7 +191,7 @@ __global__ void __launch_bounds__(1024) dg_ep_layout_kernel(const uint32_t* __re
     for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) {
         uint32_t total = 0, before = 0;
         for (uint32_t s = 0; s < world; ++s) {
-            const uint32_t c = __ldg(all_counts + static_cast<size_t>(s) * num_experts + e);
+            const uint32_t c = ld_ro(all_counts + static_cast<size_t>(s) * num_experts + e);
             if (s < rank) before += c;
             total += c;
         }
@@ -246,10 +260,10 @@ struct EpDispatchParams {
 };
 
 DG_DEVICE void ep_dispatch_pair(const EpDispatchParams& p, uint64_t pair, uint32_t lane) {
-    const int32_t lr = __ldg(p.local_rank + pair);
+    const int32_t lr = ld_ro(p.local_rank + pair);
     if (lr < 0) { if (lane == 0) p.pos_of_pair[pair] = -1; return; }
-    const uint32_t e = static_cast<uint32_t>(__ldg(p.expert_of_pair + pair));
-    const uint32_t row = __ldg(p.pair_base + e) + __ldg(p.block_base + (pair / kEpChunk) * p.num_experts + e) + static_cast<uint32_t>(lr);
+    const uint32_t e = static_cast<uint32_t>(ld_ro(p.expert_of_pair + pair));
+    const uint32_t row = ld_ro(p.pair_base + e) + ld_ro(p.block_base + (pair / kEpChunk) * p.num_experts + e) + static_cast<uint32_t>(lr);
     const uint32_t owner = e / p.experts_per_rank, slot = e - owner * p.experts_per_rank;
     const uint32_t in_slot = row - slot * p.slot_rows;      // masked layout only
     if (row >= p.capacity || (p.slot_rows != 0 && in_slot >= p.slot_rows)) { if (lane == 0) p.pos_of_pair[pair] = -1; return; }
@@ -263,25 +277,27 @@ DG_DEVICE void ep_dispatch_pair(const EpDispatchParams& p, uint64_t pair, uint32
     for (; c + 32 * (kDeep - 1) < vecs; c += 32 * kDeep) {
         uint4 v[kDeep];
         #pragma unroll
-        for (uint32_t i = 0; i < kDeep; ++i) v[i] = __ldg(src + c + 32 * i);
+        for (uint32_t i = 0; i < kDeep; ++i) v[i] = ld_ro(src + c + 32 * i);
         #pragma unroll
         for (uint32_t i = 0; i < kDeep; ++i) dst[c + 32 * i] = v[i];
     }
     for (; c + 96 < vecs; c += 128) {
-        const uint4 v0 = __ldg(src + c), v1 = __ldg(src + c + 32), v2 = __ldg(src + c + 64), v3 = __ldg(src + c + 96);
+        const uint4 v0 = ld_ro(src + c), v1 = ld_ro(src + c + 32), v2 = ld_ro(src + c + 64), v3 = ld_ro(src + c + 96);
         dst[c] = v0; dst[c + 32] = v1; dst[c + 64] = v2; dst[c + 96] = v3;
     }
-    for (; c < vecs; c += 32) dst[c] = __ldg(src + c);
+    for (; c < vecs; c += 32) dst[c] = ld_ro(src + c);
     uint32_t* dsf = p.peer_sf[owner];
     const size_t sf_base = p.slot_rows ? static_cast<size_t>(slot) * p.sf_cols * p.peer_sf_stride + in_slot : row;
     for (uint32_t w = lane; w < p.sf_cols; w += 32)
-        dsf[sf_base + static_cast<size_t>(w) * p.peer_sf_stride] = __ldg(p.sf + static_cast<size_t>(w) * p.sf_stride + tok);
+        dsf[sf_base + static_cast<size_t>(w) * p.peer_sf_stride] = ld_ro(p.sf + static_cast<size_t>(w) * p.sf_stride + tok);
 }
 
 
 // One warp per (token, j) pair; the grid may be smaller than the pair count (warps stride over the pairs), which
 // lets a caller leave room on every SM for a kernel running beside this one.
 __global__ void __launch_bounds__(256) dg_ep_dispatch_kernel(const EpDispatchParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x / 32);
     for (uint64_t pair = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; pair < p.pairs; pair += warps)
@@ -301,6 +317,8 @@ struct EpCombineParams {
 // out[t, :] = bf16( sum_j w[t, j] * rows_of_owner(t, j)[pos[t, j], :] ): the same ordered fused multiply-add
 // chain as dg_moe_combine_kernel, reading each term from the rank that computed it.  One thread owns 8 columns.
 __global__ void __launch_bounds__(256) dg_ep_combine_kernel(const EpCombineParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
     const uint32_t chunks = p.n / 8;
     // tokens x chunks fits 32 bits (checked by the host): 32-bit division instead of the 64-bit sequence
     const uint32_t total = p.tokens * chunks, stride = gridDim.x * blockDim.x;
@@ -319,11 +337,11 @@ __global__ void __launch_bounds__(256) dg_ep_combine_kernel(const EpCombineParam
             live[u] = false;
             if (j < p.topk) {
                 const size_t at = static_cast<size_t>(t) * p.topk + j;
-                const int32_t row = __ldg(p.pos_of_pair + at);
+                const int32_t row = ld_ro(p.pos_of_pair + at);
                 if (row >= 0) {
-                    const uint32_t owner = static_cast<uint32_t>(__ldg(p.expert_of_pair + at)) / p.experts_per_rank;
+                    const uint32_t owner = static_cast<uint32_t>(ld_ro(p.expert_of_pair + at)) / p.experts_per_rank;
                     live[u] = true;
-                    wj[u] = __ldg(p.weights + at);
+                    wj[u] = ld_ro(p.weights + at);
                     v[u] = *(reinterpret_cast<const uint4*>(p.peer_rows[owner] + static_cast<size_t>(row) * p.pitch) + c);
                 }
             }

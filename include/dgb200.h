@@ -173,8 +173,8 @@ size_t dg_sf_words(uint32_t rows, uint32_t k, uint32_t gran_k, uint32_t num_grou
 enum { DG_SF_RULE_REFERENCE_CPU = 0, DG_SF_RULE_RANGE_FIT = 1 };
 
 /* ops_sm100.rs:1186 (cast_bf16_to_fp8_sf_dev).  Outputs are caller-allocated: dst rows*k bytes,
- * sf dg_sf_words(rows, k, gran_k, num_groups) words (every word is written, no pre-zeroing needed
- * except for the alignment padding rows, which are left untouched). */
+ * sf dg_sf_words(rows, k, gran_k, num_groups) words (every word is written, the alignment padding rows
+ * with zeros: no pre-zeroing needed). */
 int dg_cast_bf16_to_fp8_sf(dg_ctx* ctx, const uint16_t* src, uint32_t src_ld, uint32_t rows, uint32_t k, uint32_t gran_k,
                            uint32_t num_groups, uint8_t* dst, uint32_t* sf);
 /* moe.rs:273-296 with layout.rs:218-233 (deepgemm_silu_mul_bf16), fused with the activation quantiser the
