@@ -622,6 +622,16 @@ cudaError_t configure_contiguous_kernels() {
     return e;
 }
 
+// The context's scratch for partial sums, at least `floats` long.
+int ensure_splitk_ws(dg_ctx* ctx, size_t floats) {
+    if (ctx->splitk_ws_cap >= floats) return DG_OK;
+    DG_CUDA(cudaSetDevice(ctx->ordinal));
+    if (ctx->splitk_ws) { cudaFree(ctx->splitk_ws); ctx->splitk_ws = nullptr; ctx->splitk_ws_cap = 0; }
+    DG_CUDA(cudaMalloc(&ctx->splitk_ws, floats * sizeof(float)));
+    ctx->splitk_ws_cap = floats;
+    return DG_OK;
+}
+
 int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue* epi, const Problem& pr) {
     if (out == nullptr || out->buf == nullptr) return fail(DG_ERR_SHAPE, "null output");
     if (out->kind < DG_OUT_BF16 || out->kind > DG_OUT_SWIGLU_FP8) return fail(DG_ERR_SHAPE, "invalid output kind %d", out->kind);
@@ -687,13 +697,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const uint32_t splits = plan.splits;
     const uint32_t ws_pitch = align4(pr.n);
     if (splits > 1) {
-        const size_t need = static_cast<size_t>(splits) * pr.m * ws_pitch;
-        if (ctx->splitk_ws_cap < need) {
-            DG_CUDA(cudaSetDevice(ctx->ordinal));
-            if (ctx->splitk_ws) { cudaFree(ctx->splitk_ws); ctx->splitk_ws = nullptr; ctx->splitk_ws_cap = 0; }
-            DG_CUDA(cudaMalloc(&ctx->splitk_ws, need * sizeof(float)));
-            ctx->splitk_ws_cap = need;
-        }
+        rc = ensure_splitk_ws(ctx, static_cast<size_t>(splits) * pr.m * ws_pitch);
+        if (rc) return rc;
     }
     const uint32_t sfa_words = 4 * ka->gran_k >= block_k ? 1 : block_k / (4 * ka->gran_k);
     const uint32_t sfb_words = 4 * kb->gran_k >= block_k ? 1 : block_k / (4 * kb->gran_k);
@@ -882,6 +887,70 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     return DG_OK;
 }
 
+struct F32Plan {
+    uint32_t ctas, block_n;          // a pair of CTAs with 256 x 256 tiles, or single CTAs with 128 x 128 tiles
+    uint32_t splits, kb_per_split;   // K ranges (dense problems with few tiles), in k-blocks of 128
+};
+// Costs in microseconds, fitted on B200 over 22 problems (m 68-6900, n 560-8096, k 1152-8064): a K block takes 0.36 of a 128 x 128
+// tile and 0.56 of a 256 x 256 one (a quarter as many tiles, half the SM pairs), so the pair wins wherever its waves are fewer than
+// 0.64 of the others; K ranges pay 3.5 plus their planes for the second launch, and never more than one wave.
+F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint32_t groups, uint32_t sms) {
+    const uint32_t kbs = k / 128;
+    const bool dense = type == DG_GEMM_NORMAL;
+    // row blocks: a contiguous group ends inside a tile, half a tile is lost on average
+    auto row_blocks = [&](uint32_t tile_m) {
+        if (type == DG_GEMM_M_GROUPED_CONTIGUOUS) return groups * (static_cast<double>(m) / groups / tile_m + 0.5);
+        return static_cast<double>(dense ? 1u : groups) * ceil_div(m, tile_m);
+    };
+    const double tiles = row_blocks(128) * ceil_div(n, 128), pair_tiles = row_blocks(256) * ceil_div(n, 256);
+    auto waves = [](double t, uint32_t workers) { return static_cast<double>(static_cast<uint64_t>(t / workers + 0.999)); };
+    F32Plan best = {1, 128, 1, kbs};
+    double best_cost = waves(tiles, sms) * (kbs * 0.36 + 0.6);
+    const double pair_cost = sms >= 2 ? waves(pair_tiles, sms / 2) * (kbs * 0.56 + 1.2) : best_cost;
+    // (a masked group's rows are known to the device only and usually fewer than its slot: small tiles)
+    if (type != DG_GEMM_M_GROUPED_MASKED && pair_cost < best_cost) {
+        best = {2, 256, 1, kbs};
+        best_cost = pair_cost;
+    }
+    for (uint32_t splits = 2; dense && n % 4 == 0 && splits <= 8; ++splits) {
+        const uint32_t per = ceil_div(kbs, splits);
+        if (per < 4 || per * (splits - 1) >= kbs || tiles * splits > sms) continue;
+        const double cost = per * 0.36 + 0.6 + 3.5 + static_cast<double>(splits) * m * n * 4.0 / 4e6;
+        if (cost < best_cost) {
+            best = {1, 128, splits, per};
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+template <uint32_t kCtas, uint32_t kBlockN, bool kPartial>
+cudaError_t launch_f32scale_kernel(const dg::F32ScaleParams& q, uint32_t grid, uint32_t smem, dg_ctx* ctx, const CUtensorMap* maps) {
+    auto kernel = dg::dg_gemm_f32scale_kernel<kCtas, kBlockN, kPartial>;
+    static std::atomic<uint64_t> configured{0};
+    if (ctx->ordinal >= 64 || !(configured.load() & (1ull << ctx->ordinal))) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemCapacity));
+        if (e != cudaSuccess) return e;
+        if (ctx->ordinal < 64) configured.fetch_or(1ull << ctx->ordinal);
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(dg::kF32Threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kCtas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, q, maps[0], maps[1], maps[2]);
+}
+
 int ensure_group_ends(dg_ctx* ctx, uint32_t groups) {
     if (ctx->group_ends_cap >= groups) return DG_OK;
     if (ctx->group_ends) { cudaFree(ctx->group_ends); ctx->group_ends = nullptr; ctx->group_ends_cap = 0; }
@@ -979,8 +1048,14 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     if (contiguous && align % 32 != 0) return fail(DG_ERR_UNSUPPORTED, "the exact f32-scale path needs an mk alignment of at least 32");
     if (a_ld < k || b_ld < k || a_ld % 16 != 0 || b_ld % 16 != 0) return fail(DG_ERR_SHAPE, "leading dimensions must be >= k and multiples of 16 bytes");
     if (out_ld < n || (static_cast<size_t>(out_ld) * 2) % 16 != 0) return fail(DG_ERR_SHAPE, "output ld (%u) must be >= n and a multiple of 8 elements", out_ld);
+    const F32Plan plan = choose_f32scale(type, m, n, k, groups, static_cast<uint32_t>(ctx->num_sms));
+    const uint32_t ws_pitch = align4(n);
     CUtensorMap maps[3];
     int rc;
+    if (plan.splits > 1) {
+        rc = ensure_splitk_ws(ctx, static_cast<size_t>(plan.splits) * m * ws_pitch);
+        if (rc) return rc;
+    }
     {
         uint64_t dims[3] = {k, m, a_groups};
         uint64_t strides[2] = {a_ld, static_cast<uint64_t>(a_ld) * m};
@@ -989,14 +1064,18 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
         if (rc) return rc;
         uint64_t bdims[3] = {k, n, b_groups};
         uint64_t bstrides[2] = {b_ld, static_cast<uint64_t>(b_ld) * n};
-        uint32_t bbox[3] = {128, dg::kF32BlockN, 1};
+        uint32_t bbox[3] = {128, plan.block_n / plan.ctas, 1};
         rc = encode_map(&maps[1], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, b, bdims, bstrides, bbox, CU_TENSOR_MAP_SWIZZLE_128B, "B");
         if (rc) return rc;
-        const uint64_t pitch = static_cast<uint64_t>(out_ld) * 2;
-        uint64_t ddims[3] = {n, m, a_groups};
+        const bool partial = plan.splits > 1;      // one f32 plane per K range, summed afterwards
+        const uint64_t pitch = partial ? static_cast<uint64_t>(ws_pitch) * 4 : static_cast<uint64_t>(out_ld) * 2;
+        uint64_t ddims[3] = {n, m, partial ? plan.splits : a_groups};
         uint64_t dstrides[2] = {pitch, pitch * m};
         uint32_t dbox[3] = {32, 32, 1};
-        rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, out, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_64B, "D");
+        if (partial)
+            rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ctx->splitk_ws, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_128B, "D partials");
+        else
+            rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, out, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_64B, "D");
         if (rc) return rc;
     }
     dg::F32ScaleParams q;
@@ -1005,48 +1084,41 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     p.m = m; p.n = n; p.k = k;
     p.num_groups = groups;
     p.gemm_type = type;
-    p.block_n = p.tile_n = dg::kF32BlockN;
+    p.block_n = p.tile_n = plan.block_n;
     p.block_k_elems = 128;
-    p.num_splits = 1;
+    p.num_splits = plan.splits;
+    p.kb_per_split = plan.kb_per_split;
     p.cluster_splits = 1;
     p.num_accum_stages = 2;
     p.mk_alignment = align;
     p.grouped_layout = layout;
     p.status = ctx->status;
     uint32_t stages = dg::kMaxStages;
-    while (stages > 1 && dg::f32scale_smem_bytes(stages) > kSmemCapacity) --stages;
+    while (stages > 1 && dg::f32scale_smem_bytes(plan.ctas, plan.block_n, plan.splits > 1, stages) > kSmemCapacity) --stages;
     p.num_stages = stages;
     q.sfa_t = a_sf_t;
     q.sfb = sfb;
     q.sfa_stride = align4(m);
     q.k_blocks = k / 128;
     q.n_blocks128 = ceil_div(n, 128);
-    const uint32_t smem = dg::f32scale_smem_bytes(stages);
+    const uint32_t smem = dg::f32scale_smem_bytes(plan.ctas, plan.block_n, plan.splits > 1, stages);
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    {
-        static std::atomic<uint64_t> configured{0};
-        if (ctx->ordinal >= 64 || !(configured.load() & (1ull << ctx->ordinal))) {
-            DG_CUDA(cudaFuncSetAttribute(dg::dg_gemm_f32scale_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemCapacity)));
-            if (ctx->ordinal < 64) configured.fetch_or(1ull << ctx->ordinal);
-        }
-    }
-    uint32_t grid = static_cast<uint32_t>(ctx->num_sms);
+    uint32_t grid = static_cast<uint32_t>(ctx->num_sms) / plan.ctas * plan.ctas;
     if (type == DG_GEMM_NORMAL || type == DG_GEMM_BATCHED) {
-        const uint64_t tiles = static_cast<uint64_t>(ceil_div(m, dg::kBlockM)) * ceil_div(n, dg::kF32BlockN) * (type == DG_GEMM_BATCHED ? groups : 1);
-        if (tiles < grid) grid = static_cast<uint32_t>(tiles);
+        const uint64_t ctas = static_cast<uint64_t>(ceil_div(m, dg::kBlockM * plan.ctas)) * ceil_div(n, plan.block_n) * (type == DG_GEMM_BATCHED ? groups : 1) *
+                              plan.splits * plan.ctas;
+        if (ctas < grid) grid = static_cast<uint32_t>(ctas);
     }
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(dg::kF32Threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    const cudaError_t ce = cudaLaunchKernelEx(&cfg, dg::dg_gemm_f32scale_kernel, q, maps[0], maps[1], maps[2]);
+    cudaError_t ce;
+    if (plan.ctas == 2) ce = launch_f32scale_kernel<2, 256, false>(q, grid, smem, ctx, maps);
+    else if (plan.splits > 1) ce = launch_f32scale_kernel<1, 128, true>(q, grid, smem, ctx, maps);
+    else ce = launch_f32scale_kernel<1, 128, false>(q, grid, smem, ctx, maps);
+    if (ce == cudaSuccess && plan.splits > 1) {
+        const uint64_t threads = static_cast<uint64_t>(m) * ceil_div(n, 4);
+        launch(dg::dg_splitk_reduce_kernel<true>, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, ctx->splitk_ws, plan.splits, m, n, ws_pitch,
+               1.0f, out, out_ld);
+        ce = cudaGetLastError();
+    }
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
     return DG_OK;
 }

@@ -5,24 +5,28 @@
 // which is what deepgemm/src/reference.rs:85-114 (and :133-208 for the grouped layouts) computes.  The tensor core's block
 // scaling only takes power-of-two (UE8M0) scales, so an f32 scale with a mantissa cannot ride the UMMA: here every K block
 // is multiplied on its own (tcgen05.mma kind::f8f6f4 into one of two TMEM buffers, starting from zero) and the epilogue
-// warps fold it into f32 accumulators they keep in registers: acc += (block * sfa) * sfb, the reference's order of
-// operations.  One 384-thread CTA per SM, 128 x 128 tiles: warp 0 loads A / B k-blocks with TMA, warp 1 issues the UMMAs, and
-// eight epilogue warps (4-11) each own 32 accumulator rows x 64 columns (a warp reads the TMEM lanes of its quadrant, warp % 4;
-// warps 4-7 take columns 0-63, warps 8-11 columns 64-127), read every K block's partial tile (tcgen05.ld), scale and add it,
-// and at the end store bf16 through swizzled staging and TMA.  Reading a partial tile out of TMEM per 128 of K costs more
-// than that block's tensor time even with eight warps, so this path stays well below the block-scaled kernel's rate: it
-// exists for exactness with arbitrary scales, the UE8M0 path for speed.
+// warps fold it into f32 accumulators they keep in registers: acc = fma(block, sfa * sfb, acc).
+//
+// What bounds it: every K block's partial tile has to leave TMEM (128 lanes x 4 bytes per cycle) and go through one FMA per
+// element (128 per cycle and SM), each 256 cycles for 128 x 256 elements, beside 512 cycles of tensor time; a K block costs the
+// epilogue warps ~1100 cycles all told (barrier, scales, TMEM latency), which is the limit.  The operands of a 128 x 128 tile
+// (32 KB for 256 tensor cycles) also arrive slower than the tensor core takes them.  So a CTA pair computes 256 x 256
+// (kCtas = 2, kBlockN = 256): 32 KB per CTA for 512 tensor cycles, both TMEM buffers 256 columns wide, and 128 x 256 f32
+// accumulators in the registers of eight epilogue warps (the other four give registers back for that).  Problems with too few
+// such tiles use 128 x 128 tiles of single CTAs, and cut K into ranges (f32 partial planes summed by dg_splitk_reduce_kernel)
+// when even those do not fill the SMs.  4096 x 7168 x 7168: 348 us with 128 x 128 tiles and three rounded operations per
+// element, 313 with one FMA, 260 with the pair; sixteen epilogue warps of 64 columns (96 registers) spilled and took 350.
+// Roles of the 384-thread CTA: warp 0 loads A / B k-blocks with TMA, warp 1 issues the UMMAs, warps 4-11 are the epilogue: each
+// owns 32 rows (TMEM quadrant warp % 4) x half of the tile's columns.
 #pragma once
 #include "dg_gemm_kernel.cuh"
 
 namespace dg {
 
-constexpr uint32_t kF32BlockN = 128;
-constexpr uint32_t kF32Threads = 384;      // producer, UMMA issuer, two idle warps, eight epilogue warps
-constexpr uint32_t kF32ColsPerWarp = 64;   // accumulator columns an epilogue warp keeps in registers
+constexpr uint32_t kF32Threads = 384;     // TMA producer, UMMA issuer, two idle warps, eight epilogue warps
 
 struct F32ScaleParams {
-    GemmParams g;              // shape, layout, scheduler inputs (block_n = tile_n = 128, block_k_elems = 128)
+    GemmParams g;              // shape, layout, scheduler inputs (block_n = tile_n = kBlockN, block_k_elems = 128)
     const float* sfa_t;        // activation scales, transposed: [(group * k_blocks + kb) * sfa_stride + row]
     const float* sfb;          // weight scales: [(group * n_blocks128 + n / 128) * k_blocks + kb]
     uint32_t sfa_stride;       // align4(rows per group)
@@ -33,14 +37,24 @@ struct F32ScaleParams {
 //   [4,6) D format (1 = f32), [7,10) A format (0 = e4m3), [10,13) B format, [17,23) N >> 3, [24,29) M >> 4.
 DG_DEVICE uint32_t make_idesc_f8(uint32_t m, uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 
+template <uint32_t kCtas>
 DG_DEVICE void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (kCtas == 1)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 
+// kPartial: the tile is one K range of a split problem and goes to its f32 plane (tmap_d: f32) instead of the bf16 output.
+template <uint32_t kCtas, uint32_t kBlockN, bool kPartial>
 __global__ void __launch_bounds__(kF32Threads, 1)
 dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                         const __grid_constant__ CUtensorMap tmap_d) {
@@ -48,18 +62,21 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    constexpr uint32_t kTile = kBlockM * kBlockKBytes;        // 16 KB per operand and k-block
-    constexpr uint32_t kEpiBuf = 2048;                        // 32 rows x 64 bytes of bf16 per staging buffer
+    const uint32_t cta_rank = kCtas == 2 ? cluster_cta_rank() : 0u;
+    constexpr uint32_t kLoadN = kBlockN / kCtas;              // weight rows this CTA loads
+    constexpr uint32_t kTileA = kBlockM * kBlockKBytes, kTileB = kLoadN * kBlockKBytes;
+    constexpr uint32_t kEpiBuf = kPartial ? 4096 : 2048;      // 32 rows x 32 columns
+    constexpr uint32_t kEpiWarps = 8, kWarpCols = kBlockN / 2;     // accumulator columns of an epilogue warp
     const uint32_t num_stages = p.num_stages;
 
     uint8_t* smem_a = smem;
-    uint8_t* smem_b = smem_a + num_stages * kTile;
-    uint8_t* smem_epi = smem_b + num_stages * kTile;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_epi + 16 * kEpiBuf);
-    uint64_t* bar_full = bars;
+    uint8_t* smem_b = smem_a + num_stages * kTileA;
+    uint8_t* smem_epi = smem_b + num_stages * kTileB;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_epi + kEpiWarps * kEpiBuf);
+    uint64_t* bar_full = bars;                               // a k-block's operands landed (pair: both CTAs', on rank 0)
     uint64_t* bar_empty = bars + kMaxStages;
     uint64_t* bar_tmem_full = bars + 2 * kMaxStages;         // a K block's partial tile is complete in TMEM buffer e
-    uint64_t* bar_tmem_empty = bars + 2 * kMaxStages + 2;    // the epilogue warps have read buffer e
+    uint64_t* bar_tmem_empty = bars + 2 * kMaxStages + 2;    // the epilogue warps (of both CTAs) have read buffer e
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -70,7 +87,7 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
         }
         for (uint32_t e = 0; e < 2; ++e) {
             mbar_init(bar_tmem_full + e, 1);
-            mbar_init(bar_tmem_empty + e, 8);
+            mbar_init(bar_tmem_empty + e, kEpiWarps * kCtas);
         }
         *abort_flag = 0;
         fence_mbar_init();
@@ -79,133 +96,190 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
         tma_prefetch_desc(&tmap_d);
     }
     if (warp == 1) {
-        tmem_alloc<1>(tmem_slot, 2 * kF32BlockN);
-        tmem_relinquish<1>();
+        tmem_alloc<kCtas>(tmem_slot, 2 * kBlockN);
+        tmem_relinquish<kCtas>();
     }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (kCtas == 2) cluster_sync(); else __syncthreads();
     tc_fence_after();
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t total_kb = q.k_blocks;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        Scheduler sched(p, 1);
-        Tile t;
-        uint32_t stage = 0, phase = 0;
-        bool ok = true;
-        while (ok && sched.next(t)) {
-            for (uint32_t kb = 0; kb < total_kb; ++kb) {
-                if (!mbar_wait_warp(bar_empty + stage, phase ^ 1, abort_flag, p.status, 0x100 + stage)) { ok = false; break; }
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(bar_full + stage, 2 * kTile);
-                    const int32_t kx = static_cast<int32_t>(kb * kBlockKBytes);
-                    tma_load_3d(smem_a + stage * kTile, &tmap_a, bar_full + stage, kx, static_cast<int32_t>(t.m0), static_cast<int32_t>(t.ga));
-                    tma_load_3d(smem_b + stage * kTile, &tmap_b, bar_full + stage, kx, static_cast<int32_t>(t.n0), static_cast<int32_t>(t.gb));
+    // 384 threads x 168 registers at launch = 128 x 88 + 256 x 208
+    constexpr bool kMoveRegs = kBlockN == 256;
+    if (warp < 4) {
+        if constexpr (kMoveRegs) setmaxnreg_dec<88>();
+        if (warp == 0) {
+            // ------------------------------------------------------------ TMA producer
+            Scheduler sched(p, kCtas);
+            Tile t;
+            uint32_t stage = 0, phase = 0;
+            bool ok = true;
+            const uint32_t full_addr = kCtas == 2 ? mapa_u32(smem_u32(bar_full), 0) : 0u;
+            while (ok && sched.next(t)) {
+                const int32_t row_a = static_cast<int32_t>(t.m0 + cta_rank * kBlockM), row_b = static_cast<int32_t>(t.n0 + cta_rank * kLoadN);
+                for (uint32_t kb = t.kb0; kb < t.kb1; ++kb) {
+                    if (!mbar_wait_warp(bar_empty + stage, phase ^ 1, abort_flag, p.status, 0x100 + stage)) { ok = false; break; }
+                    if (elect_one()) {
+                        const int32_t kx = static_cast<int32_t>(kb * kBlockKBytes);
+                        if constexpr (kCtas == 1) {
+                            mbar_arrive_expect_tx(bar_full + stage, kTileA + kTileB);
+                            tma_load_3d(smem_a + stage * kTileA, &tmap_a, bar_full + stage, kx, row_a, static_cast<int32_t>(t.ga));
+                            tma_load_3d(smem_b + stage * kTileB, &tmap_b, bar_full + stage, kx, row_b, static_cast<int32_t>(t.gb));
+                        } else {
+                            if (cta_rank == 0) mbar_arrive_expect_tx(bar_full + stage, 2 * (kTileA + kTileB));
+                            tma_load_3d_2cta(smem_a + stage * kTileA, &tmap_a, full_addr + stage * 8, kx, row_a, static_cast<int32_t>(t.ga));
+                            tma_load_3d_2cta(smem_b + stage * kTileB, &tmap_b, full_addr + stage * 8, kx, row_b, static_cast<int32_t>(t.gb));
+                        }
+                    }
+                    __syncwarp();
+                    if (++stage == num_stages) { stage = 0; phase ^= 1; }
                 }
-                if (++stage == num_stages) { stage = 0; phase ^= 1; }
+            }
+        } else if (warp == 1 && cta_rank == 0) {
+            // ------------------------------------------------------------- UMMA issuer
+            Scheduler sched(p, kCtas);
+            Tile t;
+            uint32_t stage = 0, phase = 0, block = 0;
+            constexpr uint32_t kM = kBlockM * kCtas;
+            const uint32_t idesc = make_idesc_f8(kM, kBlockN);
+            const bool leader_lane = elect_one();
+            bool ok = true;
+            while (ok && sched.next(t)) {
+                for (uint32_t kb = t.kb0; kb < t.kb1; ++kb, ++block) {
+                    const uint32_t e = block & 1, buf_phase = (block >> 1) & 1;
+                    if (!mbar_wait_warp(bar_tmem_empty + e, buf_phase ^ 1, abort_flag, p.status, 0x200 + e)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_full + stage, phase, abort_flag, p.status, 0x300 + stage)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t a_desc = make_smem_desc(smem_u32(smem_a + stage * kTileA), 0, 1024, 2);
+                    const uint64_t b_desc = make_smem_desc(smem_u32(smem_b + stage * kTileB), 0, 1024, 2);
+                    if (leader_lane) {
+                        #pragma unroll
+                        for (uint32_t k = 0; k < kBlockKBytes / kUmmaKBytes; ++k)
+                            umma_f8<kCtas>(tmem_base + e * kBlockN, a_desc + k * (kUmmaKBytes >> 4), b_desc + k * (kUmmaKBytes >> 4), idesc, k != 0 ? 1u : 0u);
+                        if constexpr (kCtas == 1) {
+                            umma_commit(bar_empty + stage);
+                            umma_commit(bar_tmem_full + e);
+                        } else {
+                            umma_commit_2cta(bar_empty + stage, static_cast<uint16_t>(3));
+                            umma_commit_2cta(bar_tmem_full + e, static_cast<uint16_t>(3));
+                        }
+                    }
+                    __syncwarp();
+                    if (++stage == num_stages) { stage = 0; phase ^= 1; }
+                }
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        // ------------------------------------------------------------- UMMA issuer
-        Scheduler sched(p, 1);
-        Tile t;
-        uint32_t stage = 0, phase = 0, block = 0;
-        const uint32_t idesc = make_idesc_f8(kBlockM, kF32BlockN);
-        bool ok = true;
-        while (ok && sched.next(t)) {
-            for (uint32_t kb = 0; kb < total_kb; ++kb, ++block) {
-                const uint32_t e = block & 1, buf_phase = (block >> 1) & 1;
-                if (!mbar_wait_warp(bar_tmem_empty + e, buf_phase ^ 1, abort_flag, p.status, 0x200 + e)) { ok = false; break; }
-                if (!mbar_wait_warp(bar_full + stage, phase, abort_flag, p.status, 0x300 + stage)) { ok = false; break; }
-                tc_fence_after();
-                const uint64_t a_desc = make_smem_desc(smem_u32(smem_a + stage * kTile), 0, 1024, 2);
-                const uint64_t b_desc = make_smem_desc(smem_u32(smem_b + stage * kTile), 0, 1024, 2);
-                if (elect_one()) {
-                    #pragma unroll
-                    for (uint32_t k = 0; k < kBlockKBytes / kUmmaKBytes; ++k)
-                        umma_f8(tmem_base + e * kF32BlockN, a_desc + k * (kUmmaKBytes >> 4), b_desc + k * (kUmmaKBytes >> 4), idesc, k != 0 ? 1u : 0u);
-                    umma_commit(bar_empty + stage);
-                    umma_commit(bar_tmem_full + e);
-                }
-                __syncwarp();
-                if (++stage == num_stages) { stage = 0; phase ^= 1; }
-            }
-        }
-        __syncwarp();
-    } else if (warp >= 4) {
+    } else {
         // ------------------------------------------------------------------ epilogue
-        const uint32_t ew = warp % 4, col_half = (warp - 4) / 4;       // TMEM lane quadrant; which 64 of the tile's 128 columns
-        uint8_t* buf0 = smem_epi + (warp - 4) * 2 * kEpiBuf;
-        Scheduler sched(p, 1);
+        if constexpr (kMoveRegs) setmaxnreg_inc<208>();
+        const uint32_t ew = warp % 4, col_part = (warp - 4) / 4;       // TMEM lane quadrant; which half of the tile's columns
+        uint8_t* const buf = smem_epi + (warp - 4) * kEpiBuf;
+        Scheduler sched(p, kCtas);
         Tile t;
-        uint32_t block = 0, buf_idx = 0;
+        uint32_t block = 0;
         bool ok = true;
         while (ok && sched.next(t)) {
-            const uint32_t row0 = t.m0 + ew * 32, row = row0 + lane;
+            const uint32_t row0 = t.m0 + cta_rank * kBlockM + ew * 32, row = row0 + lane, n0 = t.n0 + col_part * kWarpCols;
             const bool row_ok = row < t.m_end;
-            // the activation scale of this thread's row for K block kb, and the weight scale of the tile's 128 columns
-            const float* sfa_row = q.sfa_t + static_cast<size_t>(t.ga) * total_kb * q.sfa_stride + row;
-            const float* sfb_tile = q.sfb + (static_cast<size_t>(t.gb) * q.n_blocks128 + t.n0 / 128) * total_kb;
-            float acc[kF32ColsPerWarp];
+            // the activation scale of this thread's row for K block kb, and the weight scale of the warp's columns
+            const float* sfa_row = q.sfa_t + static_cast<size_t>(t.ga) * q.k_blocks * q.sfa_stride + row;
+            const uint32_t nb = n0 / 128 < q.n_blocks128 ? n0 / 128 : q.n_blocks128 - 1;
+            const float* sfb_tile = q.sfb + (static_cast<size_t>(t.gb) * q.n_blocks128 + nb) * q.k_blocks;
+            auto scale_a = [&](uint32_t kb) { return row_ok && kb < t.kb1 ? ld_ro(sfa_row + static_cast<size_t>(kb) * q.sfa_stride) : 0.0f; };
+            auto scale_b = [&](uint32_t kb) { return kb < t.kb1 ? ld_ro(sfb_tile + kb) : 0.0f; };
+            float acc[kWarpCols];
             #pragma unroll
-            for (uint32_t i = 0; i < kF32ColsPerWarp; ++i) acc[i] = 0.0f;
-            for (uint32_t kb = 0; kb < total_kb; ++kb, ++block) {
+            for (uint32_t i = 0; i < kWarpCols; ++i) acc[i] = 0.0f;
+            // scales are fetched two K blocks ahead of their use
+            float sa = scale_a(t.kb0), sb = scale_b(t.kb0), sa1 = scale_a(t.kb0 + 1), sb1 = scale_b(t.kb0 + 1);
+            for (uint32_t kb = t.kb0; kb < t.kb1; ++kb, ++block) {
                 const uint32_t e = block & 1, buf_phase = (block >> 1) & 1;
-                const float sa = row_ok ? ld_ro(sfa_row + static_cast<size_t>(kb) * q.sfa_stride) : 0.0f;
-                const float sb = ld_ro(sfb_tile + kb);
+                const float sa2 = scale_a(kb + 2), sb2 = scale_b(kb + 2);
+                // One factor for both scales: one rounding fewer than scaling twice.  Where their product leaves the range that keeps full
+                // precision (never with scales of quantised data) the block is multiplied by the activation scale first, in place in TMEM:
+                // a second path over the accumulators would cost every K block register moves.
+                const float both = sa * sb, mag = fabsf(both);
+                const bool one_factor = __all_sync(0xFFFFFFFFu, (mag >= 1e-30f && mag <= 1e30f) || sa == 0.0f || sb == 0.0f);
+                const float s = one_factor ? both : sb;
                 if (!mbar_wait(bar_tmem_full + e, buf_phase, abort_flag, p.status, 0x600 + e)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * kF32BlockN + col_half * kF32ColsPerWarp;
+                const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * kBlockN + col_part * kWarpCols;
+                if (!one_factor) {
+                    #pragma unroll 1
+                    for (uint32_t c = 0; c < kWarpCols; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld_32x32b_x16(taddr + c, v);
+                        tmem_ld_wait_x16(v);
+                        #pragma unroll
+                        for (uint32_t i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * sa);
+                        tmem_st_32x32b_x16(taddr + c, v);
+                    }
+                    tmem_st_wait();
+                }
+                // two elements per instruction (packed f32x2: the same IEEE operations, half the issue slots)
+                auto fold = [&](uint32_t (&v)[16], uint32_t c) {
+                    #pragma unroll
+                    for (uint32_t i = 0; i < 16; i += 2) {
+                        const float2 r = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), make_float2(s, s),
+                                                    make_float2(acc[c * 16 + i], acc[c * 16 + i + 1]));
+                        acc[c * 16 + i] = r.x;
+                        acc[c * 16 + i + 1] = r.y;
+                    }
+                };
+                // the TMEM load of the next 16 columns is in flight while the current ones are folded in
+                uint32_t va[16], vb[16];
+                tmem_ld_32x32b_x16(taddr, va);
                 #pragma unroll
-                for (uint32_t c = 0; c < kF32ColsPerWarp / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld_32x32b_x32(taddr + c * 32, v);
-                    tmem_ld_wait_x32(v);
-                    if (c + 1 == kF32ColsPerWarp / 32) {
+                for (uint32_t c = 0; c < kWarpCols / 16; c += 2) {
+                    tmem_ld_wait_x16(va);
+                    tmem_ld_32x32b_x16(taddr + (c + 1) * 16, vb);
+                    fold(va, c);
+                    tmem_ld_wait_x16(vb);
+                    if (c + 2 < kWarpCols / 16) {
+                        tmem_ld_32x32b_x16(taddr + (c + 2) * 16, va);
+                    } else {
                         // the buffer is in registers: hand it back to the UMMA warp
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_tmem_empty + e);
+                        if (lane == 0) {
+                            if constexpr (kCtas == 1) mbar_arrive(bar_tmem_empty + e);
+                            else mbar_arrive_remote(bar_tmem_empty + e, 0);
+                        }
                     }
-                    // two elements per instruction (packed f32x2: the same IEEE operations, half the issue slots)
-                    const float2 sa2 = make_float2(sa, sa), sb2 = make_float2(sb, sb);
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 32; i += 2) {
-                        const float2 x = __fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), sa2), sb2);
-                        const float2 r = __fadd2_rn(make_float2(acc[c * 32 + i], acc[c * 32 + i + 1]), x);
-                        acc[c * 32 + i] = r.x;
-                        acc[c * 32 + i + 1] = r.y;
-                    }
+                    fold(vb, c + 1);
                 }
+                sa = sa1; sb = sb1; sa1 = sa2; sb1 = sb2;
             }
             if (!ok) break;
-            // bf16 rows through 64-byte-swizzled staging, one TMA store per 32 columns (rows past the group's end are cut off by
-            // the store's 32-row granularity exactly as in the block-scaled kernel)
+            // 32 columns at a time through swizzled staging, one TMA store each (rows past the group's end are cut off by the store's
+            // 32-row granularity exactly as in the block-scaled kernel)
             #pragma unroll
-            for (uint32_t c = 0; c < kF32ColsPerWarp / 32; ++c) {
-                uint8_t* buf = buf0 + buf_idx * kEpiBuf;
-                if (lane == 0) tma_store_wait_read<1>();
+            for (uint32_t c = 0; c < kWarpCols / 32; ++c) {
+                if (lane == 0) tma_store_wait_read<0>();
                 __syncwarp();
-                const uint32_t row_addr = smem_u32(buf) + lane * 64;
-                #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    const uint32_t chunk = j ^ ((lane >> 1) & 3);
-                    st_shared_v4(row_addr + chunk * 16, pack_bf16x2(acc[c * 32 + 8 * j + 0], acc[c * 32 + 8 * j + 1]),
-                                 pack_bf16x2(acc[c * 32 + 8 * j + 2], acc[c * 32 + 8 * j + 3]), pack_bf16x2(acc[c * 32 + 8 * j + 4], acc[c * 32 + 8 * j + 5]),
-                                 pack_bf16x2(acc[c * 32 + 8 * j + 6], acc[c * 32 + 8 * j + 7]));
+                if constexpr (kPartial) {
+                    const uint32_t row_addr = smem_u32(buf) + lane * 128;
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j)
+                        st_shared_v4(row_addr + ((j ^ (lane & 7)) << 4), __float_as_uint(acc[c * 32 + 4 * j]), __float_as_uint(acc[c * 32 + 4 * j + 1]),
+                                     __float_as_uint(acc[c * 32 + 4 * j + 2]), __float_as_uint(acc[c * 32 + 4 * j + 3]));
+                } else {
+                    const uint32_t row_addr = smem_u32(buf) + lane * 64;
+                    auto bf16x2 = [&](uint32_t i) { return pack_bf16x2(acc[c * 32 + 2 * i], acc[c * 32 + 2 * i + 1]); };
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j)
+                        st_shared_v4(row_addr + ((j ^ ((lane >> 1) & 3)) << 4), bf16x2(4 * j), bf16x2(4 * j + 1), bf16x2(4 * j + 2), bf16x2(4 * j + 3));
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                const uint32_t col0 = t.n0 + col_half * kF32ColsPerWarp + c * 32;
+                const uint32_t col0 = n0 + c * 32;
                 if (lane == 0) {
                     if (col0 < p.n && row0 < t.m_end) tma_store_3d(&tmap_d, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0), static_cast<int32_t>(t.gd));
                     tma_store_commit();
                 }
-                buf_idx ^= 1;
             }
         }
         if (lane == 0) tma_store_wait<0>();
@@ -213,13 +287,15 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
     }
 
     tc_fence_before();
-    __syncthreads();
+    if constexpr (kCtas == 2) cluster_sync(); else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc<1>(tmem_base, 2 * kF32BlockN);
+        tmem_dealloc<kCtas>(tmem_base, 2 * kBlockN);
     }
 }
 
-inline uint32_t f32scale_smem_bytes(uint32_t stages) { return 1024 + stages * 2 * kBlockM * kBlockKBytes + 16 * 2048 + (2 * kMaxStages + 4) * 8 + 16; }
+inline uint32_t f32scale_smem_bytes(uint32_t ctas, uint32_t block_n, bool partial, uint32_t stages) {
+    return 1024 + stages * (kBlockM + block_n / ctas) * kBlockKBytes + 8 * (partial ? 4096 : 2048) + (2 * kMaxStages + 4) * 8 + 16;
+}
 
 }  // namespace dg

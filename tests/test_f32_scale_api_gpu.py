@@ -159,3 +159,39 @@ def test_exact_route_ragged_shapes_and_varying_scales(ctx):
     got = to_f32(out)
     assert not np.isnan(got[valid]).any()
     reference_tolerance(got[valid], want[valid])
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (1500, 4104, 256),      # 256 x 256 tiles of CTA pairs: one full wave, ragged rows and columns, two K blocks
+    (3000, 3976, 384),      # several tiles per pair, an odd number of K blocks (the accumulator buffers swap over between tiles)
+    (130, 520, 6272),       # K ranges with an uneven last one, partial planes of ragged rows and columns
+    (64, 4096, 2048),       # K ranges of four K blocks
+    (1, 8, 128),            # one row, one K block
+])
+def test_exact_route_tile_variants(ctx, m, n, k):
+    # every element against a float64 sum over the K blocks of exact block products; bf16 rounding (2^-8 of a value at most) is
+    # what separates the two, so the squared difference stays below 2^-16 of the squared sum: calc_diff <= 2^-17
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    kb, nb = k // 128, (n + 127) // 128
+    a8 = torch.randn((m, k), generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    b8 = torch.randn((n, k), generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    sfa = torch.rand((m, kb), generator=gen, device="cuda") * 0.03 + 0.004
+    sfb = torch.rand((nb, kb), generator=gen, device="cuda") * 0.03 + 0.004
+    if m % 2 == 0:
+        sfa[0, 0], sfb[0, 0] = 1e-24, 1e-24      # a product outside the range of one factor
+        sfa[1, :], sfb[0, -1] = 1e-21, 1e18
+    a64 = a8.double().view(m, kb, 128) * sfa.double().unsqueeze(-1)
+    b64 = b8.double().view(n, kb, 128) * sfb.double().repeat_interleave(128, 0)[:n].unsqueeze(-1)
+    want = a64.view(m, k) @ b64.view(n, k).t()
+    out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    a_sf_t = dg.transform_sf_dev(ctx, sfa, m, kb, 1)
+    dg.fp8_gemm_nt_dev(ctx, dg.Fp8Tensor(a8.view(torch.uint8), m, k, k), a_sf_t, dg.Fp8Tensor(b8.view(torch.uint8), n, k, k), sfb, out, n)
+    ctx.sync()
+    got = out.double()
+    assert not torch.isnan(got).any()
+    for rows in ([0], [min(1, m - 1)], range(m)):       # the rows with extreme scales on their own, then everything
+        x, y = got[list(rows)], want[list(rows)]
+        # scaled so that squares of tiny rows do not underflow
+        s = y.abs().max().clamp_min(1e-300)
+        x, y = x / s, y / s
+        assert float(1 - 2 * (x * y).sum() / (x * x + y * y).sum()) <= 2.0 ** -17
