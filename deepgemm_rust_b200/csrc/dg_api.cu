@@ -16,6 +16,7 @@
 #include "../../include/dgb200.h"
 #include "dg_cast_kernels.cuh"
 #include "dg_gemm_kernel.cuh"
+#include "dg_gemm_swap.cuh"
 #include "dg_gemm_f32scale.cuh"
 #include "dg_moe_kernels.cuh"
 
@@ -73,6 +74,8 @@ struct dg_ctx {
     uint32_t group_ends_cap = 0;
     float* splitk_ws = nullptr;         // scratch for the f32 partial products of K-split GEMMs
     size_t splitk_ws_cap = 0;           // in floats
+    uint32_t* splitk_counters = nullptr;   // K ranges that have arrived, per tile (swapped tile family); zero between launches
+    uint32_t splitk_counters_cap = 0;
     uint32_t* bridge_sf[2] = {nullptr, nullptr};   // packed scale words built from f32 scales by the f32-scale entry points
     size_t bridge_sf_cap[2] = {0, 0};              // in words
 };
@@ -120,6 +123,7 @@ int dg_ctx_destroy(dg_ctx* ctx) {
     if (ctx->status) cudaFree(ctx->status);
     if (ctx->group_ends) cudaFree(ctx->group_ends);
     if (ctx->splitk_ws) cudaFree(ctx->splitk_ws);
+    if (ctx->splitk_counters) cudaFree(ctx->splitk_counters);
     for (int i = 0; i < 2; ++i)
         if (ctx->bridge_sf[i]) cudaFree(ctx->bridge_sf[i]);
     if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -133,6 +137,7 @@ int dg_ctx_check_status(dg_ctx* ctx) {
     DG_CUDA(cudaMemcpy(&st, ctx->status, sizeof(st), cudaMemcpyDeviceToHost));
     if (st.code != 0) {
         cudaMemset(ctx->status, 0, sizeof(st));
+        if (ctx->splitk_counters) cudaMemset(ctx->splitk_counters, 0, ctx->splitk_counters_cap * sizeof(uint32_t));   // the kernel may have left some
         return fail(DG_ERR_TIMEOUT, "a device-side wait ran out: block %u, site 0x%x, parity %u", st.block, st.site, st.extra);
     }
     return DG_OK;
@@ -183,8 +188,7 @@ uint32_t dg_get_theoretical_mk_alignment_for_contiguous_layout(uint32_t arch_maj
 struct KernelPlan {
     bool swap;                 // weights on the UMMA M dimension, activation rows on UMMA N
     uint32_t ctas, umma_n, halves, stages, accum, smem;
-    uint32_t splits;           // K ranges summed by a second kernel (first tile family)
-    uint32_t cluster_splits;   // K ranges summed inside a cluster (swapped family)
+    uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
 };
 static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan);
@@ -193,21 +197,26 @@ int dg_best_config(const dg_desc* d, dg_config* out) {
     return search_config(d, 0, out, &plan);
 }
 
-// Is any of the DG_* knobs set?  They may change between two calls, so a call that sees one never uses a remembered choice.
+// What the DG_* knobs say, as a hash of their text (0 if none is set); they may change between two calls.
 // One pass over the environment takes 50 ns; asking for every knob by name 54 ns each.
-static bool any_knob_set() {
-    for (char** e = environ; e != nullptr && *e != nullptr; ++e)
-        if ((*e)[0] == 'D' && (*e)[1] == 'G' && (*e)[2] == '_') return true;
-    return false;
+static uint64_t knob_signature() {
+    uint64_t h = 0;
+    for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
+        if ((*e)[0] != 'D' || (*e)[1] != 'G' || (*e)[2] != '_') continue;
+        for (const char* c = *e; *c != 0; ++c) h = (h ^ static_cast<unsigned char>(*c)) * 0x100000001B3ull;
+        h = (h ^ '\n') * 0x100000001B3ull + 1;
+    }
+    return h;
 }
 
 // search_config with the choices of recent problems remembered: the search walks ~500 candidates (3.7 us on a B200 host, more
 // than the launch itself), and a program asks for the same few problems again and again.  The choice is a function of the
-// description, the alignment knob and the environment alone.  One small table per thread, overwritten on collision.
+// description, the alignment and the knobs alone.  One small table per thread, overwritten on collision.
 static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan) {
     struct Key {
         dg_desc desc;
         uint32_t no_k_ranges, alignment;
+        uint32_t knobs[2];
     };
     struct Entry {
         bool used;
@@ -217,10 +226,10 @@ static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     };
     constexpr uint32_t kEntries = 64;
     static thread_local Entry table[kEntries];
-    if (any_knob_set()) return search_config(d, no_k_ranges, out, plan);
-    const Key key = {*d, no_k_ranges, g_mk_alignment.load()};
-    static_assert(sizeof(Key) == 16 * sizeof(uint32_t), "compared and hashed as 16 words");
-    uint32_t words[16], hash = 0;
+    const uint64_t knobs = knob_signature();
+    const Key key = {*d, no_k_ranges, g_mk_alignment.load(), {static_cast<uint32_t>(knobs), static_cast<uint32_t>(knobs >> 32)}};
+    static_assert(sizeof(Key) == 18 * sizeof(uint32_t), "compared and hashed as 18 words");
+    uint32_t words[18], hash = 0;
     memcpy(words, &key, sizeof(key));
     for (uint32_t w : words) hash = (hash ^ w) * 0x9E3779B1u;
     Entry& e = table[(hash >> 16) % kEntries];
@@ -233,6 +242,98 @@ static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     *out = e.cfg;
     *plan = e.plan;
     return DG_OK;
+}
+
+// Is the swapped family the better one for this problem?
+static bool prefer_swapped(const dg_desc* d) {
+    (void)d;
+    return false;
+}
+
+// Tile choice of the swapped family; false if nothing fits (or the DG_* knobs leave nothing).
+static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, KernelPlan* plan) {
+    const char *force_n = getenv("DG_BLOCK_N"), *force_ctas = getenv("DG_CTAS"), *force_stages = getenv("DG_STAGES");
+    const char *force_splits = getenv("DG_SPLITS"), *force_halves = getenv("DG_K_SLABS");
+    const bool mxf4 = d->a_bits == 4 && d->b_bits == 4;
+    const uint32_t half_k = mxf4 ? 256 : 128, groups = d->num_groups ? d->num_groups : 1;
+    const bool dense = d->gemm_type == DG_GEMM_NORMAL || d->gemm_type == DG_GEMM_BATCHED;
+    const uint32_t align = g_mk_alignment.load();
+    double best_cost = 0;
+    bool found = false;
+    for (uint32_t halves = 1; halves <= 2; ++halves) {
+        if (force_halves && static_cast<uint32_t>(atoi(force_halves)) != halves) continue;
+        const uint32_t block_k = half_k * halves;
+        // kernel operand A is the caller's b (weights), kernel operand B the caller's a (activation rows)
+        const uint32_t sfa_words = 4 * d->gran_b >= block_k ? 1 : block_k / (4 * d->gran_b);
+        const uint32_t sfb_words = 4 * d->gran_a >= block_k ? 1 : block_k / (4 * d->gran_a);
+        const uint32_t total_kb = ceil_div(d->k, block_k);
+        for (uint32_t ctas = 1; ctas <= 2; ++ctas) {
+            if (force_ctas && static_cast<uint32_t>(atoi(force_ctas)) != ctas) continue;
+            if (ctas == 2 && sms < 2) continue;
+            const uint32_t step = dense ? 16 * ctas : 32, workers = sms / ctas;
+            // rows per group, as far as the host knows them
+            double rows = d->m;
+            if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
+                const double per_group = static_cast<double>(d->m) / groups;
+                rows = per_group > align / 2.0 ? per_group - align / 2.0 : per_group;
+            } else if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) {
+                rows = d->expected_m < d->m ? d->expected_m : d->m;
+            }
+            // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected, and 288 rows for
+            // groups of about 256 (half of them are a little above)
+            uint32_t bn;
+            if (dense) bn = d->m <= 256 ? ceil_div(d->m, step) * step : 256;
+            else bn = ceil_div(static_cast<uint32_t>(2 * rows) + 1, 32) * 32;
+            if (!dense && bn < 64) bn = 64;
+            if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED && bn > ceil_div(d->m, 32) * 32) bn = ceil_div(d->m, 32) * 32;
+            if (bn > 256) bn = 256;
+            if (force_n) bn = static_cast<uint32_t>(atoi(force_n));
+            if (bn == 0 || bn > dg::kSwapMaxRows || (bn > 256 && bn % 32 != 0) || (bn > 256 && dense) || bn % step != 0) continue;
+            const uint32_t sf_cols = 4 * sfa_words + ceil_div(bn, 128) * 4 * sfb_words;
+            if (bn + sf_cols > 512) continue;
+            const uint32_t m_blocks = ceil_div(d->n, 128 * ctas);
+            const uint32_t most_rows = bn < 32 ? bn : bn / 32 * 32;         // of a tile that has a neighbour
+            const double row_tiles = rows <= bn ? 1.0 : (dense ? static_cast<double>(ceil_div(d->m, most_rows)) : rows / most_rows + 0.5);
+            const double tile_rows = rows / row_tiles;
+            const uint32_t tiles = static_cast<uint32_t>(groups * row_tiles * m_blocks + 0.999);
+            const uint32_t most_splits = d->gemm_type == DG_GEMM_NORMAL ? 16 : 1;
+            for (uint32_t splits = 1; splits <= most_splits; ++splits) {
+                if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != splits) continue;
+                if (splits > 1 && total_kb < 2 * splits) continue;       // at least two k-blocks per range
+                if (splits > 1 && !force_splits && static_cast<uint64_t>(tiles) * splits > workers) continue;
+                uint32_t stages = force_stages ? static_cast<uint32_t>(atoi(force_stages)) : dg::kMaxStages;
+                if (stages > dg::kMaxStages) stages = dg::kMaxStages;
+                auto smem = [&](uint32_t st) { return dg::gemm_swap_smem_bytes(bn, ctas, d->cd_dtype, st, sfa_words, sfb_words, halves); };
+                while (stages > 1 && smem(stages) > kSmemCapacity) --stages;
+                if (smem(stages) > kSmemCapacity || (stages < 2 && !force_stages)) continue;
+                const double mma = 4.0 * (tile_rows > 66.0 ? tile_rows * 0.5 : 33.0);
+                const double feed = (16384.0 + tile_rows / ctas * 128.0) / 70.0;
+                const double per_kb = (halves * (mma > feed ? mma : feed) + 150.0) * (stages < 3 ? 1.5 : 1.0);   // two stages do not cover a load's latency
+                const double kb_per = static_cast<double>(total_kb) / splits;
+                const double waves = splits > 1 || dense ? ceil_div(tiles * splits, workers) : static_cast<double>(tiles) / workers;
+                const double cost = waves * (kb_per * per_kb + 800.0) + (splits > 1 ? 2500.0 + splits * tile_rows * 8.0 : 0.0);
+                if (!found || cost < best_cost * (1.0 - 1e-9)) {
+                    found = true;
+                    best_cost = cost;
+                    plan->swap = true;
+                    plan->ctas = ctas; plan->umma_n = bn; plan->halves = halves; plan->stages = stages; plan->accum = 2;
+                    plan->splits = splits; plan->tiles = tiles; plan->smem = smem(stages);
+                    out->swap_ab = 1;
+                    out->block_m = bn;            // activation rows per tile (an upper bound: a tile's UMMA N follows its rows)
+                    out->block_n = 128 * ctas;    // weight rows per tile
+                    out->block_k = block_k;
+                    out->cluster_m = 1;
+                    out->cluster_n = ctas;
+                    out->num_stages = stages;
+                    out->num_accum_stages = 2;
+                    out->smem_size = plan->smem;
+                    out->num_tiles = tiles;
+                    out->num_splits = splits;
+                }
+            }
+        }
+    }
+    return found;
 }
 
 // no_k_ranges: the caller adds into the output (K ranges would need the sum to be written, not added)
@@ -338,96 +439,13 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
         }
     }
     }
-    // ---- the swapped family: weight rows on UMMA M, activation rows on UMMA N (bf16 / f32 outputs).  DG_SWAP=1 selects it
-    // wherever it applies.  It is not the default anywhere yet: measured on B200 it streams the weights of skinny and
-    // small-group problems more slowly than the first family, which keeps more weight bytes in flight per SM.
+    // ---- the swapped family: weight rows on UMMA M, activation rows on UMMA N
     {
         const char* force_swap = getenv("DG_SWAP");
         const bool forced = force_swap && atoi(force_swap) != 0, forbidden = force_swap && atoi(force_swap) == 0;
-        const bool plain_out = d->cd_dtype == DG_OUT_BF16 || d->cd_dtype == DG_OUT_F32;
-        const bool dense = d->gemm_type == DG_GEMM_NORMAL || d->gemm_type == DG_GEMM_BATCHED;
-        const bool want = forced && !d->major_a_mn && !d->major_b_mn;   // MN-major operands: first family only
-        if (plain_out && want && !forbidden) {
-            uint32_t s_n = 0, s_ctas = 0, s_halves = 0, s_stages = 0, s_accum = 0, s_split = 1, s_tiles = 0;
-            double s_cost = 0;
-            for (uint32_t halves = 1; halves <= 2; ++halves) {
-                if (force_halves && static_cast<uint32_t>(atoi(force_halves)) != halves) continue;
-                const uint32_t block_k = half_k * halves;
-                // kernel operand A is the caller's b (weights), kernel operand B the caller's a (activation rows)
-                const uint32_t sfa_words = 4 * d->gran_b >= block_k ? 1 : block_k / (4 * d->gran_b);
-                const uint32_t sfb_words = 4 * d->gran_a >= block_k ? 1 : block_k / (4 * d->gran_a);
-                const uint32_t total_kb = ceil_div(d->k, block_k);
-                for (uint32_t ctas = 1; ctas <= 2; ++ctas) {
-                    if (force_ctas && static_cast<uint32_t>(atoi(force_ctas)) != ctas) continue;
-                    if (ctas == 2 && sms < 2) continue;
-                    const uint32_t step_n = 16 * ctas;
-                    // rows a tile may have: everything a dense problem has (up to 256), else 256 and the tile's UMMA N follows the group
-                    uint32_t bn = dense && d->m <= 256 ? ceil_div(d->m, step_n) * step_n : 256;
-                    if (force_n) bn = static_cast<uint32_t>(atoi(force_n));
-                    if (bn == 0 || bn > 256 || bn % step_n != 0) continue;
-                    const uint32_t sf_cols = 4 * sfa_words + ceil_div(bn, 128) * 4 * sfb_words;
-                    if (bn + sf_cols > 512) continue;
-                    const uint32_t accum = 2 * bn + sf_cols <= 512 ? 2 : 1;
-                    const uint32_t a_blocks = ceil_div(d->n, 128 * ctas);
-                    double row_blocks;
-                    if (dense) row_blocks = static_cast<double>(groups) * ceil_div(d->m, bn);
-                    else if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
-                        const double per_group = static_cast<double>(d->m) / groups;
-                        row_blocks = groups * ((per_group > align / 2.0 ? per_group - align / 2.0 : per_group) / bn + 0.5);
-                    } else row_blocks = groups * (static_cast<double>(d->expected_m ? d->expected_m : d->m) / bn + 0.5);
-                    const uint32_t tiles = static_cast<uint32_t>(row_blocks * a_blocks + 0.999);
-                    const uint32_t max_split = d->gemm_type == DG_GEMM_NORMAL ? 8 / ctas : 1;
-                    for (uint32_t split = 1; split <= max_split; ++split) {
-                        if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != split) continue;
-                        const uint32_t kb_per = ceil_div(total_kb, split);
-                        if (split > 1 && total_kb < 2 * split) continue;       // at least two k-blocks per range
-                        uint32_t stages = force_stages ? static_cast<uint32_t>(atoi(force_stages)) : dg::kMaxStages;
-                        if (stages > dg::kMaxStages) stages = dg::kMaxStages;
-                        while (stages > 1 && dg::gemm_smem_bytes(bn, ctas, d->cd_dtype, stages, sfa_words, sfb_words, halves, true) > kSmemCapacity) --stages;
-                        if (dg::gemm_smem_bytes(bn, ctas, d->cd_dtype, stages, sfa_words, sfb_words, halves, true) > kSmemCapacity) continue;
-                        if (stages < 3 && !force_stages) continue;
-                        // the exchange buffer of the K ranges lies over the stage buffers
-                        if (split > 1 && dg::gemm_stage_bytes(bn, ctas, stages, halves) < split * ceil_div(bn, split) * 512) continue;
-                        const double bytes_kb = halves * (16384.0 + bn / ctas * 128.0);                  // per CTA and k-block
-                        const double stream = kb_per * bytes_kb / 64.0;
-                        const double mma = kb_per * halves * 4.0 * (bn * 0.5 > 118.0 ? bn * 0.5 : 118.0);
-                        const double per_tile = (stream > mma ? stream : mma) + (split > 1 ? 3500.0 : (accum == 1 ? 12.0 * bn : 2.0 * bn)) + 2500.0;
-                        const double ctas_total = static_cast<double>(tiles) * split * ctas;
-                        const double waves = ctas_total <= sms ? 1.0 : ctas_total / sms;               // the hardware refills SMs as clusters finish
-                        const double hbm = (static_cast<double>(d->n) * groups * d->k * (d->b_bits / 8.0) + static_cast<double>(d->m) * d->k + 2.0 * d->m * d->n) / 3300.0;
-                        const double l2 = ctas_total * kb_per * bytes_kb / 9000.0;
-                        double cost = waves * per_tile;
-                        if (hbm > cost) cost = hbm;
-                        if (l2 > cost) cost = l2;
-                        cost += 0.1 * per_tile + l2 * 0.01;      // among equals: more CTAs in flight, fewer bytes through L2
-                        if (s_n == 0 || cost < s_cost * (1.0 - 1e-9)) {
-                            s_n = bn; s_ctas = ctas; s_halves = halves; s_stages = stages; s_accum = accum; s_split = split; s_tiles = tiles;
-                            s_cost = cost;
-                        }
-                    }
-                }
-            }
-            if (s_n != 0) {
-                const uint32_t block_k = half_k * s_halves;
-                const uint32_t sfa_words = 4 * d->gran_b >= block_k ? 1 : block_k / (4 * d->gran_b);
-                const uint32_t sfb_words = 4 * d->gran_a >= block_k ? 1 : block_k / (4 * d->gran_a);
-                plan->swap = true;
-                plan->ctas = s_ctas; plan->umma_n = s_n; plan->halves = s_halves; plan->stages = s_stages; plan->accum = s_accum;
-                plan->splits = 1; plan->cluster_splits = s_split; plan->tiles = s_tiles;
-                plan->smem = dg::gemm_smem_bytes(s_n, s_ctas, d->cd_dtype, s_stages, sfa_words, sfb_words, s_halves, true);
-                out->swap_ab = 1;
-                out->block_m = s_n;            // activation rows per tile (an upper bound: a tile's UMMA N follows its rows)
-                out->block_n = 128 * s_ctas;   // weight rows per tile
-                out->block_k = block_k;
-                out->cluster_m = 1;
-                out->cluster_n = s_ctas;
-                out->num_stages = s_stages;
-                out->num_accum_stages = s_accum;
-                out->smem_size = plan->smem;
-                out->num_tiles = s_tiles;
-                out->num_splits = s_split;
-                return DG_OK;
-            }
+        const bool applies = !swiglu && !d->major_a_mn && !d->major_b_mn;
+        if (applies && !forbidden && (forced || prefer_swapped(d))) {
+            if (search_swapped(d, sms, out, plan)) return DG_OK;
             if (forced) return fail(DG_ERR_SHAPE, "no tile configuration of the swapped family fits (DG_BLOCK_N=%s DG_CTAS=%s)", force_n ? force_n : "",
                                     force_ctas ? force_ctas : "");
         }
@@ -436,7 +454,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     const uint32_t stages = best_stages;
     plan->swap = false;
     plan->ctas = best_ctas; plan->umma_n = best_n; plan->halves = best_halves; plan->stages = best_stages; plan->accum = best_accum;
-    plan->splits = best_splits; plan->cluster_splits = 1; plan->tiles = best_tiles;
+    plan->splits = best_splits; plan->tiles = best_tiles;
     out->swap_ab = 0;
     out->block_m = 128 * best_ctas;
     out->block_n = best_n;
@@ -544,22 +562,28 @@ void launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem,
 
 // The opt-in to the full shared-memory carve-out is per kernel instantiation and per device; the first
 // call also makes the runtime load that kernel's image.
-template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, bool kSwap = false>
+// kSlabs: 0 the first tile family, else the swapped family with that many K slabs per stage.
+template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kSlabs>
+constexpr auto gemm_kernel() {
+    if constexpr (kSlabs != 0) return &dg::dg_gemm_swap_kernel<kFmt, kOut, kCtas, kSlabs>;
+    else return &dg::dg_gemm_kernel<kFmt, kOut, kCtas>;
+}
+template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kSlabs = 0>
 cudaError_t configure_kernel() {
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && (configured.load() & (1ull << dev))) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(dg::dg_gemm_kernel<kFmt, kOut, kCtas, kSwap>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<kFmt, kOut, kCtas, kSlabs>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kSmemCapacity));
     if (e == cudaSuccess && dev < 64) configured.fetch_or(1ull << dev);
     return e;
 }
 
-template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, bool kSwap = false>
+template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kSlabs = 0>
 cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream, const CUtensorMap* maps) {
-    auto kernel = dg::dg_gemm_kernel<kFmt, kOut, kCtas, kSwap>;
-    cudaError_t e = configure_kernel<kFmt, kOut, kCtas, kSwap>();
+    auto kernel = gemm_kernel<kFmt, kOut, kCtas, kSlabs>();
+    cudaError_t e = configure_kernel<kFmt, kOut, kCtas, kSlabs>();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -569,7 +593,7 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kCtas * (kSwap ? p.cluster_splits : 1u);   // swapped family: the K ranges of a tile share a cluster
+    attr[0].val.clusterDim.x = kCtas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     // the kernel waits for its predecessor itself (griddep_wait) after its set-up: let the two overlap
@@ -577,14 +601,25 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4]);
+    if constexpr (kSlabs != 0) return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
+    else return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4]);
 }
 
-template <uint32_t kFmt, uint32_t kCtas>
-cudaError_t launch_swapped(int kind, const dg::GemmParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream, const CUtensorMap* maps) {
-    if (kind == DG_OUT_BF16) return launch_kernel<kFmt, dg::kOutBf16, kCtas, true>(p, grid, smem, stream, maps);
-    if (kind == DG_OUT_F32) return launch_kernel<kFmt, dg::kOutF32, kCtas, true>(p, grid, smem, stream, maps);
+template <uint32_t kFmt, uint32_t kCtas, uint32_t kSlabs>
+cudaError_t launch_swapped_by_out(int kind, const dg::GemmParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream, const CUtensorMap* maps) {
+    if (kind == DG_OUT_BF16) return launch_kernel<kFmt, dg::kOutBf16, kCtas, kSlabs>(p, grid, smem, stream, maps);
+    if (kind == DG_OUT_F32) return launch_kernel<kFmt, dg::kOutF32, kCtas, kSlabs>(p, grid, smem, stream, maps);
+    if constexpr (kFmt != dg::kFmtBf16)
+        if (kind == DG_OUT_FP8) return launch_kernel<kFmt, dg::kOutFp8, kCtas, kSlabs>(p, grid, smem, stream, maps);
     return cudaErrorInvalidValue;
+}
+template <uint32_t kFmt>
+cudaError_t launch_swapped(const KernelPlan& plan, int kind, const dg::GemmParams& p, uint32_t grid, cudaStream_t stream, const CUtensorMap* maps) {
+    if (plan.ctas == 2)
+        return plan.halves == 2 ? launch_swapped_by_out<kFmt, 2, 2>(kind, p, grid, plan.smem, stream, maps)
+                                : launch_swapped_by_out<kFmt, 2, 1>(kind, p, grid, plan.smem, stream, maps);
+    return plan.halves == 2 ? launch_swapped_by_out<kFmt, 1, 2>(kind, p, grid, plan.smem, stream, maps)
+                            : launch_swapped_by_out<kFmt, 1, 1>(kind, p, grid, plan.smem, stream, maps);
 }
 
 template <uint32_t kFmt, uint32_t kCtas>
@@ -605,10 +640,14 @@ cudaError_t configure_contiguous_kernels_of() {
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 2>();
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 1>();
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 2>();
-    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 1, true>();
-    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 2, true>();
-    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 1, true>();
-    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 2, true>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 1, 1>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 1, 2>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 2, 1>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 2, 2>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 1, 1>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 1, 2>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 2, 1>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 2, 2>();
     return e;
 }
 // Everything dg_m_grouped_fp8_fp4_gemm_contiguous[_ends] can launch, configured (and loaded) for the current device.
@@ -697,14 +736,25 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const uint32_t splits = plan.splits;
     const uint32_t ws_pitch = align4(pr.n);
     if (splits > 1) {
-        rc = ensure_splitk_ws(ctx, static_cast<size_t>(splits) * pr.m * ws_pitch);
+        // first family: one (m, n) plane per range; swapped family: one accumulator per tile, CTA of the pair and range
+        rc = ensure_splitk_ws(ctx, swap ? static_cast<size_t>(plan.tiles) * plan.ctas * splits * ceil_div(plan.umma_n, 32) * 32 * dg::kBlockM
+                                        : static_cast<size_t>(splits) * pr.m * ws_pitch);
         if (rc) return rc;
+        const uint32_t counters = plan.tiles * plan.ctas;
+        if (swap && ctx->splitk_counters_cap < counters) {
+            DG_CUDA(cudaSetDevice(ctx->ordinal));
+            if (ctx->splitk_counters) { cudaFree(ctx->splitk_counters); ctx->splitk_counters = nullptr; ctx->splitk_counters_cap = 0; }
+            const uint32_t cap = counters < 1024 ? 1024 : counters;
+            DG_CUDA(cudaMalloc(&ctx->splitk_counters, cap * sizeof(uint32_t)));
+            DG_CUDA(cudaMemsetAsync(ctx->splitk_counters, 0, cap * sizeof(uint32_t), ctx->stream));
+            ctx->splitk_counters_cap = cap;
+        }
     }
     const uint32_t sfa_words = 4 * ka->gran_k >= block_k ? 1 : block_k / (4 * ka->gran_k);
     const uint32_t sfb_words = 4 * kb->gran_k >= block_k ? 1 : block_k / (4 * kb->gran_k);
     const uint32_t sf_block_n = ceil_div(plan.umma_n, 128) * 128;
 
-    CUtensorMap maps[5];
+    CUtensorMap maps[7];
     bool wide_k = false;
     {
         // packed e2m1 stays packed in shared memory for kind::mxf4 (16U4_ALIGN8B) and is expanded to one code per byte
@@ -727,7 +777,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         // last slab would read into the next row), otherwise the 3-D maps and one load per slab stay.
         const char* wide_env = getenv("DG_WIDE_K");
         // (not where the loads carry the evict-first hint: dense problems of a single row block, see below)
-        const bool hinted = pr.type == DG_GEMM_NORMAL && pr.m <= (swap ? plan.umma_n : 128 * plan.ctas);
+        const bool hinted = !swap && pr.type == DG_GEMM_NORMAL && pr.m <= 128 * plan.ctas;
         wide_k = plan.halves == 2 && !mxf4 && ka->bits == 8 && kb->bits == 8 && pr.k % 128 == 0 && !(!pr.bf16 && (ka->major_mn || kb->major_mn)) &&
                  !hinted && !(wide_env && strcmp(wide_env, "0") == 0);
         if (wide_k) {
@@ -738,7 +788,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
             if (rc) return rc;
             uint64_t e4[4] = {128, kb_rows, pr.k / 128, kb_groups};
             uint64_t t4[3] = {b_pitch, 128, b_pitch * kb_rows};
-            uint32_t c4[4] = {128, plan.umma_n / plan.ctas, 2, 1};
+            uint32_t c4[4] = {128, swap ? dg::swap_main_rows(plan.umma_n, plan.ctas) : plan.umma_n / plan.ctas, 2, 1};
             rc = encode_map(&maps[1], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kb->data, e4, t4, c4, CU_TENSOR_MAP_SWIZZLE_128B, "B");
             if (rc) return rc;
         } else {
@@ -746,13 +796,24 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         if (rc) return rc;
         uint64_t bdims[3] = {pr.k, kb_rows, kb_groups};
         uint64_t bstrides[2] = {b_pitch, b_pitch * kb_rows};
-        uint32_t bbox[3] = {slab, plan.umma_n / plan.ctas, 1};
+        uint32_t bbox[3] = {slab, swap ? dg::swap_main_rows(plan.umma_n, plan.ctas) : plan.umma_n / plan.ctas, 1};
         if (!pr.bf16 && kb->major_mn) {
             bdims[0] = kb_rows; bdims[1] = pr.k; bstrides[0] = kb->ld; bstrides[1] = static_cast<uint64_t>(kb->ld) * pr.k;
             bbox[0] = 128; bbox[1] = slab;
         }
         rc = encode_map(&maps[1], map_dtype(kb->bits), 3, kb->data, bdims, bstrides, bbox, CU_TENSOR_MAP_SWIZZLE_128B, "B");
         if (rc) return rc;
+        }
+        if (swap) {
+            // smaller boxes of the activations: for tiles with few rows, and for the rows of a tile beyond 256
+            uint64_t pdims[3] = {pr.k, kb_rows, kb_groups};
+            uint64_t pstrides[2] = {b_pitch, b_pitch * kb_rows};
+            uint32_t pbox[3] = {slab, dg::swap_part_rows(dg::swap_main_rows(plan.umma_n, plan.ctas)), 1};
+            rc = encode_map(&maps[5], map_dtype(kb->bits), 3, kb->data, pdims, pstrides, pbox, CU_TENSOR_MAP_SWIZZLE_128B, "B part");
+            if (rc) return rc;
+            pbox[1] = dg::kSwapTailRows;
+            rc = encode_map(&maps[6], map_dtype(kb->bits), 3, kb->data, pdims, pstrides, pbox, CU_TENSOR_MAP_SWIZZLE_128B, "B tail");
+            if (rc) return rc;
         }
     }
     const uint32_t sfa_cols = dg_sf_packed_cols(pr.k, ka->gran_k), sfb_cols = dg_sf_packed_cols(pr.k, kb->gran_k);
@@ -766,12 +827,13 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         uint64_t bdims[2] = {align4(kb_rows), static_cast<uint64_t>(sfb_cols) * kb_groups};
         uint64_t bstrides[1] = {static_cast<uint64_t>(align4(kb_rows)) * 4};
         uint32_t bbox[2] = {swiglu ? plan.umma_n / 2 : sf_block_n, sfb_words};   // fused activation: gate rows and up rows as two boxes
+        if (swap) { bbox[0] = 128; bbox[1] = 1; }
         rc = encode_map(&maps[3], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, pr.bf16 ? kb->data : kb->sf, bdims, bstrides, bbox, CU_TENSOR_MAP_SWIZZLE_NONE, "SFB");
         if (rc) return rc;
     }
     {
         // 32 rows per store; 32 columns of bf16 (64-byte rows) or f32, 128 columns of e4m3 (128-byte rows)
-        if (splits > 1) {
+        if (splits > 1 && !swap) {
             // K ranges write f32 partial tiles into the workspace, one plane per range
             uint64_t dims[3] = {pr.n, pr.m, splits};
             uint64_t strides[2] = {static_cast<uint64_t>(ws_pitch) * 4, static_cast<uint64_t>(ws_pitch) * 4 * pr.m};
@@ -783,9 +845,10 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
             const uint64_t pitch = static_cast<uint64_t>(out->ld) * d_elem;
             uint64_t dims[3] = {n_out, pr.m, a_groups};
             uint64_t strides[2] = {pitch, pitch * pr.m};
-            uint32_t box[3] = {out->kind == DG_OUT_FP8 ? 128u : 32u, 32, 1};   // the fused activation stores 32 x 32 bytes, unswizzled
+            // the fused activation and the swapped family store e4m3 as 32 x 32 bytes, unswizzled
+            uint32_t box[3] = {out->kind == DG_OUT_FP8 && !swap ? 128u : 32u, 32, 1};
             rc = encode_map(&maps[4], dt, 3, out->buf, dims, strides, box,
-                            swiglu ? CU_TENSOR_MAP_SWIZZLE_NONE : (out->kind == DG_OUT_BF16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B), "D");
+                            swiglu || (fp8_out && swap) ? CU_TENSOR_MAP_SWIZZLE_NONE : (out->kind == DG_OUT_BF16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B), "D");
         }
         if (rc) return rc;
     }
@@ -801,9 +864,14 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.block_n = plan.umma_n;
     p.block_k_elems = block_k;
     p.num_splits = splits;
-    p.cluster_splits = plan.cluster_splits;
-    p.kb_per_split = splits > 1 ? ceil_div(ceil_div(ceil_div(pr.k, block_k), splits), 4) * 4 : ceil_div(ceil_div(pr.k, block_k), plan.cluster_splits);
-    p.out_group_rows = (pr.type == DG_GEMM_M_GROUPED_MASKED || pr.type == DG_GEMM_BATCHED) ? pr.m : 0;
+    p.kb_per_split = splits > 1 ? ceil_div(ceil_div(ceil_div(pr.k, block_k), splits), 4) * 4 : ceil_div(pr.k, block_k);
+    if (swap) {
+        p.acc_stride = dg::gemm_swap_acc_stride(plan.umma_n, sfa_words, sfb_words);
+        p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
+        if (p.acc_stride == plan.umma_n) p.acc_edge_chunks = 0;
+        p.splitk_ws = ctx->splitk_ws;
+        p.splitk_counters = ctx->splitk_counters;
+    }
     p.num_stages = plan.stages;
     p.num_accum_stages = plan.accum;
     p.gran_a = ka->gran_k;
@@ -819,7 +887,11 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.mk_alignment = align;
     // groups start at multiples of `align` rows; tiles stay 128 (or 256) rows tall and simply run into the next group's rows,
     // which are computed and not stored.  Stores go out in 32-row boxes, so only an alignment of 16 needs row-exact stores.
-    p.mask_rows = (contiguous && align % 32 != 0) ? 1 : 0;
+    // A problem that the rule sends to the swapped family writes the same rows; where DG_SWAP=1 pins that family, the masked and
+    // contiguous layouts write exactly the valid rows.
+    const char* pinned = getenv("DG_SWAP");
+    const bool exact_rows = swap && !fp8_out && pinned && atoi(pinned) != 0 && (contiguous || pr.type == DG_GEMM_M_GROUPED_MASKED);
+    p.mask_rows = ((contiguous && align % 32 != 0) || exact_rows) ? 1 : 0;
     p.out_ptr = out->buf;
     p.out_ld = out->ld;
     {
@@ -837,7 +909,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.mn_b = (!pr.bf16 && kb->major_mn) ? 1 : 0;
     p.accumulate = e.accumulate ? 1 : 0;
     p.tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
-    p.has_alpha = (e.has_alpha && splits == 1) ? 1 : 0;   // with K ranges summed by the second kernel alpha is applied there
+    p.has_alpha = (e.has_alpha && (swap || splits == 1)) ? 1 : 0;   // with K ranges summed by the second kernel alpha is applied there
     p.alpha = e.alpha;
     p.sfd = out->sfd;
     p.sfd_stride = align4(pr.m);
@@ -856,26 +928,21 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     uint32_t grid = static_cast<uint32_t>(ctx->num_sms) / ctas * ctas;
     if (pr.type == DG_GEMM_NORMAL || pr.type == DG_GEMM_BATCHED)
         grid = plan.tiles * splits * ctas < grid ? plan.tiles * splits * ctas : grid;
-    // K ranges summed inside a cluster: one cluster per output tile, as many clusters as tiles
-    if (swap && plan.cluster_splits > 1) grid = plan.tiles * plan.cluster_splits * ctas;
-    const int kernel_out = splits > 1 ? DG_OUT_F32 : out->kind;
+    const int kernel_out = splits > 1 && !swap ? DG_OUT_F32 : out->kind;
     const uint32_t smem = plan.smem;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     cudaError_t ce;
     if (swap) {
-        if (pr.bf16) ce = ctas == 2 ? launch_swapped<dg::kFmtBf16, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
-                                    : launch_swapped<dg::kFmtBf16, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
-        else if (mxf4) ce = ctas == 2 ? launch_swapped<dg::kFmtMxf4, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
-                                      : launch_swapped<dg::kFmtMxf4, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
-        else ce = ctas == 2 ? launch_swapped<dg::kFmtMxf8f6f4, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
-                            : launch_swapped<dg::kFmtMxf8f6f4, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
+        if (pr.bf16) ce = launch_swapped<dg::kFmtBf16>(plan, kernel_out, p, grid, ctx->stream, maps);
+        else if (mxf4) ce = launch_swapped<dg::kFmtMxf4>(plan, kernel_out, p, grid, ctx->stream, maps);
+        else ce = launch_swapped<dg::kFmtMxf8f6f4>(plan, kernel_out, p, grid, ctx->stream, maps);
     } else if (pr.bf16) ce = ctas == 2 ? launch_by_out<dg::kFmtBf16, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
                                 : launch_by_out<dg::kFmtBf16, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
     else if (mxf4) ce = ctas == 2 ? launch_by_out<dg::kFmtMxf4, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
                                   : launch_by_out<dg::kFmtMxf4, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
     else ce = ctas == 2 ? launch_by_out<dg::kFmtMxf8f6f4, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
                         : launch_by_out<dg::kFmtMxf8f6f4, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
-    if (ce == cudaSuccess && splits > 1) {
+    if (ce == cudaSuccess && splits > 1 && !swap) {
         const uint64_t threads = static_cast<uint64_t>(pr.m) * ceil_div(pr.n, 4);
         const uint32_t blocks = static_cast<uint32_t>((threads + 255) / 256);
         const float alpha = e.has_alpha ? e.alpha : 1.0f;
@@ -1088,7 +1155,6 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     p.block_k_elems = 128;
     p.num_splits = plan.splits;
     p.kb_per_split = plan.kb_per_split;
-    p.cluster_splits = 1;
     p.num_accum_stages = 2;
     p.mk_alignment = align;
     p.grouped_layout = layout;

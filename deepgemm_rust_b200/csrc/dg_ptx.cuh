@@ -170,6 +170,11 @@ DG_DEVICE uint64_t l2_policy_evict_first() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
     return pol;
 }
+DG_DEVICE uint64_t l2_policy_evict_normal() {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
 DG_DEVICE void tma_load_3d_hint(void* smem, const void* tmap, uint64_t* bar, int32_t x, int32_t y, int32_t z, uint64_t policy) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(
@@ -182,6 +187,20 @@ DG_DEVICE void tma_load_3d_2cta_hint(void* smem, const void* tmap, uint32_t bar_
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(
             smem_u32(smem)),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z), "l"(policy)
+        : "memory");
+}
+DG_DEVICE void tma_load_4d_hint(void* smem, const void* tmap, uint64_t* bar, int32_t x, int32_t y, int32_t z, int32_t w, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;" ::"r"(
+            smem_u32(smem)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy)
+        : "memory");
+}
+DG_DEVICE void tma_load_4d_2cta_hint(void* smem, const void* tmap, uint32_t bar_cluster_addr, int32_t x, int32_t y, int32_t z, int32_t w, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;" ::"r"(
+            smem_u32(smem)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy)
         : "memory");
 }
 DG_DEVICE void tma_store_3d(const void* tmap, const void* smem, int32_t x, int32_t y, int32_t z) {
@@ -437,10 +456,6 @@ DG_DEVICE uint32_t cvt_e2m1x8(const float* v) {
 // Separate rounded multiply and add on purpose: a fused multiply-add would keep the sign of an
 // underflowing product.
 DG_DEVICE float scale_pos_zero(float v, float inv) { return __fadd_rn(__fmul_rn(v, inv), 0.0f); }
-// Store to the shared memory of a CTA of this cluster (address from mapa_u32).
-DG_DEVICE void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v) {
-    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
-}
 DG_DEVICE void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
