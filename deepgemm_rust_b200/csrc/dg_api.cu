@@ -601,7 +601,7 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    if constexpr (kSlabs != 0) return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
+    if constexpr (kSlabs != 0) return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[5], maps[6]);
     else return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4]);
 }
 
@@ -833,7 +833,10 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     }
     {
         // 32 rows per store; 32 columns of bf16 (64-byte rows) or f32, 128 columns of e4m3 (128-byte rows)
-        if (splits > 1 && !swap) {
+        if (swap) {
+            // the swapped family writes the output itself, without a map, in 16-byte pieces
+            if (reinterpret_cast<uintptr_t>(out->buf) % 16 != 0) return fail(DG_ERR_SHAPE, "D: base address must be 16-byte aligned");
+        } else if (splits > 1) {
             // K ranges write f32 partial tiles into the workspace, one plane per range
             uint64_t dims[3] = {pr.n, pr.m, splits};
             uint64_t strides[2] = {static_cast<uint64_t>(ws_pitch) * 4, static_cast<uint64_t>(ws_pitch) * 4 * pr.m};
@@ -845,10 +848,9 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
             const uint64_t pitch = static_cast<uint64_t>(out->ld) * d_elem;
             uint64_t dims[3] = {n_out, pr.m, a_groups};
             uint64_t strides[2] = {pitch, pitch * pr.m};
-            // the fused activation and the swapped family store e4m3 as 32 x 32 bytes, unswizzled
-            uint32_t box[3] = {out->kind == DG_OUT_FP8 && !swap ? 128u : 32u, 32, 1};
+            uint32_t box[3] = {out->kind == DG_OUT_FP8 ? 128u : 32u, 32, 1};   // the fused activation stores 32 x 32 bytes, unswizzled
             rc = encode_map(&maps[4], dt, 3, out->buf, dims, strides, box,
-                            swiglu || (fp8_out && swap) ? CU_TENSOR_MAP_SWIZZLE_NONE : (out->kind == DG_OUT_BF16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B), "D");
+                            swiglu ? CU_TENSOR_MAP_SWIZZLE_NONE : (out->kind == DG_OUT_BF16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B), "D");
         }
         if (rc) return rc;
     }
@@ -890,8 +892,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     // A problem that the rule sends to the swapped family writes the same rows; where DG_SWAP=1 pins that family, the masked and
     // contiguous layouts write exactly the valid rows.
     const char* pinned = getenv("DG_SWAP");
-    const bool exact_rows = swap && !fp8_out && pinned && atoi(pinned) != 0 && (contiguous || pr.type == DG_GEMM_M_GROUPED_MASKED);
-    p.mask_rows = ((contiguous && align % 32 != 0) || exact_rows) ? 1 : 0;
+    p.mask_rows = ((contiguous && align % 32 != 0) || (swap && pinned && atoi(pinned) != 0)) ? 1 : 0;
     p.out_ptr = out->buf;
     p.out_ld = out->ld;
     {

@@ -11,9 +11,9 @@
 // scale words into a ring of its own, warp 1 issues the UMMAs, warps 4-7 are the epilogue.  The accumulator holds D transposed
 // (TMEM lane = output column, TMEM column = output row):
 //   bf16  tcgen05.ld.16x256b gives every lane column pairs of one lane row, stmatrix.trans turns 8 x 8 blocks round on the way
-//         to shared memory (16 bytes of 8 output columns per row), one TMA store per warp and 32 rows
-//   f32   lane-per-column loads, one 128-byte row per store instruction
-//   e4m3  lane-per-column loads; the 32 columns of a scale block are the 32 lanes of a warp: one warp reduction per row
+//         through shared memory, 64 bytes of a row per four lanes
+//   f32   lane-per-column loads, 128 bytes of a row per store instruction
+//   e4m3  as bf16 into shared memory, then a row of 32 columns (a scale block) per lane
 // Two accumulators of up to 320 columns and the scale columns do not fit 512 TMEM columns side by side, so the second one starts
 // at acc_stride < block_n: tiles wider than that overlap the other buffer.  The epilogue drains those columns first (buffer 0
 // from its last 32 columns down, buffer 1 upwards) and reports them separately, so that the next tile's UMMAs start while the
@@ -32,9 +32,8 @@ constexpr uint32_t kSwapSfSlots = 4;      // ring of scale words, fetched ahead 
 
 struct SwapTile {
     uint32_t m0;               // first weight row (output column)
-    uint32_t n0, rows, n;      // first activation row, rows of the tile, UMMA N of all its parts (rows rounded up)
-    uint32_t row_end;          // rows at or beyond this one belong to someone else: never stored
-    bool exact;                // a store box that crosses row_end is written row by row
+    uint32_t n0, valid, n;     // first activation row, rows of the tile, UMMA N of all its parts (rows rounded up)
+    uint32_t rows;             // rows that are written
     uint32_t ga, gb, gd;       // group coordinate of the weights, of the activations and of D
     uint32_t kb0, kb1;         // k-block range
     uint32_t index, split;     // output tile and K range
@@ -43,6 +42,7 @@ struct SwapTile {
 // Walks the tile list of one CTA (pair); every role runs its own copy and sees the same sequence.
 struct SwapScheduler {
     const GemmParams& p;
+    bool grouped;
     uint32_t step, tile_m, worker, num_workers, num_m_blocks, total_kb, iter;
     uint32_t cur_group, cum_begin, row_start, rows, tile_rows, num_tiles;
 
@@ -56,15 +56,14 @@ struct SwapScheduler {
         cur_group = 0;
         cum_begin = 0;
         row_start = 0;
-        // grouped layouts store whole 32-row boxes (up to 31 rows past the group's end, its own padding): every row of a box is
-        // computed; dense boxes are cut at the matrix end by the store itself
-        const bool grouped = p.gemm_type == kGemmContiguous || p.gemm_type == kGemmMasked;
+        grouped = p.gemm_type == kGemmContiguous || p.gemm_type == kGemmMasked;
         step = grouped ? 32 : 16 * ctas;
-        if (grouped) load_group();
-        else set_rows(p.n);
+        if (!grouped) set_rows(p.n);
     }
+    // What needs global memory: call once, after griddep_wait().  The constructor belongs before it, where its time is hidden.
+    DG_DEVICE void start() { if (grouped) load_group(); }
     DG_DEVICE void set_rows(uint32_t r) {
-        // tiles of one range of rows meet at multiples of 32 rows, the height of a store box (BLOCK_N = 16 stores row by row there)
+        // tiles of one range of rows meet at multiples of 32 rows (16 for BLOCK_N = 16)
         rows = r;
         const uint32_t grid = p.block_n < 32 ? 16u : 32u, most = p.block_n / grid * grid;
         num_tiles = r <= p.block_n ? (r != 0 ? 1u : 0u) : (r + most - 1) / most;
@@ -122,10 +121,12 @@ struct SwapScheduler {
         t.m0 = mb * tile_m;
         t.n0 = row_start + nb * tile_rows;
         const uint32_t left = rows - nb * tile_rows;
-        t.rows = left < tile_rows ? left : tile_rows;
-        t.n = (t.rows + step - 1) / step * step;
-        t.exact = p.mask_rows != 0 || (num_tiles > 1 && p.block_n < 32);
-        t.row_end = t.exact && p.block_n < 32 ? t.n0 + t.rows : row_start + rows;
+        t.valid = left < tile_rows ? left : tile_rows;
+        t.n = (t.valid + step - 1) / step * step;
+        // like the first family's 32-row store boxes, a group's last rows go out with what follows them up to a multiple of 32: rows of
+        // the group's own padding (mask_rows: the neighbour may start there, nothing but valid rows)
+        t.rows = t.valid;
+        if (grouped && p.mask_rows == 0) t.rows = t.n < p.n - t.n0 ? t.n : p.n - t.n0;
         return true;
     }
 };
@@ -149,11 +150,15 @@ DG_DEVICE uint4 ld_shared_v4(uint32_t addr) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
+DG_DEVICE uint32_t ld_shared_u16(uint32_t addr) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+}
 DG_DEVICE uint64_t desc64(uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(hi) << 32 | lo; }
 
-// staging bytes of one epilogue warp and buffer (32 output rows x 32 columns), and buffers per warp (f32 leaves the room to the stages)
-constexpr uint32_t swap_epi_buf_bytes(uint32_t out_kind) { return out_kind == kOutBf16 ? 2048u : (out_kind == kOutF32 ? 4096u : 1024u); }
-constexpr uint32_t swap_epi_bufs(uint32_t out_kind) { return out_kind == kOutF32 ? 1u : 2u; }
+// staging bytes of one epilogue warp: 32 output rows x 32 columns (f32 goes out straight from registers)
+constexpr uint32_t swap_epi_buf_bytes(uint32_t out_kind) { return out_kind == kOutF32 ? 0u : 2048u; }
 
 // Activation rows of a stage, per CTA and slab: the first 256 rows of a tile, and the rows beyond.
 __host__ __device__ inline uint32_t swap_main_rows(uint32_t block_n, uint32_t ctas) { return (block_n < 256 ? block_n : 256) / ctas; }
@@ -169,12 +174,11 @@ template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kHalves>
 __global__ void __launch_bounds__(kNumThreads, 1)
 dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                    const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_b_part,
-                    const __grid_constant__ CUtensorMap tmap_b_tail) {
+                    const __grid_constant__ CUtensorMap tmap_b_part, const __grid_constant__ CUtensorMap tmap_b_tail) {
     constexpr bool kMXF4 = kFmt == kFmtMxf4, kScaled = kFmt != kFmtBf16;
     constexpr uint32_t kHalfElems = kMXF4 ? 256 : 128;      // K elements of one 128-byte slab
     constexpr uint32_t kBlockKElems = kHalves * kHalfElems;
-    constexpr uint32_t kEpiBufBytes = swap_epi_buf_bytes(kOut), kEpiBufs = swap_epi_bufs(kOut);
+    constexpr uint32_t kEpiBufBytes = swap_epi_buf_bytes(kOut);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
@@ -195,7 +199,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem_a + num_stages * a_bytes;
     uint8_t* smem_epi = smem_b + num_stages * b_bytes;
-    uint8_t* smem_sf = smem_epi + 4 * kEpiBufs * kEpiBufBytes;      // kSwapSfSlots x (weight words, activation words)
+    uint8_t* smem_sf = smem_epi + 4 * kEpiBufBytes;      // kSwapSfSlots x (weight words, activation words)
     const uint32_t sf_slot_bytes = sfa_bytes + sfb_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_sf + kSwapSfSlots * sf_slot_bytes);
     uint64_t* bar_full = bars;                       // operands and scale words of a stage in place (pair: both CTAs', on rank 0)
@@ -237,7 +241,6 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             tma_prefetch_desc(&tmap_sfa);
             tma_prefetch_desc(&tmap_sfb);
         }
-        tma_prefetch_desc(&tmap_d);
     }
     if (warp == 1) {
         tmem_alloc<kCtas>(tmem_slot, kTmemCols);
@@ -246,7 +249,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     tc_fence_before();
     if constexpr (kCtas == 2) cluster_sync(); else __syncthreads();
     tc_fence_after();
-    griddep_wait();
+    // Every role waits for the previous kernel itself, after what it can do without global memory: its first instructions have to
+    // come from memory too, ~1000 cycles that pass while that kernel still runs.
     griddep_launch_dependents();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_sfa = tmem_base + p.acc_stride + block_n;
@@ -263,6 +267,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint64_t policy = p.stream_a ? l2_policy_evict_first() : l2_policy_evict_normal();
             const uint32_t tx = (a_bytes >> p.tx_shift_a) * kCtas;
             const bool expects = cta_rank == 0, wide = p.wide_k != 0;
+            griddep_wait();
+            sched.start();
             while (ok && sched.next(t)) {
                 const int32_t row = static_cast<int32_t>(t.m0 + cta_rank * kBlockM), g = static_cast<int32_t>(t.ga);
                 for (uint32_t kb = t.kb0; kb < t.kb1; ++kb) {
@@ -301,6 +307,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t part_rows = swap_part_rows(main_rows);
             const bool expects = cta_rank == 0, wide = p.wide_k != 0;
             constexpr uint32_t kTailBytes = kSwapTailRows * kBlockKBytes;
+            griddep_wait();
+            sched.start();
             while (ok && sched.next(t)) {
                 // a pair's UMMA takes the first half of its N rows from rank 0 and the second half from rank 1
                 const uint32_t n_main = t.n < 256 ? t.n : 256u, my_rows = n_main / kCtas, my_tail = (t.n - n_main) / kCtas;
@@ -364,6 +372,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t sfa_slab = kMXF4 ? 8u : (per128_a ? 0u : 4u), sfb_slab = kMXF4 ? 8u * per_word : (per128_b ? 0u : 4u * per_word);
             const uint32_t sfa_cols[2] = {tmem_sfa, tmem_sfa + sfa_slab}, sfb_cols[2] = {tmem_sfb, tmem_sfb + sfb_slab};
             const bool throttled = p.tc_util < 100;
+            griddep_wait();
+            sched.start();
             while (ok && sched.next(t)) {
                 const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
                 if (!mbar_wait_warp(bar_tmem_empty + e, acc_phase ^ 1, abort_flag, p.status, 0x200 + e)) break;
@@ -478,9 +488,11 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 if (w.kb >= w.t.kb1) start(w);
             };
             auto needs = [&](const Walk& w, const SfPlan& plan) { return (w.kb & (plan.period - 1)) == 0 || w.kb == w.t.kb0; };
-            Walk ahead{SwapScheduler(p, kCtas, kBlockKElems)}, here{SwapScheduler(p, kCtas, kBlockKElems)};
+            Walk ahead{SwapScheduler(p, kCtas, kBlockKElems)};
+            griddep_wait();
+            ahead.sched.start();
             start(ahead);
-            start(here);
+            Walk here = ahead;
             uint32_t in_slot = 0, in_phase = 0, out_slot = 0, out_phase = 0, in_flight = 0;
             uint32_t stage = 0, phase = 0;      // of the k-block `here`
             const bool leader_lane = elect_one();
@@ -544,11 +556,13 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     } else {
         // ------------------------------------------------------------------ epilogue
         const uint32_t ew = warp - 4;              // TMEM lane quadrant: 32 output columns
-        uint8_t* buf0 = smem_epi + ew * kEpiBufs * kEpiBufBytes;
+        uint8_t* const buf = smem_epi + ew * kEpiBufBytes;
         SwapScheduler sched(p, kCtas, kBlockKElems);
         SwapTile t;
-        uint32_t it = 0, buf_idx = 0;
+        uint32_t it = 0;
         bool ok = true;
+        griddep_wait();
+        sched.start();
         while (sched.next(t)) {
             const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
             ++it;
@@ -559,6 +573,10 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * p.acc_stride;
             const uint32_t col0 = t.m0 + cta_rank * kBlockM + ew * 32;      // first output column of this warp
             const uint32_t chunks = (t.rows + 31) / 32;
+            constexpr uint32_t kElem = kOut == kOutBf16 ? 2 : (kOut == kOutF32 ? 4 : 1);
+            uint8_t* const out = static_cast<uint8_t*>(p.out_ptr) + ((static_cast<size_t>(t.gd) * p.n + t.n0) * p.out_ld + col0) * kElem;
+            const size_t pitch = static_cast<size_t>(p.out_ld) * kElem;
+            const uint32_t cols = col0 < p.m ? (p.m - col0 < 32 ? p.m - col0 : 32u) : 0u;       // columns of this warp that exist
             auto arrive = [&](uint64_t* bar) {
                 tc_fence_before();
                 __syncwarp();
@@ -567,98 +585,14 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                     else mbar_arrive_remote(bar + e, 0);
                 }
             };
-            // 32 output rows to registers: bf16 in matrix-fragment order (lanes 0-15 of the quadrant, then 16-31), else one column per lane
+            // 32 output rows to registers: in matrix-fragment order (lanes 0-15 of the quadrant, then 16-31), f32 one column per lane
             auto load_chunk = [&](uint32_t c, uint32_t (&v)[32]) {
-                if constexpr (kOut == kOutBf16) {
+                if constexpr (kOut != kOutF32) {
                     tmem_ld_16x256b_x4(taddr + c * 32, v);
                     tmem_ld_16x256b_x4(taddr + (16u << 16) + c * 32, v + 16);
                 } else {
                     tmem_ld_32x32b_x32(taddr + c * 32, v);
                 }
-            };
-            auto process = [&](uint32_t (&v)[32], uint32_t c) {
-                const uint32_t row0 = t.n0 + c * 32;
-                uint8_t* buf = buf0 + buf_idx * kEpiBufBytes;
-                if (lane == 0) tma_store_wait_read<kEpiBufs - 1>();     // the store that used this buffer last has finished reading it
-                __syncwarp();
-                if (p.has_alpha) {
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * p.alpha);
-                }
-                if constexpr (kOut == kOutBf16) {
-                    // 64-byte rows, 64B swizzle: 16-byte chunk index ^ ((row / 2) % 4); lane 8 q + i addresses columns 8 q .. 8 q + 7 of row 8 j + i
-                    const uint32_t q = lane / 8, i = lane % 8;
-                    #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) {
-                        const uint32_t row = 8 * j + i;
-                        stmatrix_x4_trans(smem_u32(buf) + row * 64 + ((q ^ ((row >> 1) & 3)) << 4),
-                                          pack_bf16x2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1])),
-                                          pack_bf16x2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])),
-                                          pack_bf16x2(__uint_as_float(v[16 + 4 * j]), __uint_as_float(v[16 + 4 * j + 1])),
-                                          pack_bf16x2(__uint_as_float(v[16 + 4 * j + 2]), __uint_as_float(v[16 + 4 * j + 3])));
-                    }
-                } else if constexpr (kOut == kOutF32) {
-                    // 128-byte rows, 128B swizzle: 16-byte chunk index ^ (row % 8)
-                    #pragma unroll
-                    for (uint32_t r = 0; r < 32; ++r)
-                        *reinterpret_cast<uint32_t*>(buf + r * 128 + (((lane / 4) ^ (r & 7)) << 4) + (lane % 4) * 4) = v[r];
-                } else {
-                    // round to bf16 first, take the block maximum over the 32 columns (lanes) of every row on the bf16 bit patterns; lane r
-                    // turns row r's maximum into its power-of-two scale
-                    uint32_t amax = 0;
-                    #pragma unroll
-                    for (uint32_t r = 0; r < 32; ++r) {
-                        v[r] = pack_bf16x2(0.0f, __uint_as_float(v[r]));        // bf16 in the upper half: widened back to f32 bits
-                        const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, (v[r] >> 16) & 0x7FFFu);
-                        amax = lane == r ? m : amax;
-                    }
-                    const uint32_t rounded = (amax + 0x7Fu - 0x60u) >> 7;
-                    uint32_t sf_exp = (rounded < 8u ? 8u : rounded) - 8u;
-                    sf_exp = sf_exp < 105u ? 105u : sf_exp;
-                    if (row0 + lane < t.row_end && col0 < p.m)
-                        reinterpret_cast<uint8_t*>(p.sfd)[(static_cast<size_t>(t.gd * (p.m / 128) + col0 / 128) * p.sfd_stride + row0 + lane) * 4 + (col0 % 128) / 32] =
-                            static_cast<uint8_t>(sf_exp);
-                    const uint32_t inv_bits = (254u - sf_exp) << 23;
-                    #pragma unroll
-                    for (uint32_t r = 0; r < 32; ++r) {
-                        const float inv = __uint_as_float(__shfl_sync(0xFFFFFFFFu, inv_bits, r));
-                        buf[r * 32 + lane] = static_cast<uint8_t>(cvt_e4m3x2(scale_pos_zero(__uint_as_float(v[r]), inv), 0.0f));
-                    }
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if constexpr (kOut != kOutFp8) {
-                    if (t.exact && row0 + 32 > t.row_end) {
-                        // the neighbour of this box's rows may start right at row_end: each lane writes its own row, if valid
-                        constexpr uint32_t kElem = kOut == kOutBf16 ? 2 : 4, kVec = 16 / kElem, kRow = 32 * kElem;
-                        if (row0 + lane < t.row_end) {
-                            uint8_t* dst = static_cast<uint8_t*>(p.out_ptr) + ((static_cast<size_t>(t.gd) * p.n + row0 + lane) * p.out_ld + col0) * kElem;
-                            #pragma unroll
-                            for (uint32_t j = 0; j < kRow / 16; ++j) {
-                                const uint32_t chunk = kOut == kOutBf16 ? (j ^ ((lane >> 1) & 3)) : (j ^ (lane & 7));
-                                const uint4 x = ld_shared_v4(smem_u32(buf) + lane * kRow + chunk * 16);
-                                const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-                                #pragma unroll
-                                for (uint32_t i = 0; i < kVec; ++i) {
-                                    if (col0 + j * kVec + i < p.m) {
-                                        if constexpr (kOut == kOutBf16) reinterpret_cast<uint16_t*>(dst)[j * kVec + i] = static_cast<uint16_t>(w[i / 2] >> (16 * (i & 1)));
-                                        else reinterpret_cast<uint32_t*>(dst)[j * kVec + i] = w[i];
-                                    }
-                                }
-                            }
-                        }
-                        __syncwarp();
-                        return;
-                    }
-                }
-                if (lane == 0) {
-                    if (col0 < p.m) {
-                        if (p.accumulate) tma_reduce_add_3d(&tmap_d, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0), static_cast<int32_t>(t.gd));
-                        else tma_store_3d(&tmap_d, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0), static_cast<int32_t>(t.gd));
-                    }
-                    tma_store_commit();
-                }
-                buf_idx = kEpiBufs - 1 - buf_idx;
             };
             if (p.num_splits > 1) {
                 // K ranges: this range's accumulator to the workspace, 16 bytes per thread and step (coalesced; read back by the same thread
@@ -691,49 +625,128 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 const bool last = *last_flag != 0;
                 named_bar_sync(1, 128);            // everyone has read the flag before the next tile may set it
                 if (!last) continue;
-                const float4* first = reinterpret_cast<const float4*>(p.splitk_ws + first_slot * tile_floats);
-                for (uint32_t c = 0; c < chunks; ++c) {
-                    uint32_t v[32];
-                    float acc[32];
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) acc[i] = 0.0f;
-                    #pragma unroll 2
-                    for (uint32_t s = 0; s < p.num_splits; ++s) {
-                        float4 x[8];
-                        #pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) x[i] = __ldcg(first + s * (tile_floats / 4) + (c * 8 + i) * 128 + et);
-                        #pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) { acc[4 * i] += x[i].x; acc[4 * i + 1] += x[i].y; acc[4 * i + 2] += x[i].z; acc[4 * i + 3] += x[i].w; }
-                    }
-                    #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) v[i] = __float_as_uint(acc[i]);
-                    process(v, c);
-                }
-                continue;
             }
             // Chunks in an order that frees the columns shared with the other accumulator first: buffer 0 from the top, buffer 1 from the
-            // bottom.  Two register sets: the TMEM load of the next chunk is in flight while the current one is converted and staged.
-            const uint32_t loads = (t.n + 31) / 32, edge = p.acc_edge_chunks < loads ? p.acc_edge_chunks : loads;
-            auto chunk_at = [&](uint32_t i) { return e == 0 ? loads - 1 - i : i; };
-            uint32_t va[32], vb[32];
-            load_chunk(chunk_at(0), va);
-            for (uint32_t i = 0; i < loads; i += 2) {
-                tmem_ld_wait_x32(va);
-                if (i + 1 == edge || (i == 0 && edge == 0)) arrive(bar_tmem_edge);
-                const bool has_b = i + 1 < loads;
-                if (has_b) load_chunk(chunk_at(i + 1), vb);
-                else arrive(bar_tmem_empty);
-                if (chunk_at(i) < chunks) process(va, chunk_at(i));
-                if (has_b) {
-                    tmem_ld_wait_x32(vb);
-                    if (i + 2 == edge) arrive(bar_tmem_edge);
-                    if (i + 2 < loads) load_chunk(chunk_at(i + 2), va);
-                    else arrive(bar_tmem_empty);
-                    if (chunk_at(i + 1) < chunks) process(vb, chunk_at(i + 1));
+            // bottom.  One pass of one loop per chunk: unrolled (or with two chunks in flight) this code outgrows the instruction cache.
+            const bool ranges = p.num_splits > 1;
+            const uint32_t loads = ranges ? chunks : (t.n + 31) / 32, edge = p.acc_edge_chunks < loads ? p.acc_edge_chunks : loads;
+            #pragma unroll 1
+            for (uint32_t i = 0; i < loads; ++i) {
+                const uint32_t c = e == 0 ? loads - 1 - i : i;
+                uint32_t v[32];
+                if (ranges) {
+                    const size_t tile_floats = static_cast<size_t>((block_n + 31) / 32) * 32 * kBlockM;
+                    const float4* first = reinterpret_cast<const float4*>(p.splitk_ws + (static_cast<size_t>(t.index) * kCtas + cta_rank) * p.num_splits * tile_floats) +
+                                          c * 1024 + threadIdx.x - 128;
+                    #pragma unroll
+                    for (uint32_t k = 0; k < 32; ++k) v[k] = 0;
+                    #pragma unroll 2
+                    for (uint32_t r = 0; r < p.num_splits; ++r) {
+                        float4 x[8];
+                        #pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k) x[k] = __ldcg(first + r * (tile_floats / 4) + k * 128);
+                        #pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k) {
+                            v[4 * k] = __float_as_uint(__uint_as_float(v[4 * k]) + x[k].x);
+                            v[4 * k + 1] = __float_as_uint(__uint_as_float(v[4 * k + 1]) + x[k].y);
+                            v[4 * k + 2] = __float_as_uint(__uint_as_float(v[4 * k + 2]) + x[k].z);
+                            v[4 * k + 3] = __float_as_uint(__uint_as_float(v[4 * k + 3]) + x[k].w);
+                        }
+                    }
+                } else {
+                    load_chunk(c, v);
+                    tmem_ld_wait_x32(v);
+                    if (i + 1 == edge || (i == 0 && edge == 0)) arrive(bar_tmem_edge);
+                    if (i + 1 == loads) arrive(bar_tmem_empty);
+                }
+                if (c >= chunks) continue;
+                // Exactly the tile's rows are written, straight from the warp: a store through TMA would hold the staging buffer for ~1000
+                // cycles, longer than a chunk takes to convert.
+                const uint32_t left = t.rows - c * 32, rows_here = left < 32 ? left : 32u;
+                uint8_t* const dst = out + c * 32 * pitch;
+                if (p.has_alpha) {
+                    #pragma unroll
+                    for (uint32_t k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * p.alpha);
+                }
+                if constexpr (kOut == kOutF32) {
+                    // one row per instruction: 32 lanes write 128 consecutive bytes
+                    float* o = reinterpret_cast<float*>(dst) + lane;
+                    #pragma unroll
+                    for (uint32_t r = 0; r < 32; ++r) {
+                        if (r < rows_here && lane < cols) *o = p.accumulate ? *o + __uint_as_float(v[r]) : __uint_as_float(v[r]);
+                        o += p.out_ld;
+                    }
+                    continue;
+                }
+                // 64-byte rows of bf16, the 16-byte pieces swizzled by (row / 2) % 4; lane 8 q + k addresses columns 8 q .. 8 q + 7 of row 8 j + k
+                __syncwarp();       // the previous chunk has been read
+                #pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t row = 8 * j + lane % 8;
+                    stmatrix_x4_trans(smem_u32(buf) + row * 64 + (((lane / 8) ^ ((row >> 1) & 3)) << 4),
+                                      pack_bf16x2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1])),
+                                      pack_bf16x2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])),
+                                      pack_bf16x2(__uint_as_float(v[16 + 4 * j]), __uint_as_float(v[16 + 4 * j + 1])),
+                                      pack_bf16x2(__uint_as_float(v[16 + 4 * j + 2]), __uint_as_float(v[16 + 4 * j + 3])));
+                }
+                __syncwarp();
+                if constexpr (kOut == kOutBf16) {
+                    // a lane takes one 16-byte piece of every eighth row: four lanes write 64 bytes of a row
+                    const uint32_t piece = lane % 4;
+                    uint8_t* at = dst + (lane / 4) * pitch + piece * 16;
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const uint32_t row = 8 * j + lane / 4, from = smem_u32(buf) + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4);
+                        if (row < rows_here && piece * 8 + 8 <= cols) {
+                            uint4 x = ld_shared_v4(from);
+                            if (p.accumulate) {
+                                const uint4 old = *reinterpret_cast<uint4*>(at);
+                                x = make_uint4(add_bf16x2(x.x, old.x), add_bf16x2(x.y, old.y), add_bf16x2(x.z, old.z), add_bf16x2(x.w, old.w));
+                            }
+                            *reinterpret_cast<uint4*>(at) = x;
+                        } else if (row < rows_here && piece * 8 < cols) {
+                            // the matrix ends inside this piece
+                            #pragma unroll 1
+                            for (uint32_t k = 0; piece * 8 + k < cols; ++k) {
+                                uint16_t* const o = reinterpret_cast<uint16_t*>(at) + k;
+                                const uint32_t y = ld_shared_u16(from + 2 * k);
+                                *o = static_cast<uint16_t>(p.accumulate ? add_bf16x2(y, *o) : y);
+                            }
+                        }
+                        at += 8 * pitch;
+                    }
+                } else {
+                    // a lane takes a row: bf16 values, maximum of their bit patterns, the power-of-two scale that brings it under 448,
+                    // 32 bytes of e4m3 (n is a multiple of 128: the columns all exist or none does)
+                    uint32_t w[16];
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const uint4 x = ld_shared_v4(smem_u32(buf) + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4));
+                        w[4 * j] = x.x; w[4 * j + 1] = x.y; w[4 * j + 2] = x.z; w[4 * j + 3] = x.w;
+                    }
+                    uint32_t amax = 0;
+                    #pragma unroll
+                    for (uint32_t k = 0; k < 16; ++k) amax = max(amax, max(w[k] & 0x7FFFu, (w[k] >> 16) & 0x7FFFu));
+                    const uint32_t rounded = (amax + 0x7Fu - 0x60u) >> 7;
+                    uint32_t sf_exp = (rounded < 8u ? 8u : rounded) - 8u;
+                    sf_exp = sf_exp < 105u ? 105u : sf_exp;
+                    const float inv = __uint_as_float((254u - sf_exp) << 23);
+                    if (lane < rows_here && cols != 0) {
+                        uint32_t q[8];
+                        #pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k)
+                            q[k] = cvt_e4m3x4(scale_pos_zero(__uint_as_float(w[2 * k] << 16), inv), scale_pos_zero(__uint_as_float(w[2 * k] & 0xFFFF0000u), inv),
+                                              scale_pos_zero(__uint_as_float(w[2 * k + 1] << 16), inv), scale_pos_zero(__uint_as_float(w[2 * k + 1] & 0xFFFF0000u), inv));
+                        uint4* const o = reinterpret_cast<uint4*>(dst + lane * pitch);
+                        o[0] = make_uint4(q[0], q[1], q[2], q[3]);
+                        o[1] = make_uint4(q[4], q[5], q[6], q[7]);
+                        if (c * 32 + lane < t.valid)
+                            reinterpret_cast<uint8_t*>(p.sfd)[(static_cast<size_t>(t.gd * (p.m / 128) + col0 / 128) * p.sfd_stride + t.n0 + c * 32 + lane) * 4 + (col0 % 128) / 32] =
+                                static_cast<uint8_t>(sf_exp);
+                    }
                 }
             }
         }
-        if (lane == 0) tma_store_wait<0>();
         __syncwarp();
     }
 
@@ -749,7 +762,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
 inline uint32_t gemm_swap_smem_bytes(uint32_t block_n, uint32_t ctas, uint32_t out_kind, uint32_t stages, uint32_t sfa_words, uint32_t sfb_words, uint32_t halves) {
     const uint32_t sf_block_n = (block_n + 127) / 128 * 128;
     const uint32_t per_stage = halves * (kBlockM + swap_main_rows(block_n, ctas) + swap_tail_rows(block_n, ctas)) * kBlockKBytes;
-    return 1024 + stages * per_stage + 4 * swap_epi_bufs(out_kind) * swap_epi_buf_bytes(out_kind) + kSwapSfSlots * (512 * sfa_words + sf_block_n * 4 * sfb_words) +
+    return 1024 + stages * per_stage + 4 * swap_epi_buf_bytes(out_kind) + kSwapSfSlots * (512 * sfa_words + sf_block_n * 4 * sfb_words) +
            (2 * kMaxStages + 2 * kSwapSfSlots + 7) * 8 + 16;
 }
 // Column where the second accumulator starts.

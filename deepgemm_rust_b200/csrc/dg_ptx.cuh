@@ -430,6 +430,10 @@ DG_DEVICE uint32_t pack_bf16x2(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
+// Sum of two bf16 pairs, each rounded once.
+DG_DEVICE uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    return pack_bf16x2(__uint_as_float(a << 16) + __uint_as_float(b << 16), __uint_as_float(a & 0xFFFF0000u) + __uint_as_float(b & 0xFFFF0000u));
+}
 DG_DEVICE uint32_t cvt_e4m3x2(float lo, float hi) {
     uint16_t r;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
