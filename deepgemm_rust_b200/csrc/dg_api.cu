@@ -588,7 +588,7 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(dg::kNumThreads, 1, 1);
+    cfg.blockDim = dim3(kSlabs != 0 ? dg::kSwapThreads : dg::kNumThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];

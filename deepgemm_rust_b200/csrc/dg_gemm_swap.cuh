@@ -7,9 +7,10 @@
 // on the same weights.  A group of R rows is cut into ceil(R / BLOCK_N) tiles of about equal height, because a narrow tile is
 // bound by its weight stream and by the issue of its instructions (~450 cycles per 128 bytes of K), not by its tensor time.
 //
-// Roles of the 256-thread CTA (one per SM, persistent): warp 0 loads weights, warp 3 activations, warp 2 loads and re-orders the
-// scale words into a ring of its own, warp 1 issues the UMMAs, warps 4-7 are the epilogue.  The accumulator holds D transposed
-// (TMEM lane = output column, TMEM column = output row):
+// Roles of the 384-thread CTA (one per SM, persistent): warp 0 loads weights, warp 3 activations, warp 2 loads and re-orders the
+// scale words into a ring of its own, warp 1 issues the UMMAs, warps 4-11 are the epilogue: two per TMEM quadrant, taking turns
+// at its 32-row chunks (a chunk is a chain of dependent steps, ~1000 cycles; with short K one warp could not keep up).  The
+// accumulator holds D transposed (TMEM lane = output column, TMEM column = output row):
 //   bf16  tcgen05.ld.16x256b gives every lane column pairs of one lane row, stmatrix.trans turns 8 x 8 blocks round on the way
 //         through shared memory, 64 bytes of a row per four lanes
 //   f32   lane-per-column loads, 128 bytes of a row per store instruction
@@ -26,6 +27,8 @@
 
 namespace dg {
 
+constexpr uint32_t kSwapThreads = 384;
+constexpr uint32_t kSwapEpiWarps = 8;
 constexpr uint32_t kSwapMaxRows = 320;    // of a tile
 constexpr uint32_t kSwapTailRows = 16;    // per CTA and box, for the rows of a tile beyond 256
 constexpr uint32_t kSwapSfSlots = 4;      // ring of scale words, fetched ahead of the k-block that needs them
@@ -171,7 +174,7 @@ __host__ __device__ inline uint32_t swap_part_rows(uint32_t main_rows) { return 
 // tmap_b brings swap_main_rows rows of the activations (and, with wide_k, both slabs of a stage), tmap_b_part swap_part_rows of
 // one slab, tmap_b_tail kSwapTailRows of one slab.
 template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kHalves>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kSwapThreads, 1)
 dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
                     const __grid_constant__ CUtensorMap tmap_b_part, const __grid_constant__ CUtensorMap tmap_b_tail) {
@@ -199,7 +202,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem_a + num_stages * a_bytes;
     uint8_t* smem_epi = smem_b + num_stages * b_bytes;
-    uint8_t* smem_sf = smem_epi + 4 * kEpiBufBytes;      // kSwapSfSlots x (weight words, activation words)
+    uint8_t* smem_sf = smem_epi + kSwapEpiWarps * kEpiBufBytes;      // kSwapSfSlots x (weight words, activation words)
     const uint32_t sf_slot_bytes = sfa_bytes + sfb_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_sf + kSwapSfSlots * sf_slot_bytes);
     uint64_t* bar_full = bars;                       // operands and scale words of a stage in place (pair: both CTAs', on rank 0)
@@ -228,8 +231,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         }
         for (uint32_t e = 0; e < 2; ++e) {
             mbar_init(bar_tmem_full + e, 1);
-            mbar_init(bar_tmem_empty + e, 4 * kCtas);
-            mbar_init(bar_tmem_edge + e, 4 * kCtas);
+            mbar_init(bar_tmem_empty + e, kSwapEpiWarps * kCtas);
+            mbar_init(bar_tmem_edge + e, kSwapEpiWarps * kCtas);
         }
         mbar_init(bar_tc, 1);
         *abort_flag = 0;
@@ -555,8 +558,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue
-        const uint32_t ew = warp - 4;              // TMEM lane quadrant: 32 output columns
-        uint8_t* const buf = smem_epi + ew * kEpiBufBytes;
+        const uint32_t ew = warp % 4, half = (warp - 4) / 4;      // TMEM lane quadrant: 32 output columns; which of its two warps
+        uint8_t* const buf = smem_epi + (warp - 4) * kEpiBufBytes;
         SwapScheduler sched(p, kCtas, kBlockKElems);
         SwapTile t;
         uint32_t it = 0;
@@ -567,7 +570,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
             ++it;
             ok = ok && mbar_wait(bar_tmem_full + e, acc_phase, abort_flag, p.status, 0x600 + e);
-            // with K ranges the four warps meet below: a warp that gave up keeps coming to those meetings, so that none waits for it
+            // with K ranges the eight warps meet below: a warp that gave up keeps coming to those meetings, so that none waits for it
             if (!ok && p.num_splits == 1) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * p.acc_stride;
@@ -599,9 +602,9 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 // positions), then count the range in; the last one sums all of them in range order
                 const size_t tile_floats = static_cast<size_t>((block_n + 31) / 32) * 32 * kBlockM;
                 const size_t first_slot = (static_cast<size_t>(t.index) * kCtas + cta_rank) * p.num_splits;
-                const uint32_t et = threadIdx.x - 128;
+                const uint32_t et = ew * 32 + lane;       // position in the 128 lanes of the accumulator
                 float4* mine = reinterpret_cast<float4*>(p.splitk_ws + (first_slot + t.split) * tile_floats);
-                for (uint32_t c = 0; ok && c < chunks; ++c) {
+                for (uint32_t c = half; ok && c < chunks; c += 2) {
                     uint32_t v[32];
                     load_chunk(c, v);
                     tmem_ld_wait_x32(v);
@@ -613,31 +616,32 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 arrive(bar_tmem_edge);
                 arrive(bar_tmem_empty);
                 __threadfence();
-                named_bar_sync(1, 128);
-                if (et == 0) {
+                named_bar_sync(1, kSwapEpiWarps * 32);
+                if (threadIdx.x == 128) {
                     uint32_t* counter = p.splitk_counters + static_cast<size_t>(t.index) * kCtas + cta_rank;
                     const bool last = ok && atomicAdd(counter, 1u) + 1 == p.num_splits;
                     if (last) *counter = 0;        // ready for the next launch
                     __threadfence();
                     *last_flag = last ? 1u : 0u;
                 }
-                named_bar_sync(1, 128);
+                named_bar_sync(1, kSwapEpiWarps * 32);
                 const bool last = *last_flag != 0;
-                named_bar_sync(1, 128);            // everyone has read the flag before the next tile may set it
+                named_bar_sync(1, kSwapEpiWarps * 32);            // everyone has read the flag before the next tile may set it
                 if (!last) continue;
             }
             // Chunks in an order that frees the columns shared with the other accumulator first: buffer 0 from the top, buffer 1 from the
             // bottom.  One pass of one loop per chunk: unrolled (or with two chunks in flight) this code outgrows the instruction cache.
             const bool ranges = p.num_splits > 1;
             const uint32_t loads = ranges ? chunks : (t.n + 31) / 32, edge = p.acc_edge_chunks < loads ? p.acc_edge_chunks : loads;
+            bool edge_done = ranges, all_done = ranges;       // (with K ranges both were reported above)
             #pragma unroll 1
-            for (uint32_t i = 0; i < loads; ++i) {
+            for (uint32_t i = half; i < loads; i += 2) {
                 const uint32_t c = e == 0 ? loads - 1 - i : i;
                 uint32_t v[32];
                 if (ranges) {
                     const size_t tile_floats = static_cast<size_t>((block_n + 31) / 32) * 32 * kBlockM;
                     const float4* first = reinterpret_cast<const float4*>(p.splitk_ws + (static_cast<size_t>(t.index) * kCtas + cta_rank) * p.num_splits * tile_floats) +
-                                          c * 1024 + threadIdx.x - 128;
+                                          c * 1024 + ew * 32 + lane;
                     #pragma unroll
                     for (uint32_t k = 0; k < 32; ++k) v[k] = 0;
                     #pragma unroll 2
@@ -656,8 +660,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 } else {
                     load_chunk(c, v);
                     tmem_ld_wait_x32(v);
-                    if (i + 1 == edge || (i == 0 && edge == 0)) arrive(bar_tmem_edge);
-                    if (i + 1 == loads) arrive(bar_tmem_empty);
+                    if (!edge_done && i + 2 >= edge) { arrive(bar_tmem_edge); edge_done = true; }
+                    if (i + 2 >= loads) { arrive(bar_tmem_empty); all_done = true; }
                 }
                 if (c >= chunks) continue;
                 // Exactly the tile's rows are written, straight from the warp: a store through TMA would hold the staging buffer for ~1000
@@ -746,6 +750,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                     }
                 }
             }
+            if (!edge_done) arrive(bar_tmem_edge);      // a tile of one chunk leaves the second warp without any
+            if (!all_done) arrive(bar_tmem_empty);
         }
         __syncwarp();
     }
@@ -762,7 +768,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
 inline uint32_t gemm_swap_smem_bytes(uint32_t block_n, uint32_t ctas, uint32_t out_kind, uint32_t stages, uint32_t sfa_words, uint32_t sfb_words, uint32_t halves) {
     const uint32_t sf_block_n = (block_n + 127) / 128 * 128;
     const uint32_t per_stage = halves * (kBlockM + swap_main_rows(block_n, ctas) + swap_tail_rows(block_n, ctas)) * kBlockKBytes;
-    return 1024 + stages * per_stage + 4 * swap_epi_buf_bytes(out_kind) + kSwapSfSlots * (512 * sfa_words + sf_block_n * 4 * sfb_words) +
+    return 1024 + stages * per_stage + kSwapEpiWarps * swap_epi_buf_bytes(out_kind) + kSwapSfSlots * (512 * sfa_words + sf_block_n * 4 * sfb_words) +
            (2 * kMaxStages + 2 * kSwapSfSlots + 7) * 8 + 16;
 }
 // Column where the second accumulator starts.
