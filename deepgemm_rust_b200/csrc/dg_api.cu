@@ -244,10 +244,36 @@ static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     return DG_OK;
 }
 
-// Is the swapped family the better one for this problem?
+// Rows of a group, as far as the host knows them: the contiguous arena's rows include its alignment padding.
+static double group_rows(const dg_desc* d) {
+    const uint32_t groups = d->num_groups ? d->num_groups : 1, align = g_mk_alignment.load();
+    if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
+        const double per_group = static_cast<double>(d->m) / groups;
+        return per_group > align / 2.0 ? per_group - align / 2.0 : per_group;
+    }
+    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return d->expected_m < d->m ? d->expected_m : d->m;
+    return d->m;
+}
+
+// Is the swapped family the better one for this problem?  Measured on B200 over 40 grouped problems: expert groups that fit one
+// tile gain 5-20 % (masked 32 x <= 256 rows, 4096 x 7168: 247 -> 199 us; contiguous 256 x 256 rows: 486 -> 430 us at
+// 4096 x 7168, 263 -> 237 us at 7168 x 2048); with less than 2048 bytes of K its start-up and the transposed epilogue show
+// (34 x 64 rows, 1792 x 1024: 22 -> 31 us), and groups of two tiles and more fill the first family's 256-row tiles as well
+// (900 rows: 750 -> 808 us).
 static bool prefer_swapped(const dg_desc* d) {
-    (void)d;
-    return false;
+    if (d->cd_dtype == DG_OUT_SWIGLU_FP8) return false;
+    const uint32_t k_bytes = d->a_bits == 4 && d->b_bits == 4 ? d->k / 2 : d->k;
+    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return k_bytes >= 2048 && group_rows(d) <= 450.0;
+    // (an arena with fewer rows per group than the alignment is one of mostly empty groups, about which nothing was measured)
+    if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS)
+        return k_bytes >= 2048 && group_rows(d) <= 450.0 && d->m / (d->num_groups ? d->num_groups : 1) >= g_mk_alignment.load();
+    // Dense e4m3, a few rows: where the weight blocks alone fill half of the SMs in one wave (four fifths above 32 rows), a CTA streams
+    // its 128 weight rows without K ranges and without a second launch (8 x 17056 x 8192: 41 -> 26 us; 28 x 9872 x 4608: 17.2 -> 15.4;
+    // 53 x 18600 x 10240: 38 -> 34).  With fewer blocks, more than one wave or more rows the first family's K ranges are as fast or
+    // faster, and an e2m1 operand (half the weight bytes) leaves the stream too thin.
+    const uint32_t blocks = ceil_div(d->n, 128), sms = d->num_sms ? d->num_sms : 148;
+    return d->gemm_type == DG_GEMM_NORMAL && d->a_bits == 8 && d->b_bits == 8 && blocks <= sms &&
+           ((d->m <= 32 && 2 * blocks >= sms) || (d->m <= 64 && 5 * blocks >= 4 * sms));
 }
 
 // Tile choice of the swapped family; false if nothing fits (or the DG_* knobs leave nothing).
@@ -257,7 +283,6 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
     const bool mxf4 = d->a_bits == 4 && d->b_bits == 4;
     const uint32_t half_k = mxf4 ? 256 : 128, groups = d->num_groups ? d->num_groups : 1;
     const bool dense = d->gemm_type == DG_GEMM_NORMAL || d->gemm_type == DG_GEMM_BATCHED;
-    const uint32_t align = g_mk_alignment.load();
     double best_cost = 0;
     bool found = false;
     for (uint32_t halves = 1; halves <= 2; ++halves) {
@@ -270,23 +295,22 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
         for (uint32_t ctas = 1; ctas <= 2; ++ctas) {
             if (force_ctas && static_cast<uint32_t>(atoi(force_ctas)) != ctas) continue;
             if (ctas == 2 && sms < 2) continue;
+            // the dense problems the rule above picks: one CTA per weight block, two slabs, no K ranges
+            const bool picked = d->gemm_type == DG_GEMM_NORMAL && !getenv("DG_SWAP");
+            if (picked && ((halves == 1 && !force_halves) || (ctas == 2 && !force_ctas))) continue;
+            // grouped layouts: pairs and one slab per stage measured best at every size (MoE layer of 256 experts: 3.88 ms against 4.28
+            // with two slabs; single CTAs 5-15 % slower)
+            if (d->gemm_type != DG_GEMM_NORMAL && d->gemm_type != DG_GEMM_BATCHED && ((halves == 2 && !force_halves) || (ctas == 1 && !force_ctas && sms >= 2))) continue;
             const uint32_t step = dense ? 16 * ctas : 32, workers = sms / ctas;
-            // rows per group, as far as the host knows them
-            double rows = d->m;
-            if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
-                const double per_group = static_cast<double>(d->m) / groups;
-                rows = per_group > align / 2.0 ? per_group - align / 2.0 : per_group;
-            } else if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) {
-                rows = d->expected_m < d->m ? d->expected_m : d->m;
-            }
-            // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected, and 288 rows for
-            // groups of about 256 (half of them are a little above)
+            const double rows = group_rows(d);
+            // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected (masked: at most
+            // a slot) and at least 64, and 288 rather than 256 for groups around that size, half of which are a little above
             uint32_t bn;
             if (dense) bn = d->m <= 256 ? ceil_div(d->m, step) * step : 256;
             else bn = ceil_div(static_cast<uint32_t>(2 * rows) + 1, 32) * 32;
             if (!dense && bn < 64) bn = 64;
             if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED && bn > ceil_div(d->m, 32) * 32) bn = ceil_div(d->m, 32) * 32;
-            if (bn > 256) bn = 256;
+            if (bn > 256) bn = d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS && halves == 1 ? 288 : 256;
             if (force_n) bn = static_cast<uint32_t>(atoi(force_n));
             if (bn == 0 || bn > dg::kSwapMaxRows || (bn > 256 && bn % 32 != 0) || (bn > 256 && dense) || bn % step != 0) continue;
             const uint32_t sf_cols = 4 * sfa_words + ceil_div(bn, 128) * 4 * sfb_words;
@@ -296,7 +320,7 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
             const double row_tiles = rows <= bn ? 1.0 : (dense ? static_cast<double>(ceil_div(d->m, most_rows)) : rows / most_rows + 0.5);
             const double tile_rows = rows / row_tiles;
             const uint32_t tiles = static_cast<uint32_t>(groups * row_tiles * m_blocks + 0.999);
-            const uint32_t most_splits = d->gemm_type == DG_GEMM_NORMAL ? 16 : 1;
+            const uint32_t most_splits = d->gemm_type == DG_GEMM_NORMAL && !picked ? 16 : 1;
             for (uint32_t splits = 1; splits <= most_splits; ++splits) {
                 if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != splits) continue;
                 if (splits > 1 && total_kb < 2 * splits) continue;       // at least two k-blocks per range
@@ -311,6 +335,7 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
                 const double per_kb = (halves * (mma > feed ? mma : feed) + 150.0) * (stages < 3 ? 1.5 : 1.0);   // two stages do not cover a load's latency
                 const double kb_per = static_cast<double>(total_kb) / splits;
                 const double waves = splits > 1 || dense ? ceil_div(tiles * splits, workers) : static_cast<double>(tiles) / workers;
+                // a k-block's barriers and copies cost ~450 cycles however narrow the tile (one slab; ~600 for two)
                 const double cost = waves * (kb_per * per_kb + 800.0) + (splits > 1 ? 2500.0 + splits * tile_rows * 8.0 : 0.0);
                 if (!found || cost < best_cost * (1.0 - 1e-9)) {
                     found = true;

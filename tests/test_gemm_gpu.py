@@ -681,3 +681,80 @@ def test_bounded_wait_reports_timeout_and_context_survives():
     c.sync()                                  # the record is cleared by the report
     run_dense(c, 128, 256, 512)               # and the same context still computes correctly
     c.close()
+
+
+@pytest.mark.parametrize("out_kind", [0, 1])
+@pytest.mark.parametrize("sizes,n,k", [
+    ([256, 257, 288, 289, 1, 0, 320, 33], 384, 2048),   # one tile, the 32 rows beyond 256, two tiles from 289 rows on; empty and tiny groups
+    ([31, 32, 64, 65, 96, 128], 264, 2176),             # tile heights of one to four store boxes, columns off the 128 grid, 17 k-blocks
+])
+def test_rule_picks_the_swapped_family_for_small_groups(ctx, sizes, n, k, out_kind):
+    # no DG_SWAP: the tile heights a group can get, through the contiguous layout; every valid row and column against the oracle
+    m_idx = np.concatenate([np.r_[np.full(s, g, np.int32), np.full((-s) % 128, -1, np.int32)] for g, s in enumerate(sizes)])
+    m_total, groups = len(m_idx), len(sizes)
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.MGroupedContiguous, m_total, n, k, groups)).swap_ab
+    _, aq, asf = fp8_operand_1d(m_total, k, 301)
+    _, bq, bsf = fp8_operand_1d(groups * n, k, 302, 128, groups)
+    d = torch.full((m_total, n), float("nan"), dtype=torch.float32 if out_kind else torch.bfloat16, device="cuda")
+    out = dg.Sm100Out.F32(d, n) if out_kind else dg.Sm100Out.Bf16(d, n)
+    dg.m_grouped_fp8_fp4_gemm_contiguous_dev(ctx, lp(aq, asf, m_total, k), dev(m_idx), lp(bq, bsf, groups * n, k), out, groups)
+    ctx.sync()
+    got = to_f32(d)
+    for g, s in enumerate(sizes):
+        if s == 0:
+            continue
+        rows = np.nonzero(m_idx == g)[0].astype(np.uint32)
+        cols = np.arange(g * n, (g + 1) * n, dtype=np.uint32)
+        check_sampled(got, None, (aq, asf, 8, 128, 1, m_total), None, (bq, bsf, 8, 128, groups, n), k, rows, cols, TIGHT_F32 if out_kind else TIGHT_BF16)
+
+
+def test_swapped_masked_fp8_output_is_the_requantised_accumulator(ctx):
+    # the e4m3 epilogue of the swapped family: one and several 32-row chunks, ragged last ones; the CPU epilogue applied to the GPU's
+    # own f32 accumulators (same tiles) gives the identical bytes and scale words on every valid row
+    masked, m_max, n, k = [1, 32, 33, 100, 0, 200], 200, 256, 2048
+    groups = len(masked)
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.MGroupedMasked, m_max, n, k, groups, 64)).swap_ab
+    _, aq, asf = fp8_operand_1d(groups * m_max, k, 311, 128, groups)
+    _, bq, bsf = fp8_operand_1d(groups * n, k, 312, 128, groups)
+    a_op, b_op, mm = lp(aq, asf, m_max, k), lp(bq, bsf, groups * n, k), dev(np.array(masked, np.int32))
+    d32 = torch.zeros((groups * m_max, n), dtype=torch.float32, device="cuda")
+    dg.m_grouped_fp8_fp4_gemm_masked_dev(ctx, a_op, mm, b_op, dg.Sm100Out.F32(d32, n), groups, 64)
+    stride = dg.sf_aligned_rows(m_max)
+    d8 = torch.zeros((groups * m_max, n), dtype=torch.uint8, device="cuda")
+    sfd = torch.zeros(groups * (n // 128) * stride, dtype=torch.int32, device="cuda")
+    dg.m_grouped_fp8_fp4_gemm_masked_dev(ctx, a_op, mm, b_op, dg.Sm100Out.Fp8(d8, n, sfd), groups, 64)
+    ctx.sync()
+    dn, got8, got_sfd = to_f32(d32), d8.cpu().numpy(), sfd.cpu().numpy().view(np.uint32).reshape(groups, n // 128, stride)
+    want8, want_sfd = np.zeros_like(got8), np.zeros(sfd.numel(), np.uint32)
+    for g in range(groups):
+        O.requant_fp8(dn[g * m_max:(g + 1) * m_max], g, stride, want8[g * m_max:(g + 1) * m_max], want_sfd)
+    want_sfd = want_sfd.reshape(groups, n // 128, stride)
+    for g, rows in enumerate(masked):
+        at = slice(g * m_max, g * m_max + rows)
+        want = O.lp_gemm_rows(aq, asf, 8, 128, groups, m_max, np.arange(at.start, at.stop, dtype=np.uint32), bq, bsf, 8, 128, groups, n,
+                              np.arange(g * n, (g + 1) * n, dtype=np.uint32), k) if rows else None
+        assert rows == 0 or O.calc_diff(dn[at], want) <= TIGHT_F32
+        assert np.array_equal(got8[at], want8[at])
+        assert np.array_equal(got_sfd[g, :, :rows], want_sfd[g, :, :rows])
+
+
+@pytest.mark.parametrize("m,n", [(1, 9480), (17, 9480), (32, 18936), (64, 18936)])
+def test_rule_picks_the_swapped_family_for_few_dense_rows(ctx, m, n):
+    k = 1280          # 75 and 148 weight blocks, the last one ragged; ten k-blocks
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).swap_ab
+    _, aq, asf = fp8_operand_1d(m, k, 321)
+    _, bq, bsf = fp8_operand_1d(n, k, 322)
+    d = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    dg.fp8_fp4_gemm_dev(ctx, lp(aq, asf, m, k), lp(bq, bsf, n, k), dg.Sm100Out.F32(d, n), dg.Sm100Epilogue(alpha=0.5))
+    ctx.sync()
+    got = to_f32(d) / 0.5
+    cols = np.r_[0:40, 120:136, 4090:4106, n - 10:n].astype(np.uint32)
+    check_sampled(got, None, (aq, asf, 8, 128, 1, m), None, (bq, bsf, 8, 128, 1, n), k, np.arange(m, dtype=np.uint32), cols, TIGHT_F32)
+    assert not np.isnan(got).any()
+    # the bf16 kernel shares the rule: its operands are rows of 2k bytes
+    a, b = (torch.randn((r, k // 2), device="cuda").bfloat16() for r in (m, n))
+    dg.bf16_gemm_dev(ctx, a, k // 2, m, b, k // 2, n, k // 2, dg.Sm100Out.F32(d, n))
+    ctx.sync()
+    want = a.float() @ b.float().t()
+    # f32 sums of k / 2 exact products in another order: k / 2 roundings of 2^-24 relative to the largest partial sum at most
+    assert float((d - want).abs().max()) <= (k // 2) * 2.0 ** -24 * float((a.float().abs() @ b.float().abs().t()).max())
