@@ -190,6 +190,7 @@ struct KernelPlan {
     uint32_t ctas, umma_n, halves, stages, accum, smem;
     uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
+    uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
 };
 static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
@@ -382,7 +383,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
 
     const char* force_splits = getenv("DG_SPLITS");
     const char* force_halves = getenv("DG_K_SLABS");
-    uint32_t best_n = 0, best_accum = 0, best_tiles = 0, best_ctas = 0, best_stages = 0, best_splits = 1, best_halves = 1;
+    uint32_t best_n = 0, best_accum = 0, best_tiles = 0, best_ctas = 0, best_stages = 0, best_splits = 1, best_halves = 1, best_epi_bufs = 2;
     double best_cost = 0;
     // a stage holds one or two 128-byte K slabs per operand; two slabs halve the per-stage bookkeeping per UMMA
     for (uint32_t halves = 1; halves <= 2; ++halves) {
@@ -435,17 +436,27 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // never straddle ranges; the partial sums cost a second small kernel (launch + S reads of the M x N f32 tile set)
             const bool may_split = d->gemm_type == DG_GEMM_NORMAL && d->cd_dtype != DG_OUT_FP8 && !swiglu && d->n % 4 == 0 && !no_k_ranges;
             for (uint32_t splits = 1; splits <= 16; ++splits) {
-                if (splits > 1 && (!may_split || halves > 1)) break;
+                if (splits > 1 && !may_split) break;
                 if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != splits) continue;
-                uint32_t kb_per = ceil_div(ceil_div(total_kb, splits), 4) * 4;
-                if (splits > 1 && (kb_per < 8 || kb_per * (splits - 1) >= total_kb)) continue;   // every range non-empty, at least 8 k-blocks
+                const uint32_t unit = 4 / halves;      // a range is whole scale words: four slabs
+                uint32_t kb_per = ceil_div(ceil_div(total_kb, splits), unit) * unit;
+                if (splits > 1 && (kb_per < 2 * unit || kb_per * (splits - 1) >= total_kb)) continue;   // every range non-empty, at least 8 k-blocks
                 if (splits == 1) kb_per = total_kb;
                 // K ranges store f32 partials whatever the caller's output type: size the staging buffers for that
                 const uint32_t kernel_out = splits > 1 ? static_cast<uint32_t>(DG_OUT_F32) : d->cd_dtype;
                 uint32_t stages = force_stages ? static_cast<uint32_t>(atoi(force_stages)) : dg::kMaxStages;
                 if (stages > dg::kMaxStages) stages = dg::kMaxStages;
-                while (stages > 1 && dg::gemm_smem_bytes(bn, ctas, kernel_out, stages, sfa_words, sfb_words, halves) > kSmemCapacity) --stages;
-                if (stages < 1 || dg::gemm_smem_bytes(bn, ctas, kernel_out, stages, sfa_words, sfb_words, halves) > kSmemCapacity) continue;
+                // f32 staging takes 32 KB; with half of it three stages of two slabs fit 256-column tiles
+                const uint32_t most_stages = stages;
+                uint32_t epi_bufs = 2;
+                auto smem = [&]() { return dg::gemm_smem_bytes(bn, ctas, kernel_out, stages, sfa_words, sfb_words, halves, epi_bufs); };
+                while (stages > 1 && smem() > kSmemCapacity) --stages;
+                if (stages < 3 && most_stages >= 3 && kernel_out == DG_OUT_F32) {
+                    stages = most_stages;
+                    epi_bufs = 1;
+                    while (stages > 1 && smem() > kSmemCapacity) --stages;
+                }
+                if (stages < 1 || smem() > kSmemCapacity) continue;
                 if (stages < 3 && !force_stages) continue;
                 const uint32_t waves = ceil_div(tiles * splits, workers);
                 const double tile_cost = kb_per * per_kb + (splits > 1 ? 2.0 * bn : epilogue) + 600.0;
@@ -458,7 +469,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
                 const double cost = (compute > l2_floor ? compute : l2_floor) + reduce;
                 if (best_n == 0 || cost < best_cost * (1.0 - 1e-9)) {
                     best_n = bn; best_cost = cost; best_accum = accum; best_tiles = tiles; best_ctas = ctas; best_stages = stages;
-                    best_splits = splits; best_halves = halves;
+                    best_splits = splits; best_halves = halves; best_epi_bufs = epi_bufs;
                 }
             }
         }
@@ -492,7 +503,8 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     out->num_stages = stages;
     out->num_accum_stages = best_accum;
     out->smem_size = dg::gemm_smem_bytes(best_n, best_ctas, best_splits > 1 ? static_cast<uint32_t>(DG_OUT_F32) : d->cd_dtype, stages, sfa_words,
-                                         sfb_words, best_halves);
+                                         sfb_words, best_halves, best_epi_bufs);
+    plan->epi_bufs = best_epi_bufs;
     out->num_tiles = best_tiles;
     out->num_splits = best_splits;
     plan->smem = out->smem_size;
@@ -891,7 +903,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.block_n = plan.umma_n;
     p.block_k_elems = block_k;
     p.num_splits = splits;
-    p.kb_per_split = splits > 1 ? ceil_div(ceil_div(ceil_div(pr.k, block_k), splits), 4) * 4 : ceil_div(pr.k, block_k);
+    const uint32_t split_unit = 4 / plan.halves;
+    p.kb_per_split = splits > 1 ? ceil_div(ceil_div(ceil_div(pr.k, block_k), splits), split_unit) * split_unit : ceil_div(pr.k, block_k);
     if (swap) {
         p.acc_stride = dg::gemm_swap_acc_stride(plan.umma_n, sfa_words, sfb_words);
         p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
@@ -900,6 +913,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         p.splitk_counters = ctx->splitk_counters;
     }
     p.num_stages = plan.stages;
+    p.epi_bufs = swap ? 2 : plan.epi_bufs;
     p.num_accum_stages = plan.accum;
     p.gran_a = ka->gran_k;
     p.gran_b = kb->gran_k;

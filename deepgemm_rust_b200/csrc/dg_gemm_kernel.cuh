@@ -78,6 +78,7 @@ struct GemmParams {
                                // for (100 - tc_util) / tc_util times the k-block's tensor time (bf16_gemm_sm100.rs:358-371)
     float alpha;
     uint32_t sfd_stride;       // output scale words: stride between word columns (fp8 output)
+    uint32_t epi_bufs;         // staging buffers of an epilogue warp: 2, or 1 where f32 staging would cost a stage of two slabs
     // second tile family only (dg_gemm_swap.cuh), where m counts weight rows and n activation rows per group
     uint32_t acc_stride;       // TMEM column where the second accumulator starts (below block_n: the two share columns)
     uint32_t acc_edge_chunks;  // 32-column chunks that hold the shared columns
@@ -255,7 +256,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem_a + num_stages * a_bytes;
     uint8_t* smem_epi = smem_b + num_stages * b_bytes;
-    uint8_t* smem_sfa = smem_epi + 8 * kEpiBufBytes;
+    uint8_t* smem_sfa = smem_epi + 4 * p.epi_bufs * kEpiBufBytes;
     uint8_t* smem_sfb = smem_sfa + num_stages * sfa_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_sfb + num_stages * sfb_bytes);
     uint64_t* bar_full = bars;                       // A/B tiles of a stage landed (pair: both CTAs' tiles, on rank 0)
@@ -585,7 +586,16 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         // in rows of kRowBytes (64 / 128 / 128 bytes, swizzled like the store's tensor map) and
         // every kSubsPerBuf steps one TMA store writes 32 rows
         const uint32_t ew = warp - 4;  // TMEM lane quadrant and 32-row slice of this CTA's 128 rows
-        uint8_t* buf0 = smem_epi + ew * 2 * kEpiBufBytes;
+        uint8_t* buf0 = smem_epi + ew * p.epi_bufs * kEpiBufBytes;
+        const uint32_t buf_flip = p.epi_bufs - 1;
+        // the buffer about to be filled must have been read by the store that used it last
+        auto wait_for_buffer = [&]() {
+            if (lane == 0) {
+                if (buf_flip) tma_store_wait_read<1>();
+                else tma_store_wait_read<0>();
+            }
+            __syncwarp();
+        };
         constexpr uint32_t kSubsPerBuf = kOut == kOutFp8 ? 4 : 1;
         constexpr uint32_t kColsPerBuf = 32 * kSubsPerBuf;
         constexpr uint32_t kRowBytes = kOut == kOutBf16 ? 64 : 128;
@@ -636,8 +646,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                     tmem_ld_wait_x32(u);
                     if (s + 1 == num_out_subs) release_accumulator();
                     uint8_t* buf = buf0 + buf_idx * kEpiBufBytes;
-                    if (lane == 0) tma_store_wait_read<1>();   // the store issued two buffers ago has finished reading this buffer
-                    __syncwarp();
+                    wait_for_buffer();
                     uint32_t amax = 0;
                     #pragma unroll
                     for (uint32_t i = 0; i < 32; i += 2) {
@@ -674,7 +683,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                             tma_store_3d(&tmap_d, buf, static_cast<int32_t>(col0), static_cast<int32_t>(row0), static_cast<int32_t>(t.gd));
                         tma_store_commit();
                     }
-                    buf_idx ^= 1;
+                    buf_idx ^= buf_flip;
                 }
                 continue;
             }
@@ -682,9 +691,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                 const uint32_t sub_in_buf = s % kSubsPerBuf;
                 uint8_t* buf = buf0 + buf_idx * kEpiBufBytes;
                 if (sub_in_buf == 0) {
-                    // the store issued two buffers ago must have finished reading this buffer
-                    if (lane == 0) tma_store_wait_read<1>();
-                    __syncwarp();
+                    wait_for_buffer();
                 }
                 if (p.has_alpha) {
                     #pragma unroll
@@ -771,7 +778,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                         }
                         tma_store_commit();
                     }
-                    buf_idx ^= 1;
+                    buf_idx ^= buf_flip;
                 }
             };
             // two register sets: the TMEM load of the next 32 columns is in flight while the current ones are
@@ -806,10 +813,10 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
 
 // Bytes of dynamic shared memory the kernel needs for a configuration (host side).
 inline uint32_t gemm_smem_bytes(uint32_t block_n, uint32_t ctas, uint32_t out_kind, uint32_t stages, uint32_t sfa_words, uint32_t sfb_words,
-                                uint32_t halves) {
+                                uint32_t halves, uint32_t epi_bufs = 2) {
     const uint32_t sf_block_n = (block_n + 127) / 128 * 128;
     const uint32_t per_stage = halves * (kBlockM * kBlockKBytes + block_n / ctas * kBlockKBytes) + 512 * sfa_words + sf_block_n * 4 * sfb_words;
-    return 1024 + stages * per_stage + 8 * epilogue_buf_bytes(out_kind) + (4 * kMaxStages + 5) * 8 + 16;
+    return 1024 + stages * per_stage + 4 * epi_bufs * epilogue_buf_bytes(out_kind) + (4 * kMaxStages + 5) * 8 + 16;
 }
 
 }  // namespace dg
