@@ -428,10 +428,17 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // max(~118, bn / 2) cycles and a CTA receives its A tile (16 KB) plus bn/ctas rows of B at ~77 bytes per cycle;
             // a single-buffered accumulator exposes the whole epilogue (~10.5 cycles per column).
             const uint32_t total_kb = ceil_div(d->k, block_k);
-            const double mma = 4.0 * (bn * 0.5 > 118.0 ? bn * 0.5 : 118.0);
+            // Dense problems have constants of their own, fitted to 205 of them (m 1-4096, n 512-16384, k 1024-16384, e4m3 / mixed / mxfp4,
+            // every width, K ranges; the choice is 2 % off the best tile on average, 4 % with the others): a scale copy costs
+            // 40 cycles, a tile 2900 from its first load to its last store, of which the last one's epilogue is exposed.
+            const bool fitted = (d->gemm_type == DG_GEMM_NORMAL || d->gemm_type == DG_GEMM_BATCHED) && !swiglu;
+            const double least_mma = fitted ? 103.0 : 118.0;
+            const double mma = 4.0 * (bn * 0.5 > least_mma ? bn * 0.5 : least_mma);
             const double feed = (16384.0 + bn / ctas * 128.0) / 77.0;
-            const double epilogue = swiglu ? (accum == 1 ? 40.0 * bn : 1.0 * bn) : (accum == 1 ? 10.5 * bn : 1.0 * bn);
-            const double per_kb = halves * (mma > feed ? mma : feed) + 150.0;
+            const double epilogue = swiglu ? (accum == 1 ? 40.0 * bn : 1.0 * bn) : (accum == 1 ? (fitted ? 9.7 : 10.5) * bn : (fitted ? 5.2 * bn : 1.0 * bn));
+            const double copies = (4 * d->gran_a > block_k ? static_cast<double>(block_k) / (4 * d->gran_a) : sfa_words) +
+                                  (4 * d->gran_b > block_k ? static_cast<double>(block_k) / (4 * d->gran_b) : sfb_words) * ceil_div(bn, 128);
+            const double per_kb = halves * (mma > feed ? mma : feed) + (fitted ? 234.0 + 40.0 * copies : 150.0);
             // K ranges (dense GEMMs with f32-summable outputs only): each range is a multiple of 4 k-blocks so scale words
             // never straddle ranges; the partial sums cost a second small kernel (launch + S reads of the M x N f32 tile set)
             const bool may_split = d->gemm_type == DG_GEMM_NORMAL && d->cd_dtype != DG_OUT_FP8 && !swiglu && d->n % 4 == 0 && !no_k_ranges;
@@ -459,12 +466,14 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
                 if (stages < 1 || smem() > kSmemCapacity) continue;
                 if (stages < 3 && !force_stages) continue;
                 const uint32_t waves = ceil_div(tiles * splits, workers);
-                const double tile_cost = kb_per * per_kb + (splits > 1 ? 2.0 * bn : epilogue) + 600.0;
-                const double reduce = splits > 1 ? 9000.0 + static_cast<double>(splits) * d->m * d->n * 4.0 / 3000.0 : 0.0;
+                const double tile_cost = kb_per * per_kb + (splits > 1 ? 3.6 * bn : epilogue) + (fitted ? 2855.0 : 600.0);
+                const double reduce = (splits > 1 ? 4450.0 + static_cast<double>(splits) * d->m * d->n * 4.0 / 1507.0 : 0.0) +
+                                      (fitted ? 4.5 * bn + (ctas == 2 ? 280.0 : 0.0) : 0.0);
                 // every CTA pulls its A slab (16 KB) and its share of B from L2 for each 128 bytes of K; with many small groups
-                // (weights read once, little reuse) that aggregate stream, ~9000 bytes per cycle on this part, is the limit
+                // (weights read once, little reuse) that aggregate stream, ~9000 bytes per cycle on this part (11000 with the reuse of
+                // dense problems), is the limit
                 const double l2_bytes = static_cast<double>(tiles) * ctas * ceil_div(d->k, half_k) * (16384.0 + bn / ctas * 128.0);
-                const double l2_floor = l2_bytes / 9000.0;
+                const double l2_floor = l2_bytes / (fitted ? 11140.0 : 9000.0);
                 const double compute = waves * tile_cost;
                 const double cost = (compute > l2_floor ? compute : l2_floor) + reduce;
                 if (best_n == 0 || cost < best_cost * (1.0 - 1e-9)) {
