@@ -301,7 +301,7 @@ typedef struct {
     uint32_t major_a_mn, major_b_mn;   /* heuristics_sm100.rs:72-73 */
 } dg_desc;
 typedef struct {
-    uint32_t swap_ab;            /* always 0: A rows ride the UMMA M dimension */
+    uint32_t swap_ab;            /* 1: weight rows ride the UMMA M dimension, activation rows UMMA N */
     uint32_t block_m, block_n, block_k;
     uint32_t cluster_m, cluster_n;
     uint32_t num_stages;
