@@ -270,11 +270,16 @@ static bool prefer_swapped(const dg_desc* d) {
         return k_bytes >= 2048 && group_rows(d) <= 450.0 && d->m / (d->num_groups ? d->num_groups : 1) >= g_mk_alignment.load();
     // Dense e4m3, a few rows: where the weight blocks alone fill half of the SMs in one wave (four fifths above 32 rows), a CTA streams
     // its 128 weight rows without K ranges and without a second launch (8 x 17056 x 8192: 41 -> 26 us; 28 x 9872 x 4608: 17.2 -> 15.4;
-    // 53 x 18600 x 10240: 38 -> 34).  With fewer blocks, more than one wave or more rows the first family's K ranges are as fast or
+    // 53 x 18600 x 10240: 38 -> 34).  With more than one wave or more rows the first family's K ranges are as fast or
     // faster, and an e2m1 operand (half the weight bytes) leaves the stream too thin.
     const uint32_t blocks = ceil_div(d->n, 128), sms = d->num_sms ? d->num_sms : 148;
+    // With fewer blocks it still wins where K is short: it takes 4.4 us + 0.31 us per 128 bytes of K whatever n is, the K ranges with
+    // their second launch 8.2 us + 0.17 us per MB of weights (up to 32 rows and from 25 blocks on, 13 problems: 3680 x 2048
+    // 12.2 -> 8.9 us, 5208 x 1536 10.6 -> 8.6, 9040 x 2560 15.3 -> 10.6; 0.99 to 1.44 times as fast; with fewer blocks 0.88 times).
+    const uint32_t slabs = ceil_div(d->k, 128);
+    const bool short_k = 6 * blocks >= sms && slabs * 0.31 < 3.8 + 0.17 * blocks * slabs * (128 * 128 / 1e6);
     return d->gemm_type == DG_GEMM_NORMAL && d->a_bits == 8 && d->b_bits == 8 && blocks <= sms &&
-           ((d->m <= 32 && 2 * blocks >= sms) || (d->m <= 64 && 5 * blocks >= 4 * sms));
+           ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));
 }
 
 // Tile choice of the swapped family; false if nothing fits (or the DG_* knobs leave nothing).

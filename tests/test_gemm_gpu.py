@@ -758,3 +758,18 @@ def test_rule_picks_the_swapped_family_for_few_dense_rows(ctx, m, n):
     want = a.float() @ b.float().t()
     # f32 sums of k / 2 exact products in another order: k / 2 roundings of 2^-24 relative to the largest partial sum at most
     assert float((d - want).abs().max()) <= (k // 2) * 2.0 ** -24 * float((a.float().abs() @ b.float().abs().t()).max())
+
+
+@pytest.mark.parametrize("m,n,k,picked", [(1, 3080, 1920, True), (32, 3080, 1920, True), (31, 9344, 4480, True), (5, 3080, 2048, False), (5, 3072, 1920, False)])
+def test_rule_picks_the_swapped_family_for_few_weight_blocks_with_short_k(ctx, m, n, k, picked):
+    # 25 weight blocks are the fewest and 15 K slabs the most for them; 24 blocks or 16 slabs keep the K ranges
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).swap_ab == picked
+    _, aq, asf = fp8_operand_1d(m, k, 331)
+    _, bq, bsf = fp8_operand_1d(n, k, 332)
+    d = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    dg.fp8_fp4_gemm_dev(ctx, lp(aq, asf, m, k), lp(bq, bsf, n, k), dg.Sm100Out.F32(d, n))
+    ctx.sync()
+    got = to_f32(d)
+    cols = np.r_[0:40, 120:136, n - 40:n].astype(np.uint32)
+    check_sampled(got, None, (aq, asf, 8, 128, 1, m), None, (bq, bsf, 8, 128, 1, n), k, np.arange(m, dtype=np.uint32), cols, TIGHT_F32)
+    assert not np.isnan(got).any()
