@@ -256,7 +256,8 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     uint8_t* smem_a = smem;
     uint8_t* smem_b = smem_a + num_stages * a_bytes;
     uint8_t* smem_epi = smem_b + num_stages * b_bytes;
-    uint8_t* smem_sfa = smem_epi + 4 * p.epi_bufs * kEpiBufBytes;
+    const uint32_t epi_bufs = kOut == kOutF32 ? p.epi_bufs : 2u;      // known at compile time where it does not vary
+    uint8_t* smem_sfa = smem_epi + 4 * epi_bufs * kEpiBufBytes;
     uint8_t* smem_sfb = smem_sfa + num_stages * sfa_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_sfb + num_stages * sfb_bytes);
     uint64_t* bar_full = bars;                       // A/B tiles of a stage landed (pair: both CTAs' tiles, on rank 0)
@@ -586,8 +587,8 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         // in rows of kRowBytes (64 / 128 / 128 bytes, swizzled like the store's tensor map) and
         // every kSubsPerBuf steps one TMA store writes 32 rows
         const uint32_t ew = warp - 4;  // TMEM lane quadrant and 32-row slice of this CTA's 128 rows
-        uint8_t* buf0 = smem_epi + ew * p.epi_bufs * kEpiBufBytes;
-        const uint32_t buf_flip = p.epi_bufs - 1;
+        uint8_t* buf0 = smem_epi + ew * epi_bufs * kEpiBufBytes;
+        const uint32_t buf_flip = epi_bufs - 1;
         // the buffer about to be filled must have been read by the store that used it last
         auto wait_for_buffer = [&]() {
             if (lane == 0) {
