@@ -317,14 +317,15 @@ DG_DEVICE void umma_block_scaled(uint32_t d_tmem, uint64_t a_desc, uint64_t b_de
 DG_DEVICE void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 DG_DEVICE void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Read-only loads of what an earlier kernel wrote.  Volatile, unlike __ldg: the compiler may move a plain read-only load above
-// griddep_wait(), where the earlier kernel may not have finished.
-DG_DEVICE uint32_t ld_ro(const uint32_t* p) { uint32_t v; asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+// Loads of what an earlier kernel wrote.  Volatile: the compiler keeps them behind griddep_wait(), before which that kernel may
+// not have finished.  Plain loads, not the non-coherent path (ld.global.nc, __ldg): that one is defined only for data nobody
+// writes while this kernel is resident, and a kernel that overlaps its predecessor is resident while its inputs are written.
+DG_DEVICE uint32_t ld_ro(const uint32_t* p) { uint32_t v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 DG_DEVICE int32_t ld_ro(const int32_t* p) { return static_cast<int32_t>(ld_ro(reinterpret_cast<const uint32_t*>(p))); }
 DG_DEVICE float ld_ro(const float* p) { return __uint_as_float(ld_ro(reinterpret_cast<const uint32_t*>(p))); }
 DG_DEVICE uint4 ld_ro(const uint4* p) {
     uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 DG_DEVICE float4 ld_ro(const float4* p) {
