@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) dg_sf_pack_kernel(const SfPackParams p) {
 
 // (batches, mn, sf_k) f32 -> (batches * sf_k, align4(mn)) f32, padding columns zero.
 // 32x32 tiles through shared memory so both the reads and the writes coalesce.
-__global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* __restrict__ src, float* __restrict__ dst, uint32_t mn,
+__global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* src, float* dst, uint32_t mn,
                                                               uint32_t sf_k, uint32_t aligned_mn) {
     griddep_wait();
     griddep_launch_dependents();
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* __res
     const uint32_t tx = threadIdx.x % 32, ty = threadIdx.x / 32;
     for (uint32_t i = ty; i < 32; i += 8) {
         const uint32_t r = r0 + i, c = c0 + tx;
-        tile[i][tx] = (r < mn && c < sf_k) ? src[(static_cast<size_t>(b) * mn + r) * sf_k + c] : 0.0f;
+        tile[i][tx] = (r < mn && c < sf_k) ? ld_ro(src + (static_cast<size_t>(b) * mn + r) * sf_k + c) : 0.0f;
     }
     __syncthreads();
     for (uint32_t i = ty; i < 32; i += 8) {
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) dg_transpose_sf_kernel(const float* __res
 // Group-end table of the contiguous layout: ends[g] = 1 + last row whose m_indices == g.
 // Step 1 (grid): atomicMax per row.  Step 2 (one block): running maximum, so a group without
 // rows inherits the previous end and the scheduler's prefix walk stays monotone.
-__global__ void __launch_bounds__(256) dg_group_ends_kernel(const int32_t* __restrict__ m_indices, uint32_t* ends, uint32_t groups,
+__global__ void __launch_bounds__(256) dg_group_ends_kernel(const int32_t* m_indices, uint32_t* ends, uint32_t groups,
                                                             uint32_t m) {
     griddep_wait();
     griddep_launch_dependents();
@@ -257,8 +257,8 @@ __global__ void __launch_bounds__(1024) dg_group_ends_scan_kernel(uint32_t* ends
 // Sum of the f32 partial products of a K-split GEMM: out[m, n] = alpha * sum_s partial[s, m, n], added in order
 // s = 0, 1, ... (deterministic), written as bf16 or f32.  One thread owns 4 columns (16-byte loads).
 template <bool kBf16>
-__global__ void __launch_bounds__(256) dg_splitk_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, uint32_t n,
-                                                               uint32_t pitch, float alpha, void* __restrict__ out, uint32_t out_ld) {
+__global__ void __launch_bounds__(256) dg_splitk_reduce_kernel(const float* partial, uint32_t splits, uint32_t m, uint32_t n,
+                                                               uint32_t pitch, float alpha, void* out, uint32_t out_ld) {
     griddep_wait();                // launched beside the tail of the GEMM that writes the partials
     griddep_launch_dependents();
     const uint32_t chunks = (n + 3) / 4;
@@ -311,12 +311,12 @@ __global__ void dg_expire_wait_kernel(Status* status, uint64_t limit_ns) {
 }
 
 // Packed e2m1 -> one code per byte (low nibble), 16 bytes in, 32 bytes out per thread.
-__global__ void __launch_bounds__(256) dg_unpack_fp4_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint64_t packed_len) {
+__global__ void __launch_bounds__(256) dg_unpack_fp4_kernel(const uint8_t* src, uint8_t* dst, uint64_t packed_len) {
     griddep_wait();
     griddep_launch_dependents();
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
     if (i + 16 <= packed_len) {
-        const uint4 v = *reinterpret_cast<const uint4*>(src + i);
+        const uint4 v = ld_ro(reinterpret_cast<const uint4*>(src + i));
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
         uint32_t o[8];
         #pragma unroll

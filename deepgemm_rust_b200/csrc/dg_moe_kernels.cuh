@@ -8,8 +8,8 @@
 namespace dg {
 
 // dst row i = src row idx[i] (row_bytes, a multiple of 16); idx[i] < 0 writes zeros.
-__global__ void __launch_bounds__(256) dg_gather_rows_kernel(const uint8_t* __restrict__ src, size_t src_pitch, const int32_t* __restrict__ idx,
-                                                             uint32_t n_dst, uint32_t row_bytes, uint8_t* __restrict__ dst, size_t dst_pitch) {
+__global__ void __launch_bounds__(256) dg_gather_rows_kernel(const uint8_t* src, size_t src_pitch, const int32_t* idx,
+                                                             uint32_t n_dst, uint32_t row_bytes, uint8_t* dst, size_t dst_pitch) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
@@ -27,9 +27,9 @@ __global__ void __launch_bounds__(256) dg_gather_rows_kernel(const uint8_t* __re
 
 // Send row i = [k data bytes of token idx[i] | its sf_cols scale words | zero padding up to out_pitch].
 // Scale words come from the packed layout sf[c * sf_stride + token].
-__global__ void __launch_bounds__(256) dg_moe_pack_rows_kernel(const uint8_t* __restrict__ data, uint32_t k, const uint32_t* __restrict__ sf,
-                                                               uint32_t sf_stride, uint32_t sf_cols, const int32_t* __restrict__ idx, uint32_t n,
-                                                               uint8_t* __restrict__ out, size_t out_pitch) {
+__global__ void __launch_bounds__(256) dg_moe_pack_rows_kernel(const uint8_t* data, uint32_t k, const uint32_t* sf,
+                                                               uint32_t sf_stride, uint32_t sf_cols, const int32_t* idx, uint32_t n,
+                                                               uint8_t* out, size_t out_pitch) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(256) dg_moe_pack_rows_kernel(const uint8_t* __
 
 // Arena row i takes received row idx[i]: data bytes to dst_data, scale words to the packed layout
 // dst_sf[c * dst_sf_stride + i].  idx[i] < 0 (alignment padding) writes zero data and zero scales.
-__global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* __restrict__ in, size_t in_pitch, uint32_t k, uint32_t sf_cols,
-                                                                 const int32_t* __restrict__ idx, uint32_t n_dst, uint8_t* __restrict__ dst_data,
-                                                                 uint32_t* __restrict__ dst_sf, uint32_t dst_sf_stride) {
+__global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* in, size_t in_pitch, uint32_t k, uint32_t sf_cols,
+                                                                 const int32_t* idx, uint32_t n_dst, uint8_t* dst_data,
+                                                                 uint32_t* dst_sf, uint32_t dst_sf_stride) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
@@ -70,9 +70,9 @@ __global__ void __launch_bounds__(256) dg_moe_unpack_rows_kernel(const uint8_t* 
 
 // out[t, :] = bf16( sum_j w[t, j] * rows[pos[t, j], :] ), f32 accumulation in order j = 0..topk-1
 // with one fused multiply-add per term; pos < 0 skips the term.  One thread owns 8 columns.
-__global__ void __launch_bounds__(256) dg_moe_combine_kernel(const uint16_t* __restrict__ rows, size_t pitch, const int32_t* __restrict__ pos,
-                                                             const float* __restrict__ w, uint32_t tokens, uint32_t topk, uint32_t n,
-                                                             uint16_t* __restrict__ out, size_t out_pitch) {
+__global__ void __launch_bounds__(256) dg_moe_combine_kernel(const uint16_t* rows, size_t pitch, const int32_t* pos,
+                                                             const float* w, uint32_t tokens, uint32_t topk, uint32_t n,
+                                                             uint16_t* out, size_t out_pitch) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t chunks = n / 8;
@@ -121,8 +121,8 @@ constexpr uint32_t kEpChunk = 256;   // pairs per block of the ranking kernel
 // local_rank[p] = number of earlier pairs of the same chunk with the same expert;
 // block_hist[b * num_experts + e] = pairs of chunk b routed to expert e.  Expert ids outside
 // [0, num_experts) are dropped (rank -1): such a pair is neither sent nor reduced.
-__global__ void __launch_bounds__(kEpChunk) dg_ep_rank_pairs_kernel(const int32_t* __restrict__ expert_of_pair, uint32_t pairs, uint32_t num_experts,
-                                                                    int32_t* __restrict__ local_rank, uint32_t* __restrict__ block_hist) {
+__global__ void __launch_bounds__(kEpChunk) dg_ep_rank_pairs_kernel(const int32_t* expert_of_pair, uint32_t pairs, uint32_t num_experts,
+                                                                    int32_t* local_rank, uint32_t* block_hist) {
     griddep_wait();
     griddep_launch_dependents();
     extern __shared__ uint32_t ep_hist[];
@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kEpChunk) dg_ep_rank_pairs_kernel(const int32_
 // Exclusive scan over chunks, per expert, in place; counts[e] = this rank's pairs for expert e.  One warp per expert:
 // 32 chunks per round (independent loads, shuffle scan), so a scan over hundreds of chunks costs a handful of memory
 // round trips instead of one per chunk.
-__global__ void __launch_bounds__(256) dg_ep_block_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t num_blocks, uint32_t num_experts,
-                                                               uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(256) dg_ep_block_scan_kernel(uint32_t* block_hist, uint32_t num_blocks, uint32_t num_experts,
+                                                               uint32_t* counts) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
@@ -177,9 +177,9 @@ __global__ void __launch_bounds__(256) dg_ep_block_scan_kernel(uint32_t* __restr
 // slot_rows != 0 selects the masked layout instead: local expert l owns the fixed slot of rows [l * slot_rows,
 // (l + 1) * slot_rows), group_ends[l] is then its valid row count (the masked GEMM's masked_m), and the overflow flag is
 // raised when some expert receives more than slot_rows rows (or the slots exceed `capacity`).
-__global__ void __launch_bounds__(1024) dg_ep_layout_kernel(const uint32_t* __restrict__ all_counts, uint32_t world, uint32_t rank, uint32_t num_experts,
-                                                            uint32_t alignment, uint32_t capacity, uint32_t slot_rows, uint32_t* __restrict__ pair_base,
-                                                            uint32_t* __restrict__ group_ends, uint32_t* __restrict__ totals) {
+__global__ void __launch_bounds__(1024) dg_ep_layout_kernel(const uint32_t* all_counts, uint32_t world, uint32_t rank, uint32_t num_experts,
+                                                            uint32_t alignment, uint32_t capacity, uint32_t slot_rows, uint32_t* pair_base,
+                                                            uint32_t* group_ends, uint32_t* totals) {
     griddep_wait();
     griddep_launch_dependents();
     extern __shared__ uint32_t ep_smem[];

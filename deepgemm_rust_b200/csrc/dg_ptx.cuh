@@ -320,6 +320,8 @@ DG_DEVICE void griddep_launch_dependents() { asm volatile("griddepcontrol.launch
 // Loads of what an earlier kernel wrote.  Volatile: the compiler keeps them behind griddep_wait(), before which that kernel may
 // not have finished.  Plain loads, not the non-coherent path (ld.global.nc, __ldg): that one is defined only for data nobody
 // writes while this kernel is resident, and a kernel that overlaps its predecessor is resident while its inputs are written.
+// For the same reason no input pointer of such a kernel is __restrict__: through `const T* __restrict__` the compiler takes
+// the data for constant, and may use the non-coherent path or load ahead of griddep_wait() by itself.
 DG_DEVICE uint32_t ld_ro(const uint32_t* p) { uint32_t v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 DG_DEVICE int32_t ld_ro(const int32_t* p) { return static_cast<int32_t>(ld_ro(reinterpret_cast<const uint32_t*>(p))); }
 DG_DEVICE float ld_ro(const float* p) { return __uint_as_float(ld_ro(reinterpret_cast<const uint32_t*>(p))); }

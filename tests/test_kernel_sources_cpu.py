@@ -17,3 +17,15 @@ def test_no_non_coherent_loads():
     # they are resident; the non-coherent load path is defined only for data that is read-only for a kernel's whole lifetime
     for name, text in device_sources():
         assert not re.search(r"ld\.global\.nc|__ldg\s*\(", text), name
+
+
+def test_overlapped_kernels_declare_no_constant_inputs():
+    # through `const T* __restrict__` the compiler may move a load above griddep_wait() or onto the non-coherent path
+    overlapped = 0
+    for name, text in device_sources():
+        for head in re.split(r"__global__", text)[1:]:
+            signature, _, body = head.partition(") {")
+            if "griddep_wait()" in body:
+                overlapped += 1
+                assert not re.search(r"\bconst\b[^,(]*\*\s*__restrict__", signature), (name, signature)
+    assert overlapped >= 15      # the pattern still finds the kernels

@@ -130,3 +130,24 @@ def test_group_ends_and_unpack(ctx):
         got = dg.unpack_fp4_raw_dev(ctx, dev(src), n).cpu().numpy()
         assert np.array_equal(got[0::2], src & 0xF) and np.array_equal(got[1::2], src >> 4)
     ctx.sync()
+
+
+def test_kernels_read_what_the_one_before_them_wrote(ctx):
+    # chains on one stream without a synchronisation between them: every kernel starts while its predecessor runs, and has to see
+    # that one's output, not what its (reused) input buffer held before
+    rows, k = 200, 1024
+    srcs = [randn_bf16(rows, k, seed=900 + i) for i in range(8)]
+    scales = [np.random.default_rng(950 + i).random((132, 60), dtype=np.float32) for i in range(8)]
+    dev_srcs, dev_scales = [dev(s, torch.bfloat16) for s in srcs], [dev(s) for s in scales]
+    codes, turned = [], []
+    for _ in range(3):
+        codes, turned = [], []
+        for x, s in zip(dev_srcs, dev_scales):
+            q, _ = dg.cast_bf16_to_fp4_packed_sf_dev(ctx, x, k, rows, k, 1, 1)
+            codes.append(dg.unpack_fp4_raw_dev(ctx, q, q.numel() - 5))        # an odd length: whole vectors and a tail of bytes
+            turned.append(dg.transform_sf_dev(ctx, dg.transform_sf_dev(ctx, s, 132, 60), 60, 132))
+    ctx.sync()
+    for src, s, c, t in zip(srcs, scales, codes, turned):
+        want = O.cast_bf16_to_fp4_packed_sf(src, k, 1, 1)[0].reshape(-1)[:-5]
+        assert np.array_equal(c.cpu().numpy(), np.stack([want & 15, want >> 4], 1).reshape(-1))
+        assert np.array_equal(t.cpu().numpy(), s)
