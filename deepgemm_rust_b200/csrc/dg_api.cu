@@ -594,9 +594,9 @@ bool pdl_enabled() {
 // fully serialised form.)  Grids of more than 4096 blocks are launched serialised: early blocks move in beside a persistent
 // GEMM, whose SMs are then stuck with its shared-memory carve-out (a small L1) until the grid is through; on an MoE layer of
 // 8192 tokens that cost the activation and combine kernels more (40 us of 4.9 ms) than the ~2 us of overlap bring.
-// Errors are collected by cudaGetLastError, as for a <<<>>> launch.
+// Returns the launch's own result: cudaGetLastError would also hand out what an earlier call that failed had left behind.
 template <typename... Params, typename... Args>
-void launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
@@ -608,7 +608,7 @@ void launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() && static_cast<uint64_t>(grid.x) * grid.y * grid.z <= 4096 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
 // The opt-in to the full shared-memory carve-out is per kernel instantiation and per device; the first
@@ -1000,9 +1000,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         const uint64_t threads = static_cast<uint64_t>(pr.m) * ceil_div(pr.n, 4);
         const uint32_t blocks = static_cast<uint32_t>((threads + 255) / 256);
         const float alpha = e.has_alpha ? e.alpha : 1.0f;
-        launch(out->kind == DG_OUT_BF16 ? dg::dg_splitk_reduce_kernel<true> : dg::dg_splitk_reduce_kernel<false>, blocks, 256, 0, ctx->stream,
-               ctx->splitk_ws, splits, pr.m, pr.n, ws_pitch, alpha, out->buf, out->ld);
-        ce = cudaGetLastError();
+        ce = launch(out->kind == DG_OUT_BF16 ? dg::dg_splitk_reduce_kernel<true> : dg::dg_splitk_reduce_kernel<false>, blocks, 256, 0, ctx->stream,
+                    ctx->splitk_ws, splits, pr.m, pr.n, ws_pitch, alpha, out->buf, out->ld);
     }
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
     return DG_OK;
@@ -1083,9 +1082,8 @@ int ensure_group_ends(dg_ctx* ctx, uint32_t groups) {
 
 int run_group_ends(dg_ctx* ctx, const int32_t* m_indices, uint32_t m, uint32_t groups, uint32_t* ends) {
     DG_CUDA(cudaMemsetAsync(ends, 0, static_cast<size_t>(groups) * 4, ctx->stream));
-    if (m > 0) launch(dg::dg_group_ends_kernel, ceil_div(m, 256), 256, 0, ctx->stream, m_indices, ends, groups, m);
-    launch(dg::dg_group_ends_scan_kernel, 1, 1024, 0, ctx->stream, ends, groups);
-    DG_CUDA(cudaGetLastError());
+    if (m > 0) DG_CUDA(launch(dg::dg_group_ends_kernel, ceil_div(m, 256), 256, 0, ctx->stream, m_indices, ends, groups, m));
+    DG_CUDA(launch(dg::dg_group_ends_scan_kernel, 1, 1024, 0, ctx->stream, ends, groups));
     return DG_OK;
 }
 
@@ -1235,9 +1233,8 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     else ce = launch_f32scale_kernel<1, 128, false>(q, grid, smem, ctx, maps);
     if (ce == cudaSuccess && plan.splits > 1) {
         const uint64_t threads = static_cast<uint64_t>(m) * ceil_div(n, 4);
-        launch(dg::dg_splitk_reduce_kernel<true>, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, ctx->splitk_ws, plan.splits, m, n, ws_pitch,
-               1.0f, out, out_ld);
-        ce = cudaGetLastError();
+        ce = launch(dg::dg_splitk_reduce_kernel<true>, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, ctx->splitk_ws, plan.splits, m, n,
+                    ws_pitch, 1.0f, out, out_ld);
     }
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
     return DG_OK;
@@ -1429,12 +1426,11 @@ static int cast_common(dg_ctx* ctx, const uint16_t* src, uint32_t src_ld, uint32
     if (units > 0x7FFFFFFFull) return fail(DG_ERR_SHAPE, "matrix too large for one launch");
     const uint32_t blocks = static_cast<uint32_t>(units);
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    if (silu_mul && gran == 32) launch(dg::dg_cast_kernel<32, false, true>, blocks, 256, 0, ctx->stream, p);
-    else if (silu_mul) launch(dg::dg_cast_kernel<128, false, true>, blocks, 256, 0, ctx->stream, p);
-    else if (fp4) launch(dg::dg_cast_kernel<32, true>, blocks, 256, 0, ctx->stream, p);
-    else if (gran == 32) launch(dg::dg_cast_kernel<32, false>, blocks, 256, 0, ctx->stream, p);
-    else launch(dg::dg_cast_kernel<128, false>, blocks, 256, 0, ctx->stream, p);
-    DG_CUDA(cudaGetLastError());
+    if (silu_mul && gran == 32) DG_CUDA(launch(dg::dg_cast_kernel<32, false, true>, blocks, 256, 0, ctx->stream, p));
+    else if (silu_mul) DG_CUDA(launch(dg::dg_cast_kernel<128, false, true>, blocks, 256, 0, ctx->stream, p));
+    else if (fp4) DG_CUDA(launch(dg::dg_cast_kernel<32, true>, blocks, 256, 0, ctx->stream, p));
+    else if (gran == 32) DG_CUDA(launch(dg::dg_cast_kernel<32, false>, blocks, 256, 0, ctx->stream, p));
+    else DG_CUDA(launch(dg::dg_cast_kernel<128, false>, blocks, 256, 0, ctx->stream, p));
     return DG_OK;
 }
 
@@ -1464,8 +1460,7 @@ int dg_transform_sf(dg_ctx* ctx, const float* sf, uint32_t mn, uint32_t sf_k, ui
     if (mn == 0 || sf_k == 0 || num_batches == 0) return DG_OK;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     dim3 grid(ceil_div(align4(mn), 32), ceil_div(sf_k, 32), num_batches);
-    launch(dg::dg_transpose_sf_kernel, grid, 256, 0, ctx->stream, sf, dst, mn, sf_k, align4(mn));
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_transpose_sf_kernel, grid, 256, 0, ctx->stream, sf, dst, mn, sf_k, align4(mn)));
     return DG_OK;
 }
 
@@ -1484,8 +1479,7 @@ static int sf_pack_common(dg_ctx* ctx, const float* src, uint32_t src_ld, uint32
     p.mode = mode;
     const uint64_t total = static_cast<uint64_t>(rows) * p.cols;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    launch(dg::dg_sf_pack_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ctx->stream, p);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_sf_pack_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ctx->stream, p));
     return DG_OK;
 }
 
@@ -1519,8 +1513,7 @@ int dg_unpack_fp4_raw(dg_ctx* ctx, const uint8_t* src, size_t packed_len, uint8_
         return fail(DG_ERR_SHAPE, "src and dst must be 16-byte aligned");
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     const uint64_t threads = (packed_len + 15) / 16;
-    launch(dg::dg_unpack_fp4_kernel, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, src, dst, packed_len);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_unpack_fp4_kernel, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, src, dst, packed_len));
     return DG_OK;
 }
 
@@ -1543,8 +1536,7 @@ int dg_gather_rows(dg_ctx* ctx, const void* src, size_t src_pitch, const int32_t
         return fail(DG_ERR_SHAPE, "rows, pitches and base addresses must be multiples of 16 bytes");
     if (n_dst == 0) return DG_OK;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    launch(dg::dg_gather_rows_kernel, ceil_div(n_dst, 8), 256, 0, ctx->stream, static_cast<const uint8_t*>(src), src_pitch, idx, n_dst, row_bytes, static_cast<uint8_t*>(dst), dst_pitch);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_gather_rows_kernel, ceil_div(n_dst, 8), 256, 0, ctx->stream, static_cast<const uint8_t*>(src), src_pitch, idx, n_dst, row_bytes, static_cast<uint8_t*>(dst), dst_pitch));
     return DG_OK;
 }
 
@@ -1555,8 +1547,7 @@ int dg_moe_pack_rows(dg_ctx* ctx, const uint8_t* data, uint32_t k, const uint32_
         return fail(DG_ERR_SHAPE, "k and out_pitch must be multiples of 16 and out_pitch >= k + 4 * sf_cols");
     if (n == 0) return DG_OK;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    launch(dg::dg_moe_pack_rows_kernel, ceil_div(n, 8), 256, 0, ctx->stream, data, k, sf, sf_stride, sf_cols, idx, n, out, out_pitch);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_moe_pack_rows_kernel, ceil_div(n, 8), 256, 0, ctx->stream, data, k, sf, sf_stride, sf_cols, idx, n, out, out_pitch));
     return DG_OK;
 }
 
@@ -1568,8 +1559,7 @@ int dg_moe_unpack_rows(dg_ctx* ctx, const uint8_t* in, size_t in_pitch, uint32_t
     if (dst_sf_stride < n_dst) return fail(DG_ERR_SHAPE, "scale stride smaller than the row count");
     if (n_dst == 0) return DG_OK;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    launch(dg::dg_moe_unpack_rows_kernel, ceil_div(n_dst, 8), 256, 0, ctx->stream, in, in_pitch, k, sf_cols, idx, n_dst, dst_data, dst_sf, dst_sf_stride);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_moe_unpack_rows_kernel, ceil_div(n_dst, 8), 256, 0, ctx->stream, in, in_pitch, k, sf_cols, idx, n_dst, dst_data, dst_sf, dst_sf_stride));
     return DG_OK;
 }
 
@@ -1580,8 +1570,7 @@ int dg_moe_combine(dg_ctx* ctx, const uint16_t* rows, size_t pitch, const int32_
     if (tokens == 0 || n == 0) return DG_OK;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     const uint64_t threads = static_cast<uint64_t>(tokens) * (n / 8);
-    launch(dg::dg_moe_combine_kernel, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, rows, pitch, pos, weights, tokens, topk, n, out, out_pitch);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_moe_combine_kernel, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, rows, pitch, pos, weights, tokens, topk, n, out, out_pitch));
     return DG_OK;
 }
 
@@ -1641,9 +1630,8 @@ int dg_ep_count(dg_ctx* ctx, const int32_t* expert_of_pair, uint32_t pairs, uint
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     const uint32_t chunks = ceil_div(pairs, dg::kEpChunk);
     if (chunks > 0)
-        launch(dg::dg_ep_rank_pairs_kernel, chunks, dg::kEpChunk, num_experts * sizeof(uint32_t), ctx->stream, expert_of_pair, pairs, num_experts, local_rank, block_hist);
-    launch(dg::dg_ep_block_scan_kernel, ceil_div(num_experts, 8), 256, 0, ctx->stream, block_hist, chunks, num_experts, counts);
-    DG_CUDA(cudaGetLastError());
+        DG_CUDA(launch(dg::dg_ep_rank_pairs_kernel, chunks, dg::kEpChunk, num_experts * sizeof(uint32_t), ctx->stream, expert_of_pair, pairs, num_experts, local_rank, block_hist));
+    DG_CUDA(launch(dg::dg_ep_block_scan_kernel, ceil_div(num_experts, 8), 256, 0, ctx->stream, block_hist, chunks, num_experts, counts));
     return DG_OK;
 }
 
@@ -1654,8 +1642,7 @@ int dg_ep_layout(dg_ctx* ctx, const uint32_t* all_counts, uint32_t world, uint32
         return fail(DG_ERR_SHAPE, "need 1 <= world <= 1024, rank < world, num_experts <= 4096 and a multiple of world");
     if (alignment == 0) return fail(DG_ERR_SHAPE, "alignment must be positive");
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    launch(dg::dg_ep_layout_kernel, 1, 1024, 3 * num_experts * sizeof(uint32_t), ctx->stream, all_counts, world, rank, num_experts, alignment, capacity, slot_rows, pair_base, group_ends, totals);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_ep_layout_kernel, 1, 1024, 3 * num_experts * sizeof(uint32_t), ctx->stream, all_counts, world, rank, num_experts, alignment, capacity, slot_rows, pair_base, group_ends, totals));
     return DG_OK;
 }
 
@@ -1680,8 +1667,7 @@ int dg_ep_dispatch(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* lo
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     uint32_t blocks = ceil_div(pairs, 8);
     if (max_blocks != 0 && blocks > max_blocks) blocks = max_blocks;
-    launch(dg::dg_ep_dispatch_kernel, blocks, 256, 0, ctx->stream, p);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_ep_dispatch_kernel, blocks, 256, 0, ctx->stream, p));
     return DG_OK;
 }
 
@@ -1702,8 +1688,7 @@ int dg_ep_combine(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* pos
     if (threads > 0xFFFFFF00ull) return fail(DG_ERR_SHAPE, "tokens x n / 8 must fit 32 bits");
     uint32_t blocks = static_cast<uint32_t>((threads + 255) / 256);
     if (max_blocks != 0 && blocks > max_blocks) blocks = max_blocks;
-    launch(dg::dg_ep_combine_kernel, blocks, 256, 0, ctx->stream, p);
-    DG_CUDA(cudaGetLastError());
+    DG_CUDA(launch(dg::dg_ep_combine_kernel, blocks, 256, 0, ctx->stream, p));
     return DG_OK;
 }
 

@@ -773,3 +773,18 @@ def test_rule_picks_the_swapped_family_for_few_weight_blocks_with_short_k(ctx, m
     cols = np.r_[0:40, 120:136, n - 40:n].astype(np.uint32)
     check_sampled(got, None, (aq, asf, 8, 128, 1, m), None, (bq, bsf, 8, 128, 1, n), k, np.arange(m, dtype=np.uint32), cols, TIGHT_F32)
     assert not np.isnan(got).any()
+
+
+def test_a_failed_call_does_not_fail_the_next_one(ctx):
+    # the allocation of 2^50 bytes is refused by the host and leaves its error with the runtime; the calls after it launch well and
+    # have to say so (K ranges: two launches; quantiser: one; group table: a memset and two)
+    m, n, k = 8, 2112, 7168
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).num_splits > 1
+    x = torch.randn((m, k), device="cuda").bfloat16()
+    calls = [lambda: run_dense(ctx, m, n, k), lambda: dg.cast_bf16_to_fp8_sf_dev(ctx, x, k, m, k, 128),
+             lambda: dg.psum_from_m_indices_dev(ctx, torch.zeros(128, dtype=torch.int32, device="cuda"), 1)]
+    for call in calls:
+        with pytest.raises(dg.DgError):
+            dg.peer_alloc(ctx, 1 << 50, False)
+        call()
+    ctx.sync()
