@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 
 #include "../../include/dgb200.h"
@@ -64,20 +65,28 @@ uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 }  // namespace
 
+// A device buffer that grows on demand.
+struct ScratchBuffer {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    bool captured = false;      // a captured graph may hold its address: it stays until the context goes
+};
+struct ScratchBlock {
+    void* ptr;
+    ScratchBlock* next;
+};
+
 struct dg_ctx {
     int ordinal = 0;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
     int num_sms = 0;
     dg::Status* status = nullptr;       // device word block the kernels report into
-    uint32_t* group_ends = nullptr;     // scratch for the contiguous layout's group-end table
-    uint32_t group_ends_cap = 0;
-    float* splitk_ws = nullptr;         // scratch for the f32 partial products of K-split GEMMs
-    size_t splitk_ws_cap = 0;           // in floats
-    uint32_t* splitk_counters = nullptr;   // K ranges that have arrived, per tile (swapped tile family); zero between launches
-    uint32_t splitk_counters_cap = 0;
-    uint32_t* bridge_sf[2] = {nullptr, nullptr};   // packed scale words built from f32 scales by the f32-scale entry points
-    size_t bridge_sf_cap[2] = {0, 0};              // in words
+    ScratchBuffer group_ends;           // group-end table of the contiguous layout
+    ScratchBuffer splitk_ws;            // f32 partial products of K-split GEMMs
+    ScratchBuffer splitk_counters;      // K ranges that have arrived, per tile (swapped tile family); zero between launches
+    ScratchBuffer bridge_sf[2];         // packed scale words built from f32 scales by the f32-scale entry points
+    ScratchBlock* replaced = nullptr;   // outgrown buffers that a captured graph may still use
 };
 
 extern "C" {
@@ -121,11 +130,13 @@ int dg_ctx_destroy(dg_ctx* ctx) {
     if (ctx == nullptr) return DG_OK;
     cudaSetDevice(ctx->ordinal);
     if (ctx->status) cudaFree(ctx->status);
-    if (ctx->group_ends) cudaFree(ctx->group_ends);
-    if (ctx->splitk_ws) cudaFree(ctx->splitk_ws);
-    if (ctx->splitk_counters) cudaFree(ctx->splitk_counters);
-    for (int i = 0; i < 2; ++i)
-        if (ctx->bridge_sf[i]) cudaFree(ctx->bridge_sf[i]);
+    for (ScratchBuffer* b : {&ctx->group_ends, &ctx->splitk_ws, &ctx->splitk_counters, &ctx->bridge_sf[0], &ctx->bridge_sf[1]})
+        if (b->ptr) cudaFree(b->ptr);
+    while (ScratchBlock* block = ctx->replaced) {
+        ctx->replaced = block->next;
+        cudaFree(block->ptr);
+        delete block;
+    }
     if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return DG_OK;
@@ -137,7 +148,7 @@ int dg_ctx_check_status(dg_ctx* ctx) {
     DG_CUDA(cudaMemcpy(&st, ctx->status, sizeof(st), cudaMemcpyDeviceToHost));
     if (st.code != 0) {
         cudaMemset(ctx->status, 0, sizeof(st));
-        if (ctx->splitk_counters) cudaMemset(ctx->splitk_counters, 0, ctx->splitk_counters_cap * sizeof(uint32_t));   // the kernel may have left some
+        if (ctx->splitk_counters.ptr) cudaMemset(ctx->splitk_counters.ptr, 0, ctx->splitk_counters.bytes);   // the kernel may have left some
         return fail(DG_ERR_TIMEOUT, "a device-side wait ran out: block %u, site 0x%x, parity %u", st.block, st.site, st.extra);
     }
     return DG_OK;
@@ -712,13 +723,40 @@ cudaError_t configure_contiguous_kernels() {
     return e;
 }
 
-// The context's scratch for partial sums, at least `floats` long.
-int ensure_splitk_ws(dg_ctx* ctx, size_t floats) {
-    if (ctx->splitk_ws_cap >= floats) return DG_OK;
-    DG_CUDA(cudaSetDevice(ctx->ordinal));
-    if (ctx->splitk_ws) { cudaFree(ctx->splitk_ws); ctx->splitk_ws = nullptr; ctx->splitk_ws_cap = 0; }
-    DG_CUDA(cudaMalloc(&ctx->splitk_ws, floats * sizeof(float)));
-    ctx->splitk_ws_cap = floats;
+// Makes one of the context's scratch buffers at least `bytes` long (all zero when it is new, if `zeroed`).  The stream may
+// be capturing: allocations are then made in the relaxed mode, outside the graph, and a buffer whose address went into a graph is
+// never freed before the context, so that the graph can be replayed after the buffer was outgrown.
+int reserve(dg_ctx* ctx, ScratchBuffer* buf, size_t bytes, bool zeroed = false) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const bool capturing = cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+    if (buf->bytes < bytes) {
+        DG_CUDA(cudaSetDevice(ctx->ordinal));
+        if (buf->ptr && (buf->captured || capturing)) {
+            ScratchBlock* block = new (std::nothrow) ScratchBlock{buf->ptr, ctx->replaced};
+            if (block == nullptr) return fail(DG_ERR_DRIVER, "out of host memory");
+            ctx->replaced = block;
+        } else if (buf->ptr) {
+            cudaFree(buf->ptr);
+        }
+        *buf = ScratchBuffer();
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        DG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        void* ptr = nullptr;
+        cudaError_t e = cudaMalloc(&ptr, bytes);
+        if (e == cudaSuccess && zeroed) {
+            cudaStream_t side = nullptr;        // not the context's stream: a captured fill would only run with the graph
+            e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaMemsetAsync(ptr, 0, bytes, side);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(side);
+            if (side) cudaStreamDestroy(side);
+            if (e != cudaSuccess) cudaFree(ptr);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return fail(DG_ERR_DRIVER, "allocating %zu bytes of scratch: %s", bytes, cudaGetErrorString(e));
+        buf->ptr = ptr;
+        buf->bytes = bytes;
+    }
+    buf->captured |= capturing;
     return DG_OK;
 }
 
@@ -788,19 +826,14 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const uint32_t ws_pitch = align4(pr.n);
     if (splits > 1) {
         // first family: one (m, n) plane per range; swapped family: one accumulator per tile, CTA of the pair and range
-        rc = ensure_splitk_ws(ctx, swap ? static_cast<size_t>(plan.tiles) * plan.ctas * splits * ceil_div(plan.umma_n, 32) * 32 * dg::kBlockM
-                                        : static_cast<size_t>(splits) * pr.m * ws_pitch);
+        rc = reserve(ctx, &ctx->splitk_ws, sizeof(float) * (swap ? static_cast<size_t>(plan.tiles) * plan.ctas * splits * ceil_div(plan.umma_n, 32) * 32 * dg::kBlockM
+                                                                 : static_cast<size_t>(splits) * pr.m * ws_pitch));
         if (rc) return rc;
         const uint32_t counters = plan.tiles * plan.ctas;
-        if (swap && ctx->splitk_counters_cap < counters) {
-            DG_CUDA(cudaSetDevice(ctx->ordinal));
-            if (ctx->splitk_counters) { cudaFree(ctx->splitk_counters); ctx->splitk_counters = nullptr; ctx->splitk_counters_cap = 0; }
-            const uint32_t cap = counters < 1024 ? 1024 : counters;
-            DG_CUDA(cudaMalloc(&ctx->splitk_counters, cap * sizeof(uint32_t)));
-            DG_CUDA(cudaMemsetAsync(ctx->splitk_counters, 0, cap * sizeof(uint32_t), ctx->stream));
-            ctx->splitk_counters_cap = cap;
-        }
+        if (swap) rc = reserve(ctx, &ctx->splitk_counters, sizeof(uint32_t) * (counters < 1024 ? 1024 : counters), true);
+        if (rc) return rc;
     }
+    float* const splitk_ws = static_cast<float*>(ctx->splitk_ws.ptr);
     const uint32_t sfa_words = 4 * ka->gran_k >= block_k ? 1 : block_k / (4 * ka->gran_k);
     const uint32_t sfb_words = 4 * kb->gran_k >= block_k ? 1 : block_k / (4 * kb->gran_k);
     const uint32_t sf_block_n = ceil_div(plan.umma_n, 128) * 128;
@@ -892,7 +925,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
             uint64_t dims[3] = {pr.n, pr.m, splits};
             uint64_t strides[2] = {static_cast<uint64_t>(ws_pitch) * 4, static_cast<uint64_t>(ws_pitch) * 4 * pr.m};
             uint32_t box[3] = {32, 32, 1};
-            rc = encode_map(&maps[4], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ctx->splitk_ws, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "D partials");
+            rc = encode_map(&maps[4], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, splitk_ws, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "D partials");
         } else {
             const CUtensorMapDataType dt = out->kind == DG_OUT_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                            : (fp8_out ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
@@ -923,8 +956,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         p.acc_stride = dg::gemm_swap_acc_stride(plan.umma_n, sfa_words, sfb_words);
         p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
         if (p.acc_stride == plan.umma_n) p.acc_edge_chunks = 0;
-        p.splitk_ws = ctx->splitk_ws;
-        p.splitk_counters = ctx->splitk_counters;
+        p.splitk_ws = splitk_ws;
+        p.splitk_counters = static_cast<uint32_t*>(ctx->splitk_counters.ptr);
     }
     p.num_stages = plan.stages;
     p.epi_bufs = swap ? 2 : plan.epi_bufs;
@@ -1001,7 +1034,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         const uint32_t blocks = static_cast<uint32_t>((threads + 255) / 256);
         const float alpha = e.has_alpha ? e.alpha : 1.0f;
         ce = launch(out->kind == DG_OUT_BF16 ? dg::dg_splitk_reduce_kernel<true> : dg::dg_splitk_reduce_kernel<false>, blocks, 256, 0, ctx->stream,
-                    ctx->splitk_ws, splits, pr.m, pr.n, ws_pitch, alpha, out->buf, out->ld);
+                    splitk_ws, splits, pr.m, pr.n, ws_pitch, alpha, out->buf, out->ld);
     }
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
     return DG_OK;
@@ -1071,13 +1104,10 @@ cudaError_t launch_f32scale_kernel(const dg::F32ScaleParams& q, uint32_t grid, u
     return cudaLaunchKernelEx(&cfg, kernel, q, maps[0], maps[1], maps[2]);
 }
 
-int ensure_group_ends(dg_ctx* ctx, uint32_t groups) {
-    if (ctx->group_ends_cap >= groups) return DG_OK;
-    if (ctx->group_ends) { cudaFree(ctx->group_ends); ctx->group_ends = nullptr; ctx->group_ends_cap = 0; }
-    const uint32_t cap = groups < 1024 ? 1024 : groups;
-    DG_CUDA(cudaMalloc(&ctx->group_ends, static_cast<size_t>(cap) * 4));
-    ctx->group_ends_cap = cap;
-    return DG_OK;
+int ensure_group_ends(dg_ctx* ctx, uint32_t groups, uint32_t** ends) {
+    const int rc = reserve(ctx, &ctx->group_ends, sizeof(uint32_t) * (groups < 1024 ? 1024 : groups));
+    *ends = static_cast<uint32_t*>(ctx->group_ends.ptr);
+    return rc;
 }
 
 int run_group_ends(dg_ctx* ctx, const int32_t* m_indices, uint32_t m, uint32_t groups, uint32_t* ends) {
@@ -1126,11 +1156,12 @@ int dg_m_grouped_fp8_fp4_gemm_contiguous(dg_ctx* ctx, const dg_lp_operand* a, co
     if (!ctx || !a || !b || !out || !m_indices) return fail(DG_ERR_SHAPE, "null argument");
     if (num_groups == 0) return fail(DG_ERR_SHAPE, "num_groups must be positive");
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    int rc = ensure_group_ends(ctx, num_groups);
+    uint32_t* ends = nullptr;
+    int rc = ensure_group_ends(ctx, num_groups, &ends);
     if (rc) return rc;
-    rc = run_group_ends(ctx, m_indices, a->rows, num_groups, ctx->group_ends);
+    rc = run_group_ends(ctx, m_indices, a->rows, num_groups, ends);
     if (rc) return rc;
-    return dg_m_grouped_fp8_fp4_gemm_contiguous_ends(ctx, a, ctx->group_ends, b, out, num_groups, epi);
+    return dg_m_grouped_fp8_fp4_gemm_contiguous_ends(ctx, a, ends, b, out, num_groups, epi);
 }
 
 int dg_m_grouped_fp8_fp4_gemm_masked(dg_ctx* ctx, const dg_lp_operand* a, const int32_t* masked_m, const dg_lp_operand* b,
@@ -1172,9 +1203,10 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     CUtensorMap maps[3];
     int rc;
     if (plan.splits > 1) {
-        rc = ensure_splitk_ws(ctx, static_cast<size_t>(plan.splits) * m * ws_pitch);
+        rc = reserve(ctx, &ctx->splitk_ws, sizeof(float) * plan.splits * m * ws_pitch);
         if (rc) return rc;
     }
+    float* const splitk_ws = static_cast<float*>(ctx->splitk_ws.ptr);
     {
         uint64_t dims[3] = {k, m, a_groups};
         uint64_t strides[2] = {a_ld, static_cast<uint64_t>(a_ld) * m};
@@ -1192,7 +1224,7 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
         uint64_t dstrides[2] = {pitch, pitch * m};
         uint32_t dbox[3] = {32, 32, 1};
         if (partial)
-            rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ctx->splitk_ws, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_128B, "D partials");
+            rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, splitk_ws, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_128B, "D partials");
         else
             rc = encode_map(&maps[2], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, out, ddims, dstrides, dbox, CU_TENSOR_MAP_SWIZZLE_64B, "D");
         if (rc) return rc;
@@ -1233,7 +1265,7 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     else ce = launch_f32scale_kernel<1, 128, false>(q, grid, smem, ctx, maps);
     if (ce == cudaSuccess && plan.splits > 1) {
         const uint64_t threads = static_cast<uint64_t>(m) * ceil_div(n, 4);
-        ce = launch(dg::dg_splitk_reduce_kernel<true>, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, ctx->splitk_ws, plan.splits, m, n,
+        ce = launch(dg::dg_splitk_reduce_kernel<true>, static_cast<uint32_t>((threads + 255) / 256), 256, 0, ctx->stream, splitk_ws, plan.splits, m, n,
                     ws_pitch, 1.0f, out, out_ld);
     }
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
@@ -1256,33 +1288,32 @@ static int bridge_common(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_t 
             const uint32_t* table = layout;
             if (contiguous) {
                 // the group-end table the scheduler walks, built from m_indices in the context's scratch
-                int rc = ensure_group_ends(ctx, groups);
+                uint32_t* ends = nullptr;
+                int rc = ensure_group_ends(ctx, groups, &ends);
                 if (rc) return rc;
                 DG_CUDA(cudaSetDevice(ctx->ordinal));
-                rc = run_group_ends(ctx, reinterpret_cast<const int32_t*>(layout), m, groups, ctx->group_ends);
+                rc = run_group_ends(ctx, reinterpret_cast<const int32_t*>(layout), m, groups, ends);
                 if (rc) return rc;
-                table = ctx->group_ends;
+                table = ends;
             }
             return launch_f32scale(ctx, type, a, a_ld, a_sf_t, b, b_ld, sfb, m, n, k, groups, table, out, out_ld);
         }
     }
     const size_t need[2] = {dg_sf_words(m * a_groups, k, 128, a_groups), dg_sf_words(n * b_groups, k, 128, b_groups)};
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    for (int i = 0; i < 2; ++i) {
-        if (ctx->bridge_sf_cap[i] >= need[i]) continue;
-        if (ctx->bridge_sf[i]) { cudaFree(ctx->bridge_sf[i]); ctx->bridge_sf[i] = nullptr; ctx->bridge_sf_cap[i] = 0; }
-        DG_CUDA(cudaMalloc(&ctx->bridge_sf[i], need[i] * 4));
-        ctx->bridge_sf_cap[i] = need[i];
-    }
+    int rc = reserve(ctx, &ctx->bridge_sf[0], need[0] * 4);
+    if (rc == DG_OK) rc = reserve(ctx, &ctx->bridge_sf[1], need[1] * 4);
+    if (rc) return rc;
+    uint32_t *const sfa_words = static_cast<uint32_t*>(ctx->bridge_sf[0].ptr), *const sfb_words = static_cast<uint32_t*>(ctx->bridge_sf[1].ptr);
     // padding rows of the packed layouts must read as a valid exponent
-    DG_CUDA(cudaMemsetAsync(ctx->bridge_sf[0], 0, need[0] * 4, ctx->stream));
-    DG_CUDA(cudaMemsetAsync(ctx->bridge_sf[1], 0, need[1] * 4, ctx->stream));
-    int rc = dg_transform_sf_t_packed_ue8m0(ctx, a_sf_t, m * a_groups, k, 128, a_groups, ctx->bridge_sf[0]);
+    DG_CUDA(cudaMemsetAsync(sfa_words, 0, need[0] * 4, ctx->stream));
+    DG_CUDA(cudaMemsetAsync(sfb_words, 0, need[1] * 4, ctx->stream));
+    rc = dg_transform_sf_t_packed_ue8m0(ctx, a_sf_t, m * a_groups, k, 128, a_groups, sfa_words);
     if (rc) return rc;
-    rc = dg_transform_sf2d_packed_ue8m0(ctx, sfb, k / 128, n * b_groups, k, b_groups, ctx->bridge_sf[1]);
+    rc = dg_transform_sf2d_packed_ue8m0(ctx, sfb, k / 128, n * b_groups, k, b_groups, sfb_words);
     if (rc) return rc;
-    dg_lp_operand a_op = {a, ctx->bridge_sf[0], m, k, a_ld, 8, 128, 0, static_cast<size_t>(m) * a_groups * a_ld, need[0]};
-    dg_lp_operand b_op = {b, ctx->bridge_sf[1], type == DG_GEMM_BATCHED || type == DG_GEMM_NORMAL ? n : n * groups, k, b_ld, 8, 128, 0,
+    dg_lp_operand a_op = {a, sfa_words, m, k, a_ld, 8, 128, 0, static_cast<size_t>(m) * a_groups * a_ld, need[0]};
+    dg_lp_operand b_op = {b, sfb_words, type == DG_GEMM_BATCHED || type == DG_GEMM_NORMAL ? n : n * groups, k, b_ld, 8, 128, 0,
                           static_cast<size_t>(n) * b_groups * b_ld, need[1]};
     dg_out o = {DG_OUT_BF16, out, out_ld, nullptr, static_cast<size_t>(m) * a_groups * out_ld, 0};
     switch (type) {
