@@ -76,16 +76,25 @@ struct ScratchBlock {
     ScratchBlock* next;
 };
 
+// What the calls of one stream share: they run one after the other.
+struct Scratch {
+    cudaStream_t stream = nullptr;
+    bool orphaned = false;              // the stream was the context's own and is destroyed; another may get its handle
+    ScratchBuffer group_ends;           // group-end table of the contiguous layout
+    ScratchBuffer splitk_ws;            // f32 partial products of K-split GEMMs
+    ScratchBuffer splitk_counters;      // K ranges that have arrived, per tile (swapped tile family); zero between launches
+    ScratchBuffer bridge_sf[2];         // packed scale words built from f32 scales by the f32-scale entry points
+    Scratch* next = nullptr;
+};
+
 struct dg_ctx {
     int ordinal = 0;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
     int num_sms = 0;
     dg::Status* status = nullptr;       // device word block the kernels report into
-    ScratchBuffer group_ends;           // group-end table of the contiguous layout
-    ScratchBuffer splitk_ws;            // f32 partial products of K-split GEMMs
-    ScratchBuffer splitk_counters;      // K ranges that have arrived, per tile (swapped tile family); zero between launches
-    ScratchBuffer bridge_sf[2];         // packed scale words built from f32 scales by the f32-scale entry points
+    Scratch first;                      // one set per stream the context has been used on
+    Scratch* scratch = &first;          // of `stream`
     ScratchBlock* replaced = nullptr;   // outgrown buffers that a captured graph may still use
 };
 
@@ -115,6 +124,7 @@ static int ctx_create(int ordinal, void* stream, bool adopt, dg_ctx** out) {
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return fail(DG_ERR_DRIVER, "cudaStreamCreate failed"); }
         c->owns_stream = true;
     }
+    c->first.stream = c->stream;
     if (cudaMalloc(&c->status, sizeof(dg::Status)) != cudaSuccess || cudaMemset(c->status, 0, sizeof(dg::Status)) != cudaSuccess) {
         delete c;
         return fail(DG_ERR_DRIVER, "allocating the device status word failed");
@@ -130,8 +140,12 @@ int dg_ctx_destroy(dg_ctx* ctx) {
     if (ctx == nullptr) return DG_OK;
     cudaSetDevice(ctx->ordinal);
     if (ctx->status) cudaFree(ctx->status);
-    for (ScratchBuffer* b : {&ctx->group_ends, &ctx->splitk_ws, &ctx->splitk_counters, &ctx->bridge_sf[0], &ctx->bridge_sf[1]})
-        if (b->ptr) cudaFree(b->ptr);
+    for (Scratch *set = &ctx->first, *next; set != nullptr; set = next) {
+        next = set->next;
+        for (ScratchBuffer* b : {&set->group_ends, &set->splitk_ws, &set->splitk_counters, &set->bridge_sf[0], &set->bridge_sf[1]})
+            if (b->ptr) cudaFree(b->ptr);
+        if (set != &ctx->first) delete set;
+    }
     while (ScratchBlock* block = ctx->replaced) {
         ctx->replaced = block->next;
         cudaFree(block->ptr);
@@ -148,7 +162,8 @@ int dg_ctx_check_status(dg_ctx* ctx) {
     DG_CUDA(cudaMemcpy(&st, ctx->status, sizeof(st), cudaMemcpyDeviceToHost));
     if (st.code != 0) {
         cudaMemset(ctx->status, 0, sizeof(st));
-        if (ctx->splitk_counters.ptr) cudaMemset(ctx->splitk_counters.ptr, 0, ctx->splitk_counters.bytes);   // the kernel may have left some
+        for (Scratch* set = &ctx->first; set != nullptr; set = set->next)
+            if (set->splitk_counters.ptr) cudaMemset(set->splitk_counters.ptr, 0, set->splitk_counters.bytes);   // the kernel may have left some
         return fail(DG_ERR_TIMEOUT, "a device-side wait ran out: block %u, site 0x%x, parity %u", st.block, st.site, st.extra);
     }
     return DG_OK;
@@ -168,9 +183,27 @@ int dg_ctx_num_sms(const dg_ctx* ctx, int* out) {
 void* dg_ctx_stream(const dg_ctx* ctx) { return ctx ? ctx->stream : nullptr; }
 int dg_ctx_set_stream(dg_ctx* ctx, void* cuda_stream) {
     if (ctx == nullptr) return fail(DG_ERR_SHAPE, "null context");
-    if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+    const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    // work queued on the old stream may still run beside the new stream's: that one gets scratch of its own
+    const bool ends = ctx->owns_stream && ctx->stream;
+    Scratch* set = ctx->scratch;
+    if (ends || stream != ctx->stream)
+        for (set = &ctx->first; set != nullptr; set = set->next)
+            if (set->stream == stream && !set->orphaned && !(ends && set == ctx->scratch)) break;
+    if (set == nullptr) {
+        set = new (std::nothrow) Scratch;
+        if (set == nullptr) return fail(DG_ERR_DRIVER, "out of host memory");
+        set->stream = stream;
+        set->next = ctx->first.next;
+        ctx->first.next = set;
+    }
+    if (ends) {
+        ctx->scratch->orphaned = true;
+        cudaStreamDestroy(ctx->stream);
+    }
     ctx->owns_stream = false;
-    ctx->stream = static_cast<cudaStream_t>(cuda_stream);
+    ctx->stream = stream;
+    ctx->scratch = set;
     return DG_OK;
 }
 
@@ -723,7 +756,7 @@ cudaError_t configure_contiguous_kernels() {
     return e;
 }
 
-// Makes one of the context's scratch buffers at least `bytes` long (all zero when it is new, if `zeroed`).  The stream may
+// Makes a scratch buffer of the context's present stream at least `bytes` long (all zero when it is new, if `zeroed`).  The stream may
 // be capturing: allocations are then made in the relaxed mode, outside the graph, and a buffer whose address went into a graph is
 // never freed before the context, so that the graph can be replayed after the buffer was outgrown.
 int reserve(dg_ctx* ctx, ScratchBuffer* buf, size_t bytes, bool zeroed = false) {
@@ -826,14 +859,14 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const uint32_t ws_pitch = align4(pr.n);
     if (splits > 1) {
         // first family: one (m, n) plane per range; swapped family: one accumulator per tile, CTA of the pair and range
-        rc = reserve(ctx, &ctx->splitk_ws, sizeof(float) * (swap ? static_cast<size_t>(plan.tiles) * plan.ctas * splits * ceil_div(plan.umma_n, 32) * 32 * dg::kBlockM
+        rc = reserve(ctx, &ctx->scratch->splitk_ws, sizeof(float) * (swap ? static_cast<size_t>(plan.tiles) * plan.ctas * splits * ceil_div(plan.umma_n, 32) * 32 * dg::kBlockM
                                                                  : static_cast<size_t>(splits) * pr.m * ws_pitch));
         if (rc) return rc;
         const uint32_t counters = plan.tiles * plan.ctas;
-        if (swap) rc = reserve(ctx, &ctx->splitk_counters, sizeof(uint32_t) * (counters < 1024 ? 1024 : counters), true);
+        if (swap) rc = reserve(ctx, &ctx->scratch->splitk_counters, sizeof(uint32_t) * (counters < 1024 ? 1024 : counters), true);
         if (rc) return rc;
     }
-    float* const splitk_ws = static_cast<float*>(ctx->splitk_ws.ptr);
+    float* const splitk_ws = static_cast<float*>(ctx->scratch->splitk_ws.ptr);
     const uint32_t sfa_words = 4 * ka->gran_k >= block_k ? 1 : block_k / (4 * ka->gran_k);
     const uint32_t sfb_words = 4 * kb->gran_k >= block_k ? 1 : block_k / (4 * kb->gran_k);
     const uint32_t sf_block_n = ceil_div(plan.umma_n, 128) * 128;
@@ -957,7 +990,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
         if (p.acc_stride == plan.umma_n) p.acc_edge_chunks = 0;
         p.splitk_ws = splitk_ws;
-        p.splitk_counters = static_cast<uint32_t*>(ctx->splitk_counters.ptr);
+        p.splitk_counters = static_cast<uint32_t*>(ctx->scratch->splitk_counters.ptr);
     }
     p.num_stages = plan.stages;
     p.epi_bufs = swap ? 2 : plan.epi_bufs;
@@ -1105,8 +1138,8 @@ cudaError_t launch_f32scale_kernel(const dg::F32ScaleParams& q, uint32_t grid, u
 }
 
 int ensure_group_ends(dg_ctx* ctx, uint32_t groups, uint32_t** ends) {
-    const int rc = reserve(ctx, &ctx->group_ends, sizeof(uint32_t) * (groups < 1024 ? 1024 : groups));
-    *ends = static_cast<uint32_t*>(ctx->group_ends.ptr);
+    const int rc = reserve(ctx, &ctx->scratch->group_ends, sizeof(uint32_t) * (groups < 1024 ? 1024 : groups));
+    *ends = static_cast<uint32_t*>(ctx->scratch->group_ends.ptr);
     return rc;
 }
 
@@ -1203,10 +1236,10 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     CUtensorMap maps[3];
     int rc;
     if (plan.splits > 1) {
-        rc = reserve(ctx, &ctx->splitk_ws, sizeof(float) * plan.splits * m * ws_pitch);
+        rc = reserve(ctx, &ctx->scratch->splitk_ws, sizeof(float) * plan.splits * m * ws_pitch);
         if (rc) return rc;
     }
-    float* const splitk_ws = static_cast<float*>(ctx->splitk_ws.ptr);
+    float* const splitk_ws = static_cast<float*>(ctx->scratch->splitk_ws.ptr);
     {
         uint64_t dims[3] = {k, m, a_groups};
         uint64_t strides[2] = {a_ld, static_cast<uint64_t>(a_ld) * m};
@@ -1301,10 +1334,10 @@ static int bridge_common(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_t 
     }
     const size_t need[2] = {dg_sf_words(m * a_groups, k, 128, a_groups), dg_sf_words(n * b_groups, k, 128, b_groups)};
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    int rc = reserve(ctx, &ctx->bridge_sf[0], need[0] * 4);
-    if (rc == DG_OK) rc = reserve(ctx, &ctx->bridge_sf[1], need[1] * 4);
+    int rc = reserve(ctx, &ctx->scratch->bridge_sf[0], need[0] * 4);
+    if (rc == DG_OK) rc = reserve(ctx, &ctx->scratch->bridge_sf[1], need[1] * 4);
     if (rc) return rc;
-    uint32_t *const sfa_words = static_cast<uint32_t*>(ctx->bridge_sf[0].ptr), *const sfb_words = static_cast<uint32_t*>(ctx->bridge_sf[1].ptr);
+    uint32_t *const sfa_words = static_cast<uint32_t*>(ctx->scratch->bridge_sf[0].ptr), *const sfb_words = static_cast<uint32_t*>(ctx->scratch->bridge_sf[1].ptr);
     // padding rows of the packed layouts must read as a valid exponent
     DG_CUDA(cudaMemsetAsync(sfa_words, 0, need[0] * 4, ctx->stream));
     DG_CUDA(cudaMemsetAsync(sfb_words, 0, need[1] * 4, ctx->stream));

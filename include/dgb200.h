@@ -42,6 +42,7 @@ int dg_ctx_sync(dg_ctx* ctx);
 /* device.rs:124 (num_sms) */
 int dg_ctx_num_sms(const dg_ctx* ctx, int* out);
 void* dg_ctx_stream(const dg_ctx* ctx);
+/* Work queued before keeps running on the old stream: every stream a context is used on has scratch of its own, freed with the context. */
 int dg_ctx_set_stream(dg_ctx* ctx, void* cuda_stream);
 /* Reads the device status word without synchronising the stream first (the caller has). */
 int dg_ctx_check_status(dg_ctx* ctx);

@@ -195,3 +195,34 @@ def test_exact_route_tile_variants(ctx, m, n, k):
         s = y.abs().max().clamp_min(1e-300)
         x, y = x / s, y / s
         assert float(1 - 2 * (x * y).sum() / (x * x + y * y).sum()) <= 2.0 ** -17
+
+
+def test_one_context_on_two_streams(ctx):
+    # calls on different streams run beside each other; each stream's K ranges have their partial planes to themselves
+    gen = torch.Generator(device="cuda").manual_seed(77)
+    m, n, k = 64, 2048, 7168
+    b = dg.Fp8Tensor(torch.randn((n, k), generator=gen, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8), n, k, k)
+    sfb = torch.rand((n // 128, k // 128), generator=gen, device="cuda")
+    acts = [dg.Fp8Tensor(torch.randn((m, k), generator=gen, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8), m, k, k) for _ in range(2)]
+    sfas = [dg.transform_sf_dev(ctx, torch.rand((m, k // 128), generator=gen, device="cuda"), m, k // 128) for _ in range(2)]
+    want = [torch.zeros((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    for a, sfa, out in zip(acts, sfas, want):
+        dg.fp8_gemm_nt_dev(ctx, a, sfa, b, sfb, out, n)
+    ctx.sync()
+    torch.cuda.synchronize()
+    c = dg.DgContext(0, own_stream=True)      # its own stream goes with the first switch
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = [[torch.zeros((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(20)] for _ in range(2)]
+    torch.cuda.synchronize()
+    dg.fp8_gemm_nt_dev(c, acts[0], sfas[0], b, sfb, got[0][0], n)
+    for i in range(20):
+        for s in range(2):
+            c.set_stream(streams[s].cuda_stream)
+            dg.fp8_gemm_nt_dev(c, acts[s], sfas[s], b, sfb, got[s][i], n)
+    torch.cuda.synchronize()
+    for s in range(2):
+        for out in got[s]:
+            assert torch.equal(out, want[s])
+    c.set_stream(streams[0].cuda_stream)      # the same stream again
+    c.sync()
+    c.close()
