@@ -305,24 +305,27 @@ static double group_rows(const dg_desc* d) {
 // 4096 x 7168, 263 -> 237 us at 7168 x 2048); with less than 2048 bytes of K its start-up and the transposed epilogue show
 // (34 x 64 rows, 1792 x 1024: 22 -> 31 us), and groups of two tiles and more fill the first family's 256-row tiles as well
 // (900 rows: 750 -> 808 us).
+// Only with per-128 scales on both sides: a per-32 operand (every e2m1 one) brings new scale words with each k-block, which one
+// warp re-orders for a narrow tile.  Over 90 grouped problems with one it took 1.6 to 4.9 times as long as the first family
+// (64 x 12 rows, 1984 x 3072, e4m3 x e2m1: 72 -> 222 us), over 20 dense ones up to 1.7 times (2 x 11992 x 10752: 34 -> 57 us).
 static bool prefer_swapped(const dg_desc* d) {
     if (d->cd_dtype == DG_OUT_SWIGLU_FP8) return false;
-    const uint32_t k_bytes = d->a_bits == 4 && d->b_bits == 4 ? d->k / 2 : d->k;
-    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return k_bytes >= 2048 && group_rows(d) <= 450.0;
+    if (d->a_bits != 8 || d->b_bits != 8 || d->gran_a != 128 || d->gran_b != 128) return false;
+    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return d->k >= 2048 && group_rows(d) <= 450.0;
     // (an arena with fewer rows per group than the alignment is one of mostly empty groups, about which nothing was measured)
     if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS)
-        return k_bytes >= 2048 && group_rows(d) <= 450.0 && d->m / (d->num_groups ? d->num_groups : 1) >= g_mk_alignment.load();
+        return d->k >= 2048 && group_rows(d) <= 450.0 && d->m / (d->num_groups ? d->num_groups : 1) >= g_mk_alignment.load();
     // Dense e4m3, a few rows: where the weight blocks alone fill half of the SMs in one wave (four fifths above 32 rows), a CTA streams
     // its 128 weight rows without K ranges and without a second launch (8 x 17056 x 8192: 41 -> 26 us; 28 x 9872 x 4608: 17.2 -> 15.4;
     // 53 x 18600 x 10240: 38 -> 34).  With more than one wave or more rows the first family's K ranges are as fast or
-    // faster, and an e2m1 operand (half the weight bytes) leaves the stream too thin.
+    // faster.
     const uint32_t blocks = ceil_div(d->n, 128), sms = d->num_sms ? d->num_sms : 148;
     // With fewer blocks it still wins where K is short: it takes 4.4 us + 0.31 us per 128 bytes of K whatever n is, the K ranges with
     // their second launch 8.2 us + 0.17 us per MB of weights (up to 32 rows and from 25 blocks on, 13 problems: 3680 x 2048
     // 12.2 -> 8.9 us, 5208 x 1536 10.6 -> 8.6, 9040 x 2560 15.3 -> 10.6; 0.99 to 1.44 times as fast; with fewer blocks 0.88 times).
     const uint32_t slabs = ceil_div(d->k, 128);
     const bool short_k = 6 * blocks >= sms && slabs * 0.31 < 3.8 + 0.17 * blocks * slabs * (128 * 128 / 1e6);
-    return d->gemm_type == DG_GEMM_NORMAL && d->a_bits == 8 && d->b_bits == 8 && blocks <= sms &&
+    return d->gemm_type == DG_GEMM_NORMAL && blocks <= sms &&
            ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));
 }
 

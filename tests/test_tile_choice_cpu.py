@@ -1,0 +1,25 @@
+"""Which tile family a problem gets, through dg_best_config (no GPU: the choice is host code).  The lines are measured ones; the
+figures stand beside the rule in csrc/dg_api.cu."""
+import pytest
+
+import deepgemm_rust_b200 as dg
+
+NORMAL, CONTIGUOUS, MASKED = dg.GemmType.Normal, dg.GemmType.MGroupedContiguous, dg.GemmType.MGroupedMasked
+E4M3, F32, FP8_OUT = {}, {"cd_dtype": 1}, {"cd_dtype": 2}
+PER_32 = [{"a_bits": 8, "b_bits": 4, "gran_b": 32}, {"a_bits": 4, "b_bits": 4, "gran_a": 32, "gran_b": 32}, {"gran_a": 32}, {"gran_b": 32}]
+
+
+def choice(*sizes, **kw):
+    return dg.best_config(dg.Sm100Desc(*sizes, **kw))
+
+
+@pytest.mark.parametrize("operands", PER_32)
+@pytest.mark.parametrize("out", [E4M3, F32])
+@pytest.mark.parametrize("sizes", [
+    (MASKED, 256, 4096, 7168, 32, 128), (MASKED, 128, 7168, 2048, 32, 32),          # decode steps of a layer of 32 experts
+    (CONTIGUOUS, 65536, 4096, 7168, 256), (CONTIGUOUS, 8192, 5824, 6144, 22),       # small expert groups
+    (NORMAL, 2, 11992, 10752), (NORMAL, 32, 18936, 4096),                           # few dense rows
+])
+def test_operands_with_per_32_scales_keep_the_first_family(sizes, out, operands):
+    assert choice(*sizes).swap_ab                     # with per-128 scales
+    assert not choice(*sizes, **operands, **out).swap_ab
