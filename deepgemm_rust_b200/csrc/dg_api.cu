@@ -483,7 +483,10 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // Dense problems have constants of their own, fitted to 205 of them (m 1-4096, n 512-16384, k 1024-16384, e4m3 / mixed / mxfp4,
             // every width, K ranges; the choice is 2 % off the best tile on average, 4 % with the others): a scale copy costs
             // 40 cycles, a tile 2900 from its first load to its last store, of which the last one's epilogue is exposed.
-            const bool fitted = (d->gemm_type == DG_GEMM_NORMAL || d->gemm_type == DG_GEMM_BATCHED) && !swiglu;
+            // What was not in that fit keeps the constants and the choices it had before it, which measured better there: batched problems
+            // (60 of them, 1.01 times as long on average with the fitted constants, 1.22 at worst: 10 x 420 x 1792 x 512, f32), and
+            // e4m3 operands with per-32 scales (30 problems, 1.02 and 1.28: 972 x 8704 x 1024, f32).
+            const bool fitted = d->gemm_type == DG_GEMM_NORMAL && !swiglu && (d->a_bits == 4 || d->gran_a == 128) && (d->b_bits == 4 || d->gran_b == 128);
             const double least_mma = fitted ? 103.0 : 118.0;
             const double mma = 4.0 * (bn * 0.5 > least_mma ? bn * 0.5 : least_mma);
             const double feed = (16384.0 + bn / ctas * 128.0) / 77.0;
@@ -495,7 +498,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // never straddle ranges; the partial sums cost a second small kernel (launch + S reads of the M x N f32 tile set)
             const bool may_split = d->gemm_type == DG_GEMM_NORMAL && d->cd_dtype != DG_OUT_FP8 && !swiglu && d->n % 4 == 0 && !no_k_ranges;
             for (uint32_t splits = 1; splits <= 16; ++splits) {
-                if (splits > 1 && !may_split) break;
+                if (splits > 1 && (!may_split || (halves > 1 && !fitted))) break;
                 if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != splits) continue;
                 const uint32_t unit = 4 / halves;      // a range is whole scale words: four slabs
                 uint32_t kb_per = ceil_div(ceil_div(total_kb, splits), unit) * unit;
@@ -510,7 +513,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
                 uint32_t epi_bufs = 2;
                 auto smem = [&]() { return dg::gemm_smem_bytes(bn, ctas, kernel_out, stages, sfa_words, sfb_words, halves, epi_bufs); };
                 while (stages > 1 && smem() > kSmemCapacity) --stages;
-                if (stages < 3 && most_stages >= 3 && kernel_out == DG_OUT_F32) {
+                if (fitted && stages < 3 && most_stages >= 3 && kernel_out == DG_OUT_F32) {
                     stages = most_stages;
                     epi_bufs = 1;
                     while (stages > 1 && smem() > kSmemCapacity) --stages;
@@ -518,8 +521,9 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
                 if (stages < 1 || smem() > kSmemCapacity) continue;
                 if (stages < 3 && !force_stages) continue;
                 const uint32_t waves = ceil_div(tiles * splits, workers);
-                const double tile_cost = kb_per * per_kb + (splits > 1 ? 3.6 * bn : epilogue) + (fitted ? 2855.0 : 600.0);
-                const double reduce = (splits > 1 ? 4450.0 + static_cast<double>(splits) * d->m * d->n * 4.0 / 1507.0 : 0.0) +
+                const double tile_cost = kb_per * per_kb + (splits > 1 ? (fitted ? 3.6 : 2.0) * bn : epilogue) + (fitted ? 2855.0 : 600.0);
+                const double plane_bytes = static_cast<double>(splits) * d->m * d->n * 4.0;
+                const double reduce = (splits > 1 ? (fitted ? 4450.0 + plane_bytes / 1507.0 : 9000.0 + plane_bytes / 3000.0) : 0.0) +
                                       (fitted ? 4.5 * bn + (ctas == 2 ? 280.0 : 0.0) : 0.0);
                 // every CTA pulls its A slab (16 KB) and its share of B from L2 for each 128 bytes of K; with many small groups
                 // (weights read once, little reuse) that aggregate stream, ~9000 bytes per cycle on this part (11000 with the reuse of

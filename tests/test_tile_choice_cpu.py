@@ -23,3 +23,16 @@ def choice(*sizes, **kw):
 def test_operands_with_per_32_scales_keep_the_first_family(sizes, out, operands):
     assert choice(*sizes).swap_ab                     # with per-128 scales
     assert not choice(*sizes, **operands, **out).swap_ab
+
+
+@pytest.mark.parametrize("sizes,kw,tile", [
+    ((dg.GemmType.Batched, 420, 1792, 512, 10), F32, (256, 192, 256, 1)),
+    ((dg.GemmType.Batched, 24, 3200, 512, 12), FP8_OUT, (128, 128, 128, 1)),
+    ((dg.GemmType.Batched, 876, 3072, 2048, 6), E4M3, (256, 224, 256, 1)),
+    ((NORMAL, 972, 8704, 1024), {"gran_a": 32, "gran_b": 32, **F32}, (256, 160, 256, 1)),
+])
+def test_problems_outside_the_fit_of_the_dense_costs_keep_their_tiles(sizes, kw, tile):
+    # the cost constants of dense problems were fitted to unbatched ones, e4m3 with per-128 scales or e2m1; these measured 5-28 %
+    # slower with the tiles the fitted constants gave them
+    c = choice(*sizes, **kw)
+    assert (c.block_m, c.block_n, c.block_k, c.num_splits) == tile
