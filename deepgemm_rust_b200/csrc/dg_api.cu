@@ -356,13 +356,21 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
             if (d->gemm_type != DG_GEMM_NORMAL && d->gemm_type != DG_GEMM_BATCHED && ((halves == 2 && !force_halves) || (ctas == 1 && !force_ctas && sms >= 2))) continue;
             const uint32_t step = dense ? 16 * ctas : 32, workers = sms / ctas;
             const double rows = group_rows(d);
-            // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected (masked: at most
-            // a slot) and at least 64, and 288 rather than 256 for groups around that size, half of which are a little above
+            // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected and at least 64, in the
+            // contiguous layout 288 rather than 256 for groups around that size, half of which are a little above.
+            // A masked problem's expected rows are a hint about the mean only, and a hot group's weights pass through an SM once per tile:
+            // with a hint of 1, tiles of 64 rows took up to 4.3 times as long as the first family (13 groups of up to 903 rows,
+            // 2304 x 4096: 92 -> 390 us).  So at least 128 rows, and a quarter of the slot.  128 rows cost nothing where the hint is right
+            // (1-16 rows, 30 problems: 0.99 of the time on average; 256 rows took 3 % more in a decode step of 62 experts x 2 rows).
             uint32_t bn;
             if (dense) bn = d->m <= 256 ? ceil_div(d->m, step) * step : 256;
             else bn = ceil_div(static_cast<uint32_t>(2 * rows) + 1, 32) * 32;
             if (!dense && bn < 64) bn = 64;
-            if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED && bn > ceil_div(d->m, 32) * 32) bn = ceil_div(d->m, 32) * 32;
+            if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) {
+                const uint32_t least = d->m / 4 > 128 ? ceil_div(d->m / 4, 32) * 32 : 128, slot = ceil_div(d->m, 32) * 32;
+                if (bn < least) bn = least;
+                if (bn > slot) bn = slot;
+            }
             if (bn > 256) bn = d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS && halves == 1 ? 288 : 256;
             if (force_n) bn = static_cast<uint32_t>(atoi(force_n));
             if (bn == 0 || bn > dg::kSwapMaxRows || (bn > 256 && bn % 32 != 0) || (bn > 256 && dense) || bn % step != 0) continue;

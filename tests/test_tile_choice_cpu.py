@@ -36,3 +36,11 @@ def test_problems_outside_the_fit_of_the_dense_costs_keep_their_tiles(sizes, kw,
     # slower with the tiles the fitted constants gave them
     c = choice(*sizes, **kw)
     assert (c.block_m, c.block_n, c.block_k, c.num_splits) == tile
+
+
+@pytest.mark.parametrize("slot,height", [(64, 64), (76, 96), (128, 128), (250, 128), (516, 160), (924, 256), (4096, 256)])
+@pytest.mark.parametrize("expected", [1, 16])
+def test_a_weak_hint_does_not_shorten_the_tiles_of_a_masked_problem(slot, height, expected):
+    # expected_m is a hint about the mean of the groups; a group may fill its slot whatever it says
+    c = choice(MASKED, slot, 4096, 7168, 32, expected, **FP8_OUT)
+    assert c.swap_ab and c.block_m == height
