@@ -300,30 +300,42 @@ static double group_rows(const dg_desc* d) {
     return d->m;
 }
 
-// Is the swapped family the better one for this problem?  Measured on B200 over 40 grouped problems: expert groups that fit one
-// tile gain 5-20 % (masked 32 x <= 256 rows, 4096 x 7168: 247 -> 199 us; contiguous 256 x 256 rows: 486 -> 430 us at
-// 4096 x 7168, 263 -> 237 us at 7168 x 2048); with less than 2048 bytes of K its start-up and the transposed epilogue show
-// (34 x 64 rows, 1792 x 1024: 22 -> 31 us), and groups of two tiles and more fill the first family's 256-row tiles as well
-// (900 rows: 750 -> 808 us).
+// Is the swapped family the better one for this problem?  Measured on B200 over 920 grouped problems (4-128 groups of 4-1200 rows,
+// equal and skewed, n 128-7168, k 1024-7168), both families side by side.  It wins where a group's rows fit one tile and there is
+// enough to stream (masked 32 x <= 256 rows, 4096 x 7168: 247 -> 199 us; contiguous 256 x 256 rows: 486 -> 430 us at 4096 x 7168,
+// 263 -> 237 us at 7168 x 2048).  It loses
+//   with few tiles: below half a wave of pair tiles (masked) or one wave (contiguous) it took 1.2-1.3 times as long over 300 problems,
+//     because its tiles are 256 weight rows wide where the first family goes down to 32;
+//   with short K, where its start-up and the transposed epilogue show: below 2048 bytes 1.17-1.24 times on average (34 x 64 rows,
+//     1792 x 1024: 22 -> 31 us).  Up to 28 slabs of 128 bytes it is the better one for e4m3 output (the first family then has
+//     tiles of 128 and 256 columns only), for masked groups with 4096 columns and two waves, and for contiguous groups of 160-320
+//     rows (one tile of its, two of the other's); else it takes up to 1.4 times as long (20 x 36 rows, 1792 x 2048: 17.9 -> 24.5 us);
+//   with fewer than 2048 columns in the contiguous layout (up to 1.4 times: 28 x 40 rows, 1088 x 6144: 54 -> 75 us);
+//   with groups of two tiles and more, which fill the first family's 256-row tiles as well (900 rows: 750 -> 808 us).
+// With these lines it is chosen for a third of them; on average they take 0.95 (masked) and 0.99 (contiguous) of the first family's
+// time, at most 1.34; chosen wherever K had 2048 bytes and groups up to 450 rows it was 0.99 and 1.02, at most 2.0.
 // Only with per-128 scales on both sides: a per-32 operand (every e2m1 one) brings new scale words with each k-block, which one
 // warp re-orders for a narrow tile.  Over 90 grouped problems with one it took 1.6 to 4.9 times as long as the first family
 // (64 x 12 rows, 1984 x 3072, e4m3 x e2m1: 72 -> 222 us), over 20 dense ones up to 1.7 times (2 x 11992 x 10752: 34 -> 57 us).
 static bool prefer_swapped(const dg_desc* d) {
     if (d->cd_dtype == DG_OUT_SWIGLU_FP8) return false;
     if (d->a_bits != 8 || d->b_bits != 8 || d->gran_a != 128 || d->gran_b != 128) return false;
-    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return d->k >= 2048 && group_rows(d) <= 450.0;
-    // (an arena with fewer rows per group than the alignment is one of mostly empty groups, about which nothing was measured)
-    if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS)
-        return d->k >= 2048 && group_rows(d) <= 450.0 && d->m / (d->num_groups ? d->num_groups : 1) >= g_mk_alignment.load();
+    const uint32_t sms = d->num_sms ? d->num_sms : 148, slabs = ceil_div(d->k, 128), groups = d->num_groups ? d->num_groups : 1;
+    if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED || d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
+        const double rows = group_rows(d), waves = static_cast<double>(groups) * ceil_div(d->n, 256) / (sms / 2.0);
+        if (d->k < 2048 || rows > 450.0) return false;
+        if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return waves >= 0.5 && (d->cd_dtype == DG_OUT_FP8 || slabs >= 28 || (waves >= 2.0 && d->n >= 4096));
+        // (an arena with fewer rows per group than the alignment is one of mostly empty groups, about which nothing was measured)
+        return waves >= 1.0 && d->n >= 2048 && (slabs >= 28 || (rows >= 160.0 && rows <= 320.0)) && d->m / groups >= g_mk_alignment.load();
+    }
     // Dense e4m3, a few rows: where the weight blocks alone fill half of the SMs in one wave (four fifths above 32 rows), a CTA streams
     // its 128 weight rows without K ranges and without a second launch (8 x 17056 x 8192: 41 -> 26 us; 28 x 9872 x 4608: 17.2 -> 15.4;
     // 53 x 18600 x 10240: 38 -> 34).  With more than one wave or more rows the first family's K ranges are as fast or
     // faster.
-    const uint32_t blocks = ceil_div(d->n, 128), sms = d->num_sms ? d->num_sms : 148;
+    const uint32_t blocks = ceil_div(d->n, 128);
     // With fewer blocks it still wins where K is short: it takes 4.4 us + 0.31 us per 128 bytes of K whatever n is, the K ranges with
     // their second launch 8.2 us + 0.17 us per MB of weights (up to 32 rows and from 25 blocks on, 13 problems: 3680 x 2048
     // 12.2 -> 8.9 us, 5208 x 1536 10.6 -> 8.6, 9040 x 2560 15.3 -> 10.6; 0.99 to 1.44 times as fast; with fewer blocks 0.88 times).
-    const uint32_t slabs = ceil_div(d->k, 128);
     const bool short_k = 6 * blocks >= sms && slabs * 0.31 < 3.8 + 0.17 * blocks * slabs * (128 * 128 / 1e6);
     return d->gemm_type == DG_GEMM_NORMAL && blocks <= sms &&
            ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));

@@ -685,8 +685,8 @@ def test_bounded_wait_reports_timeout_and_context_survives():
 
 @pytest.mark.parametrize("out_kind", [0, 1])
 @pytest.mark.parametrize("sizes,n,k", [
-    ([256, 257, 288, 289, 1, 0, 320, 33], 384, 2048),   # one tile, the 32 rows beyond 256, two tiles from 289 rows on; empty and tiny groups
-    ([31, 32, 64, 65, 96, 128], 264, 2176),             # tile heights of one to four store boxes, columns off the 128 grid, 17 k-blocks
+    ([256, 257, 288, 289, 1, 0, 320, 33], 2432, 2048),  # one tile, the 32 rows beyond 256, two tiles from 289 rows on; empty and tiny groups
+    ([31, 32, 64, 65, 96, 128], 3208, 3712),            # tile heights of one to four store boxes, columns off the 128 grid, 29 k-blocks
 ])
 def test_rule_picks_the_swapped_family_for_small_groups(ctx, sizes, n, k, out_kind):
     # no DG_SWAP: the tile heights a group can get, through the contiguous layout; every valid row and column against the oracle
@@ -711,7 +711,7 @@ def test_rule_picks_the_swapped_family_for_small_groups(ctx, sizes, n, k, out_ki
 def test_swapped_masked_fp8_output_is_the_requantised_accumulator(ctx):
     # the e4m3 epilogue of the swapped family: one and several 32-row chunks, ragged last ones; the CPU epilogue applied to the GPU's
     # own f32 accumulators (same tiles) gives the identical bytes and scale words on every valid row
-    masked, m_max, n, k = [1, 32, 33, 100, 0, 200], 200, 256, 2048
+    masked, m_max, n, k = [1, 32, 33, 100, 0, 200], 200, 1664, 3584
     groups = len(masked)
     assert dg.best_config(dg.Sm100Desc(dg.GemmType.MGroupedMasked, m_max, n, k, groups, 64)).swap_ab
     _, aq, asf = fp8_operand_1d(groups * m_max, k, 311, 128, groups)

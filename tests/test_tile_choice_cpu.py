@@ -44,3 +44,25 @@ def test_a_weak_hint_does_not_shorten_the_tiles_of_a_masked_problem(slot, height
     # expected_m is a hint about the mean of the groups; a group may fill its slot whatever it says
     c = choice(MASKED, slot, 4096, 7168, 32, expected, **FP8_OUT)
     assert c.swap_ab and c.block_m == height
+
+
+@pytest.mark.parametrize("sizes,kw,swapped", [
+    # decode steps of 32 experts: e4m3 output, then bf16 with short K
+    ((MASKED, 256, 4096, 7168, 32, 128), FP8_OUT, True), ((MASKED, 128, 7168, 2048, 32, 32), E4M3, True),
+    # masked: half a wave of pair tiles (37 of 74), 28 slabs of K, 4096 columns
+    ((MASKED, 128, 256, 7168, 37, 32), E4M3, True), ((MASKED, 128, 256, 7168, 36, 32), FP8_OUT, False),
+    ((MASKED, 128, 2048, 3584, 32, 32), E4M3, True), ((MASKED, 128, 2048, 3456, 32, 32), E4M3, False),
+    ((MASKED, 128, 2048, 2048, 32, 32), FP8_OUT, True), ((MASKED, 128, 2048, 1920, 32, 32), FP8_OUT, False),
+    ((MASKED, 128, 4096, 2048, 10, 32), E4M3, True), ((MASKED, 128, 4096, 2048, 9, 32), E4M3, False), ((MASKED, 128, 3968, 2048, 64, 32), F32, False),
+    ((MASKED, 1024, 4096, 7168, 32, 450), E4M3, True), ((MASKED, 1024, 4096, 7168, 32, 451), E4M3, False),
+    # prefill of 256 experts, about 256 rows each and 64 of padding
+    ((CONTIGUOUS, 98304, 4096, 7168, 256), E4M3, True), ((CONTIGUOUS, 98304, 7168, 2048, 256), E4M3, True),
+    # contiguous: a wave of pair tiles, 2048 columns, groups that fit one tile where K is short
+    ((CONTIGUOUS, 10 * 256, 2048, 3584, 10), E4M3, True), ((CONTIGUOUS, 9 * 256, 2048, 3584, 9), E4M3, False),
+    ((CONTIGUOUS, 64 * 256, 2040, 7168, 64), E4M3, False), ((CONTIGUOUS, 64 * 256, 2048, 3456, 64), E4M3, True),
+    ((CONTIGUOUS, 64 * 128, 2048, 3456, 64), E4M3, False), ((CONTIGUOUS, 64 * 512, 2048, 3456, 64), E4M3, False),
+    ((CONTIGUOUS, 64 * 512, 2048, 3584, 64), E4M3, True), ((CONTIGUOUS, 64 * 520, 2048, 3584, 64), E4M3, False),
+    ((CONTIGUOUS, 20 * 128, 1792, 2048, 20), E4M3, False), ((CONTIGUOUS, 6 * 128, 264, 2176, 6), E4M3, False),
+])
+def test_family_of_a_grouped_problem(sizes, kw, swapped):
+    assert choice(*sizes, **kw).swap_ab == swapped
