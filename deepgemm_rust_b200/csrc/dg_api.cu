@@ -289,13 +289,13 @@ static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     return DG_OK;
 }
 
-// Rows of a group, as far as the host knows them: the contiguous arena's rows include its alignment padding.
+// Rows of a group of the contiguous layout, as far as the host knows them: the arena's rows include the alignment padding.
+static double contiguous_rows(uint32_t m, uint32_t groups) {
+    const double per_group = static_cast<double>(m) / groups, padding = g_mk_alignment.load() / 2.0;
+    return per_group > padding ? per_group - padding : per_group;
+}
 static double group_rows(const dg_desc* d) {
-    const uint32_t groups = d->num_groups ? d->num_groups : 1, align = g_mk_alignment.load();
-    if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) {
-        const double per_group = static_cast<double>(d->m) / groups;
-        return per_group > align / 2.0 ? per_group - align / 2.0 : per_group;
-    }
+    if (d->gemm_type == DG_GEMM_M_GROUPED_CONTIGUOUS) return contiguous_rows(d->m, d->num_groups ? d->num_groups : 1);
     if (d->gemm_type == DG_GEMM_M_GROUPED_MASKED) return d->expected_m < d->m ? d->expected_m : d->m;
     return d->m;
 }
@@ -660,6 +660,11 @@ bool pdl_enabled() {
     return on;
 }
 
+bool print_configs() {
+    static const bool on = [] { const char* v = getenv("DG_PRINT_CONFIGS"); return v && strcmp(v, "0") != 0; }();
+    return on;
+}
+
 // Launches a kernel that calls griddep_wait() itself before its first access to global memory, so that its start-up overlaps the
 // end of the kernel before it in the stream.  (Also the cheaper launch for the host: 2.0 us against 2.4 us measured for the
 // fully serialised form.)  Grids of more than 4096 blocks are launched serialised: early blocks move in beside a persistent
@@ -874,8 +879,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const dg_lp_operand* kb = swap ? a : b;
     const uint32_t ka_rows = swap ? pr.n : pr.m, kb_rows = swap ? pr.m : pr.n;              // per group
     const uint32_t ka_groups = swap ? b_groups : a_groups, kb_groups = swap ? a_groups : b_groups;
-    static const bool print_cfg = [] { const char* v = getenv("DG_PRINT_CONFIGS"); return v && strcmp(v, "0") != 0; }();
-    if (print_cfg)
+    if (print_configs())
         fprintf(stderr, "[dgb200] type=%u m=%u n=%u k=%u groups=%u -> swap_ab=%u block=%ux%ux%u ctas=%u stages=%u accum=%u smem=%u tiles~%u splits=%u\n",
                 pr.type, pr.m, pr.n, pr.k, pr.groups, cfg.swap_ab, cfg.block_m, cfg.block_n, cfg.block_k, plan.ctas, cfg.num_stages,
                 cfg.num_accum_stages, cfg.smem_size, cfg.num_tiles, cfg.num_splits);
@@ -1110,9 +1114,11 @@ struct F32Plan {
 F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint32_t groups, uint32_t sms) {
     const uint32_t kbs = k / 128;
     const bool dense = type == DG_GEMM_NORMAL;
-    // row blocks: a contiguous group ends inside a tile, half a tile is lost on average
+    // row blocks: a contiguous group ends inside a tile, half a tile is lost on average.  Its padding makes no tiles: counted as rows it
+    // made three waves of 128-row tiles out of what is one or two, and small groups got tiles of 256 rows, half of them empty
+    // (12 groups of 87 rows, 1152 x 3456: 22.6 us with 128-row tiles, 28.7 with 256).
     auto row_blocks = [&](uint32_t tile_m) {
-        if (type == DG_GEMM_M_GROUPED_CONTIGUOUS) return groups * (static_cast<double>(m) / groups / tile_m + 0.5);
+        if (type == DG_GEMM_M_GROUPED_CONTIGUOUS) return groups * (contiguous_rows(m, groups) / tile_m + 0.5);
         return static_cast<double>(dense ? 1u : groups) * ceil_div(m, tile_m);
     };
     const double tiles = row_blocks(128) * ceil_div(n, 128), pair_tiles = row_blocks(256) * ceil_div(n, 256);
@@ -1259,6 +1265,9 @@ static int launch_f32scale(dg_ctx* ctx, uint32_t type, const uint8_t* a, uint32_
     if (a_ld < k || b_ld < k || a_ld % 16 != 0 || b_ld % 16 != 0) return fail(DG_ERR_SHAPE, "leading dimensions must be >= k and multiples of 16 bytes");
     if (out_ld < n || (static_cast<size_t>(out_ld) * 2) % 16 != 0) return fail(DG_ERR_SHAPE, "output ld (%u) must be >= n and a multiple of 8 elements", out_ld);
     const F32Plan plan = choose_f32scale(type, m, n, k, groups, static_cast<uint32_t>(ctx->num_sms));
+    if (print_configs())
+        fprintf(stderr, "[dgb200] f32 scales: type=%u m=%u n=%u k=%u groups=%u -> block=%ux%u ctas=%u splits=%u\n", type, m, n, k, groups, 128 * plan.ctas,
+                plan.block_n, plan.ctas, plan.splits);
     const uint32_t ws_pitch = align4(n);
     CUtensorMap maps[3];
     int rc;

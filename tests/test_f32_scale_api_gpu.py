@@ -17,6 +17,8 @@ from tests.helpers import dev, to_f32
 
 pytestmark = pytest.mark.gpu
 import os
+import subprocess
+import sys
 
 # (route, activation scale, weight scale)
 ROUTES = [("exact", 0.01, 0.02), ("exact", 2.0 ** -6, 2.0 ** -5), ("exponent", 2.0 ** -6, 2.0 ** -5)]
@@ -226,3 +228,25 @@ def test_one_context_on_two_streams(ctx):
     c.set_stream(streams[0].cuda_stream)      # the same stream again
     c.sync()
     c.close()
+
+
+def test_small_contiguous_groups_get_small_tiles():
+    # arenas of 128 rows per group: a group fits one tile of 128 rows and all tiles one wave of the SMs; the arena's padding must not
+    # be taken for rows that make a second wave of them
+    code = """
+import torch, deepgemm_rust_b200 as dg
+ctx = dg.DgContext(0)
+for groups, rows, n, k in ((12, 128, 1152, 3456), (18, 128, 1024, 512)):
+    m = groups * rows
+    a, b = (dg.Fp8Tensor(torch.zeros((r, k), dtype=torch.uint8, device="cuda"), r, k, k) for r in (m, groups * n))
+    sfa_t = dg.transform_sf_dev(ctx, torch.ones((m, k // 128), device="cuda"), m, k // 128)
+    out = torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+    index = torch.arange(groups, dtype=torch.int32, device="cuda").repeat_interleave(rows)
+    dg.m_grouped_fp8_gemm_nt_contiguous_dev(ctx, a, sfa_t, b, torch.ones((groups * n // 128, k // 128), device="cuda"), out, n, index, groups)
+ctx.sync()
+"""
+    run = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                         env={**os.environ, "DG_PRINT_CONFIGS": "1"})
+    assert run.returncode == 0, run.stderr
+    lines = [line for line in run.stderr.splitlines() if "f32 scales" in line]
+    assert len(lines) == 2 and all("block=128x128 ctas=1" in line for line in lines), lines
