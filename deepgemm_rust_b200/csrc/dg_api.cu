@@ -500,9 +500,9 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // max(~118, bn / 2) cycles and a CTA receives its A tile (16 KB) plus bn/ctas rows of B at ~77 bytes per cycle;
             // a single-buffered accumulator exposes the whole epilogue (~10.5 cycles per column).
             const uint32_t total_kb = ceil_div(d->k, block_k);
-            // Dense problems have constants of their own, fitted to 205 of them (m 1-4096, n 512-16384, k 1024-16384, e4m3 / mixed / mxfp4,
-            // every width, K ranges; the choice is 2 % off the best tile on average, 4 % with the others): a scale copy costs
-            // 40 cycles, a tile 2900 from its first load to its last store, of which the last one's epilogue is exposed.
+            // Dense problems have constants of their own.  For one wave they were fitted to 205 problems (m 1-4096, n 512-16384, k 1024-16384,
+            // e4m3 / mixed / mxfp4, every width, K ranges; the choice is 2 % off the best of these tiles on average, 4 % with the others): a
+            // scale copy costs 40 cycles, a tile 2900 from its first load to its last store, of which the last one's epilogue is exposed.
             // What was not in that fit keeps the constants and the choices it had before it, which measured better there: batched problems
             // (60 of them, 1.01 times as long on average with the fitted constants, 1.22 at worst: 10 x 420 x 1792 x 512, f32), and
             // e4m3 operands with per-32 scales (30 problems, 1.02 and 1.28: 972 x 8704 x 1024, f32).
@@ -550,7 +550,17 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
                 // dense problems), is the limit
                 const double l2_bytes = static_cast<double>(tiles) * ctas * ceil_div(d->k, half_k) * (16384.0 + bn / ctas * 128.0);
                 const double l2_floor = l2_bytes / (fitted ? 11140.0 : 9000.0);
-                const double compute = waves * tile_cost;
+                double compute = waves * tile_cost;
+                if (fitted && splits == 1 && waves > 1) {
+                    // A further wave starts while the one before it is stored: with two accumulators only the longer of main loop and stores
+                    // counts, with one the epilogue comes on top; f32 tiles store twice the bytes.  Over 152 problems of several waves
+                    // (m 512-8192, n 1536-24576, k 512-8192, bf16 and f32 outputs, 20 tiles each) the choice is 1.1 % off the best of them,
+                    // 3.8 % with the first wave's cost for every wave, which took 256-column tiles and their exposed epilogues where narrower
+                    // ones are faster: 2894 x 6144 x 1024 20.0 -> 26.7 us, 7467 x 3448 x 2560 with f32 output 63.6 -> 80.2.
+                    const double loop = kb_per * per_kb, store = kernel_out == DG_OUT_F32 ? 2.0 * bn : 1.0 * bn;
+                    const double hidden = loop + bn > 10.0 * store ? loop + bn : 10.0 * store;
+                    compute = tile_cost + (waves - 1.0) * ((accum == 1 ? loop + 12.0 * store : hidden) + 1000.0);
+                }
                 const double cost = (compute > l2_floor ? compute : l2_floor) + reduce;
                 if (best_n == 0 || cost < best_cost * (1.0 - 1e-9)) {
                     best_n = bn; best_cost = cost; best_accum = accum; best_tiles = tiles; best_ctas = ctas; best_stages = stages;
