@@ -1049,10 +1049,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.mk_alignment = align;
     // groups start at multiples of `align` rows; tiles stay 128 (or 256) rows tall and simply run into the next group's rows,
     // which are computed and not stored.  Stores go out in 32-row boxes, so only an alignment of 16 needs row-exact stores.
-    // A problem that the rule sends to the swapped family writes the same rows; where DG_SWAP=1 pins that family, the masked and
-    // contiguous layouts write exactly the valid rows.
-    const char* pinned = getenv("DG_SWAP");
-    p.mask_rows = ((contiguous && align % 32 != 0) || (swap && pinned && atoi(pinned) != 0)) ? 1 : 0;
+    // Both tile families write the same rows: a group's own and its padding up to the next multiple of 32.
+    p.mask_rows = (contiguous && align % 32 != 0) ? 1 : 0;
     p.out_ptr = out->buf;
     p.out_ld = out->ld;
     {

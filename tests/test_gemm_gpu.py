@@ -425,12 +425,12 @@ def test_m_grouped_masked(ctx, masked, m_max, n, k, ctas, family, monkeypatch):
     assert not np.isnan(dn[valid]).any()
     diff = O.calc_diff(dn[valid], want[valid])
     assert diff <= TIGHT_BF16, diff
-    # rows of a group whose tiles were never scheduled keep the caller's contents (no stray writes)
+    # rows beyond a group's last 32-row store keep the caller's contents (no stray writes), in both tile families
     for g in range(groups):
-        # first family: whole 128- or 256-row tiles; swapped family: exactly the valid rows
-        first_untouched = g * m_max + (masked[g] if family == "1" else ((masked[g] + 128 * ctas - 1) // (128 * ctas)) * 128 * ctas)
+        first_untouched = g * m_max + (masked[g] + 31) // 32 * 32
         if first_untouched < (g + 1) * m_max:
             assert np.isnan(dn[first_untouched:(g + 1) * m_max]).all()
+
 
 
 def test_bmm_and_fp8_requant_epilogue(ctx):
@@ -788,3 +788,36 @@ def test_a_failed_call_does_not_fail_the_next_one(ctx):
             dg.peer_alloc(ctx, 1 << 50, False)
         call()
     ctx.sync()
+
+
+@pytest.mark.parametrize("family", [None, "0", "1"])
+@pytest.mark.parametrize("n,k", [(256, 512), (4096, 3584)])      # the rule's choice: the first family, the swapped one
+def test_grouped_calls_write_the_same_rows_whichever_family_runs(ctx, n, k, family, monkeypatch):
+    # a group's own rows and its padding up to the next multiple of 32 (at most its slot) are written, nothing else
+    pin_family(monkeypatch, family)
+    masked, m_max = [37, 1, 0, 100, 33, 64], 100
+    groups = len(masked)
+    if family is None:
+        assert dg.best_config(dg.Sm100Desc(dg.GemmType.MGroupedMasked, m_max, n, k, groups, 39)).swap_ab == (k == 3584)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+
+    def quantised(rows, batches):
+        return dg.cast_bf16_to_fp8_sf_dev(ctx, torch.randn((rows, k), generator=gen, device="cuda").bfloat16(), k, rows, k, 128, batches)
+    b = dg.LpOperand(*quantised(groups * n, groups), groups * n, k, k)
+    d = torch.full((groups * m_max, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dg.m_grouped_fp8_fp4_gemm_masked_dev(ctx, dg.LpOperand(*quantised(groups * m_max, groups), m_max, k, k), dev(np.array(masked, np.int32)), b,
+                                         dg.Sm100Out.Bf16(d, n), groups, 39)
+    ctx.sync()
+    written = ~torch.isnan(d).view(groups, m_max, n)
+    for g, rows in enumerate(masked):
+        upto = min((rows + 31) // 32 * 32, m_max)
+        assert written[g, :upto].all() and not written[g, upto:].any()
+    m_idx, starts = contiguous_layout(masked)
+    d = torch.full((len(m_idx), n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dg.m_grouped_fp8_fp4_gemm_contiguous_dev(ctx, dg.LpOperand(*quantised(len(m_idx), 1), len(m_idx), k, k), dev(m_idx), b, dg.Sm100Out.Bf16(d, n), groups)
+    ctx.sync()
+    want = np.zeros(len(m_idx), bool)
+    for start, rows in zip(starts, masked):
+        want[start:start + (rows + 31) // 32 * 32] = True
+    got = (~torch.isnan(d)).cpu().numpy()
+    assert (got == want[:, None]).all()
