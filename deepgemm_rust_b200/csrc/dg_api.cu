@@ -225,9 +225,9 @@ uint32_t dg_get_mk_alignment_for_contiguous_layout(void) { return g_mk_alignment
 uint32_t dg_get_theoretical_mk_alignment_for_contiguous_layout(uint32_t arch_major) { return arch_major == 10 ? 256u : 128u; }
 
 // ------------------------------------------------------------------------- heuristics
-// Tile choice for 148 SMs / 227 KB shared memory / 512 TMEM columns.  A rows always ride the
-// UMMA M dimension (128 per tile); BLOCK_N is picked from the widths the epilogue of the output
-// type can store, minimising waves x per-tile cost; stages fill the shared memory left over.
+// Tile choice for 148 SMs / 227 KB shared memory / 512 TMEM columns.  In the first tile family A rows ride the UMMA M dimension (128
+// per CTA); BLOCK_N is picked from the widths the epilogue of the output type can store, minimising waves x per-tile cost; stages
+// fill the shared memory left over.  prefer_swapped says which problems the second family gets, with weight rows on UMMA M.
 // What the launcher needs to know about a choice (the public dg_config describes the same choice in the reference's terms).
 struct KernelPlan {
     bool swap;                 // weights on the UMMA M dimension, activation rows on UMMA N
@@ -360,7 +360,8 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
         for (uint32_t ctas = 1; ctas <= 2; ++ctas) {
             if (force_ctas && static_cast<uint32_t>(atoi(force_ctas)) != ctas) continue;
             if (ctas == 2 && sms < 2) continue;
-            // the dense problems the rule above picks: one CTA per weight block, two slabs, no K ranges
+            // the dense problems the rule above picks: one CTA per weight block, two slabs, no K ranges (those, pairs and one slab only
+            // where DG_SWAP=1 pins the family: in the dense problems it was measured on, the first family's K ranges are the faster ones)
             const bool picked = d->gemm_type == DG_GEMM_NORMAL && !getenv("DG_SWAP");
             if (picked && ((halves == 1 && !force_halves) || (ctas == 2 && !force_ctas))) continue;
             // grouped layouts: pairs and one slab per stage measured best at every size (MoE layer of 256 experts: 3.88 ms against 4.28
@@ -371,8 +372,8 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
             // tile height: everything a dense problem has up to 256 rows; where groups vary, twice what is expected and at least 64, in the
             // contiguous layout 288 rather than 256 for groups around that size, half of which are a little above.
             // A masked problem's expected rows are a hint about the mean only, and a hot group's weights pass through an SM once per tile:
-            // with a hint of 1, tiles of 64 rows took up to 4.3 times as long as the first family (13 groups of up to 903 rows,
-            // 2304 x 4096: 92 -> 390 us).  So at least 128 rows, and a quarter of the slot.  128 rows cost nothing where the hint is right
+            // with a hint of 1, tiles of 64 rows took up to 2.0 times as long as the first family (15 groups of up to 336 rows,
+            // 3712 x 3072: 59 -> 99 us).  So at least 128 rows, and a quarter of the slot.  128 rows cost nothing where the hint is right
             // (1-16 rows, 30 problems: 0.99 of the time on average; 256 rows took 3 % more in a decode step of 62 experts x 2 rows).
             uint32_t bn;
             if (dense) bn = d->m <= 256 ? ceil_div(d->m, step) * step : 256;
@@ -408,7 +409,8 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
                 const double per_kb = (halves * (mma > feed ? mma : feed) + 150.0) * (stages < 3 ? 1.5 : 1.0);   // two stages do not cover a load's latency
                 const double kb_per = static_cast<double>(total_kb) / splits;
                 const double waves = splits > 1 || dense ? ceil_div(tiles * splits, workers) : static_cast<double>(tiles) / workers;
-                // a k-block's barriers and copies cost ~450 cycles however narrow the tile (one slab; ~600 for two)
+                // decides only where DG_SWAP=1 pins the family for a dense or batched problem, between pairs, slabs and K ranges: by its
+                // rule every problem has one candidate here
                 const double cost = waves * (kb_per * per_kb + 800.0) + (splits > 1 ? 2500.0 + splits * tile_rows * 8.0 : 0.0);
                 if (!found || cost < best_cost * (1.0 - 1e-9)) {
                     found = true;
@@ -884,7 +886,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     rc = choose_config(&desc, e.accumulate ? 1u : 0u, &cfg, &plan);
     if (rc) return rc;
     const bool swap = plan.swap;
-    // the swapped family runs the same kernel with the operands' roles exchanged: its operand A (UMMA M side) is the weights
+    // the swapped family's kernel takes the operands with their roles exchanged: its operand A (UMMA M side) is the weights
     const dg_lp_operand* ka = swap ? b : a;
     const dg_lp_operand* kb = swap ? a : b;
     const uint32_t ka_rows = swap ? pr.n : pr.m, kb_rows = swap ? pr.m : pr.n;              // per group

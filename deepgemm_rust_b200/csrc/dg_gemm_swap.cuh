@@ -3,9 +3,10 @@
 //
 // What it is for: problems with few activation rows per weight matrix (expert groups of up to a few hundred rows).  The first
 // family pads a group to 128 or 256 rows on UMMA M; here a group of r rows costs r rounded up to 32 columns of tensor work, and
-// every weight byte passes through an SM once per tile of up to 320 rows: above 256 rows a k-step is two UMMAs (256 + the rest)
-// on the same weights.  A group of R rows is cut into ceil(R / BLOCK_N) tiles of about equal height, because a narrow tile is
-// bound by its weight stream and by the issue of its instructions (~450 cycles per 128 bytes of K), not by its tensor time.
+// every weight byte passes through an SM once per tile: above 256 rows (288 by the rule, up to 320 where DG_BLOCK_N asks for it) a
+// k-step is two UMMAs (256 + the rest) on the same weights.  A group of R rows is cut into ceil(R / BLOCK_N) tiles of about equal
+// height, because a narrow tile is bound by its weight stream and by the issue of its instructions (~450 cycles per 128 bytes of
+// K), not by its tensor time.
 //
 // Roles of the 384-thread CTA (one per SM, persistent): warp 0 loads weights, warp 3 activations, warp 2 loads and re-orders the
 // scale words into a ring of its own, warp 1 issues the UMMAs, warps 4-11 are the epilogue: two per TMEM quadrant, taking turns
@@ -19,9 +20,9 @@
 // at acc_stride < block_n: tiles wider than that overlap the other buffer.  The epilogue drains those columns first (buffer 0
 // from its last 32 columns down, buffer 1 upwards) and reports them separately, so that the next tile's UMMAs start while the
 // rest is still being stored; narrower tiles never wait.
-// Dense problems with few tiles cut K into ranges, one per CTA (pair): every range writes its f32 accumulator to a workspace in
-// the epilogue's register order, the last range of a tile to arrive (a counter per tile) adds them in range order and stores the
-// tile.  Nobody waits for anybody, the sum does not depend on who is last, and there is no second launch.
+// K ranges, one per CTA (pair), for dense problems where DG_SWAP=1 pins this family (by its rule it gets none): every range writes
+// its f32 accumulator to a workspace in the epilogue's register order, the last range of a tile to arrive (a counter per tile)
+// adds them in range order and stores the tile.  Nobody waits for anybody, the sum does not depend on who is last, and there is no second launch.
 #pragma once
 #include "dg_gemm_kernel.cuh"
 

@@ -149,9 +149,9 @@ int dg_fp8_fp4_bmm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, 
 /* The older f32-scale API (deepgemm/src/ops.rs:328 fp8_gemm_nt_dev, :422 / :535 the grouped variants, :635
  * fp8_bmm_nt_dev), which on Blackwell the reference routes through ops_sm100.rs:1414-1605.  a: e4m3 (rows, a_ld);
  * a_sf_t: the output of dg_transform_sf for a's (rows, k/128) f32 scales; b: e4m3 (num_groups * n, b_ld); sfb:
- * (num_groups * n / 128, k/128) f32 tile scales; out: bf16.  Exactly like the reference's bridge, only the exponent of
- * each f32 scale is used (scales must be powers of two to be exact).  Packed scale words are built in
- * context-owned scratch. */
+ * (num_groups * n / 128, k/128) f32 tile scales; out: bf16.  Every scale is applied exactly, K block by K block, as in
+ * reference.rs:85-208.  With DG_F32_SCALES=exponent in the environment the calls do what the reference's bridge does: only the
+ * exponent of each f32 scale is used (scales must be powers of two to be exact), packed into context-owned scratch. */
 int dg_fp8_gemm_nt(dg_ctx* ctx, const uint8_t* a, uint32_t a_ld, const float* a_sf_t, const uint8_t* b, uint32_t b_ld, const float* sfb, uint32_t m,
                    uint32_t n, uint32_t k, uint16_t* out, uint32_t out_ld);
 int dg_m_grouped_fp8_gemm_nt_contiguous(dg_ctx* ctx, const uint8_t* a, uint32_t a_ld, const float* a_sf_t, const uint8_t* b, uint32_t b_ld,
