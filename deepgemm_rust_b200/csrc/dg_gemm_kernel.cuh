@@ -83,6 +83,7 @@ struct GemmParams {
     uint32_t acc_stride;       // TMEM column where the second accumulator starts (below block_n: the two share columns)
     uint32_t acc_edge_chunks;  // 32-column chunks that hold the shared columns
     float* splitk_ws;          // K ranges: f32 accumulators, one per tile, CTA of the pair and range
+    uint32_t table_groups;     // groups whose rows and tiles are copied to shared memory (16 bytes each); the others are read where they are used
     uint32_t* splitk_counters; // K ranges that have arrived, per tile and CTA of the pair; zero between launches
     const uint32_t* grouped_layout;  // contiguous: end row of each group; masked: valid rows per group
     uint32_t* sfd;

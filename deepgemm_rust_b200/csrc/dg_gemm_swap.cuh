@@ -49,6 +49,7 @@ struct SwapScheduler {
     bool grouped;
     uint32_t step, tile_m, worker, num_workers, num_m_blocks, total_kb, iter;
     uint32_t cur_group, cum_begin, row_start, rows, tile_rows, num_tiles;
+    const uint4* table;      // shared memory: (row_start, rows, num_tiles, tile_rows) of the first table_groups groups
 
     DG_DEVICE SwapScheduler(const GemmParams& params, uint32_t ctas, uint32_t block_k_elems) : p(params) {
         tile_m = kBlockM * ctas;
@@ -60,12 +61,16 @@ struct SwapScheduler {
         cur_group = 0;
         cum_begin = 0;
         row_start = 0;
+        table = nullptr;
         grouped = p.gemm_type == kGemmContiguous || p.gemm_type == kGemmMasked;
         step = grouped ? 32 : 16 * ctas;
         if (!grouped) set_rows(p.n);
     }
-    // What needs global memory: call once, after griddep_wait().  The constructor belongs before it, where its time is hidden.
-    DG_DEVICE void start() { if (grouped) load_group(); }
+    // What needs the group table: call once, after open_groups().  The constructor belongs before it, where its time is hidden.
+    DG_DEVICE void start(const uint4* group_table) {
+        table = group_table;
+        if (grouped) load_group();
+    }
     DG_DEVICE void set_rows(uint32_t r) {
         // tiles of one range of rows meet at multiples of 32 rows (16 for BLOCK_N = 16)
         rows = r;
@@ -73,17 +78,29 @@ struct SwapScheduler {
         num_tiles = r <= p.block_n ? (r != 0 ? 1u : 0u) : (r + most - 1) / most;
         tile_rows = num_tiles > 1 ? ((r + num_tiles - 1) / num_tiles + grid - 1) / grid * grid : r;
     }
-    DG_DEVICE void load_group() {
-        if (cur_group >= p.num_groups) return;
+    // rows and tiles of a group, from global memory
+    DG_DEVICE void read_group(uint32_t g) {
         if (p.gemm_type == kGemmContiguous) {
-            const uint32_t prev_end = cur_group == 0 ? 0u : ld_ro(p.grouped_layout + cur_group - 1);
-            uint32_t end = ld_ro(p.grouped_layout + cur_group);
+            const uint32_t prev_end = g == 0 ? 0u : ld_ro(p.grouped_layout + g - 1);
+            uint32_t end = ld_ro(p.grouped_layout + g);
             end = end < p.n ? end : p.n;
             row_start = (prev_end + p.mk_alignment - 1) / p.mk_alignment * p.mk_alignment;
             set_rows(end > row_start ? end - row_start : 0u);
         } else {
-            const int32_t valid = static_cast<int32_t>(ld_ro(p.grouped_layout + cur_group));
+            const int32_t valid = static_cast<int32_t>(ld_ro(p.grouped_layout + g));
             set_rows(valid <= 0 ? 0u : (static_cast<uint32_t>(valid) < p.n ? static_cast<uint32_t>(valid) : p.n));
+        }
+    }
+    DG_DEVICE void load_group() {
+        if (cur_group >= p.num_groups) return;
+        if (cur_group < p.table_groups) {
+            const uint4 x = table[cur_group];
+            row_start = x.x;
+            rows = x.y;
+            num_tiles = x.z;
+            tile_rows = x.w;
+        } else {
+            read_group(cur_group);
         }
     }
     DG_DEVICE bool next(SwapTile& t) {
@@ -214,9 +231,11 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     uint64_t* bar_tmem_empty = bar_tmem_full + 2;
     uint64_t* bar_tmem_edge = bar_tmem_full + 4;     // the columns shared with the other accumulator are in registers
     uint64_t* bar_tc = bar_tmem_full + 6;            // the UMMAs of a k-block finished (only with a duty cycle below 100 %)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tmem_full + 7);
+    uint64_t* bar_table = bar_tmem_full + 7;         // the group table is in shared memory
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tmem_full + 8);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     volatile uint32_t* last_flag = tmem_slot + 2;
+    uint4* const group_table = reinterpret_cast<uint4*>((reinterpret_cast<uintptr_t>(tmem_slot + 3) + 15) & ~uintptr_t(15));
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < num_stages; ++s) {
@@ -236,6 +255,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             mbar_init(bar_tmem_edge + e, kSwapEpiWarps * kCtas);
         }
         mbar_init(bar_tc, 1);
+        mbar_init(bar_table, kSwapEpiWarps);
         *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&tmap_a);
@@ -256,6 +276,14 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     // Every role waits for the previous kernel itself, after what it can do without global memory: its first instructions have to
     // come from memory too, ~1000 cycles that pass while that kernel still runs.
     griddep_launch_dependents();
+    // Grouped layouts: the epilogue warps, which have nothing to do yet, bring the groups' rows and tiles into shared memory.  Every
+    // role walks the groups one after the other, two to five of them between two tiles; fetched from global memory (~700 cycles each)
+    // they stopped the weight loads for that long, where a tile of 16 k-blocks takes 9000 cycles (64 masked groups of up to 64 rows,
+    // 2048 x 2048: 62.4 -> 59.4 us; contiguous 64 x 128 rows, 4096 x 3584: 227 -> 216).
+    auto groups_ready = [&]() {
+        griddep_wait();
+        return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x700);
+    };
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_sfa = tmem_base + p.acc_stride + block_n;
     const uint32_t tmem_sfb = tmem_sfa + 4 * plan_a.words;
@@ -271,8 +299,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint64_t policy = p.stream_a ? l2_policy_evict_first() : l2_policy_evict_normal();
             const uint32_t tx = (a_bytes >> p.tx_shift_a) * kCtas;
             const bool expects = cta_rank == 0, wide = p.wide_k != 0;
-            griddep_wait();
-            sched.start();
+            ok = groups_ready();
+            sched.start(group_table);
             while (ok && sched.next(t)) {
                 const int32_t row = static_cast<int32_t>(t.m0 + cta_rank * kBlockM), g = static_cast<int32_t>(t.ga);
                 for (uint32_t kb = t.kb0; kb < t.kb1; ++kb) {
@@ -311,8 +339,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t part_rows = swap_part_rows(main_rows);
             const bool expects = cta_rank == 0, wide = p.wide_k != 0;
             constexpr uint32_t kTailBytes = kSwapTailRows * kBlockKBytes;
-            griddep_wait();
-            sched.start();
+            ok = groups_ready();
+            sched.start(group_table);
             while (ok && sched.next(t)) {
                 // a pair's UMMA takes the first half of its N rows from rank 0 and the second half from rank 1
                 const uint32_t n_main = t.n < 256 ? t.n : 256u, my_rows = n_main / kCtas, my_tail = (t.n - n_main) / kCtas;
@@ -376,8 +404,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t sfa_slab = kMXF4 ? 8u : (per128_a ? 0u : 4u), sfb_slab = kMXF4 ? 8u * per_word : (per128_b ? 0u : 4u * per_word);
             const uint32_t sfa_cols[2] = {tmem_sfa, tmem_sfa + sfa_slab}, sfb_cols[2] = {tmem_sfb, tmem_sfb + sfb_slab};
             const bool throttled = p.tc_util < 100;
-            griddep_wait();
-            sched.start();
+            ok = __all_sync(0xFFFFFFFFu, groups_ready());
+            sched.start(group_table);
             while (ok && sched.next(t)) {
                 const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
                 if (!mbar_wait_warp(bar_tmem_empty + e, acc_phase ^ 1, abort_flag, p.status, 0x200 + e)) break;
@@ -493,14 +521,13 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             };
             auto needs = [&](const Walk& w, const SfPlan& plan) { return (w.kb & (plan.period - 1)) == 0 || w.kb == w.t.kb0; };
             Walk ahead{SwapScheduler(p, kCtas, kBlockKElems)};
-            griddep_wait();
-            ahead.sched.start();
+            bool ok = __all_sync(0xFFFFFFFFu, groups_ready());
+            ahead.sched.start(group_table);
             start(ahead);
             Walk here = ahead;
             uint32_t in_slot = 0, in_phase = 0, out_slot = 0, out_phase = 0, in_flight = 0;
             uint32_t stage = 0, phase = 0;      // of the k-block `here`
             const bool leader_lane = elect_one();
-            bool ok = true;
             while (ok && here.live) {
                 while (ahead.live && in_flight < kSwapSfSlots - 1) {      // a free slot never holds up words that have landed
                     if (!mbar_wait_warp(bar_sf_empty + in_slot, in_phase ^ 1, abort_flag, p.status, 0x400 + in_slot)) { ok = false; break; }
@@ -564,9 +591,17 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         SwapScheduler sched(p, kCtas, kBlockKElems);
         SwapTile t;
         uint32_t it = 0;
-        bool ok = true;
-        griddep_wait();
-        sched.start();
+        if (p.table_groups != 0) {
+            griddep_wait();
+            for (uint32_t g = threadIdx.x - 128; g < p.table_groups; g += kSwapEpiWarps * 32) {
+                sched.read_group(g);
+                group_table[g] = make_uint4(sched.row_start, sched.rows, sched.num_tiles, sched.tile_rows);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_table);
+        }
+        bool ok = groups_ready();
+        sched.start(group_table);
         while (sched.next(t)) {
             const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
             ++it;
@@ -765,12 +800,12 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     }
 }
 
-// Bytes of dynamic shared memory the kernel needs for a configuration (host side).
+// Bytes of dynamic shared memory the kernel needs for a configuration, without the group table (host side).
 inline uint32_t gemm_swap_smem_bytes(uint32_t block_n, uint32_t ctas, uint32_t out_kind, uint32_t stages, uint32_t sfa_words, uint32_t sfb_words, uint32_t halves) {
     const uint32_t sf_block_n = (block_n + 127) / 128 * 128;
     const uint32_t per_stage = halves * (kBlockM + swap_main_rows(block_n, ctas) + swap_tail_rows(block_n, ctas)) * kBlockKBytes;
     return 1024 + stages * per_stage + kSwapEpiWarps * swap_epi_buf_bytes(out_kind) + kSwapSfSlots * (512 * sfa_words + sf_block_n * 4 * sfb_words) +
-           (2 * kMaxStages + 2 * kSwapSfSlots + 7) * 8 + 16;
+           (2 * kMaxStages + 2 * kSwapSfSlots + 8) * 8 + 32;
 }
 // Column where the second accumulator starts.
 inline uint32_t gemm_swap_acc_stride(uint32_t block_n, uint32_t sfa_words, uint32_t sfb_words) {

@@ -820,3 +820,44 @@ def test_grouped_calls_write_the_same_rows_whichever_family_runs(ctx, n, k, fami
         want[start:start + (rows + 31) // 32 * 32] = True
     got = (~torch.isnan(d)).cpu().numpy()
     assert (got == want[:, None]).all()
+
+
+@pytest.mark.parametrize("masked", [True, False])
+def test_swapped_family_with_more_groups_than_its_table_holds(ctx, masked, monkeypatch):
+    # the swapped kernel keeps the rows and tiles of the first groups in what its stages leave of shared memory (room for a few hundred
+    # here) and reads the others from global memory: groups on both sides of that line, empty ones among them
+    pin_family(monkeypatch, "1")
+    groups, n, k, slot = 2000, 128, 512, 16
+    sizes = np.random.default_rng(7).integers(0, slot + 1, groups).astype(np.int32)
+    sizes[[0, 1, groups - 1]] = [slot, 0, 3]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def operand(rows, g):
+        x = torch.randn((rows, k), generator=gen, device="cuda", dtype=torch.bfloat16)
+        return dg.cast_bf16_to_fp8_sf_dev(ctx, x, k, rows, k, 128, g)
+    (aq, asf), (bq, bsf) = operand(groups * slot, groups if masked else 1), operand(groups * n, groups)
+    d = torch.full((groups * slot, n), float("nan"), dtype=torch.float32, device="cuda")
+    b_op, out = dg.LpOperand(bq, bsf, groups * n, k, k), dg.Sm100Out.F32(d, n)
+    if masked:
+        dg.m_grouped_fp8_fp4_gemm_masked_dev(ctx, dg.LpOperand(aq, asf, slot, k, k), dev(sizes), b_op, out, groups, slot // 2)
+    else:
+        previous = dg.get_mk_alignment_for_contiguous_layout()
+        dg.set_mk_alignment_for_contiguous_layout(16)
+        try:
+            ends = dev((np.arange(groups) * slot + sizes).astype(np.int32))
+            dg.m_grouped_fp8_fp4_gemm_contiguous_ends_dev(ctx, dg.LpOperand(aq, asf, groups * slot, k, k), ends, b_op, out, groups)
+        finally:
+            dg.set_mk_alignment_for_contiguous_layout(previous)
+    ctx.sync()
+    dn = to_f32(d)
+    aq, asf, bq, bsf = (t.cpu().numpy() for t in (aq, asf, bq, bsf))
+    asf, bsf = asf.view(np.uint32), bsf.view(np.uint32)
+    for g in (0, 2, 300, 500, 501, 700, 1000, groups - 2, groups - 1):
+        v = int(sizes[g])
+        rows = np.arange(g * slot, g * slot + v, dtype=np.uint32)
+        if v:
+            want = O.lp_gemm_rows(aq, asf, 8, 128, groups if masked else 1, slot if masked else groups * slot, rows, bq, bsf, 8, 128, groups, n,
+                                  np.arange(g * n, (g + 1) * n, dtype=np.uint32), k)
+            assert O.calc_diff(dn[rows], want) <= TIGHT_F32
+    valid = np.concatenate([np.arange(g * slot, g * slot + sizes[g]) for g in range(groups)]).astype(np.int64)
+    assert not np.isnan(dn[valid]).any()
