@@ -1762,6 +1762,21 @@ int dg_ep_layout(dg_ctx* ctx, const uint32_t* all_counts, uint32_t world, uint32
     return DG_OK;
 }
 
+// Pieces a row of `steps` warp loads is cut into, one warp each: of seven loads where that gives enough warps, of fewer down to one
+// where it does not.  Seven: 8192 rows of 7168 columns combine in 219 us with pieces of 7 loads, 224 with 4, 226 with 14; dispatch 96, 100
+// and 98.
+static uint32_t row_segments(uint32_t rows, uint32_t steps, uint64_t enough) {
+    if (steps == 0) return 1;
+    uint32_t per = 7;
+    while (per > 1 && static_cast<uint64_t>(rows) * ceil_div(steps, per) < enough) --per;
+    return ceil_div(steps, per);
+}
+// Eight pieces per block, those of a row next to each other; max_blocks (0: no bound) bounds the grid.
+static uint32_t piece_blocks(uint32_t rows, uint32_t segments, uint32_t max_blocks) {
+    const uint32_t blocks = static_cast<uint32_t>((static_cast<uint64_t>(rows) * segments + 7) / 8);
+    return max_blocks != 0 && blocks > max_blocks ? max_blocks : blocks;
+}
+
 int dg_ep_dispatch(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* local_rank, const uint32_t* block_base, const uint32_t* pair_base,
                    uint32_t pairs, uint32_t topk, uint32_t num_experts, uint32_t world, const uint8_t* data, uint32_t k, const uint32_t* sf,
                    uint32_t sf_stride, uint32_t sf_cols, void* const* peer_data, void* const* peer_sf, uint32_t peer_sf_stride,
@@ -1781,9 +1796,8 @@ int dg_ep_dispatch(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* lo
     p.pairs = pairs; p.topk = topk; p.k = k; p.sf_cols = sf_cols; p.sf_stride = sf_stride; p.peer_sf_stride = peer_sf_stride;
     p.num_experts = num_experts; p.experts_per_rank = num_experts / world; p.capacity = capacity; p.slot_rows = slot_rows;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    uint32_t blocks = ceil_div(pairs, 8);
-    if (max_blocks != 0 && blocks > max_blocks) blocks = max_blocks;
-    DG_CUDA(launch(dg::dg_ep_dispatch_kernel, blocks, 256, 0, ctx->stream, p));
+    p.segments = row_segments(pairs / topk, ceil_div(k, 512), 4ull * ctx->num_sms);
+    DG_CUDA(launch(dg::dg_ep_dispatch_kernel, piece_blocks(pairs / topk, p.segments, max_blocks), 256, 0, ctx->stream, p));
     return DG_OK;
 }
 
@@ -1800,11 +1814,9 @@ int dg_ep_combine(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* pos
     p.out = out; p.pitch = pitch; p.out_pitch = out_pitch;
     p.tokens = tokens; p.topk = topk; p.n = n; p.experts_per_rank = num_experts / world;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    const uint64_t threads = static_cast<uint64_t>(tokens) * (n / 8);
-    if (threads > 0xFFFFFF00ull) return fail(DG_ERR_SHAPE, "tokens x n / 8 must fit 32 bits");
-    uint32_t blocks = static_cast<uint32_t>((threads + 255) / 256);
-    if (max_blocks != 0 && blocks > max_blocks) blocks = max_blocks;
-    DG_CUDA(launch(dg::dg_ep_combine_kernel, blocks, 256, 0, ctx->stream, p));
+    if (static_cast<uint64_t>(tokens) * (n / 8) > 0xFFFFFF00ull) return fail(DG_ERR_SHAPE, "tokens x n / 8 must fit 32 bits");
+    p.segments = row_segments(tokens, ceil_div(n, 256), 32ull * ctx->num_sms);
+    DG_CUDA(launch(dg::dg_ep_combine_kernel, piece_blocks(tokens, p.segments, max_blocks), 256, 0, ctx->stream, p));
     return DG_OK;
 }
 

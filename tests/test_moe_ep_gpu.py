@@ -366,3 +366,39 @@ def test_peer_exchange_refuses_a_context_on_another_stream():
     finally:
         pe.close()
         own.close()
+
+
+@pytest.mark.parametrize("tokens,topk,hidden,n,max_blocks", [
+    (1, 1, 512, 8, 0),                # one warp load per row, one column chunk
+    (5, 9, 7680, 264, 0),             # 15 loads per row and 2 chunk steps, the last one ragged; a second look-up of result rows
+    (40, 33, 1024, 2056, 3),          # a second look-up of arena rows; warps that stride over the work
+    (5000, 8, 4096, 2304, 0),         # rows cut into pieces of several loads
+])
+def test_peer_exchange_row_pieces(ctx, tokens, topk, hidden, n, max_blocks):
+    # dispatch and combine cut rows into pieces, one warp each: rows, scale words and sums bit for bit, whatever the cut
+    experts = 40
+    rng = np.random.default_rng(tokens)
+    topi = np.stack([rng.permutation(experts)[:topk] for _ in range(tokens)]).astype(np.int32)
+    topi[rng.random(topi.shape) < 0.1] = -1                           # dropped pairs
+    topw = rng.random((tokens, topk), dtype=np.float32)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, hidden), generator=gen, device="cuda", dtype=torch.bfloat16)
+    xq, xsf = dg.cast_bf16_to_fp8_sf_dev(ctx, x, hidden, tokens, hidden, 128)
+    pe = PeerExpertParallel(ctx, experts, topk, tokens, hidden, n)
+    try:
+        pe.max_blocks = max_blocks
+        pe.result.copy_(torch.randn(pe.result.shape, generator=gen, device="cuda", dtype=torch.bfloat16))
+        pe.dispatch(dev(topi), xq, xsf)
+        out = pe.combine(dev(topw))
+        ctx.sync()
+        pos, _, _ = arena_layout(topi.reshape(-1), experts)
+        assert np.array_equal(pe.pos_of_pair.cpu().numpy()[:pos.size], pos)
+        live = torch.from_numpy(np.nonzero(pos >= 0)[0]).cuda()
+        rows = torch.from_numpy(pos).cuda()[live]
+        assert torch.equal(pe.arena[rows], xq[live // topk])
+        assert torch.equal(pe.arena_sf.view(pe.sf_cols, pe.sf_stride)[:, rows], xsf.view(pe.sf_cols, -1)[:, live // topk])
+        y_bits = pe.result.view(torch.int16).cpu().numpy().view(np.uint16)
+        want = O.moe_combine(y_bits, pos.reshape(tokens, topk).astype(np.int32), topw)
+        assert np.array_equal(out.view(torch.int16).cpu().numpy().view(np.uint16), want)
+    finally:
+        pe.close()
