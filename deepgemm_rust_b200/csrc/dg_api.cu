@@ -1097,6 +1097,12 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         grid = plan.tiles * splits * ctas < grid ? plan.tiles * splits * ctas : grid;
     const int kernel_out = splits > 1 && !swap ? DG_OUT_F32 : out->kind;
     const uint32_t smem = plan.smem;
+    if (!swap && (pr.type == DG_GEMM_NORMAL || pr.type == DG_GEMM_BATCHED) && kernel_out == DG_OUT_F32 &&
+        static_cast<uint64_t>(plan.tiles) * splits <= static_cast<uint32_t>(ctx->num_sms) / ctas) {
+        // one tile per CTA (pair): does the operand ring hold the CTA's 128 rows of it?
+        const uint32_t ring = plan.stages * plan.halves * (dg::kBlockM + plan.umma_n / ctas) * dg::kBlockKBytes;
+        p.stage_in_ring = dg::kBlockM * plan.umma_n * 4 <= ring ? 1 : 0;
+    }
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     cudaError_t ce;
     if (swap) {

@@ -861,3 +861,18 @@ def test_swapped_family_with_more_groups_than_its_table_holds(ctx, masked, monke
             assert O.calc_diff(dn[rows], want) <= TIGHT_F32
     valid = np.concatenate([np.arange(g * slot, g * slot + sizes[g]) for g in range(groups)]).astype(np.int64)
     assert not np.isnan(dn[valid]).any()
+
+
+@pytest.mark.parametrize("m,n", [(128, 256), (200, 500), (77, 36)])
+@pytest.mark.parametrize("ctas,block_n,stages", [
+    (1, 256, 2), (1, 256, 3),      # the operand ring is too small for the tile's f32 outputs, and just holds them
+    (2, 256, 3), (2, 256, 4),      # (four stages: to the byte)
+    (1, 32, 4), (2, 96, 3),
+])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_dense_f32_staged_in_the_operand_ring(ctx, m, n, ctas, block_n, stages, splits, monkeypatch):
+    # one tile per CTA and f32 outputs (a K range's partial sums too): they are staged where the operands were, if they fit
+    pin_family(monkeypatch, "0")
+    for name, value in (("DG_CTAS", ctas), ("DG_BLOCK_N", block_n), ("DG_STAGES", stages), ("DG_K_SLABS", 1), ("DG_SPLITS", splits)):
+        monkeypatch.setenv(name, str(value))
+    run_dense(ctx, m, n, 2048, out_kind=1, alpha=0.5, seed=m, b_tile_scales=False)
