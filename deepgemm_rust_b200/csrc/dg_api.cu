@@ -1032,7 +1032,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         p.acc_stride = dg::gemm_swap_acc_stride(plan.umma_n, sfa_words, sfb_words);
         p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
         if (p.acc_stride == plan.umma_n) p.acc_edge_chunks = 0;
-        if (pr.type == DG_GEMM_M_GROUPED_CONTIGUOUS || pr.type == DG_GEMM_M_GROUPED_MASKED) {
+        if (dg::swap_has_table(plan.ctas, plan.halves) && (pr.type == DG_GEMM_M_GROUPED_CONTIGUOUS || pr.type == DG_GEMM_M_GROUPED_MASKED)) {
             // the group table takes what the stages leave of the shared memory
             const uint32_t room = (kSmemCapacity - plan.smem) / 16;
             p.table_groups = pr.groups < room ? pr.groups : room;

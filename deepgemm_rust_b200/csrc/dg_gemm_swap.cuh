@@ -43,7 +43,9 @@ struct SwapTile {
     uint32_t index, split;     // output tile and K range
 };
 
-// Walks the tile list of one CTA (pair); every role runs its own copy and sees the same sequence.
+// Walks the tile list of one CTA (pair); every role runs its own copy and sees the same sequence.  kTable: the kernel keeps a table of
+// the groups in shared memory.
+template <bool kTable>
 struct SwapScheduler {
     const GemmParams& p;
     bool grouped;
@@ -61,14 +63,13 @@ struct SwapScheduler {
         cur_group = 0;
         cum_begin = 0;
         row_start = 0;
-        table = nullptr;
         grouped = p.gemm_type == kGemmContiguous || p.gemm_type == kGemmMasked;
         step = grouped ? 32 : 16 * ctas;
         if (!grouped) set_rows(p.n);
     }
     // What needs the group table: call once, after open_groups().  The constructor belongs before it, where its time is hidden.
     DG_DEVICE void start(const uint4* group_table) {
-        table = group_table;
+        if constexpr (kTable) table = group_table;
         if (grouped) load_group();
     }
     DG_DEVICE void set_rows(uint32_t r) {
@@ -93,15 +94,17 @@ struct SwapScheduler {
     }
     DG_DEVICE void load_group() {
         if (cur_group >= p.num_groups) return;
-        if (cur_group < p.table_groups) {
-            const uint4 x = table[cur_group];
-            row_start = x.x;
-            rows = x.y;
-            num_tiles = x.z;
-            tile_rows = x.w;
-        } else {
-            read_group(cur_group);
+        if constexpr (kTable) {
+            if (cur_group < p.table_groups) {
+                const uint4 x = table[cur_group];
+                row_start = x.x;
+                rows = x.y;
+                num_tiles = x.z;
+                tile_rows = x.w;
+                return;
+            }
         }
+        read_group(cur_group);
     }
     DG_DEVICE bool next(SwapTile& t) {
         uint32_t idx = worker + (iter++) * num_workers;
@@ -181,6 +184,10 @@ DG_DEVICE uint64_t desc64(uint32_t lo, uint32_t hi) { return static_cast<uint64_
 // staging bytes of one epilogue warp: 32 output rows x 32 columns (f32 goes out straight from registers)
 constexpr uint32_t swap_epi_buf_bytes(uint32_t out_kind) { return out_kind == kOutF32 ? 0u : 2048u; }
 
+// Kernels with a group table: the form that the grouped layouts get by the rule.  In the others, which the dense problems get, its code
+// costs 2 % (5 x 17888 x 9216: 31.0 -> 31.8 us).
+__host__ __device__ constexpr bool swap_has_table(uint32_t ctas, uint32_t halves) { return ctas == 2 && halves == 1; }
+
 // Activation rows of a stage, per CTA and slab: the first 256 rows of a tile, and the rows beyond.
 __host__ __device__ inline uint32_t swap_main_rows(uint32_t block_n, uint32_t ctas) { return (block_n < 256 ? block_n : 256) / ctas; }
 __host__ __device__ inline uint32_t swap_tail_rows(uint32_t block_n, uint32_t ctas) {
@@ -199,6 +206,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     constexpr bool kMXF4 = kFmt == kFmtMxf4, kScaled = kFmt != kFmtBf16;
     constexpr uint32_t kHalfElems = kMXF4 ? 256 : 128;      // K elements of one 128-byte slab
     constexpr uint32_t kBlockKElems = kHalves * kHalfElems;
+    constexpr bool kTable = swap_has_table(kCtas, kHalves);
+    using Scheduler = SwapScheduler<kTable>;
     constexpr uint32_t kEpiBufBytes = swap_epi_buf_bytes(kOut);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -282,7 +291,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     // 2048 x 2048: 62.4 -> 59.4 us; contiguous 64 x 128 rows, 4096 x 3584: 227 -> 216).
     auto groups_ready = [&]() {
         griddep_wait();
-        return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x700);
+        if constexpr (kTable) return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x700);
+        else return true;
     };
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_sfa = tmem_base + p.acc_stride + block_n;
@@ -291,7 +301,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     if (warp == 0) {
         // ------------------------------------------------------------ weights: one lane, one or two loads per stage
         if (elect_one()) {
-            SwapScheduler sched(p, kCtas, kBlockKElems);
+            Scheduler sched(p, kCtas, kBlockKElems);
             SwapTile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
@@ -331,7 +341,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         // ------------------------------------------------------------ activations: few large boxes, even where a tile needs fewer rows
         // (a load costs its issuing lane ~70 cycles whatever its size)
         if (elect_one()) {
-            SwapScheduler sched(p, kCtas, kBlockKElems);
+            Scheduler sched(p, kCtas, kBlockKElems);
             SwapTile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
@@ -385,7 +395,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     } else if (warp == 1) {
         // ------------------------------------------------------------- UMMA issuer
         if (cta_rank == 0) {
-            SwapScheduler sched(p, kCtas, kBlockKElems);
+            Scheduler sched(p, kCtas, kBlockKElems);
             SwapTile t;
             uint32_t stage = 0, phase = 0, it = 0, tc_phase = 0, prev_n = 0, slot = 0;
             bool ok = true;
@@ -404,7 +414,8 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
             const uint32_t sfa_slab = kMXF4 ? 8u : (per128_a ? 0u : 4u), sfb_slab = kMXF4 ? 8u * per_word : (per128_b ? 0u : 4u * per_word);
             const uint32_t sfa_cols[2] = {tmem_sfa, tmem_sfa + sfa_slab}, sfb_cols[2] = {tmem_sfb, tmem_sfb + sfb_slab};
             const bool throttled = p.tc_util < 100;
-            ok = __all_sync(0xFFFFFFFFu, groups_ready());
+            ok = groups_ready();
+            if constexpr (kTable) ok = __all_sync(0xFFFFFFFFu, ok);
             sched.start(group_table);
             while (ok && sched.next(t)) {
                 const uint32_t e = it & 1, acc_phase = (it >> 1) & 1;
@@ -509,7 +520,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         if constexpr (kScaled) {
             // walks the k-blocks that need new words: `ahead` issues loads, `here` re-orders what landed
             struct Walk {
-                SwapScheduler sched;
+                Scheduler sched;
                 SwapTile t;
                 uint32_t kb;
                 bool live;
@@ -520,8 +531,9 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                 if (w.kb >= w.t.kb1) start(w);
             };
             auto needs = [&](const Walk& w, const SfPlan& plan) { return (w.kb & (plan.period - 1)) == 0 || w.kb == w.t.kb0; };
-            Walk ahead{SwapScheduler(p, kCtas, kBlockKElems)};
-            bool ok = __all_sync(0xFFFFFFFFu, groups_ready());
+            Walk ahead{Scheduler(p, kCtas, kBlockKElems)};
+            bool ok = groups_ready();
+            if constexpr (kTable) ok = __all_sync(0xFFFFFFFFu, ok);
             ahead.sched.start(group_table);
             start(ahead);
             Walk here = ahead;
@@ -588,17 +600,19 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
         // ------------------------------------------------------------------ epilogue
         const uint32_t ew = warp % 4, half = (warp - 4) / 4;      // TMEM lane quadrant: 32 output columns; which of its two warps
         uint8_t* const buf = smem_epi + (warp - 4) * kEpiBufBytes;
-        SwapScheduler sched(p, kCtas, kBlockKElems);
+        Scheduler sched(p, kCtas, kBlockKElems);
         SwapTile t;
         uint32_t it = 0;
-        if (p.table_groups != 0) {
-            griddep_wait();
-            for (uint32_t g = threadIdx.x - 128; g < p.table_groups; g += kSwapEpiWarps * 32) {
-                sched.read_group(g);
-                group_table[g] = make_uint4(sched.row_start, sched.rows, sched.num_tiles, sched.tile_rows);
+        if constexpr (kTable) {
+            if (p.table_groups != 0) {
+                griddep_wait();
+                for (uint32_t g = threadIdx.x - 128; g < p.table_groups; g += kSwapEpiWarps * 32) {
+                    sched.read_group(g);
+                    group_table[g] = make_uint4(sched.row_start, sched.rows, sched.num_tiles, sched.tile_rows);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_table);
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_table);
         }
         bool ok = groups_ready();
         sched.start(group_table);
