@@ -25,6 +25,7 @@
 // adds them in range order and stores the tile.  Nobody waits for anybody, the sum does not depend on who is last, and there is no second launch.
 #pragma once
 #include "dg_gemm_kernel.cuh"
+#include "dg_ring.cuh"
 
 namespace dg {
 
@@ -216,8 +217,10 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     const uint32_t cta_rank = kCtas == 2 ? cluster_cta_rank() : 0u;
     const uint32_t block_n = p.block_n;
     const uint32_t sf_block_n = (block_n + 127) / 128 * 128;
-    const SfPlan plan_a = sf_plan(p.gran_a, kBlockKElems), plan_b = sf_plan(p.gran_b, kBlockKElems);
-    const uint32_t sf_period = plan_a.period < plan_b.period ? plan_a.period : plan_b.period;      // k-blocks between two loads of scale words
+    SfPlan plan_a = sf_plan(p.gran_a, kBlockKElems), plan_b = sf_plan(p.gran_b, kBlockKElems);
+    const uint32_t new_words = plan_a.period < plan_b.period ? plan_a.period : plan_b.period;
+    const uint32_t sf_period = scale_period(p.num_stages, new_words);      // k-blocks between two loads of scale words
+    if (sf_period != new_words) plan_a.period = plan_b.period = sf_period;
     const uint32_t sfa_bytes = 512 * plan_a.words, sfb_bytes = sf_block_n * 4 * plan_b.words;
     const uint32_t main_rows = swap_main_rows(block_n, kCtas), tail_rows = swap_tail_rows(block_n, kCtas);
     constexpr uint32_t a_half = kBlockM * kBlockKBytes, a_bytes = a_half * kHalves;

@@ -876,3 +876,41 @@ def test_dense_f32_staged_in_the_operand_ring(ctx, m, n, ctas, block_n, stages, 
     for name, value in (("DG_CTAS", ctas), ("DG_BLOCK_N", block_n), ("DG_STAGES", stages), ("DG_K_SLABS", 1), ("DG_SPLITS", splits)):
         monkeypatch.setenv(name, str(value))
     run_dense(ctx, m, n, 2048, out_kind=1, alpha=0.5, seed=m, b_tile_scales=False)
+
+
+@pytest.mark.parametrize("ctas", [1, 2])
+@pytest.mark.parametrize("stages,slabs", [(1, 1), (2, 1), (3, 1), (1, 2)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_swapped_family_with_fewer_stages_than_a_scale_word_has_k_blocks(ctx, stages, slabs, ctas, splits, monkeypatch):
+    # a short ring: scale words are fetched for every k-block (tests/test_operand_ring_cpu.py plays the protocol); K ranges may start
+    # inside a scale word
+    pin_family(monkeypatch, "1")
+    for name, value in (("DG_CTAS", ctas), ("DG_STAGES", stages), ("DG_K_SLABS", slabs), ("DG_SPLITS", splits), ("DG_BLOCK_N", 96)):
+        monkeypatch.setenv(name, str(value))
+    cfg = dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, 90, 1000, 4736))
+    assert cfg.swap_ab and cfg.num_stages == stages and cfg.block_k == 128 * slabs
+    run_dense(ctx, 90, 1000, 4736, seed=stages)
+    run_dense(ctx, 200, 520, 4736, out_kind=1, seed=stages)
+
+
+@pytest.mark.parametrize("block_n", [288, 320])
+def test_swapped_single_cta_tiles_whose_ring_has_three_stages(ctx, block_n, monkeypatch):
+    pin_family(monkeypatch, "1")
+    monkeypatch.setenv("DG_CTAS", "1")
+    monkeypatch.setenv("DG_BLOCK_N", str(block_n))
+    sizes, n, k = [320, 1, 0, 289, 256], 1000, 3712
+    m_idx = np.concatenate([np.r_[np.full(s, g, np.int32), np.full((-s) % 128, -1, np.int32)] for g, s in enumerate(sizes)])
+    m_total, groups = len(m_idx), len(sizes)
+    cfg = dg.best_config(dg.Sm100Desc(dg.GemmType.MGroupedContiguous, m_total, n, k, groups))
+    assert cfg.swap_ab and cfg.num_stages == 3 and cfg.block_m == block_n and cfg.block_k == 128
+    _, aq, asf = fp8_operand_1d(m_total, k, 401)
+    _, bq, bsf = fp8_operand_1d(groups * n, k, 402, 128, groups)
+    d = torch.full((m_total, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dg.m_grouped_fp8_fp4_gemm_contiguous_dev(ctx, lp(aq, asf, m_total, k), dev(m_idx), lp(bq, bsf, groups * n, k), dg.Sm100Out.Bf16(d, n), groups)
+    ctx.sync()
+    got = to_f32(d)
+    for g, s in enumerate(sizes):
+        if s:
+            rows = np.nonzero(m_idx == g)[0].astype(np.uint32)
+            check_sampled(got, None, (aq, asf, 8, 128, 1, m_total), None, (bq, bsf, 8, 128, groups, n), k, rows,
+                          np.arange(g * n, (g + 1) * n, dtype=np.uint32), TIGHT_BF16)
