@@ -1769,17 +1769,16 @@ int dg_ep_layout(dg_ctx* ctx, const uint32_t* all_counts, uint32_t world, uint32
 }
 
 // Pieces a row of `steps` warp loads is cut into, one warp each: of seven loads where that gives enough warps, of fewer down to one
-// where it does not.  Seven: 8192 rows of 7168 columns combine in 219 us with pieces of 7 loads, 224 with 4, 226 with 14; dispatch 96, 100
-// and 98.
+// where it does not.  (8192 rows of 7168 columns: combine takes 219 us with pieces of 7 loads, 224 with 4, 226 with 14.)
 static uint32_t row_segments(uint32_t rows, uint32_t steps, uint64_t enough) {
     if (steps == 0) return 1;
-    uint32_t per = 7;
+    uint32_t per = dg::kEpPieceLoads;
     while (per > 1 && static_cast<uint64_t>(rows) * ceil_div(steps, per) < enough) --per;
     return ceil_div(steps, per);
 }
 // Eight pieces per block, those of a row next to each other; max_blocks (0: no bound) bounds the grid.
-static uint32_t piece_blocks(uint32_t rows, uint32_t segments, uint32_t max_blocks) {
-    const uint32_t blocks = static_cast<uint32_t>((static_cast<uint64_t>(rows) * segments + 7) / 8);
+static uint32_t piece_blocks(uint64_t pieces, uint32_t max_blocks) {
+    const uint32_t blocks = static_cast<uint32_t>((pieces + 7) / 8);
     return max_blocks != 0 && blocks > max_blocks ? max_blocks : blocks;
 }
 
@@ -1802,8 +1801,30 @@ int dg_ep_dispatch(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* lo
     p.pairs = pairs; p.topk = topk; p.k = k; p.sf_cols = sf_cols; p.sf_stride = sf_stride; p.peer_sf_stride = peer_sf_stride;
     p.num_experts = num_experts; p.experts_per_rank = num_experts / world; p.capacity = capacity; p.slot_rows = slot_rows;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
-    p.segments = row_segments(pairs / topk, ceil_div(k, 512), 4ull * ctx->num_sms);
-    DG_CUDA(launch(dg::dg_ep_dispatch_kernel, piece_blocks(pairs / topk, p.segments, max_blocks), 256, 0, ctx->stream, p));
+    // A warp per pair and piece while that makes at most 14 warps per SM, pieces as short as 7 warps per SM allow (top-8, both ways of work
+    // side by side: 128 tokens of 2048 / 4096 / 5120 / 7168 bytes 2.56 / 2.96 / 3.15 / 3.47 us against 3.13 / 3.20 / 3.38 / 3.41 with a
+    // warp per token and piece; 256 tokens of 4096 / 5120 / 7168 bytes 3.73 / 4.06 / 4.86 against 3.57 / 3.89 / 4.59; with top-1 and
+    // top-2 within 4 % of each other).  Beyond, pieces of seven loads where they make six warps per SM, else shorter ones (256 tokens of
+    // 7168 bytes: four pieces 4.59 us, three 5.23, two 6.66; 512 of 2048 bytes: two 3.53, one 4.61).
+    const uint32_t loads = k == 0 ? 1 : ceil_div(k, 512), tokens = pairs / topk, sms = static_cast<uint32_t>(ctx->num_sms);
+    if (static_cast<uint64_t>(pairs) * ceil_div(loads, dg::kEpPieceLoads) <= 14ull * sms) {
+        p.piece_loads = dg::kEpPieceLoads;
+        while (p.piece_loads > 1 && static_cast<uint64_t>(pairs) * ceil_div(loads, p.piece_loads - 1) <= 7ull * sms) --p.piece_loads;
+        p.pieces = ceil_div(loads, p.piece_loads);
+        p.piece_loads = ceil_div(loads, p.pieces);
+        dim3 grid(ceil_div(pairs, 8), p.pieces, 1);
+        if (max_blocks != 0) {
+            if (grid.y > max_blocks) grid.y = max_blocks;
+            if (grid.x > max_blocks / grid.y) grid.x = max_blocks / grid.y;
+        }
+        DG_CUDA(launch(dg::dg_ep_dispatch_pairs_kernel, grid, 256, 0, ctx->stream, p));
+        return DG_OK;
+    }
+    p.pieces = row_segments(tokens, loads, 6ull * sms);
+    p.piece_loads = ceil_div(loads, p.pieces);
+    const uint64_t units = static_cast<uint64_t>(tokens) * ceil_div(topk, 32) * p.pieces;
+    if (units > 0xFFFFFFFFull) return fail(DG_ERR_SHAPE, "tokens x pieces of a row must fit 32 bits");
+    DG_CUDA(launch(dg::dg_ep_dispatch_tokens_kernel, piece_blocks(units, max_blocks), 256, 0, ctx->stream, p));
     return DG_OK;
 }
 
@@ -1822,7 +1843,7 @@ int dg_ep_combine(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* pos
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     if (static_cast<uint64_t>(tokens) * (n / 8) > 0xFFFFFF00ull) return fail(DG_ERR_SHAPE, "tokens x n / 8 must fit 32 bits");
     p.segments = row_segments(tokens, ceil_div(n, 256), 32ull * ctx->num_sms);
-    DG_CUDA(launch(dg::dg_ep_combine_kernel, piece_blocks(tokens, p.segments, max_blocks), 256, 0, ctx->stream, p));
+    DG_CUDA(launch(dg::dg_ep_combine_kernel, piece_blocks(static_cast<uint64_t>(tokens) * p.segments, max_blocks), 256, 0, ctx->stream, p));
     return DG_OK;
 }
 

@@ -241,6 +241,10 @@ __global__ void __launch_bounds__(1024) dg_ep_layout_kernel(const uint32_t* all_
     }
 }
 
+// Warp loads (512 bytes) of a row that one warp of the dispatch holds, at most.  Eight take the per-token kernel from 64 to 76 registers
+// (8192 tokens, top-8: 7168 bytes 93.8 -> 92.7 us, but 2048 bytes 28.9 -> 30.8; 1024 tokens x 7168 bytes 11.8 -> 15.6).
+constexpr uint32_t kEpPieceLoads = 7;
+
 struct EpDispatchParams {
     const int32_t* expert_of_pair;   // (pairs)
     const int32_t* local_rank;       // (pairs)
@@ -252,76 +256,111 @@ struct EpDispatchParams {
     uint32_t* const* peer_sf;        // [world] arena scale words, sf[c * peer_sf_stride + row]
     int32_t* pos_of_pair;            // (pairs) arena row on the owner, -1 if dropped
     uint32_t pairs, topk, k, sf_cols, sf_stride, peer_sf_stride, num_experts, experts_per_rank, capacity;
-    uint32_t segments;               // of a token's row, one warp each
+    uint32_t pieces, piece_loads;    // a token's row is cut into `pieces` of piece_loads warp loads, one warp each
     uint32_t slot_rows;              // masked layout: rows per expert slot (0: contiguous layout); the arena's scale words are then
                                      // laid out per slot, sf[(slot * sf_cols + c) * peer_sf_stride + row in slot]
 };
 
-// One warp per (token, segment of its row): the segment is read once and stored to the arena rows of the token's top-k experts (a warp
-// per pair read every token top-k times from L2 and walked five dependent loads per row).  A lane per expert works out where its
-// copy goes; the whole warp then stores to one row after the other.  Bound by the stores (topk x k bytes per token): 8192 tokens x 7168
-// bytes, top-8: 120 -> 95 us (a decode step's 128 tokens: 4.1 -> 4.8, a few loads per warp).  The grid may be smaller than the work
-// (warps stride over it), which lets a caller leave room on every SM for a kernel running beside this one.
-__global__ void __launch_bounds__(256) dg_ep_dispatch_kernel(const EpDispatchParams p) {
+// Arena row of a pair that has a rank among its expert's pairs, -1 if it does not fit; where its data and scale words go.
+DG_DEVICE int32_t ep_arena_row(const EpDispatchParams& p, uint32_t pair, uint32_t local_rank, uint8_t*& dst, uint32_t*& dst_sf) {
+    const uint32_t e = static_cast<uint32_t>(ld_ro(p.expert_of_pair + pair));
+    const uint32_t row = ld_ro(p.pair_base + e) + ld_ro(p.block_base + static_cast<size_t>(pair / kEpChunk) * p.num_experts + e) + local_rank;
+    const uint32_t owner = e / p.experts_per_rank, slot = e - owner * p.experts_per_rank;
+    const uint32_t in_slot = row - slot * p.slot_rows;      // masked layout only
+    if (row >= p.capacity || (p.slot_rows != 0 && in_slot >= p.slot_rows)) return -1;
+    dst = p.peer_data[owner] + static_cast<size_t>(row) * p.k;
+    dst_sf = p.peer_sf[owner] + (p.slot_rows ? static_cast<size_t>(slot) * p.sf_cols * p.peer_sf_stride + in_slot : row);
+    return static_cast<int32_t>(row);
+}
+
+// Few tokens: one warp per (pair, piece of its token's row); grid.y is the piece.  Bound by the chain of dependent loads that leads to
+// the arena row, beside which the piece is already on its way.  Top-8, 7168-byte rows: 16 tokens 2.1 us, 128 tokens 3.3 (a warp per
+// token's piece, which stores to its experts' rows one after the other: 4.1 and 4.5; a warp per pair with a whole row, fetched after the
+// chain: 3.5 and 3.7); 2048-byte rows 2.0 and 2.4 (3.5 and 3.6; 2.2 and 2.4).
+__global__ void __launch_bounds__(256) dg_ep_dispatch_pairs_kernel(const EpDispatchParams p) {
     griddep_wait();
     griddep_launch_dependents();
-    const uint32_t lane = threadIdx.x % 32;
-    const uint32_t vecs = p.k / 16, per_segment = ((vecs + 31) / 32 + p.segments - 1) / p.segments * 32;      // whole warp loads
-    const uint32_t units = p.pairs / p.topk * p.segments, warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t unit = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; unit < units; unit += warps) {
-        const uint32_t tok = unit / p.segments, segment = unit - tok * p.segments;
-        const uint32_t first = segment * per_segment, end = first + per_segment < vecs ? first + per_segment : vecs;
-        const uint4* src = reinterpret_cast<const uint4*>(p.data + static_cast<size_t>(tok) * p.k);
-        constexpr uint32_t kDeep = 7;          // loads in flight per lane before the first store
-        uint4 v[kDeep];
-        auto fetch = [&](uint32_t c0) {
+    const uint32_t lane = threadIdx.x % 32, vecs = p.k / 16;
+    const uint32_t piece_words = (p.sf_cols + p.pieces - 1) / p.pieces;
+    for (uint64_t at = blockIdx.x * 8 + threadIdx.x / 32; at < p.pairs; at += gridDim.x * 8) {
+        const uint32_t pair = static_cast<uint32_t>(at), tok = pair / p.topk;
+        const int32_t lr = ld_ro(p.local_rank + pair);
+        for (uint32_t piece = blockIdx.y; piece < p.pieces; piece += gridDim.y) {
+            const uint4* src = reinterpret_cast<const uint4*>(p.data + static_cast<size_t>(tok) * p.k);
+            const uint32_t first = piece * p.piece_loads * 32 + lane, past = (piece + 1) * p.piece_loads * 32, end = past < vecs ? past : vecs;
+            const uint32_t word0 = piece * piece_words, words = word0 + piece_words < p.sf_cols ? word0 + piece_words : p.sf_cols;
+            uint4 v[kEpPieceLoads];
             #pragma unroll
-            for (uint32_t i = 0; i < kDeep; ++i)
-                if (c0 + 32 * i + lane < end) v[i] = ld_ro(src + c0 + 32 * i + lane);
-        };
-        fetch(first);      // on its way while the rows are looked up
-        for (uint32_t j0 = 0; j0 < p.topk; j0 += 32) {
-            // where the copy of expert j0 + lane goes: null if it is dropped
-            const uint32_t here = p.topk - j0 < 32 ? p.topk - j0 : 32;
+            for (uint32_t i = 0; i < kEpPieceLoads; ++i) {
+                if (i >= p.piece_loads) break;
+                if (first + 32 * i < end) v[i] = ld_ro(src + first + 32 * i);
+            }
+            const uint32_t word = word0 + lane;
+            uint32_t x = 0;
+            if (word < words) x = ld_ro(p.sf + static_cast<size_t>(word) * p.sf_stride + tok);
             uint8_t* dst = nullptr;
             uint32_t* dst_sf = nullptr;
-            if (lane < here) {
-                const uint32_t pair = tok * p.topk + j0 + lane;
-                const int32_t lr = ld_ro(p.local_rank + pair);
-                int32_t pos = -1;
-                if (lr >= 0) {
-                    const uint32_t e = static_cast<uint32_t>(ld_ro(p.expert_of_pair + pair));
-                    const uint32_t row = ld_ro(p.pair_base + e) + ld_ro(p.block_base + static_cast<size_t>(pair / kEpChunk) * p.num_experts + e) + static_cast<uint32_t>(lr);
-                    const uint32_t owner = e / p.experts_per_rank, slot = e - owner * p.experts_per_rank;
-                    const uint32_t in_slot = row - slot * p.slot_rows;      // masked layout only
-                    if (row < p.capacity && (p.slot_rows == 0 || in_slot < p.slot_rows)) {
-                        pos = static_cast<int32_t>(row);
-                        dst = p.peer_data[owner] + static_cast<size_t>(row) * p.k;
-                        dst_sf = p.peer_sf[owner] + (p.slot_rows ? static_cast<size_t>(slot) * p.sf_cols * p.peer_sf_stride + in_slot : row);
-                    }
-                }
-                if (segment == 0) p.pos_of_pair[pair] = pos;
+            const int32_t row = lr < 0 ? -1 : ep_arena_row(p, pair, static_cast<uint32_t>(lr), dst, dst_sf);
+            if (piece == 0 && lane == 0) p.pos_of_pair[pair] = row;
+            if (row < 0) continue;
+            uint4* to = reinterpret_cast<uint4*>(dst);
+            #pragma unroll
+            for (uint32_t i = 0; i < kEpPieceLoads; ++i) {
+                if (i >= p.piece_loads) break;
+                if (first + 32 * i < end) to[first + 32 * i] = v[i];
             }
-            const uint64_t dst_bits = reinterpret_cast<uint64_t>(dst), sf_bits = reinterpret_cast<uint64_t>(dst_sf);
-            for (uint32_t c0 = first; c0 < end; c0 += 32 * kDeep) {
-                if (c0 != first || j0 != 0) fetch(c0);
-                for (uint32_t j = 0; j < here; ++j) {
-                    uint4* to = reinterpret_cast<uint4*>(__shfl_sync(0xFFFFFFFFu, dst_bits, j));
-                    if (to == nullptr) continue;
-                    #pragma unroll
-                    for (uint32_t i = 0; i < kDeep; ++i)
-                        if (c0 + 32 * i + lane < end) to[c0 + 32 * i + lane] = v[i];
-                }
-            }
-            if (segment + 1 == p.segments) {
-                // scale words: one (word, expert) per lane and step
-                const uint32_t words = p.sf_cols * here;
-                for (uint32_t i0 = 0; i0 < words; i0 += 32) {
-                    const uint32_t i = i0 + lane, w = i / here, j = i - w * here;
-                    uint32_t* to = reinterpret_cast<uint32_t*>(__shfl_sync(0xFFFFFFFFu, sf_bits, j));
-                    if (i < words && to != nullptr) to[static_cast<size_t>(w) * p.peer_sf_stride] = ld_ro(p.sf + static_cast<size_t>(w) * p.sf_stride + tok);
-                }
-            }
+            if (word < words) dst_sf[static_cast<size_t>(word) * p.peer_sf_stride] = x;
+            for (uint32_t w = word + 32; w < words; w += 32)
+                dst_sf[static_cast<size_t>(w) * p.peer_sf_stride] = ld_ro(p.sf + static_cast<size_t>(w) * p.sf_stride + tok);
+        }
+    }
+}
+
+// Many tokens: one warp per (token, up to 32 of its experts, piece of its row): the piece is read once and stored to the experts' arena
+// rows.  A lane per expert works out where its copy goes; the whole warp then stores to one row after the other.  Bound by the stores
+// (topk x k bytes per token): 8192 tokens, top-8: rows of 7168 bytes 94 us (a warp per pair, which reads every token top-k times from L2 and looks
+// its row up as often: 118), 5120 bytes 69 (94), 4096 bytes 55 (71), 2048 bytes 29 (50).
+// In both kernels the grid may be smaller than the work (warps stride over it), which lets a caller leave room on every SM for a
+// kernel running beside this one.
+__global__ void __launch_bounds__(256) dg_ep_dispatch_tokens_kernel(const EpDispatchParams p) {
+    griddep_wait();
+    griddep_launch_dependents();
+    const uint32_t lane = threadIdx.x % 32, vecs = p.k / 16;
+    const uint32_t parts = (p.topk + 31) / 32;
+    const uint32_t units = p.pairs / p.topk * parts * p.pieces;      // fits 32 bits (checked by the host), the next one of a warp need not
+    for (uint64_t at = blockIdx.x * 8 + threadIdx.x / 32; at < units; at += static_cast<uint64_t>(gridDim.x) * 8) {
+        const uint32_t unit = static_cast<uint32_t>(at);
+        const uint32_t row_part = unit / p.pieces, piece = unit - row_part * p.pieces;
+        const uint32_t tok = row_part / parts, j0 = (row_part - tok * parts) * 32, here = p.topk - j0 < 32 ? p.topk - j0 : 32;
+        const uint4* src = reinterpret_cast<const uint4*>(p.data + static_cast<size_t>(tok) * p.k);
+        const uint32_t first = piece * p.piece_loads * 32 + lane, past = (piece + 1) * p.piece_loads * 32, end = past < vecs ? past : vecs;
+        uint4 v[kEpPieceLoads];      // on its way while the rows are looked up
+        #pragma unroll
+        for (uint32_t i = 0; i < kEpPieceLoads; ++i)
+            if (first + 32 * i < end) v[i] = ld_ro(src + first + 32 * i);
+        // where the copy of expert j0 + lane goes: null if it is dropped
+        uint8_t* dst = nullptr;
+        uint32_t* dst_sf = nullptr;
+        if (lane < here) {
+            const uint32_t pair = tok * p.topk + j0 + lane;
+            const int32_t lr = ld_ro(p.local_rank + pair);
+            const int32_t row = lr < 0 ? -1 : ep_arena_row(p, pair, static_cast<uint32_t>(lr), dst, dst_sf);
+            if (piece == 0) p.pos_of_pair[pair] = row;
+        }
+        const uint64_t dst_bits = reinterpret_cast<uint64_t>(dst), sf_bits = reinterpret_cast<uint64_t>(dst_sf);
+        for (uint32_t j = 0; j < here; ++j) {
+            uint4* to = reinterpret_cast<uint4*>(__shfl_sync(0xFFFFFFFFu, dst_bits, j));
+            if (to == nullptr) continue;
+            #pragma unroll
+            for (uint32_t i = 0; i < kEpPieceLoads; ++i)
+                if (first + 32 * i < end) to[first + 32 * i] = v[i];
+        }
+        // scale words: one (word, expert) per lane and step, the steps dealt out over the pieces
+        const uint32_t words = p.sf_cols * here;
+        for (uint32_t i0 = piece * 32; i0 < words; i0 += p.pieces * 32) {
+            const uint32_t i = i0 + lane, w = i / here, j = i - w * here;
+            uint32_t* to = reinterpret_cast<uint32_t*>(__shfl_sync(0xFFFFFFFFu, sf_bits, j));
+            if (i < words && to != nullptr) to[static_cast<size_t>(w) * p.peer_sf_stride] = ld_ro(p.sf + static_cast<size_t>(w) * p.sf_stride + tok);
         }
     }
 }

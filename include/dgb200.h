@@ -266,8 +266,9 @@ int dg_ep_layout(dg_ctx* ctx, const uint32_t* all_counts, uint32_t world, uint32
  * sf[c * peer_sf_stride + row]), entry `rank` being the local buffers.  Padding rows are not written.
  * slot_rows: as given to dg_ep_layout; in the masked layout the scale words go to the per-slot layout the masked GEMM
  * reads, sf[(slot * sf_cols + c) * peer_sf_stride + row in slot] with peer_sf_stride = dg_sf_aligned_rows(slot_rows).
- * max_blocks: 0 launches one warp per pair; a positive value bounds the grid (256-thread blocks striding over the
- * pairs), e.g. 2 x the SM count to leave room on every SM for a GEMM running beside the exchange. */
+ * max_blocks: 0 launches as many 256-thread blocks as there is work (a warp takes a piece of a token's row); a positive value
+ * bounds the grid, whose warps then stride over the pieces, e.g. 2 x the SM count to leave room on every SM for a GEMM running
+ * beside the exchange. */
 int dg_ep_dispatch(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* local_rank, const uint32_t* block_base, const uint32_t* pair_base,
                    uint32_t pairs, uint32_t topk, uint32_t num_experts, uint32_t world, const uint8_t* data, uint32_t k, const uint32_t* sf,
                    uint32_t sf_stride, uint32_t sf_cols, void* const* peer_data, void* const* peer_sf, uint32_t peer_sf_stride,

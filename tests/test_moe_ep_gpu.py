@@ -371,8 +371,11 @@ def test_peer_exchange_refuses_a_context_on_another_stream():
 @pytest.mark.parametrize("tokens,topk,hidden,n,max_blocks", [
     (1, 1, 512, 8, 0),                # one warp load per row, one column chunk
     (5, 9, 7680, 264, 0),             # 15 loads per row and 2 chunk steps, the last one ragged; a second look-up of result rows
-    (40, 33, 1024, 2056, 3),          # a second look-up of arena rows; warps that stride over the work
+    (40, 33, 1024, 2056, 3),          # warps that stride over the work
     (5000, 8, 4096, 2304, 0),         # rows cut into pieces of several loads
+    (129, 16, 512, 264, 0), (130, 16, 512, 264, 0),         # on a B200 the last size of a warp per pair, the first of a warp per token
+    (200, 33, 4608, 264, 5),          # a warp per token with a second part of its experts, pieces of nine loads' rows; few blocks
+    (9, 3, 7680, 264, 2),             # a warp per pair, more pieces than blocks
 ])
 def test_peer_exchange_row_pieces(ctx, tokens, topk, hidden, n, max_blocks):
     # dispatch and combine cut rows into pieces, one warp each: rows, scale words and sums bit for bit, whatever the cut
