@@ -1769,7 +1769,7 @@ int dg_ep_layout(dg_ctx* ctx, const uint32_t* all_counts, uint32_t world, uint32
 }
 
 // Pieces a row of `steps` warp loads is cut into, one warp each: of seven loads where that gives enough warps, of fewer down to one
-// where it does not.  (8192 rows of 7168 columns: combine takes 219 us with pieces of 7 loads, 224 with 4, 226 with 14.)
+// where it does not.
 static uint32_t row_segments(uint32_t rows, uint32_t steps, uint64_t enough) {
     if (steps == 0) return 1;
     uint32_t per = dg::kEpPieceLoads;
@@ -1842,7 +1842,13 @@ int dg_ep_combine(dg_ctx* ctx, const int32_t* expert_of_pair, const int32_t* pos
     p.tokens = tokens; p.topk = topk; p.n = n; p.experts_per_rank = num_experts / world;
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     if (static_cast<uint64_t>(tokens) * (n / 8) > 0xFFFFFF00ull) return fail(DG_ERR_SHAPE, "tokens x n / 8 must fit 32 bits");
-    p.segments = row_segments(tokens, ceil_div(n, 256), 32ull * ctx->num_sms);
+    // Pieces as short as one wave allows (32 warps per SM), of seven steps at most.  A wave and a bit costs two: 1024 tokens x 7168 (28
+    // steps), top-8: pieces of 7 steps 24.4 us (one wave), 6: 31.2, 5: 28.1, 4: 25.8, 2: 26.0, 1: 28.2; 512 tokens 4: 10.7, 3: 12.8; x 5120 3:
+    // 8.0, 4: 10.2; 256 tokens x 7168 2: 6.1, 1: 6.4.  Beyond one wave seven is within 3 % of the best where it divides the row (8192 x
+    // 7168: 166.8, 4: 165.5, 14: 169.8) and within 15 % elsewhere (2048 x 4096, 16 steps: 33.0, 4: 29.1).
+    uint32_t steps = 1;
+    while (steps < 7 && static_cast<uint64_t>(tokens) * ceil_div(ceil_div(n, 256), steps) > 32ull * ctx->num_sms) ++steps;
+    p.segments = ceil_div(ceil_div(n, 256), steps);
     DG_CUDA(launch(dg::dg_ep_combine_kernel, piece_blocks(static_cast<uint64_t>(tokens) * p.segments, max_blocks), 256, 0, ctx->stream, p));
     return DG_OK;
 }

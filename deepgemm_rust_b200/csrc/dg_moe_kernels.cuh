@@ -379,10 +379,11 @@ struct EpCombineParams {
 // out[t, :] = bf16( sum_j w[t, j] * rows_of_owner(t, j)[pos[t, j], :] ): the same ordered fused multiply-add
 // chain as dg_moe_combine_kernel, reading each term from the rank that computed it.  One warp per (token, segment of its row), a lane
 // 8 columns at a time: where the token's top-k rows are is worked out once per warp, a lane per row (every thread looking up all of
-// them for its 8 columns cost 32 loads beside the 8 that move data).  Bound by reading topk x n x 2 bytes per token: 8192 tokens x
-// 7168 columns, top-8: 238 -> 219 us; 128 tokens: 6.0 -> 5.6.  Two steps unrolled (238 us), or one row after the other in longer runs
-// (226-331 us), leave fewer loads in flight.
-__global__ void __launch_bounds__(256) dg_ep_combine_kernel(const EpCombineParams p) {
+// them for its 8 columns cost 32 loads beside the 8 that move data).  Bound by reading topk x n x 2 bytes per token, and so by the loads
+// in flight: 32 warps per SM (at most 64 registers; without the bound the compiler takes 79), and nothing done for rows beyond the top-k
+// (which branches skip as a whole).  8192 tokens x 7168 columns, top-8: 236 us with a thread per 8 columns, 220 by pieces with 79
+// registers and 8 rows whatever top-k is, 163.5 now; 1024 tokens 33.5, 36.9, 24.3; 128 tokens 5.7, 5.2, 4.1, of them with top-2 3.4, 4.2, 2.6.
+__global__ void __launch_bounds__(256, 4) dg_ep_combine_kernel(const EpCombineParams p) {
     griddep_wait();
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
@@ -411,14 +412,17 @@ __global__ void __launch_bounds__(256) dg_ep_combine_kernel(const EpCombineParam
             float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
             for (uint32_t j0 = 0; j0 < p.topk; j0 += kDeep) {
                 if (p.topk > kDeep) look_up(j0, row_bits, weight);
+                const uint32_t here = p.topk - j0 < kDeep ? p.topk - j0 : kDeep;
                 uint4 v[kDeep];
                 #pragma unroll
                 for (uint32_t u = 0; u < kDeep; ++u) {
+                    if (u >= here) break;
                     const uint4* row = reinterpret_cast<const uint4*>(__shfl_sync(0xFFFFFFFFu, row_bits, u));
                     if (row != nullptr && c < end) v[u] = *(row + c);
                 }
                 #pragma unroll
                 for (uint32_t u = 0; u < kDeep; ++u) {
+                    if (u >= here) break;
                     if (__shfl_sync(0xFFFFFFFFu, row_bits, u) == 0) continue;
                     const float wj = __shfl_sync(0xFFFFFFFFu, weight, u);
                     const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};

@@ -376,6 +376,7 @@ def test_peer_exchange_refuses_a_context_on_another_stream():
     (129, 16, 512, 264, 0), (130, 16, 512, 264, 0),         # on a B200 the last size of a warp per pair, the first of a warp per token
     (200, 33, 4608, 264, 5),          # a warp per token with a second part of its experts, pieces of nine loads' rows; few blocks
     (9, 3, 7680, 264, 2),             # a warp per pair, more pieces than blocks
+    (600, 8, 512, 4104, 0),           # result rows in pieces of three steps, the last one ragged
 ])
 def test_peer_exchange_row_pieces(ctx, tokens, topk, hidden, n, max_blocks):
     # dispatch and combine cut rows into pieces, one warp each: rows, scale words and sums bit for bit, whatever the cut
