@@ -235,6 +235,7 @@ struct KernelPlan {
     uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
     uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
+    uint32_t table_groups;     // groups whose rows and tiles are kept in shared memory (swapped family)
 };
 static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
@@ -418,6 +419,10 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
                     plan->swap = true;
                     plan->ctas = ctas; plan->umma_n = bn; plan->halves = halves; plan->stages = stages; plan->accum = 2;
                     plan->splits = splits; plan->tiles = tiles; plan->smem = smem(stages);
+                    // the group table takes what the stages leave of the shared memory
+                    const uint32_t room = !dense && dg::swap_has_table(ctas, halves) ? (kSmemCapacity - plan->smem) / 16 : 0;
+                    plan->table_groups = groups < room ? groups : room;
+                    plan->smem += plan->table_groups * 16;
                     out->swap_ab = 1;
                     out->block_m = bn;            // activation rows per tile (an upper bound: a tile's UMMA N follows its rows)
                     out->block_n = 128 * ctas;    // weight rows per tile
@@ -587,7 +592,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     const uint32_t stages = best_stages;
     plan->swap = false;
     plan->ctas = best_ctas; plan->umma_n = best_n; plan->halves = best_halves; plan->stages = best_stages; plan->accum = best_accum;
-    plan->splits = best_splits; plan->tiles = best_tiles;
+    plan->splits = best_splits; plan->tiles = best_tiles; plan->table_groups = 0;
     out->swap_ab = 0;
     out->block_m = 128 * best_ctas;
     out->block_n = best_n;
@@ -1032,12 +1037,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         p.acc_stride = dg::gemm_swap_acc_stride(plan.umma_n, sfa_words, sfb_words);
         p.acc_edge_chunks = ceil_div(plan.umma_n, 32) - p.acc_stride / 32;
         if (p.acc_stride == plan.umma_n) p.acc_edge_chunks = 0;
-        if (dg::swap_has_table(plan.ctas, plan.halves) && (pr.type == DG_GEMM_M_GROUPED_CONTIGUOUS || pr.type == DG_GEMM_M_GROUPED_MASKED)) {
-            // the group table takes what the stages leave of the shared memory
-            const uint32_t room = (kSmemCapacity - plan.smem) / 16;
-            p.table_groups = pr.groups < room ? pr.groups : room;
-            plan.smem += p.table_groups * 16;
-        }
+        p.table_groups = plan.table_groups;
         p.splitk_ws = splitk_ws;
         p.splitk_counters = static_cast<uint32_t*>(ctx->scratch->splitk_counters.ptr);
     }

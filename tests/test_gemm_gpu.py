@@ -824,8 +824,8 @@ def test_grouped_calls_write_the_same_rows_whichever_family_runs(ctx, n, k, fami
 
 @pytest.mark.parametrize("masked", [True, False])
 def test_swapped_family_with_more_groups_than_its_table_holds(ctx, masked, monkeypatch):
-    # the swapped kernel keeps the rows and tiles of the first groups in what its stages leave of shared memory (room for a few hundred
-    # here) and reads the others from global memory: groups on both sides of that line, empty ones among them
+    # the swapped kernel keeps the rows and tiles of the first groups in what its stages leave of shared memory (room for 362 masked
+    # and 106 contiguous ones here) and reads the others from global memory: groups on both sides of that line, empty ones among them
     pin_family(monkeypatch, "1")
     groups, n, k, slot = 2000, 128, 512, 16
     sizes = np.random.default_rng(7).integers(0, slot + 1, groups).astype(np.int32)

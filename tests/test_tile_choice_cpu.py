@@ -38,6 +38,21 @@ def test_problems_outside_the_fit_of_the_dense_costs_keep_their_tiles(sizes, kw,
     assert (c.block_m, c.block_n, c.block_k, c.num_splits) == tile
 
 
+@pytest.mark.parametrize("layout", [CONTIGUOUS, MASKED])
+def test_shared_memory_of_a_choice_counts_the_group_table(layout, monkeypatch):
+    # 16 bytes per group beside what the stages take, as many as fit; none for single CTAs, whose kernels have no table
+    monkeypatch.setenv("DG_STAGES", "6")
+
+    def smem(groups):
+        c = choice(layout, 256 * (groups if layout == CONTIGUOUS else 1), 4096, 7168, groups, 128)
+        assert c.swap_ab
+        return c.smem_size
+    assert smem(200) - smem(100) == 16 * 100
+    assert smem(1 << 14) == dg.SM100_SMEM_CAPACITY // 16 * 16
+    monkeypatch.setenv("DG_CTAS", "1")
+    assert smem(200) == smem(100)
+
+
 @pytest.mark.parametrize("slot,height", [(64, 64), (76, 96), (128, 128), (250, 128), (516, 160), (924, 256), (4096, 256)])
 @pytest.mark.parametrize("expected", [1, 16])
 def test_a_weak_hint_does_not_shorten_the_tiles_of_a_masked_problem(slot, height, expected):
