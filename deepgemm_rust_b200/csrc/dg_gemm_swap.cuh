@@ -68,7 +68,7 @@ struct SwapScheduler {
         step = grouped ? 32 : 16 * ctas;
         if (!grouped) set_rows(p.n);
     }
-    // What needs the group table: call once, after open_groups().  The constructor belongs before it, where its time is hidden.
+    // What needs the group table: call once, after groups_ready().  The constructor belongs before it, where its time is hidden.
     DG_DEVICE void start(const uint4* group_table) {
         if constexpr (kTable) table = group_table;
         if (grouped) load_group();
@@ -294,7 +294,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     // 2048 x 2048: 62.4 -> 59.4 us; contiguous 64 x 128 rows, 4096 x 3584: 227 -> 216).
     auto groups_ready = [&]() {
         griddep_wait();
-        if constexpr (kTable) return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x700);
+        if constexpr (kTable) return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x680);
         else return true;
     };
     const uint32_t tmem_base = *tmem_slot;

@@ -29,3 +29,15 @@ def test_overlapped_kernels_declare_no_constant_inputs():
                 overlapped += 1
                 assert not re.search(r"\bconst\b[^,(]*\*\s*__restrict__", signature), (name, signature)
     assert overlapped >= 15      # the pattern still finds the kernels
+
+
+def test_a_wait_that_ran_out_can_be_told_from_every_other():
+    # the status record names the wait by its site; 0x700 is the self-test's, as the public header says
+    sites = {}
+    for name, text in device_sources():
+        found = re.findall(r"(?:p\.)?status, (\([^)]*\)|0x[0-9a-f]+)", text)
+        codes = [int(c, 16) for f in found for c in re.findall(r"0x[0-9a-f]+", f)]
+        assert len(codes) == len(set(codes)), (name, [hex(c) for c in codes])
+        sites[name] = codes
+    assert [name for name, codes in sites.items() if 0x700 in codes] == ["dg_cast_kernels.cuh"]
+    assert sum(map(len, sites.values())) >= 20      # the pattern still finds the waits
