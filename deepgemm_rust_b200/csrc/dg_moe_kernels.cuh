@@ -388,9 +388,9 @@ __global__ void __launch_bounds__(256, 4) dg_ep_combine_kernel(const EpCombinePa
     griddep_launch_dependents();
     const uint32_t lane = threadIdx.x % 32;
     const uint32_t chunks = p.n / 8, per_segment = ((chunks + 31) / 32 + p.segments - 1) / p.segments * 32;
-    const uint32_t units = p.tokens * p.segments, warps = gridDim.x * (blockDim.x / 32);
+    const uint32_t units = p.tokens * p.segments, warps = gridDim.x * 8;      // fit 32 bits (checked by the host); a unit and a stride need not
     constexpr uint32_t kDeep = 8;      // rows whose loads are in flight before the first use
-    for (uint32_t unit = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; unit < units; unit += warps) {
+    for (uint32_t unit = blockIdx.x * 8 + threadIdx.x / 32; unit < units; unit = units - unit > warps ? unit + warps : units) {
         const uint32_t t = unit / p.segments, segment = unit - t * p.segments;
         const uint32_t first = segment * per_segment, end = first + per_segment < chunks ? first + per_segment : chunks;
         auto look_up = [&](uint32_t j, uint64_t& row_bits, float& weight) {

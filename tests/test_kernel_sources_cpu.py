@@ -41,3 +41,13 @@ def test_a_wait_that_ran_out_can_be_told_from_every_other():
         sites[name] = codes
     assert [name for name, codes in sites.items() if 0x700 in codes] == ["dg_cast_kernels.cuh"]
     assert sum(map(len, sites.values())) >= 20      # the pattern still finds the waits
+
+
+def test_loops_over_a_grid_end():
+    # work that fits 32 bits may end less than one stride below 2^32: a 32-bit counter that only adds would wrap round and never end
+    strided = 0
+    for name, text in device_sources():
+        loops = re.findall(r"for \((\w+) \w+ = [^;]*blockIdx\.x[^;]*;[^;]*;[^)]*\+=", text)
+        assert all(kind == "uint64_t" for kind in loops), (name, loops)
+        strided += len(loops)
+    assert strided >= 2      # the pattern still finds the loops
