@@ -510,6 +510,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             // Dense problems have constants of their own.  For one wave they were fitted to 205 problems (m 1-4096, n 512-16384, k 1024-16384,
             // e4m3 / mixed / mxfp4, every width, K ranges; the choice is 2 % off the best of these tiles on average, 4 % with the others): a
             // scale copy costs 40 cycles, a tile 2900 from its first load to its last store, of which the last one's epilogue is exposed.
+            // (Fitted when the copies were loops and f32 outputs of a single tile were staged in two buffers; both are cheaper since.)
             // What was not in that fit keeps the constants and the choices it had before it, which measured better there: batched problems
             // (60 of them, 1.01 times as long on average with the fitted constants, 1.22 at worst: 10 x 420 x 1792 x 512, f32), and
             // e4m3 operands with per-32 scales (30 problems, 1.02 and 1.28: 972 x 8704 x 1024, f32).

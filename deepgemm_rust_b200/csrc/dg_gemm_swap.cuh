@@ -290,8 +290,10 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
     griddep_launch_dependents();
     // Grouped layouts: the epilogue warps, which have nothing to do yet, bring the groups' rows and tiles into shared memory.  Every
     // role walks the groups one after the other, two to five of them between two tiles; fetched from global memory (~700 cycles each)
-    // they stopped the weight loads for that long, where a tile of 16 k-blocks takes 9000 cycles (64 masked groups of up to 64 rows,
-    // 2048 x 2048: 62.4 -> 59.4 us; contiguous 64 x 128 rows, 4096 x 3584: 227 -> 216).
+    // they stopped the weight loads for that long, where a tile of 16 k-blocks takes 9000 cycles (masked groups of up to 32 rows, 2048 x
+    // 2048: 128 of them 114.7 -> 103.9 us; of up to 64 rows, 64 of them 62.1 -> 57.1; contiguous 256 x 128 rows, 2048 x 3584: 397 ->
+    // 375).  Read from the table or not in turn, 4-64 masked groups of up to 128 rows and K of 2048-7168 gain 1-10 %, most with many groups
+    // and short K.
     auto groups_ready = [&]() {
         griddep_wait();
         if constexpr (kTable) return p.table_groups == 0 || mbar_wait(bar_table, 0, abort_flag, p.status, 0x680);
