@@ -1132,8 +1132,9 @@ struct F32Plan {
     uint32_t splits, kb_per_split;   // K ranges (dense problems with few tiles), in k-blocks of 128
 };
 // Costs in microseconds, fitted on B200 over 22 problems (m 68-6900, n 560-8096, k 1152-8064): a K block takes 0.36 of a 128 x 128
-// tile and 0.56 of a 256 x 256 one (a quarter as many tiles, half the SM pairs), so the pair wins wherever its waves are fewer than
-// 0.64 of the others; K ranges pay 3.5 plus their planes for the second launch, and never more than one wave.
+// tile and 0.45 of a 256 x 256 one (a quarter as many tiles, half the SM pairs), so the pair wins wherever its waves are fewer than
+// 0.8 of the others.  (Over the 40 problems that went over to the pair when its 0.56 became 0.45, it takes 0.93 of the other's time,
+// 0.87 to 1.01: 1315 x 4000 x 5376 54.1 -> 47.8 us, 6432 x 1344 x 2432 37.5 -> 38.0.)  K ranges pay 3.5 plus their planes for the second launch, and never more than one wave.
 F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint32_t groups, uint32_t sms) {
     const uint32_t kbs = k / 128;
     const bool dense = type == DG_GEMM_NORMAL;
@@ -1148,7 +1149,7 @@ F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint3
     auto waves = [](double t, uint32_t workers) { return static_cast<double>(static_cast<uint64_t>(t / workers + 0.999)); };
     F32Plan best = {1, 128, 1, kbs};
     double best_cost = waves(tiles, sms) * (kbs * 0.36 + 0.6);
-    const double pair_cost = sms >= 2 ? waves(pair_tiles, sms / 2) * (kbs * 0.56 + 1.2) : best_cost;
+    const double pair_cost = sms >= 2 ? waves(pair_tiles, sms / 2) * (kbs * 0.45 + 1.2) : best_cost;
     // (a masked group's rows are known to the device only and usually fewer than its slot: small tiles)
     if (type != DG_GEMM_M_GROUPED_MASKED && pair_cost < best_cost) {
         best = {2, 256, 1, kbs};

@@ -8,14 +8,17 @@
 // warps fold it into f32 accumulators they keep in registers: acc = fma(block, sfa * sfb, acc).
 //
 // What bounds it: every K block's partial tile has to leave TMEM (128 lanes x 4 bytes per cycle) and go through one FMA per
-// element (128 per cycle and SM), each 256 cycles for 128 x 256 elements, beside 512 cycles of tensor time; a K block costs the
-// epilogue warps ~1100 cycles all told (barrier, scales, TMEM latency), which is the limit.  The operands of a 128 x 128 tile
+// element (128 per cycle and SM), each 256 cycles for 128 x 256 elements, beside 512 cycles of tensor time; a K block takes ~950
+// cycles all told.  The two TMEM buffers are what couples the two sides: a buffer is filled (512), seen to be full, read and folded (~470),
+// and seen to be empty, ~850 cycles of hand-over in it, once per two K blocks.  The operands of a 128 x 128 tile
 // (32 KB for 256 tensor cycles) also arrive slower than the tensor core takes them.  So a CTA pair computes 256 x 256
 // (kCtas = 2, kBlockN = 256): 32 KB per CTA for 512 tensor cycles, both TMEM buffers 256 columns wide, and 128 x 256 f32
 // accumulators in the registers of eight epilogue warps (the other four give registers back for that).  Problems with too few
 // such tiles use 128 x 128 tiles of single CTAs, and cut K into ranges (f32 partial planes summed by dg_splitk_reduce_kernel)
 // when even those do not fill the SMs.  4096 x 7168 x 7168: 348 us with 128 x 128 tiles and three rounded operations per
-// element, 313 with one FMA, 260 with the pair; sixteen epilogue warps of 64 columns (96 registers) spilled and took 350.
+// element, 313 with one FMA, 260 with the pair, 237 with the pair's shorter loop; sixteen epilogue warps of 64 columns (96 registers) spilled
+// and took 350.  Four buffers of 128 columns (a half of the pair's tile each, N = 128) were no faster than two; loads of 32 columns, scalar FMAs and
+// asking early whether the next block is complete (which holds up the release of the present one) were slower.
 // Roles of the 384-thread CTA: warp 0 loads A / B k-blocks with TMA, warp 1 issues the UMMAs, warps 4-11 are the epilogue: each
 // owns 32 rows (TMEM quadrant warp % 4) x half of the tile's columns.
 #pragma once
@@ -61,7 +64,8 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
     const GemmParams& p = q.g;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t lane = threadIdx.x % 32;
+    const uint32_t warp = kCtas == 2 ? __shfl_sync(0xFFFFFFFFu, threadIdx.x / 32, 0) : threadIdx.x / 32;      // pair: known to be the same in every lane
     const uint32_t cta_rank = kCtas == 2 ? cluster_cta_rank() : 0u;
     constexpr uint32_t kLoadN = kBlockN / kCtas;              // weight rows this CTA loads
     constexpr uint32_t kTileA = kBlockM * kBlockKBytes, kTileB = kLoadN * kBlockKBytes;
@@ -76,8 +80,8 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
     uint64_t* bar_full = bars;                               // a k-block's operands landed (pair: both CTAs', on rank 0)
     uint64_t* bar_empty = bars + kMaxStages;
     uint64_t* bar_tmem_full = bars + 2 * kMaxStages;         // a K block's partial tile is complete in TMEM buffer e
-    uint64_t* bar_tmem_empty = bars + 2 * kMaxStages + 2;    // the epilogue warps (of both CTAs) have read buffer e
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
+    uint64_t* bar_tmem_empty = bar_tmem_full + 2;            // the epilogue warps (of both CTAs) have read buffer e
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tmem_empty + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     if (threadIdx.x == 0) {
@@ -104,12 +108,12 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
     tc_fence_after();
     griddep_wait();
     griddep_launch_dependents();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = kCtas == 2 ? __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0) : *tmem_slot;
 
-    // 384 threads x 168 registers at launch = 128 x 88 + 256 x 208
+    // 384 threads x 168 registers at launch = 128 x 72 + 256 x 216
     constexpr bool kMoveRegs = kBlockN == 256;
     if (warp < 4) {
-        if constexpr (kMoveRegs) setmaxnreg_dec<88>();
+        if constexpr (kMoveRegs) setmaxnreg_dec<72>();
         if (warp == 0) {
             // ------------------------------------------------------------ TMA producer
             Scheduler sched(p, kCtas);
@@ -162,8 +166,8 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                             umma_commit(bar_empty + stage);
                             umma_commit(bar_tmem_full + e);
                         } else {
-                            umma_commit_2cta(bar_empty + stage, static_cast<uint16_t>(3));
                             umma_commit_2cta(bar_tmem_full + e, static_cast<uint16_t>(3));
+                            umma_commit_2cta(bar_empty + stage, static_cast<uint16_t>(3));
                         }
                     }
                     __syncwarp();
@@ -174,51 +178,52 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue
-        if constexpr (kMoveRegs) setmaxnreg_inc<208>();
+        if constexpr (kMoveRegs) setmaxnreg_inc<216>();
         const uint32_t ew = warp % 4, col_part = (warp - 4) / 4;       // TMEM lane quadrant; which half of the tile's columns
         uint8_t* const buf = smem_epi + (warp - 4) * kEpiBuf;
+        const bool leader = elect_one();
+        const uint32_t tmem_mine = tmem_base + ((ew * 32) << 16) + col_part * kWarpCols;
+        const uint32_t empty_addr = kCtas == 2 ? mapa_u32(smem_u32(bar_tmem_empty), 0) : smem_u32(bar_tmem_empty);
         Scheduler sched(p, kCtas);
         Tile t;
-        uint32_t block = 0;
+        uint32_t e = 0, phase = 0;
         bool ok = true;
         while (ok && sched.next(t)) {
             const uint32_t row0 = t.m0 + cta_rank * kBlockM + ew * 32, row = row0 + lane, n0 = t.n0 + col_part * kWarpCols;
-            const bool row_ok = row < t.m_end;
             // the activation scale of this thread's row for K block kb, and the weight scale of the warp's columns
-            const float* sfa_row = q.sfa_t + static_cast<size_t>(t.ga) * q.k_blocks * q.sfa_stride + row;
             const uint32_t nb = n0 / 128 < q.n_blocks128 ? n0 / 128 : q.n_blocks128 - 1;
-            const float* sfb_tile = q.sfb + (static_cast<size_t>(t.gb) * q.n_blocks128 + nb) * q.k_blocks;
-            auto scale_a = [&](uint32_t kb) { return row_ok && kb < t.kb1 ? ld_ro(sfa_row + static_cast<size_t>(kb) * q.sfa_stride) : 0.0f; };
-            auto scale_b = [&](uint32_t kb) { return kb < t.kb1 ? ld_ro(sfb_tile + kb) : 0.0f; };
+            const float* next_a = q.sfa_t + (static_cast<size_t>(t.ga) * q.k_blocks + t.kb0) * q.sfa_stride + row;
+            const float* next_b = q.sfb + (static_cast<size_t>(t.gb) * q.n_blocks128 + nb) * q.k_blocks + t.kb0;
+            const uint32_t stride = q.sfa_stride;
+            const bool row_ok = row < t.m_end;
+            auto load_scales = [&](float& sa, float& sb) {
+                sa = 0.0f;
+                if (row_ok) sa = ld_ro(next_a);
+                sb = ld_ro(next_b);
+                next_a += stride;
+                ++next_b;
+            };
             float acc[kWarpCols];
             #pragma unroll
             for (uint32_t i = 0; i < kWarpCols; ++i) acc[i] = 0.0f;
-            // scales are fetched two K blocks ahead of their use
-            float sa = scale_a(t.kb0), sb = scale_b(t.kb0), sa1 = scale_a(t.kb0 + 1), sb1 = scale_b(t.kb0 + 1);
-            for (uint32_t kb = t.kb0; kb < t.kb1; ++kb, ++block) {
-                const uint32_t e = block & 1, buf_phase = (block >> 1) & 1;
-                const float sa2 = scale_a(kb + 2), sb2 = scale_b(kb + 2);
-                // One factor for both scales: one rounding fewer than scaling twice.  Where their product leaves the range that keeps full
-                // precision (never with scales of quantised data) the block is multiplied by the activation scale first, in place in TMEM:
-                // a second path over the accumulators would cost every K block register moves.
-                const float both = sa * sb, mag = fabsf(both);
-                const bool one_factor = __all_sync(0xFFFFFFFFu, (mag >= 1e-30f && mag <= 1e30f) || sa == 0.0f || sb == 0.0f);
-                const float s = one_factor ? both : sb;
-                if (!mbar_wait(bar_tmem_full + e, buf_phase, abort_flag, p.status, 0x600 + e)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t taddr = tmem_base + ((ew * 32) << 16) + e * kBlockN + col_part * kWarpCols;
-                if (!one_factor) {
-                    #pragma unroll 1
-                    for (uint32_t c = 0; c < kWarpCols; c += 16) {
-                        uint32_t v[16];
-                        tmem_ld_32x32b_x16(taddr + c, v);
-                        tmem_ld_wait_x16(v);
-                        #pragma unroll
-                        for (uint32_t i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * sa);
-                        tmem_st_32x32b_x16(taddr + c, v);
-                    }
-                    tmem_st_wait();
+            uint32_t left = t.kb1 - t.kb0, va[16], vb[16];
+            // One factor for both scales: one rounding fewer than scaling twice.  Where their product leaves the range that keeps full
+            // precision (never with scales of quantised data) the block is multiplied by the activation scale first, in place in TMEM:
+            // a second path over the accumulators would cost every K block register moves.
+            auto in_range = [](float s) { return fabsf(s) >= 1e-30f && fabsf(s) <= 1e30f; };
+            auto rescale = [&](uint32_t taddr, float sa) {
+                #pragma unroll 1
+                for (uint32_t c = 0; c < kWarpCols; c += 16) {
+                    tmem_ld_32x32b_x16(taddr + c, va);
+                    tmem_ld_wait_x16(va);
+                    #pragma unroll
+                    for (uint32_t i = 0; i < 16; ++i) va[i] = __float_as_uint(__uint_as_float(va[i]) * sa);
+                    tmem_st_32x32b_x16(taddr + c, va);
                 }
+                tmem_st_wait();
+            };
+            // the K block in buffer e, whose first 16 columns are already on their way to va
+            auto fold_block = [&](uint32_t taddr, float s) {
                 // two elements per instruction (packed f32x2: the same IEEE operations, half the issue slots)
                 auto fold = [&](uint32_t (&v)[16], uint32_t c) {
                     #pragma unroll
@@ -230,8 +235,6 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                     }
                 };
                 // the TMEM load of the next 16 columns is in flight while the current ones are folded in
-                uint32_t va[16], vb[16];
-                tmem_ld_32x32b_x16(taddr, va);
                 #pragma unroll
                 for (uint32_t c = 0; c < kWarpCols / 16; c += 2) {
                     tmem_ld_wait_x16(va);
@@ -244,14 +247,61 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                         // the buffer is in registers: hand it back to the UMMA warp
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) {
-                            if constexpr (kCtas == 1) mbar_arrive(bar_tmem_empty + e);
-                            else mbar_arrive_remote(bar_tmem_empty + e, 0);
+                        if constexpr (kCtas == 1) {
+                            if (lane == 0) mbar_arrive(bar_tmem_empty + e);
+                        } else if (leader) {
+                            mbar_arrive_cluster(empty_addr + e * 8);
                         }
                     }
                     fold(vb, c + 1);
                 }
-                sa = sa1; sb = sb1; sa1 = sa2; sb1 = sb2;
+                phase ^= e;
+                e ^= 1;
+                --left;
+            };
+            float sa = 0.0f, sb = 0.0f, sa1 = 0.0f, sb1 = 0.0f;      // the scales are fetched two K blocks ahead of their use
+            load_scales(sa, sb);
+            if (left > 1) load_scales(sa1, sb1);
+            if constexpr (kCtas == 2) {
+                // With 128 accumulators in registers every instruction beside the 64 FMAs and 8 loads of a K block shows: two K blocks a turn,
+                // each with scale registers of its own that are loaded again as soon as they have been used (handed from one name to the
+                // next they had to arrive within the turn they were asked for in), addresses in uniform registers, the factor worked out
+                // beside the first load.  210 -> 140 instructions per warp and K block.
+                auto k_block = [&](float& a, float& b) {
+                    if (!mbar_wait(bar_tmem_full + e, phase, abort_flag, p.status, 0x600 + e)) return false;
+                    tc_fence_after();
+                    const uint32_t taddr = tmem_mine + e * kBlockN;
+                    tmem_ld_32x32b_x16(taddr, va);
+                    float s = a * b;
+                    if (!__all_sync(0xFFFFFFFFu, in_range(s)) && !__all_sync(0xFFFFFFFFu, in_range(s) || a == 0.0f || b == 0.0f)) {
+                        tmem_ld_wait_x16(va);
+                        rescale(taddr, a);
+                        s = b;
+                        tmem_ld_32x32b_x16(taddr, va);
+                    }
+                    if (left > 2) load_scales(a, b);
+                    fold_block(taddr, s);
+                    return true;
+                };
+                while (ok && left != 0) {
+                    ok = k_block(sa, sb);
+                    if (ok && left != 0) ok = k_block(sa1, sb1);
+                }
+            } else {
+                // 64 accumulators: registers to spare, and the shorter code starts sooner (150 x 1000 x 1152: 8.7 us, 8.9 with the other loop)
+                while (left != 0) {
+                    float sa2 = 0.0f, sb2 = 0.0f;
+                    if (left > 2) load_scales(sa2, sb2);
+                    const float both = sa * sb;
+                    const bool one_factor = __all_sync(0xFFFFFFFFu, in_range(both) || sa == 0.0f || sb == 0.0f);
+                    if (!mbar_wait(bar_tmem_full + e, phase, abort_flag, p.status, 0x600 + e)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t taddr = tmem_mine + e * kBlockN;
+                    if (!one_factor) rescale(taddr, sa);
+                    tmem_ld_32x32b_x16(taddr, va);
+                    fold_block(taddr, one_factor ? both : sb);
+                    sa = sa1; sb = sb1; sa1 = sa2; sb1 = sb2;
+                }
             }
             if (!ok) break;
             // 32 columns at a time through swizzled staging, one TMA store each (rows past the group's end are cut off by the store's

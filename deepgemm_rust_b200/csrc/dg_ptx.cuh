@@ -45,6 +45,10 @@ DG_DEVICE void mbar_arrive_remote(uint64_t* bar, uint32_t cta) {
         "r"(cta)
         : "memory");
 }
+// Arrive on a barrier given by its shared::cluster address.
+DG_DEVICE void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
 DG_DEVICE bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(

@@ -250,3 +250,25 @@ ctx.sync()
     assert run.returncode == 0, run.stderr
     lines = [line for line in run.stderr.splitlines() if "f32 scales" in line]
     assert len(lines) == 2 and all("block=128x128 ctas=1" in line for line in lines), lines
+
+
+@pytest.mark.parametrize("k_blocks", [1, 2, 3, 6])
+def test_pair_tiles_of_few_k_blocks(ctx, k_blocks):
+    # 48 tiles of 256 x 256 (the choice for this many rows): their K blocks go two a turn, so odd and even counts, one and two among them;
+    # rows and columns off the tile grid, and scales whose product leaves the range in which one factor stands for both
+    rng = np.random.default_rng(k_blocks)
+    m, n, k = 2040, 1400, 128 * k_blocks
+    a, b = lcg_e4m3(31, m, k), lcg_e4m3(32, n, k)
+    sfa = (rng.random((m, k_blocks)) * 0.03 + 0.001).astype(np.float32)
+    sfb = (rng.random((-(-n // 128), k_blocks)) * 0.03 + 0.001).astype(np.float32)
+    sfa[300:400] *= 1e-15
+    sfb[2:4] *= 1e-15
+    a_sf_t = dg.transform_sf_dev(ctx, dev(sfa), m, k_blocks, 1)
+    out = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+    dg.fp8_gemm_nt_dev(ctx, dg.Fp8Tensor(dev(a), m, k, k), a_sf_t, dg.Fp8Tensor(dev(b), n, k, k), dev(sfb), out, n)
+    ctx.sync()
+    fa = dev(a).view(torch.float8_e4m3fn).double() * dev(sfa).double().repeat_interleave(128, 1)
+    fb = dev(b).view(torch.float8_e4m3fn).double() * dev(sfb).double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)
+    want, size = fa @ fb.T, fa.abs() @ fb.abs().T
+    # one bf16 rounding (8 significant bits: 2^-8 of the value at most), and f32 sums: fewer than 32 roundings of 2^-24 of the terms' magnitudes
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 32 * 2.0 ** -24 * size).all())
