@@ -222,6 +222,7 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                 }
                 tmem_st_wait();
             };
+            auto block_done = [&]() { return mbar_wait(bar_tmem_full + e, phase, abort_flag, p.status, 0x600 + e); };
             // the K block in buffer e, whose first 16 columns are already on their way to va
             auto fold_block = [&](uint32_t taddr, float s) {
                 // two elements per instruction (packed f32x2: the same IEEE operations, half the issue slots)
@@ -268,7 +269,7 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                 // next they had to arrive within the turn they were asked for in), addresses in uniform registers, the factor worked out
                 // beside the first load.  210 -> 140 instructions per warp and K block.
                 auto k_block = [&](float& a, float& b) {
-                    if (!mbar_wait(bar_tmem_full + e, phase, abort_flag, p.status, 0x600 + e)) return false;
+                    if (!block_done()) return false;
                     tc_fence_after();
                     const uint32_t taddr = tmem_mine + e * kBlockN;
                     tmem_ld_32x32b_x16(taddr, va);
@@ -294,7 +295,7 @@ dg_gemm_f32scale_kernel(const __grid_constant__ F32ScaleParams q, const __grid_c
                     if (left > 2) load_scales(sa2, sb2);
                     const float both = sa * sb;
                     const bool one_factor = __all_sync(0xFFFFFFFFu, in_range(both) || sa == 0.0f || sb == 0.0f);
-                    if (!mbar_wait(bar_tmem_full + e, phase, abort_flag, p.status, 0x600 + e)) { ok = false; break; }
+                    if (!block_done()) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t taddr = tmem_mine + e * kBlockN;
                     if (!one_factor) rescale(taddr, sa);
