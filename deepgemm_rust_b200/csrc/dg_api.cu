@@ -19,6 +19,7 @@
 #include "dg_gemm_kernel.cuh"
 #include "dg_gemm_swap.cuh"
 #include "dg_gemm_f32scale.cuh"
+#include "dg_gemm_wide.cuh"
 #include "dg_moe_kernels.cuh"
 
 namespace {
@@ -235,9 +236,13 @@ struct KernelPlan {
     uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
     uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
+    uint32_t block_n2;         // wide tiles: columns of the second half (0: not a wide tile)
     uint32_t table_groups;     // groups whose rows and tiles are kept in shared memory (swapped family)
 };
-static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan);
+// What a call rules out that its description does not tell: K ranges (the caller adds into the output: their sum is written, not added), wide
+// tiles (no bf16 operands).
+constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2;
+static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
     KernelPlan plan;
     return search_config(d, 0, out, &plan);
@@ -258,10 +263,10 @@ static uint64_t knob_signature() {
 // search_config with the choices of recent problems remembered: the search walks ~500 candidates (3.7 us on a B200 host, more
 // than the launch itself), and a program asks for the same few problems again and again.  The choice is a function of the
 // description, the alignment and the knobs alone.  One small table per thread, overwritten on collision.
-static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan) {
+static int choose_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan) {
     struct Key {
         dg_desc desc;
-        uint32_t no_k_ranges, alignment;
+        uint32_t limits, alignment;
         uint32_t knobs[2];
     };
     struct Entry {
@@ -273,14 +278,14 @@ static int choose_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
     constexpr uint32_t kEntries = 64;
     static thread_local Entry table[kEntries];
     const uint64_t knobs = knob_signature();
-    const Key key = {*d, no_k_ranges, g_mk_alignment.load(), {static_cast<uint32_t>(knobs), static_cast<uint32_t>(knobs >> 32)}};
+    const Key key = {*d, limits, g_mk_alignment.load(), {static_cast<uint32_t>(knobs), static_cast<uint32_t>(knobs >> 32)}};
     static_assert(sizeof(Key) == 18 * sizeof(uint32_t), "compared and hashed as 18 words");
     uint32_t words[18], hash = 0;
     memcpy(words, &key, sizeof(key));
     for (uint32_t w : words) hash = (hash ^ w) * 0x9E3779B1u;
     Entry& e = table[(hash >> 16) % kEntries];
     if (!e.used || memcmp(&e.key, &key, sizeof(key)) != 0) {
-        const int rc = search_config(d, no_k_ranges, &e.cfg, &e.plan);
+        const int rc = search_config(d, limits, &e.cfg, &e.plan);
         e.used = rc == DG_OK;
         if (rc) return rc;
         e.key = key;
@@ -340,6 +345,89 @@ static bool prefer_swapped(const dg_desc* d) {
     const bool short_k = 6 * blocks >= sms && slabs * 0.31 < 3.8 + 0.17 * blocks * slabs * (128 * 128 / 1e6);
     return d->gemm_type == DG_GEMM_NORMAL && blocks <= sms &&
            ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));
+}
+
+// How a dense problem's tiles of two halves are dealt out to the CTA pairs.
+struct WideWaves {
+    uint32_t whole;      // tiles computed whole, in full waves
+    uint32_t units;      // those, and single halves
+    uint32_t halves;     // length of the schedule in halves
+};
+static WideWaves wide_waves(uint32_t m, uint32_t n, uint32_t block_n, uint32_t pairs) {
+    const uint32_t across = ceil_div(n, block_n), m_blocks = ceil_div(m, 256), tiles = m_blocks * (across / 2), all = m_blocks * across;
+    WideWaves w;
+    const uint32_t waves = all / (2 * pairs), full = waves * pairs < tiles ? waves * pairs : tiles, rest = all - 2 * full;
+    // What is left over the full waves goes out as single halves, at most two per pair: whole tiles and the halves without a second one do not
+    // deal out evenly.
+    w.whole = full;
+    w.units = full + rest;
+    w.halves = 2 * waves + (all == 2 * pairs * waves ? 0 : (rest <= pairs ? 1 : 2));
+    return w;
+}
+
+// Wide tiles (dg_gemm_wide.cuh) for a problem that costs `other` in the first family's other tiles; false if those are the better ones (or
+// the only ones), unless `forced`.
+// Measured under the power cap that long runs settle at, both in turn.  Contiguous groups of 450-6500 rows, from three waves of tiles on
+// (27 problems, k 1024-6656, n 1024-6848): 0.96 of the other tiles' time on average, 0.92 to 1.02; with fewer waves up to 1.14.  Dense problems, from two and
+// a half waves on (50 of them, k 1024-16384): the constants below are fitted to those, and with them the 33 that are chosen take
+// 0.98 of the time, 0.90 to 1.05.  Halves of 160 columns were slower than both (5841 x 3720 x 11776 mxfp4: 114 -> 124 us).  Masked and batched problems, and
+// e4m3 operands with per-32 scales, were not measured and keep the other tiles.
+static bool search_wide(const dg_desc* d, uint32_t sms, double other, bool forced, dg_config* out, KernelPlan* plan) {
+    if (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32) return false;
+    if (d->major_a_mn || d->major_b_mn || sms < 2 || d->gemm_type == DG_GEMM_BATCHED) return false;
+    if (!forced && (d->gemm_type == DG_GEMM_M_GROUPED_MASKED || (d->a_bits == 8 && d->gran_a != 128) || (d->b_bits == 8 && d->gran_b != 128))) return false;
+    const uint32_t block_k = d->a_bits == 4 && d->b_bits == 4 ? 256 : 128, groups = d->num_groups ? d->num_groups : 1, pairs = sms / 2;
+    const uint32_t sfa_words = 4 * d->gran_a >= block_k ? 1 : block_k / (4 * d->gran_a), sfb_words = 4 * d->gran_b >= block_k ? 1 : block_k / (4 * d->gran_b);
+    const uint32_t total_kb = ceil_div(d->k, block_k);
+    const bool dense = d->gemm_type == DG_GEMM_NORMAL;
+    bool found = false;
+    double best = 0;
+    for (uint32_t most = 224; most >= 192; most -= 32) {
+        uint32_t bn = most, bn2 = most, tiles;
+        double halves;
+        if (dense) {
+            const WideWaves w = wide_waves(d->m, d->n, bn, pairs);
+            tiles = w.units;
+            halves = w.halves;
+        } else {
+            // a group's columns in tiles of about equal width
+            if (most != 224) break;
+            const uint32_t across = ceil_div(d->n, 2 * most), width = ceil_div(ceil_div(d->n, across), 32) * 32;
+            bn = ceil_div(width / 2, 32) * 32;
+            bn2 = width - bn;
+            if (bn2 == 0) break;
+            tiles = static_cast<uint32_t>(groups * (group_rows(d) / 256 + 0.5) * across + 0.999);
+            halves = 2.0 * ceil_div(tiles, pairs);
+        }
+        if (bn + bn2 + 4 * sfa_words + 8 * ceil_div(bn, 128) * sfb_words > 512) continue;
+        uint32_t epi_bufs = 2, stages = 4;
+        auto smem = [&]() { return dg::gemm_wide_smem_bytes(bn, d->cd_dtype, stages, sfa_words, sfb_words, epi_bufs); };
+        if (smem() > kSmemCapacity) epi_bufs = 1;
+        while (stages < dg::kMaxStages && smem() <= kSmemCapacity) ++stages;
+        while (stages > 3 && smem() > kSmemCapacity) --stages;
+        if (smem() > kSmemCapacity) continue;
+        const double cost = halves * (total_kb * (2.0 * bn + 130.0) + 1500.0 + (d->cd_dtype == DG_OUT_F32 ? 1000.0 : 0.0)) + 8000.0;
+        if (!forced && (dense ? halves < 5 || cost >= other : halves < 6 || group_rows(d) < 450.0)) continue;
+        if (found && cost >= best) continue;
+        found = true;
+        best = cost;
+        plan->swap = false;
+        plan->ctas = 2; plan->umma_n = bn; plan->block_n2 = bn2; plan->halves = 1; plan->stages = stages; plan->accum = 1;
+        plan->splits = 1; plan->tiles = tiles; plan->epi_bufs = epi_bufs; plan->table_groups = 0;
+        plan->smem = smem();
+        out->swap_ab = 0;
+        out->block_m = 256;
+        out->block_n = bn;            // of each of the tile's two accumulators
+        out->block_k = block_k;
+        out->cluster_m = 2;
+        out->cluster_n = 1;
+        out->num_stages = stages;
+        out->num_accum_stages = 2;
+        out->smem_size = plan->smem;
+        out->num_tiles = tiles;
+        out->num_splits = 1;
+    }
+    return found;
 }
 
 // Tile choice of the swapped family; false if nothing fits (or the DG_* knobs leave nothing).
@@ -422,6 +510,7 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
                     // the group table takes what the stages leave of the shared memory
                     const uint32_t room = !dense && dg::swap_has_table(ctas, halves) ? (kSmemCapacity - plan->smem) / 16 : 0;
                     plan->table_groups = groups < room ? groups : room;
+                    plan->block_n2 = 0;
                     plan->smem += plan->table_groups * 16;
                     out->swap_ab = 1;
                     out->block_m = bn;            // activation rows per tile (an upper bound: a tile's UMMA N follows its rows)
@@ -441,8 +530,7 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
     return found;
 }
 
-// no_k_ranges: the caller adds into the output (K ranges would need the sum to be written, not added)
-static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out, KernelPlan* plan) {
+static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan) {
     if (d == nullptr || out == nullptr) return fail(DG_ERR_SHAPE, "null argument");
     if ((d->a_bits != 8 && d->a_bits != 4) || (d->b_bits != 8 && d->b_bits != 4)) return fail(DG_ERR_SHAPE, "operand bits must be 8 or 4");
     if ((d->major_a_mn && d->a_bits == 4) || (d->major_b_mn && d->b_bits == 4)) return fail(DG_ERR_SHAPE, "FP4 operands must be K-major");
@@ -524,7 +612,7 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
             const double per_kb = halves * (mma > feed ? mma : feed) + (fitted ? 234.0 + 40.0 * copies : 150.0);
             // K ranges (dense GEMMs with f32-summable outputs only): each range is a multiple of 4 k-blocks so scale words
             // never straddle ranges; the partial sums cost a second small kernel (launch + S reads of the M x N f32 tile set)
-            const bool may_split = d->gemm_type == DG_GEMM_NORMAL && d->cd_dtype != DG_OUT_FP8 && !swiglu && d->n % 4 == 0 && !no_k_ranges;
+            const bool may_split = d->gemm_type == DG_GEMM_NORMAL && d->cd_dtype != DG_OUT_FP8 && !swiglu && d->n % 4 == 0 && !(limits & kNoKRanges);
             for (uint32_t splits = 1; splits <= 16; ++splits) {
                 if (splits > 1 && (!may_split || (halves > 1 && !fitted))) break;
                 if (force_splits && static_cast<uint32_t>(atoi(force_splits)) != splits) continue;
@@ -590,7 +678,14 @@ static int search_config(const dg_desc* d, uint32_t no_k_ranges, dg_config* out,
         }
     }
     if (best_n == 0) return fail(DG_ERR_SHAPE, "no tile configuration fits (DG_BLOCK_N=%s DG_CTAS=%s)", force_n ? force_n : "", force_ctas ? force_ctas : "");
+    const bool pinned = force_n || force_ctas || force_stages || force_splits || force_halves;
+    {
+        const char* wide = getenv("DG_WIDE_TILE");       // 0: never, 1: wherever they apply
+        const bool forced = wide && atoi(wide) != 0, forbidden = (wide && atoi(wide) == 0) || (limits & kNoWideTiles) || pinned;
+        if (!forbidden && search_wide(d, sms, best_cost, forced, out, plan)) return DG_OK;
+    }
     const uint32_t stages = best_stages;
+    plan->block_n2 = 0;
     plan->swap = false;
     plan->ctas = best_ctas; plan->umma_n = best_n; plan->halves = best_halves; plan->stages = best_stages; plan->accum = best_accum;
     plan->splits = best_splits; plan->tiles = best_tiles; plan->table_groups = 0;
@@ -707,10 +802,12 @@ cudaError_t launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_
 
 // The opt-in to the full shared-memory carve-out is per kernel instantiation and per device; the first
 // call also makes the runtime load that kernel's image.
-// kSlabs: 0 the first tile family, else the swapped family with that many K slabs per stage.
+// kSlabs: 0 the first tile family, kWideTiles its wide tiles, else the swapped family with that many K slabs per stage.
+constexpr uint32_t kWideTiles = 3;
 template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kSlabs>
 constexpr auto gemm_kernel() {
-    if constexpr (kSlabs != 0) return &dg::dg_gemm_swap_kernel<kFmt, kOut, kCtas, kSlabs>;
+    if constexpr (kSlabs == kWideTiles) return &dg::dg_gemm_wide_kernel<kFmt, kOut>;
+    else if constexpr (kSlabs != 0) return &dg::dg_gemm_swap_kernel<kFmt, kOut, kCtas, kSlabs>;
     else return &dg::dg_gemm_kernel<kFmt, kOut, kCtas>;
 }
 template <uint32_t kFmt, uint32_t kOut, uint32_t kCtas, uint32_t kSlabs = 0>
@@ -733,7 +830,7 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(kSlabs != 0 ? dg::kSwapThreads : dg::kNumThreads, 1, 1);
+    cfg.blockDim = dim3(kSlabs == kWideTiles ? dg::kWideThreads : (kSlabs != 0 ? dg::kSwapThreads : dg::kNumThreads), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -746,7 +843,7 @@ cudaError_t launch_kernel(const dg::GemmParams& p, uint32_t grid, uint32_t smem,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    if constexpr (kSlabs != 0) return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[5], maps[6]);
+    if constexpr (kSlabs != 0 && kSlabs != kWideTiles) return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[5], maps[6]);
     else return cudaLaunchKernelEx(&cfg, kernel, p, maps[0], maps[1], maps[2], maps[3], maps[4]);
 }
 
@@ -779,8 +876,15 @@ cudaError_t launch_by_out(int kind, const dg::GemmParams& p, uint32_t grid, uint
 }
 
 template <uint32_t kFmt>
+cudaError_t launch_wide(int kind, const dg::GemmParams& p, uint32_t grid, uint32_t smem, cudaStream_t stream, const CUtensorMap* maps) {
+    if (kind == DG_OUT_BF16) return launch_kernel<kFmt, dg::kOutBf16, 2, kWideTiles>(p, grid, smem, stream, maps);
+    return launch_kernel<kFmt, dg::kOutF32, 2, kWideTiles>(p, grid, smem, stream, maps);
+}
+
+template <uint32_t kFmt>
 cudaError_t configure_contiguous_kernels_of() {
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = configure_kernel<kFmt, dg::kOutBf16, 2, kWideTiles>();
+    if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 2, kWideTiles>();
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 1>();
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutBf16, 2>();
     if (e == cudaSuccess) e = configure_kernel<kFmt, dg::kOutF32, 1>();
@@ -889,7 +993,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
                     (!pr.bf16 && b->major_mn) ? 1u : 0u};
     dg_config cfg;
     KernelPlan plan;
-    rc = choose_config(&desc, e.accumulate ? 1u : 0u, &cfg, &plan);
+    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles : 0u), &cfg, &plan);
     if (rc) return rc;
     const bool swap = plan.swap;
     // the swapped family's kernel takes the operands with their roles exchanged: its operand A (UMMA M side) is the weights
@@ -1026,7 +1130,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.m = swap ? pr.n : pr.m;     // rows of the kernel's operand A per group (swapped family: weight rows)
     p.n = swap ? pr.m : n_out;
     p.k = pr.k;
-    p.tile_n = swiglu ? plan.umma_n / 2 : plan.umma_n;
+    p.tile_n = swiglu ? plan.umma_n / 2 : plan.umma_n + plan.block_n2;
+    p.block_n2 = plan.block_n2;
     p.num_groups = pr.groups;
     p.gemm_type = pr.type;
     p.block_n = plan.umma_n;
@@ -1095,10 +1200,14 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     const uint32_t ctas = plan.ctas;
     uint32_t grid = static_cast<uint32_t>(ctx->num_sms) / ctas * ctas;
     if (pr.type == DG_GEMM_NORMAL || pr.type == DG_GEMM_BATCHED)
-        grid = plan.tiles * splits * ctas < grid ? plan.tiles * splits * ctas : grid;
+    {
+        const uint32_t units = plan.tiles * splits;
+        if (plan.block_n2 != 0) p.whole_tiles = wide_waves(pr.m, pr.n, plan.umma_n, grid / 2).whole;
+        grid = units * ctas < grid ? units * ctas : grid;
+    }
     const int kernel_out = splits > 1 && !swap ? DG_OUT_F32 : out->kind;
     const uint32_t smem = plan.smem;
-    if (!swap && (pr.type == DG_GEMM_NORMAL || pr.type == DG_GEMM_BATCHED) && kernel_out == DG_OUT_F32 &&
+    if (!swap && plan.block_n2 == 0 && (pr.type == DG_GEMM_NORMAL || pr.type == DG_GEMM_BATCHED) && kernel_out == DG_OUT_F32 &&
         static_cast<uint64_t>(plan.tiles) * splits <= static_cast<uint32_t>(ctx->num_sms) / ctas) {
         // one tile per CTA (pair): does the operand ring hold the CTA's 128 rows of it?
         const uint32_t ring = plan.stages * plan.halves * (dg::kBlockM + plan.umma_n / ctas) * dg::kBlockKBytes;
@@ -1110,6 +1219,9 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
         if (pr.bf16) ce = launch_swapped<dg::kFmtBf16>(plan, kernel_out, p, grid, ctx->stream, maps);
         else if (mxf4) ce = launch_swapped<dg::kFmtMxf4>(plan, kernel_out, p, grid, ctx->stream, maps);
         else ce = launch_swapped<dg::kFmtMxf8f6f4>(plan, kernel_out, p, grid, ctx->stream, maps);
+    } else if (plan.block_n2 != 0) {
+        if (mxf4) ce = launch_wide<dg::kFmtMxf4>(kernel_out, p, grid, smem, ctx->stream, maps);
+        else ce = launch_wide<dg::kFmtMxf8f6f4>(kernel_out, p, grid, smem, ctx->stream, maps);
     } else if (pr.bf16) ce = ctas == 2 ? launch_by_out<dg::kFmtBf16, 2>(kernel_out, p, grid, smem, ctx->stream, maps)
                                 : launch_by_out<dg::kFmtBf16, 1>(kernel_out, p, grid, smem, ctx->stream, maps);
     else if (mxf4) ce = ctas == 2 ? launch_by_out<dg::kFmtMxf4, 2>(kernel_out, p, grid, smem, ctx->stream, maps)

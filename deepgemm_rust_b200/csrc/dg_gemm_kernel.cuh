@@ -80,6 +80,9 @@ struct GemmParams {
     uint32_t sfd_stride;       // output scale words: stride between word columns (fp8 output)
     uint32_t stage_in_ring;    // no CTA computes more than one tile, and the operand ring holds a staging buffer for every store of a tile (f32)
     uint32_t epi_bufs;         // staging buffers of an epilogue warp: 2, or 1 where f32 staging would cost a stage of two slabs
+    // wide tiles only (dg_gemm_wide.cuh)
+    uint32_t block_n2;         // columns of a tile's second half
+    uint32_t whole_tiles;      // dense: tiles from this one on are computed as two halves by two CTA pairs
     // second tile family only (dg_gemm_swap.cuh), where m counts weight rows and n activation rows per group
     uint32_t acc_stride;       // TMEM column where the second accumulator starts (below block_n: the two share columns)
     uint32_t acc_edge_chunks;  // 32-column chunks that hold the shared columns
@@ -171,19 +174,8 @@ struct Scheduler {
             } else if (idx >= per_group * p.num_groups) {
                 return false;
             }
-            const uint32_t g = idx / per_group, r = idx - g * per_group;
-            // bands of 2048 rows, rows fastest inside a band: the tiles in flight at any moment form a
-            // patch about as tall as it is wide (148 tiles of 128 x 224..256), which is what minimises the
-            // A rows plus B rows a wave pulls from DRAM, and a band's A rows stay in L2 for its next wave
-            const uint32_t kBand = 2048 / tile_m;
-            const uint32_t per_band = kBand * num_n_blocks;
-            const uint32_t band = r / per_band, in_band = r - band * per_band;
-            const uint32_t first_m = band * kBand;
-            const uint32_t rows_here = num_m_blocks - first_m < kBand ? num_m_blocks - first_m : kBand;
-            const uint32_t nb = in_band / rows_here, mb = first_m + (in_band - nb * rows_here);
-            t.m0 = mb * tile_m;
-            t.m_end = p.m;
-            t.n0 = nb * p.tile_n;
+            const uint32_t g = idx / per_group;
+            dense_tile(idx - g * per_group, t);
             t.ga = t.gb = g;
             t.gd = p.num_splits > 1 ? split_k : g;
             return true;
@@ -205,6 +197,22 @@ struct Scheduler {
         t.ga = p.gemm_type == kGemmContiguous ? 0u : cur_group;
         t.gd = t.ga;
         return true;
+    }
+
+    // where tile r of a dense problem (or of one of a batch) lies
+    DG_DEVICE void dense_tile(uint32_t r, Tile& t) const {
+        // bands of 2048 rows, rows fastest inside a band: the tiles in flight at any moment form a
+        // patch about as tall as it is wide (148 tiles of 128 x 224..256), which is what minimises the
+        // A rows plus B rows a wave pulls from DRAM, and a band's A rows stay in L2 for its next wave
+        const uint32_t kBand = 2048 / tile_m;
+        const uint32_t per_band = kBand * num_n_blocks;
+        const uint32_t band = r / per_band, in_band = r - band * per_band;
+        const uint32_t first_m = band * kBand;
+        const uint32_t rows_here = num_m_blocks - first_m < kBand ? num_m_blocks - first_m : kBand;
+        const uint32_t nb = in_band / rows_here, mb = first_m + (in_band - nb * rows_here);
+        t.m0 = mb * tile_m;
+        t.m_end = p.m;
+        t.n0 = nb * p.tile_n;
     }
 };
 

@@ -180,7 +180,6 @@ DG_DEVICE uint32_t ld_shared_u16(uint32_t addr) {
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
     return v;
 }
-DG_DEVICE uint64_t desc64(uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(hi) << 32 | lo; }
 
 // staging bytes of one epilogue warp: 32 output rows x 32 columns (f32 goes out straight from registers)
 constexpr uint32_t swap_epi_buf_bytes(uint32_t out_kind) { return out_kind == kOutF32 ? 0u : 2048u; }
