@@ -20,6 +20,7 @@
 #include "dg_gemm_swap.cuh"
 #include "dg_gemm_f32scale.cuh"
 #include "dg_gemm_wide.cuh"
+#include "dg_gemm_skinny.cuh"
 #include "dg_moe_kernels.cuh"
 
 namespace {
@@ -236,12 +237,13 @@ struct KernelPlan {
     uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
     uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
+    uint32_t skinny;           // tiles of 8 activation rows of the kernel for few of them (0: another kernel)
     uint32_t block_n2;         // wide tiles: columns of the second half (0: not a wide tile)
     uint32_t table_groups;     // groups whose rows and tiles are kept in shared memory (swapped family)
 };
 // What a call rules out that its description does not tell: K ranges (the caller adds into the output: their sum is written, not added), wide
 // tiles (no bf16 operands).
-constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2;
+constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2, kNoSkinny = 4;
 static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
     KernelPlan plan;
@@ -345,6 +347,32 @@ static bool prefer_swapped(const dg_desc* d) {
     const bool short_k = 6 * blocks >= sms && slabs * 0.31 < 3.8 + 0.17 * blocks * slabs * (128 * 128 / 1e6);
     return d->gemm_type == DG_GEMM_NORMAL && blocks <= sms &&
            ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));
+}
+
+// Is the kernel for a handful of activation rows (dg_gemm_skinny.cuh) the one for this problem?  Measured behind the activation quantiser
+// over 170 problems (m 1-32, n 512-24576, k 1024-16384): it takes 8.5 us (what the host needs for the two calls) wherever the weights
+// are below 15 MB, where the first family's K ranges with their second launch take 12.4 and the swapped family's blocks 10.  Up to 8 rows
+// that lasts, at 4 TB/s, to about 60 MB (1 x 4640 x 7680: 18.7 -> 11.8 us; 4 x 9024 x 6656: 21.4 -> 17.2; 2 x 5976 x 11264: 21.8 -> 22.0), to 40 where the
+// swapped family fills the SMs (3 x 12904 x 3584: 15.2 -> 15.6).  With two tiles of rows the multiply itself shows: to 24 MB and 12288 of K
+// (16 x 5712 x 3584: 13.9 -> 10.5; 15 x 896 x 15872: 12.8 -> 13.6; 9 x 2864 x 13824: 17.5 -> 22.7), with four to 8 MB (28 x 1352 x 3584: 12.3 -> 8.7;
+// 32 x 2112 x 7168: 12.3 -> 12.5).
+static bool prefer_skinny(const dg_desc* d) {
+    const char *knob = getenv("DG_SKINNY"), *family = getenv("DG_SWAP");
+    if ((knob && atoi(knob) == 0) || family) return false;       // a pinned family is one of the other two
+    if (d->gemm_type != DG_GEMM_NORMAL || d->k % 128 != 0 || (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32)) return false;
+    if (d->a_bits != 8 || d->b_bits != 8 || d->gran_a != 128 || d->gran_b != 128 || d->major_a_mn || d->major_b_mn) return false;
+    const uint32_t sms = d->num_sms ? d->num_sms : 148;
+    const double mb = static_cast<double>(d->n) * d->k * 1e-6;
+    if (d->m <= 8) return mb <= (2 * ceil_div(d->n, 128) >= sms ? 40.0 : 60.0);
+    if (d->m <= 16) return mb <= 24.0 && d->k <= 12288;
+    return d->m <= 32 && mb <= 8.0;
+}
+// Warps of its blocks.  Blocks of 16 columns that all fit at once share K among as many warps as there are; with more blocks it is
+// several of them per SM that keep loads in flight (8 x 2112 x 7168 with 4 / 8 / 16 warps: 9.5 / 8.1 / 8.0 us; 1 x 4096 x 7168: 12.7 / 10.7 / 11.6;
+// 16 x 7168 x 2048: 8.4 / 9.4 / 11.5).
+static uint32_t skinny_warps(uint32_t n, uint32_t sms) {
+    const uint32_t blocks = ceil_div(n, dg::kSkinnyCols);
+    return blocks <= sms ? 16 : (blocks <= 2 * sms ? 8 : 4);
 }
 
 // How a dense problem's tiles of two halves are dealt out to the CTA pairs.
@@ -550,6 +578,24 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
 
     const char* force_splits = getenv("DG_SPLITS");
     const char* force_halves = getenv("DG_K_SLABS");
+    const bool pinned = force_n || force_ctas || force_stages || force_splits || force_halves;
+    plan->skinny = 0;
+    if (!(limits & kNoSkinny) && !pinned && prefer_skinny(d)) {
+        plan->swap = false;
+        plan->skinny = d->m <= 8 ? 1 : (d->m <= 16 ? 2 : 4);
+        plan->ctas = 1; plan->umma_n = dg::kSkinnyCols; plan->halves = 1; plan->stages = 1; plan->accum = 1; plan->smem = 0; plan->splits = 1;
+        plan->tiles = ceil_div(d->n, dg::kSkinnyCols); plan->epi_bufs = 0; plan->block_n2 = 0; plan->table_groups = 0;
+        out->swap_ab = 0;
+        out->block_m = 8 * plan->skinny;
+        out->block_n = dg::kSkinnyCols;
+        out->block_k = 128;
+        out->cluster_m = out->cluster_n = 1;
+        out->num_stages = out->num_accum_stages = 1;
+        out->smem_size = static_cast<uint32_t>(sizeof(float)) * skinny_warps(d->n, sms) * 8 * plan->skinny * (dg::kSkinnyCols + 1);
+        out->num_tiles = plan->tiles;
+        out->num_splits = 1;
+        return DG_OK;
+    }
     uint32_t best_n = 0, best_accum = 0, best_tiles = 0, best_ctas = 0, best_stages = 0, best_splits = 1, best_halves = 1, best_epi_bufs = 2;
     double best_cost = 0;
     // a stage holds one or two 128-byte K slabs per operand; two slabs halve the per-stage bookkeeping per UMMA
@@ -678,7 +724,6 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
         }
     }
     if (best_n == 0) return fail(DG_ERR_SHAPE, "no tile configuration fits (DG_BLOCK_N=%s DG_CTAS=%s)", force_n ? force_n : "", force_ctas ? force_ctas : "");
-    const bool pinned = force_n || force_ctas || force_stages || force_splits || force_halves;
     {
         const char* wide = getenv("DG_WIDE_TILE");       // 0: never, 1: wherever they apply
         const bool forced = wide && atoi(wide) != 0, forbidden = (wide && atoi(wide) == 0) || (limits & kNoWideTiles) || pinned;
@@ -947,6 +992,29 @@ int reserve(dg_ctx* ctx, ScratchBuffer* buf, size_t bytes, bool zeroed = false) 
     return DG_OK;
 }
 
+int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue& e, const Problem& pr, uint32_t tiles) {
+    // what the tensor maps of the other kernels ask for
+    if (reinterpret_cast<uintptr_t>(a->data) % 16 != 0 || reinterpret_cast<uintptr_t>(b->data) % 16 != 0 || reinterpret_cast<uintptr_t>(a->sf) % 16 != 0 ||
+        reinterpret_cast<uintptr_t>(b->sf) % 16 != 0 || reinterpret_cast<uintptr_t>(out->buf) % 16 != 0)
+        return fail(DG_ERR_SHAPE, "operands, scales and output must be 16-byte aligned");
+    dg::SkinnyParams p = {static_cast<const uint8_t*>(a->data), static_cast<const uint8_t*>(b->data), a->sf, b->sf, out->buf, pr.m, pr.n, pr.k / 128,
+                          a->ld, b->ld, align4(pr.m), align4(pr.n), out->ld, e.has_alpha ? 1u : 0u, e.accumulate ? 1u : 0u, e.alpha};
+    DG_CUDA(cudaSetDevice(ctx->ordinal));
+    const bool f32 = out->kind == DG_OUT_F32;
+    const dim3 grid(ceil_div(pr.n, dg::kSkinnyCols));
+    auto run = [&](auto kernel, uint32_t warps) { return launch(kernel, grid, warps * 32, 0, ctx->stream, p); };
+    auto with_warps = [&](auto count) {
+        constexpr uint32_t kWarps = decltype(count)::value;
+        if (tiles == 4) return f32 ? run(dg::dg_gemm_skinny_kernel<4, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<4, kWarps, false>, kWarps);
+        if (tiles == 1) return f32 ? run(dg::dg_gemm_skinny_kernel<1, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<1, kWarps, false>, kWarps);
+        return f32 ? run(dg::dg_gemm_skinny_kernel<2, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<2, kWarps, false>, kWarps);
+    };
+    const uint32_t warps = skinny_warps(pr.n, static_cast<uint32_t>(ctx->num_sms));
+    const cudaError_t ce = warps == 4 ? with_warps(std::integral_constant<uint32_t, 4>()) : (warps == 8 ? with_warps(std::integral_constant<uint32_t, 8>()) : with_warps(std::integral_constant<uint32_t, 16>()));
+    if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
+    return DG_OK;
+}
+
 int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue* epi, const Problem& pr) {
     if (out == nullptr || out->buf == nullptr) return fail(DG_ERR_SHAPE, "null output");
     if (out->kind < DG_OUT_BF16 || out->kind > DG_OUT_SWIGLU_FP8) return fail(DG_ERR_SHAPE, "invalid output kind %d", out->kind);
@@ -993,7 +1061,8 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
                     (!pr.bf16 && b->major_mn) ? 1u : 0u};
     dg_config cfg;
     KernelPlan plan;
-    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles : 0u), &cfg, &plan);
+    const uint32_t tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
+    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles | kNoSkinny : 0u) | (tc_util < 100 ? kNoSkinny : 0u), &cfg, &plan);
     if (rc) return rc;
     const bool swap = plan.swap;
     // the swapped family's kernel takes the operands with their roles exchanged: its operand A (UMMA M side) is the weights
@@ -1006,6 +1075,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
                 pr.type, pr.m, pr.n, pr.k, pr.groups, cfg.swap_ab, cfg.block_m, cfg.block_n, cfg.block_k, plan.ctas, cfg.num_stages,
                 cfg.num_accum_stages, cfg.smem_size, cfg.num_tiles, cfg.num_splits);
 
+    if (plan.skinny != 0) return launch_skinny(ctx, a, b, out, e, pr, plan.skinny);
     const bool mxf4 = a->bits == 4 && b->bits == 4;
     const uint32_t block_k = cfg.block_k;
     const uint32_t splits = plan.splits;
@@ -1181,7 +1251,7 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     p.mn_a = (!pr.bf16 && ka->major_mn) ? 1 : 0;
     p.mn_b = (!pr.bf16 && kb->major_mn) ? 1 : 0;
     p.accumulate = e.accumulate ? 1 : 0;
-    p.tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
+    p.tc_util = tc_util;
     p.has_alpha = (e.has_alpha && (swap || splits == 1)) ? 1 : 0;   // with K ranges summed by the second kernel alpha is applied there
     p.alpha = e.alpha;
     p.sfd = out->sfd;

@@ -1,0 +1,108 @@
+"""The dense kernel for a handful of activation rows, against a f64 product of the dequantised operands."""
+import pytest
+import torch
+
+import deepgemm_rust_b200 as dg
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = dg.DgContext(0)
+    yield c
+    c.sync()
+    c.close()
+
+
+def operand(rows, k, ld, seed, exponents=(118, 136)):
+    """Any e4m3 code but NaN and any scale of a range, in the packed layout: (operand, its values in f64)."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    data = torch.randint(0, 256, (rows, ld), generator=gen, device="cuda", dtype=torch.uint8)
+    data[(data & 0x7F) == 0x7F] = 0
+    stride, cols = dg.sf_aligned_rows(rows), dg.sf_packed_cols(k, 128)
+    e = torch.randint(*exponents, (4 * cols, stride), generator=gen, device="cuda", dtype=torch.int32)
+    sf = (e.view(cols, 4, stride) << torch.tensor([0, 8, 16, 24], device="cuda", dtype=torch.int32).view(1, 4, 1)).sum(1, dtype=torch.int32)
+    scale = torch.exp2(e[:k // 128, :rows].double() - 127).T.repeat_interleave(128, 1)
+    return dg.LpOperand(data, sf.view(-1), rows, k, ld, 8, 128), data[:, :k].view(torch.float8_e4m3fn).double() * scale
+
+
+def is_skinny(m, n, k):
+    c = dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k))
+    return not c.swap_ab and c.block_n == 16
+
+
+@pytest.mark.parametrize("m,n,k,skinny", [
+    (8, 2112, 7168, True), (1, 4096, 14592, True), (8, 4096, 14720, False), (8, 9344, 4352, True), (8, 9352, 4352, False), (16, 5856, 4096, True),
+    (16, 5864, 4096, False), (9, 512, 12288, True), (9, 512, 12416, False), (32, 1952, 4096, True), (17, 1960, 4096, False), (33, 512, 1024, False),
+    (8, 2112, 7200, False),
+])
+def test_which_problems_get_it(m, n, k, skinny):
+    assert is_skinny(m, n, k) == skinny
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n,k", [
+    (8, 128), (16, 256), (24, 2048),              # one block, a block and a part; fewer K blocks than warps, and as many
+    (2368, 2176), (2376, 384), (4736, 640), (4744, 1152),      # either side of the lines between 16, 8 and 4 warps; odd numbers of K blocks per warp
+])
+@pytest.mark.parametrize("f32", [True, False])
+def test_product(ctx, m, n, k, f32):
+    assert is_skinny(m, n, k)
+    (a, fa), (b, fb) = operand(m, k, k + 16, 1), operand(n, k, k + 32, 2)
+    ld = n + 8
+    d = torch.full((m, ld), 7.0, dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+    dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d, ld) if f32 else dg.Sm100Out.Bf16(d, ld))
+    ctx.sync()
+    want, size = fa @ fb.T, fa.abs() @ fb.abs().T
+    # f32 sums: fewer than 128 roundings of 2^-24 of the terms' magnitudes (8 instructions per K block, 17 blocks at most, 16 warps); a bf16 result
+    # is rounded once more, 8 significant bits
+    bound = 128 * 2.0 ** -24 * size + (0.0 if f32 else 2.0 ** -8) * want.abs()
+    assert bool(((d[:, :n].double() - want).abs() <= bound).all())
+    assert bool((d[:, n:] == 7.0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("f32", [True, False])
+@pytest.mark.parametrize("m", [3, 12])
+def test_epilogue(ctx, m, f32):
+    n, k = 536, 1280
+    (a, fa), (b, fb) = operand(m, k, k, 3), operand(n, k, k, 4)
+    dtype, kind = (torch.float32, dg.Sm100Out.F32) if f32 else (torch.bfloat16, dg.Sm100Out.Bf16)
+    want, size = fa @ fb.T, fa.abs() @ fb.abs().T
+    unit = 2.0 ** -23 if f32 else 2.0 ** -8
+    d = torch.zeros((m, n), dtype=dtype, device="cuda")
+    dg.fp8_fp4_gemm_dev(ctx, a, b, kind(d, n), dg.Sm100Epilogue(alpha=-0.375))
+    ctx.sync()
+    assert bool(((d.double() + 0.375 * want).abs() <= 128 * 2.0 ** -24 * size + unit * want.abs()).all())
+    old = (torch.randn((m, n), generator=torch.Generator(device="cuda").manual_seed(5), device="cuda") * size.mean().sqrt()).to(dtype)
+    d = old.clone()
+    dg.fp8_fp4_gemm_dev(ctx, a, b, kind(d, n), dg.Sm100Epilogue(accumulate=True))
+    ctx.sync()
+    # the product and the sum are each rounded to the output type
+    assert bool(((d.double() - old.double() - want).abs() <= 128 * 2.0 ** -24 * size + unit * (2 * want.abs() + old.double().abs())).all())
+
+
+@pytest.mark.gpu
+def test_scales_and_codes_at_the_ends_of_their_range(ctx, monkeypatch):
+    # exponents far apart whose product is ordinary, scales of 2^-127, NaN scales and NaN codes: as the block-scaled tensor core has them
+    m, n, k = 5, 64, 512
+    a, fa = operand(m, k, k, 6, (230, 234))
+    b, fb = operand(n, k, k, 7, (20, 24))
+    words = b.sf.view(1, n)
+    words[0, 3] = 0                                   # 2^-127
+    words[0, 9] = words[0, 9] | 0xFF                  # NaN in the first K block of one column
+    a.data[2, 300] = 0x7F                             # NaN in a row
+    out = []
+    for skinny in ("1", "0"):
+        monkeypatch.setenv("DG_SKINNY", skinny)
+        d = torch.zeros((m, n), dtype=torch.float32, device="cuda")
+        dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d, n))
+        ctx.sync()
+        out.append(d)
+    assert torch.equal(out[0].isnan(), out[1].isnan())
+    assert bool(out[0][2].isnan().all()) and bool(out[0][:, 9].isnan().all()) and int(out[0].isnan().sum()) == n + m - 1
+    size = (fa.abs() @ fb.abs().T)
+    ok = ~out[0].isnan()
+    ok[:, 3] = False
+    assert bool(((out[0].double() - out[1].double()).abs() <= 2 * 128 * 2.0 ** -24 * size)[ok].all())
+    assert bool(torch.isclose(out[0][:2, 3], out[1][:2, 3], rtol=1e-4, atol=0).all())
