@@ -119,6 +119,7 @@ _set_mk = _proto("dg_set_mk_alignment_for_contiguous_layout", C.c_int, _u32)
 _get_mk = _proto("dg_get_mk_alignment_for_contiguous_layout", _u32)
 _get_mk_theory = _proto("dg_get_theoretical_mk_alignment_for_contiguous_layout", _u32, _u32)
 _best_config = _proto("dg_best_config", C.c_int, C.POINTER(_Desc), C.POINTER(_Config))
+_uses_few_rows_kernel = _proto("dg_uses_few_rows_kernel", C.c_int, C.POINTER(_Desc))
 
 SF_RULE_REFERENCE_CPU = 0
 SF_RULE_RANGE_FIT = 1
@@ -611,10 +612,19 @@ class Sm100Config:
 SM100_SMEM_CAPACITY = 232448
 
 
+def _desc(desc: Sm100Desc) -> _Desc:
+    return _Desc(desc.gemm_type, desc.m, desc.n, desc.k, desc.num_groups, desc.expected_m or desc.m, desc.a_bits, desc.b_bits,
+                 desc.gran_a, desc.gran_b, desc.cd_dtype, desc.num_sms, int(desc.major_a_mn), int(desc.major_b_mn))
+
+
+def uses_few_rows_kernel(desc: Sm100Desc) -> bool:
+    """Whether a dense call of this description goes to the kernel for a handful of activation rows, not to the tiles of best_config."""
+    return bool(_uses_few_rows_kernel(C.byref(_desc(desc))))
+
+
 def best_config(desc: Sm100Desc) -> Sm100Config:
     """heuristics_sm100.rs:455"""
-    d = _Desc(desc.gemm_type, desc.m, desc.n, desc.k, desc.num_groups, desc.expected_m or desc.m, desc.a_bits, desc.b_bits,
-              desc.gran_a, desc.gran_b, desc.cd_dtype, desc.num_sms, int(desc.major_a_mn), int(desc.major_b_mn))
+    d = _desc(desc)
     c = _Config()
     _check(_best_config(C.byref(d), C.byref(c)))
     return Sm100Config(bool(c.swap_ab), c.block_m, c.block_n, c.block_k, c.cluster_m, c.cluster_n, c.num_stages,

@@ -237,13 +237,12 @@ struct KernelPlan {
     uint32_t splits;           // K ranges: summed by a second kernel (first tile family) or by the last range to arrive (swapped)
     uint32_t tiles;
     uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
-    uint32_t skinny;           // tiles of 8 activation rows of the kernel for few of them (0: another kernel)
     uint32_t block_n2;         // wide tiles: columns of the second half (0: not a wide tile)
     uint32_t table_groups;     // groups whose rows and tiles are kept in shared memory (swapped family)
 };
 // What a call rules out that its description does not tell: K ranges (the caller adds into the output: their sum is written, not added), wide
 // tiles (no bf16 operands).
-constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2, kNoSkinny = 4;
+constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2;
 static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
     KernelPlan plan;
@@ -357,16 +356,19 @@ static bool prefer_swapped(const dg_desc* d) {
 // (16 x 5712 x 3584: 13.9 -> 10.5; 15 x 896 x 15872: 12.8 -> 13.6; 9 x 2864 x 13824: 17.5 -> 22.7), with four to 8 MB (28 x 1352 x 3584: 12.3 -> 8.7;
 // 32 x 2112 x 7168: 12.3 -> 12.5).
 static bool prefer_skinny(const dg_desc* d) {
-    const char *knob = getenv("DG_SKINNY"), *family = getenv("DG_SWAP");
-    if ((knob && atoi(knob) == 0) || family) return false;       // a pinned family is one of the other two
     if (d->gemm_type != DG_GEMM_NORMAL || d->k % 128 != 0 || (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32)) return false;
     if (d->a_bits != 8 || d->b_bits != 8 || d->gran_a != 128 || d->gran_b != 128 || d->major_a_mn || d->major_b_mn) return false;
     const uint32_t sms = d->num_sms ? d->num_sms : 148;
     const double mb = static_cast<double>(d->n) * d->k * 1e-6;
-    if (d->m <= 8) return mb <= (2 * ceil_div(d->n, 128) >= sms ? 40.0 : 60.0);
-    if (d->m <= 16) return mb <= 24.0 && d->k <= 12288;
-    return d->m <= 32 && mb <= 8.0;
+    const bool few = d->m <= 8 ? mb <= (2 * ceil_div(d->n, 128) >= sms ? 40.0 : 60.0) : (d->m <= 16 ? mb <= 24.0 && d->k <= 12288 : d->m <= 32 && mb <= 8.0);
+    if (!few || knob_signature() == 0) return few;
+    // DG_SKINNY=0 turns it off, and so does a knob that asks for something of another kernel
+    for (const char* knob : {"DG_SWAP", "DG_BLOCK_N", "DG_CTAS", "DG_STAGES", "DG_SPLITS", "DG_K_SLABS"})
+        if (getenv(knob)) return false;
+    const char* skinny = getenv("DG_SKINNY");
+    return !(skinny && atoi(skinny) == 0);
 }
+int dg_uses_few_rows_kernel(const dg_desc* d) { return d != nullptr && prefer_skinny(d) ? 1 : 0; }
 // Warps of its blocks.  Blocks of 16 columns that all fit at once share K among as many warps as there are; with more blocks it is
 // several of them per SM that keep loads in flight (8 x 2112 x 7168 with 4 / 8 / 16 warps: 9.5 / 8.1 / 8.0 us; 1 x 4096 x 7168: 12.7 / 10.7 / 11.6;
 // 16 x 7168 x 2048: 8.4 / 9.4 / 11.5).
@@ -579,23 +581,6 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
     const char* force_splits = getenv("DG_SPLITS");
     const char* force_halves = getenv("DG_K_SLABS");
     const bool pinned = force_n || force_ctas || force_stages || force_splits || force_halves;
-    plan->skinny = 0;
-    if (!(limits & kNoSkinny) && !pinned && prefer_skinny(d)) {
-        plan->swap = false;
-        plan->skinny = d->m <= 8 ? 1 : (d->m <= 16 ? 2 : 4);
-        plan->ctas = 1; plan->umma_n = dg::kSkinnyCols; plan->halves = 1; plan->stages = 1; plan->accum = 1; plan->smem = 0; plan->splits = 1;
-        plan->tiles = ceil_div(d->n, dg::kSkinnyCols); plan->epi_bufs = 0; plan->block_n2 = 0; plan->table_groups = 0;
-        out->swap_ab = 0;
-        out->block_m = 8 * plan->skinny;
-        out->block_n = dg::kSkinnyCols;
-        out->block_k = 128;
-        out->cluster_m = out->cluster_n = 1;
-        out->num_stages = out->num_accum_stages = 1;
-        out->smem_size = static_cast<uint32_t>(sizeof(float)) * skinny_warps(d->n, sms) * 8 * plan->skinny * (dg::kSkinnyCols + 1);
-        out->num_tiles = plan->tiles;
-        out->num_splits = 1;
-        return DG_OK;
-    }
     uint32_t best_n = 0, best_accum = 0, best_tiles = 0, best_ctas = 0, best_stages = 0, best_splits = 1, best_halves = 1, best_epi_bufs = 2;
     double best_cost = 0;
     // a stage holds one or two 128-byte K slabs per operand; two slabs halve the per-stage bookkeeping per UMMA
@@ -992,7 +977,8 @@ int reserve(dg_ctx* ctx, ScratchBuffer* buf, size_t bytes, bool zeroed = false) 
     return DG_OK;
 }
 
-int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue& e, const Problem& pr, uint32_t tiles) {
+int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue& e, const Problem& pr) {
+    const uint32_t tiles = pr.m <= 8 ? 1 : (pr.m <= 16 ? 2 : 4);      // of 8 activation rows
     // what the tensor maps of the other kernels ask for
     if (reinterpret_cast<uintptr_t>(a->data) % 16 != 0 || reinterpret_cast<uintptr_t>(b->data) % 16 != 0 || reinterpret_cast<uintptr_t>(a->sf) % 16 != 0 ||
         reinterpret_cast<uintptr_t>(b->sf) % 16 != 0 || reinterpret_cast<uintptr_t>(out->buf) % 16 != 0)
@@ -1010,6 +996,7 @@ int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, c
         return f32 ? run(dg::dg_gemm_skinny_kernel<2, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<2, kWarps, false>, kWarps);
     };
     const uint32_t warps = skinny_warps(pr.n, static_cast<uint32_t>(ctx->num_sms));
+    if (print_configs()) fprintf(stderr, "[dgb200] few rows: m=%u n=%u k=%u -> block=%ux%u warps=%u\n", pr.m, pr.n, pr.k, 8 * tiles, dg::kSkinnyCols, warps);
     const cudaError_t ce = warps == 4 ? with_warps(std::integral_constant<uint32_t, 4>()) : (warps == 8 ? with_warps(std::integral_constant<uint32_t, 8>()) : with_warps(std::integral_constant<uint32_t, 16>()));
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
     return DG_OK;
@@ -1059,10 +1046,11 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
     dg_desc desc = {pr.type, pr.m, pr.n, pr.k, pr.groups, pr.expected_m, a->bits, b->bits, a->gran_k, b->gran_k,
                     static_cast<uint32_t>(out->kind), static_cast<uint32_t>(ctx->num_sms), (!pr.bf16 && a->major_mn) ? 1u : 0u,
                     (!pr.bf16 && b->major_mn) ? 1u : 0u};
+    const uint32_t tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
+    if (!pr.bf16 && tc_util == 100 && prefer_skinny(&desc)) return launch_skinny(ctx, a, b, out, e, pr);
     dg_config cfg;
     KernelPlan plan;
-    const uint32_t tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
-    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles | kNoSkinny : 0u) | (tc_util < 100 ? kNoSkinny : 0u), &cfg, &plan);
+    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles : 0u), &cfg, &plan);
     if (rc) return rc;
     const bool swap = plan.swap;
     // the swapped family's kernel takes the operands with their roles exchanged: its operand A (UMMA M side) is the weights
@@ -1075,7 +1063,6 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
                 pr.type, pr.m, pr.n, pr.k, pr.groups, cfg.swap_ab, cfg.block_m, cfg.block_n, cfg.block_k, plan.ctas, cfg.num_stages,
                 cfg.num_accum_stages, cfg.smem_size, cfg.num_tiles, cfg.num_splits);
 
-    if (plan.skinny != 0) return launch_skinny(ctx, a, b, out, e, pr, plan.skinny);
     const bool mxf4 = a->bits == 4 && b->bits == 4;
     const uint32_t block_k = cfg.block_k;
     const uint32_t splits = plan.splits;

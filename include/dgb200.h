@@ -314,6 +314,9 @@ typedef struct {
 } dg_config;
 /* heuristics_sm100.rs:455 (best_config) */
 int dg_best_config(const dg_desc* desc, dg_config* out);
+/* 1 if a dense e4m3 call of this description (without a duty cycle) goes to the kernel for a handful of activation rows, which has no
+ * tiles of the kind dg_best_config describes (it then describes what the problem would get otherwise, with DG_SKINNY=0); else 0. */
+int dg_uses_few_rows_kernel(const dg_desc* desc);
 
 #ifdef __cplusplus
 }

@@ -26,8 +26,7 @@ def operand(rows, k, ld, seed, exponents=(118, 136)):
 
 
 def is_skinny(m, n, k):
-    c = dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k))
-    return not c.swap_ab and c.block_n == 16
+    return dg.uses_few_rows_kernel(dg.Sm100Desc(dg.GemmType.Normal, m, n, k))
 
 
 @pytest.mark.parametrize("m,n,k,skinny", [
