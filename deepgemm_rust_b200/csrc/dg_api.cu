@@ -1922,8 +1922,14 @@ int dg_ep_count(dg_ctx* ctx, const int32_t* expert_of_pair, uint32_t pairs, uint
     if (num_experts == 0 || num_experts > 8192) return fail(DG_ERR_SHAPE, "num_experts must be in [1, 8192]");
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     const uint32_t chunks = ceil_div(pairs, dg::kEpChunk);
-    if (chunks > 0)
-        DG_CUDA(launch(dg::dg_ep_rank_pairs_kernel, chunks, dg::kEpChunk, num_experts * sizeof(uint32_t), ctx->stream, expert_of_pair, pairs, num_experts, local_rank, block_hist));
+    // Up to four chunks (a decode step of 128 tokens, top-8) one block is as fast as the two launches or 2 us faster; eight take it 2 us longer.
+    if (chunks <= 4) {
+        DG_CUDA(launch(dg::dg_ep_rank_pairs_kernel<true>, 1, dg::kEpChunk, num_experts * sizeof(uint32_t), ctx->stream, expert_of_pair, pairs, num_experts, local_rank,
+                       block_hist, counts));
+        return DG_OK;
+    }
+    DG_CUDA(launch(dg::dg_ep_rank_pairs_kernel<false>, chunks, dg::kEpChunk, num_experts * sizeof(uint32_t), ctx->stream, expert_of_pair, pairs, num_experts, local_rank,
+                   block_hist, counts));
     DG_CUDA(launch(dg::dg_ep_block_scan_kernel, ceil_div(num_experts, 8), 256, 0, ctx->stream, block_hist, chunks, num_experts, counts));
     return DG_OK;
 }

@@ -293,6 +293,26 @@ def test_pair_ranking_is_a_stable_counting_sort(ctx):
             assert lr[p] == -1
 
 
+@pytest.mark.parametrize("pairs", [1, 31, 33, 255, 256, 257, 1023, 1024, 1025])
+@pytest.mark.parametrize("experts", [1, 7, 300])
+def test_pair_ranking_of_few_chunks(ctx, pairs, experts):
+    # up to four chunks of 256 pairs go through one block and one launch; ids out of range among them
+    ids = np.random.default_rng(pairs).integers(-1, experts + 1, pairs).astype(np.int32)
+    local_rank = torch.full((pairs,), 9, dtype=torch.int32, device="cuda")
+    hist = torch.full((dg.ep_block_hist_words(pairs, experts),), 9, dtype=torch.int32, device="cuda")
+    counts = torch.full((experts,), 9, dtype=torch.int32, device="cuda")
+    dg.ep_count_dev(ctx, dev(ids), pairs, experts, local_rank, hist, counts)
+    ctx.sync()
+    ok = (ids >= 0) & (ids < experts)
+    one_hot = (ids[:, None] == np.arange(experts)[None, :]).astype(np.int64)
+    before = np.cumsum(one_hot, 0) - one_hot
+    rank = np.where(ok, before[np.arange(pairs), np.where(ok, ids, 0)], -1)
+    starts = before[::256]                                     # pairs of the chunks before each chunk
+    assert np.array_equal(counts.cpu().numpy(), one_hot.sum(0)) and np.array_equal(hist.cpu().numpy().reshape(-1, experts), starts)
+    in_chunk = np.where(ok, rank - starts[np.arange(pairs) // 256, np.where(ok, ids, 0)], -1)
+    assert np.array_equal(local_rank.cpu().numpy(), in_chunk)
+
+
 def test_peer_exchange_masked_layout(ctx):
     # decode-style step: every local expert owns a fixed slot of rows, the exchange writes token rows and their scale words
     # straight into the (experts, slot_rows, k) operand of the masked grouped GEMM and hands it the per-expert row counts
