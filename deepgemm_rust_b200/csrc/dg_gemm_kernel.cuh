@@ -80,9 +80,6 @@ struct GemmParams {
     uint32_t sfd_stride;       // output scale words: stride between word columns (fp8 output)
     uint32_t stage_in_ring;    // no CTA computes more than one tile, and the operand ring holds a staging buffer for every store of a tile (f32)
     uint32_t epi_bufs;         // staging buffers of an epilogue warp: 2, or 1 where f32 staging would cost a stage of two slabs
-    // wide tiles only (dg_gemm_wide.cuh)
-    uint32_t block_n2;         // columns of a tile's second half
-    uint32_t whole_tiles;      // dense: tiles from this one on are computed as two halves by two CTA pairs
     // second tile family only (dg_gemm_swap.cuh), where m counts weight rows and n activation rows per group
     uint32_t acc_stride;       // TMEM column where the second accumulator starts (below block_n: the two share columns)
     uint32_t acc_edge_chunks;  // 32-column chunks that hold the shared columns
@@ -93,6 +90,9 @@ struct GemmParams {
     uint32_t* sfd;
     Status* status;
     long long* prof;           // debug builds only
+    // wide tiles only (dg_gemm_wide.cuh)
+    uint32_t block_n2;         // columns of a tile's second half
+    uint32_t whole_tiles;      // dense: tiles from this one on are computed as two halves by two CTA pairs
     uint32_t debug_flags;      // debug builds only: 1 = epilogue only releases the accumulator, 2 = no scale-factor traffic
 };
 
