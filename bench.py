@@ -227,7 +227,7 @@ def phase_us(record):
 
 def gemm_kernel(dg, *sizes, **kw):
     """Name of the kernel the library's tile choice runs for a problem."""
-    return "dg_gemm_swap_kernel" if dg.best_config(dg.Sm100Desc(*sizes, **kw)).swap_ab else "dg_gemm_kernel"
+    return dg.kernel_name(dg.Sm100Desc(*sizes, **kw))
 
 
 class DenseWork:

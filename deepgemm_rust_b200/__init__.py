@@ -119,7 +119,7 @@ _set_mk = _proto("dg_set_mk_alignment_for_contiguous_layout", C.c_int, _u32)
 _get_mk = _proto("dg_get_mk_alignment_for_contiguous_layout", _u32)
 _get_mk_theory = _proto("dg_get_theoretical_mk_alignment_for_contiguous_layout", _u32, _u32)
 _best_config = _proto("dg_best_config", C.c_int, C.POINTER(_Desc), C.POINTER(_Config))
-_uses_few_rows_kernel = _proto("dg_uses_few_rows_kernel", C.c_int, C.POINTER(_Desc))
+_kernel_name = _proto("dg_kernel_name", C.c_char_p, C.POINTER(_Desc))
 
 SF_RULE_REFERENCE_CPU = 0
 SF_RULE_RANGE_FIT = 1
@@ -617,9 +617,10 @@ def _desc(desc: Sm100Desc) -> _Desc:
                  desc.gran_a, desc.gran_b, desc.cd_dtype, desc.num_sms, int(desc.major_a_mn), int(desc.major_b_mn))
 
 
-def uses_few_rows_kernel(desc: Sm100Desc) -> bool:
-    """Whether a dense call of this description goes to the kernel for a handful of activation rows, not to the tiles of best_config."""
-    return bool(_uses_few_rows_kernel(C.byref(_desc(desc))))
+def kernel_name(desc: Sm100Desc) -> Optional[str]:
+    """The kernel that a call of this description launches."""
+    name = _kernel_name(C.byref(_desc(desc)))
+    return name.decode() if name else None
 
 
 def best_config(desc: Sm100Desc) -> Sm100Config:

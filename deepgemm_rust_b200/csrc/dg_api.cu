@@ -368,7 +368,14 @@ static bool prefer_skinny(const dg_desc* d) {
     const char* skinny = getenv("DG_SKINNY");
     return !(skinny && atoi(skinny) == 0);
 }
-int dg_uses_few_rows_kernel(const dg_desc* d) { return d != nullptr && prefer_skinny(d) ? 1 : 0; }
+const char* dg_kernel_name(const dg_desc* d) {
+    if (d == nullptr) return nullptr;
+    if (prefer_skinny(d)) return "dg_gemm_skinny_kernel";
+    dg_config cfg;
+    KernelPlan plan;
+    if (search_config(d, 0, &cfg, &plan)) return nullptr;
+    return plan.swap ? "dg_gemm_swap_kernel" : (plan.block_n2 != 0 ? "dg_gemm_wide_kernel" : "dg_gemm_kernel");
+}
 // Warps of its blocks.  Blocks of 16 columns that all fit at once share K among as many warps as there are; with more blocks it is
 // several of them per SM that keep loads in flight (8 x 2112 x 7168 with 4 / 8 / 16 warps: 9.5 / 8.1 / 8.0 us; 1 x 4096 x 7168: 12.7 / 10.7 / 11.6;
 // 16 x 7168 x 2048: 8.4 / 9.4 / 11.5).

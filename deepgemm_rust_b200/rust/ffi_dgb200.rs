@@ -159,7 +159,7 @@ extern "C" {
     pub fn dg_get_mk_alignment_for_contiguous_layout() -> u32;
     pub fn dg_get_theoretical_mk_alignment_for_contiguous_layout(arch_major: u32) -> u32;
     pub fn dg_best_config(desc: *const RawDesc, out: *mut RawConfig) -> c_int;
-    pub fn dg_uses_few_rows_kernel(desc: *const RawDesc) -> c_int;
+    pub fn dg_kernel_name(desc: *const RawDesc) -> *const c_char;
 }
 
 /// Status code of the C ABI -> the crate's error type (types.rs:9-21).  A device-side wait that ran

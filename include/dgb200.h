@@ -314,9 +314,10 @@ typedef struct {
 } dg_config;
 /* heuristics_sm100.rs:455 (best_config) */
 int dg_best_config(const dg_desc* desc, dg_config* out);
-/* 1 if a dense e4m3 call of this description (without a duty cycle) goes to the kernel for a handful of activation rows, which has no
- * tiles of the kind dg_best_config describes (it then describes what the problem would get otherwise, with DG_SKINNY=0); else 0. */
-int dg_uses_few_rows_kernel(const dg_desc* desc);
+/* The kernel that an e4m3 / e2m1 call of this description launches (without accumulation and duty cycle); null if none fits.  Where it is
+ * dg_gemm_skinny_kernel, the one for a handful of dense activation rows, which has no tiles of this kind, dg_best_config describes what the
+ * problem gets with DG_SKINNY=0. */
+const char* dg_kernel_name(const dg_desc* desc);
 
 #ifdef __cplusplus
 }

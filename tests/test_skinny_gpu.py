@@ -26,7 +26,7 @@ def operand(rows, k, ld, seed, exponents=(118, 136)):
 
 
 def is_skinny(m, n, k):
-    return dg.uses_few_rows_kernel(dg.Sm100Desc(dg.GemmType.Normal, m, n, k))
+    return dg.kernel_name(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)) == "dg_gemm_skinny_kernel"
 
 
 @pytest.mark.parametrize("m,n,k,skinny", [

@@ -5,9 +5,6 @@ import torch
 
 import deepgemm_rust_b200 as dg
 
-pytestmark = pytest.mark.gpu
-
-
 @pytest.fixture(scope="module")
 def ctx():
     c = dg.DgContext(0)
@@ -47,6 +44,7 @@ def both(ctx, monkeypatch, run):
 SIZES = [(1, 392, 128), (300, 456, 1152), (257, 680, 640), (2100, 4296, 384), (4352, 1800, 256), (4000, 4488, 128), (2560, 8288, 640)]
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", SIZES)
 @pytest.mark.parametrize("a_bits,b_bits", [(8, 8), (8, 4), (4, 8), (4, 4)])
 def test_dense(ctx, monkeypatch, m, n, k, a_bits, b_bits):
@@ -59,6 +57,7 @@ def test_dense(ctx, monkeypatch, m, n, k, a_bits, b_bits):
     both(ctx, monkeypatch, run)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("epilogue", [dict(alpha=-0.5), dict(accumulate=True), dict(tc_util=60)])
 @pytest.mark.parametrize("f32", [True, False])
 @pytest.mark.parametrize("gran_a,gran_b", [(128, 128), (32, 128), (32, 32)])
@@ -73,6 +72,7 @@ def test_outputs_and_scales(ctx, monkeypatch, epilogue, f32, gran_a, gran_b):
     both(ctx, monkeypatch, run)
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("alignment", [16, 128])
 @pytest.mark.parametrize("n", [456, 1096])
 @pytest.mark.parametrize("f32", [True, False])
@@ -108,3 +108,18 @@ def test_grouped(ctx, monkeypatch, alignment, n, f32):
             both(ctx, patch, masked)
     finally:
         dg.set_mk_alignment_for_contiguous_layout(128)
+
+
+CONTIGUOUS = dg.GemmType.MGroupedContiguous
+
+
+@pytest.mark.parametrize("sizes,kw,wide", [
+    ((dg.GemmType.Normal, 4096, 7168, 16384), {}, True), ((dg.GemmType.Normal, 4096, 7168, 7168), dict(a_bits=4, b_bits=4, gran_a=32, gran_b=32), True),
+    ((dg.GemmType.Normal, 4096, 7168, 16384), dict(gran_a=32), False), ((dg.GemmType.Normal, 4096, 7168, 16384), dict(cd_dtype=2), False),
+    ((dg.GemmType.Normal, 1024, 4096, 7168), {}, False),                                       # one wave
+    ((CONTIGUOUS, 32 * 2112, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 520, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 512, 4096, 7168, 32), {}, False),
+    ((CONTIGUOUS, 4 * 1024, 2048, 7168, 4), {}, False),                                        # less than three waves
+    ((dg.GemmType.MGroupedMasked, 2048, 4096, 7168, 32, 2048), {}, False), ((dg.GemmType.Batched, 2048, 4096, 7168, 16), {}, False),
+])
+def test_which_problems_get_them(sizes, kw, wide):
+    assert (dg.kernel_name(dg.Sm100Desc(*sizes, **kw)) == "dg_gemm_wide_kernel") == wide
