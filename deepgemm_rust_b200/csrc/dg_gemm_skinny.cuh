@@ -3,11 +3,11 @@
 // What bounds such a call is not the weight stream but everything around it: with the tiles of the first family 8 x 2112 x 7168 took
 // 10.5 us, of which the 15 MB of weights are 2.4: the start-up of a kernel with tensor maps, TMEM and rings, its drain, f32 planes of the
 // K ranges, and a second launch that sums them.  Here a block owns 16 weight rows (output columns) over the whole of K; its warps deal
-// the K blocks out among themselves and bring them from global memory straight to registers, where they become f16 (exactly) fragments of
-// the warp-wide matrix instruction; the warps' sums meet in shared memory.  One launch, no workspace, nothing set up before the
-// first load.  Quantiser and GEMM together: 8 x 2112 x 7168 12.1 -> 8.0 us, which is what the host needs for the two calls; 3 x 6664 x 4608
-// 16.5 -> 10.7.  With more rows or weights the multiply (two conversions and a share of the instructions per four codes) and the latency of
-// plain loads show, and the tensor-memory kernels are the better ones.
+// the K blocks out among themselves and bring them from global memory straight to registers, where a 16-byte piece of a row is a lane's share of two
+// warp-wide matrix instructions (e4m3 in, f32 sums); the warps' sums meet in shared memory.  One launch, no workspace, nothing set up
+// before the first load.  Quantiser and GEMM together: 8 x 2112 x 7168 12.1 -> 8.0 us, which is what the host needs for the two calls;
+// 3 x 6664 x 4608 16.5 -> 10.7.  (With the codes turned into f16 first, for the instruction of half the depth: the same error, up to 6 %
+// slower.)  With more rows or weights the latency of plain loads shows, and the tensor-memory kernels are the better ones.
 //
 // A K block of 128 is multiplied on its own, scaled by the two power-of-two scales and added to f32 sums.  The order of K inside a block
 // is the same for both operands and otherwise free, so that a lane's 16-byte pieces of a row are its share of the fragments.
@@ -29,14 +29,8 @@ struct SkinnyParams {
     float alpha;
 };
 
-// Two e4m3 codes -> two f16 values (exact: e4m3 is a subset).
-DG_DEVICE uint32_t e4m3x2_to_f16x2(uint32_t two) {
-    uint32_t r;
-    asm("{\n\t.reg .b16 h;\n\tcvt.u16.u32 h, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, h;\n\t}\n" : "=r"(r) : "r"(two));
-    return r;
-}
-DG_DEVICE void mma_16x8x16_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+DG_DEVICE void mma_16x8x32_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -49,7 +43,7 @@ DG_DEVICE float scale_by_exponents(float x, uint32_t ea, uint32_t eb) {
 
 // kTiles: activation rows in tiles of 8.  kWarps of a block share K.
 template <uint32_t kTiles, uint32_t kWarps, bool kF32>
-__global__ void __launch_bounds__(kWarps * 32) dg_gemm_skinny_kernel(const __grid_constant__ SkinnyParams p) {
+__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kernel(const __grid_constant__ SkinnyParams p) {
     __shared__ float sums[kWarps][kTiles * 8][kSkinnyCols + 1];
     griddep_wait();
     griddep_launch_dependents();
@@ -90,14 +84,12 @@ __global__ void __launch_bounds__(kWarps * 32) dg_gemm_skinny_kernel(const __gri
         for (uint32_t j = 0; j < 2; ++j) {
             const uint32_t w0[4] = {c.w[0][j].x, c.w[0][j].y, c.w[0][j].z, c.w[0][j].w}, w1[4] = {c.w[1][j].x, c.w[1][j].y, c.w[1][j].z, c.w[1][j].w};
             #pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                const uint32_t a0 = e4m3x2_to_f16x2(w0[q]), a1 = e4m3x2_to_f16x2(w1[q]), a2 = e4m3x2_to_f16x2(w0[q] >> 16), a3 = e4m3x2_to_f16x2(w1[q] >> 16);
+            for (uint32_t q = 0; q < 4; q += 2)
                 #pragma unroll
                 for (uint32_t i = 0; i < kTiles; ++i) {
                     const uint32_t y[4] = {c.x[i][j].x, c.x[i][j].y, c.x[i][j].z, c.x[i][j].w};
-                    mma_16x8x16_f16(d[i], a0, a1, a2, a3, e4m3x2_to_f16x2(y[q]), e4m3x2_to_f16x2(y[q] >> 16));
+                    mma_16x8x32_e4m3(d[i], w0[q], w1[q], w0[q + 1], w1[q + 1], y[q], y[q + 1]);
                 }
-            }
         }
         const uint32_t shift = 8 * (kb & 3);
         #pragma unroll

@@ -30,8 +30,9 @@ def is_skinny(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k,skinny", [
-    (8, 2112, 7168, True), (1, 4096, 14592, True), (8, 4096, 14720, False), (8, 9344, 4352, True), (8, 9352, 4352, False), (16, 5856, 4096, True),
-    (16, 5864, 4096, False), (9, 512, 12288, True), (9, 512, 12416, False), (32, 1952, 4096, True), (17, 1960, 4096, False), (33, 512, 1024, False),
+    (8, 2112, 7168, True), (1, 4096, 15616, True), (8, 4096, 15744, False), (8, 9344, 5248, True), (8, 9352, 5248, False), (16, 5856, 4096, True),
+    (16, 5864, 4096, False), (9, 512, 12288, True), (9, 512, 12416, False), (9, 2376, 7168, True), (9, 2376, 7296, False), (32, 1952, 4096, True),
+    (17, 1960, 4096, False), (17, 512, 4224, False), (33, 512, 1024, False),
     (8, 2112, 7200, False),
 ])
 def test_which_problems_get_it(m, n, k, skinny):
