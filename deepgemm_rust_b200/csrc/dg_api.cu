@@ -351,8 +351,8 @@ static bool prefer_swapped(const dg_desc* d) {
 // Is the kernel for a handful of activation rows (dg_gemm_skinny.cuh) the one for this problem?  Measured behind the activation quantiser
 // over 300 problems (m 1-32, n 512-24576, k 1024-16384): it takes 8.5 us (what the host needs for the two calls) wherever the weights
 // are below 15 MB, where the first family's K ranges with their second launch take 12.4 and the swapped family's blocks 10.  Up to 8 rows
-// that lasts, at 4 TB/s, to 64 MB (1 x 4640 x 7680: 18.7 -> 11.8 us; 4 x 9024 x 6656: 21.9 -> 16.3; 3 x 5200 x 13312: 22.0 -> 22.5), to 48 where the
-// swapped family fills the SMs (3 x 12904 x 3584: 15.4 -> 15.2).  With two tiles of rows the multiply itself shows: to 24 MB, and with fewer blocks than
+// that lasts, at 4 TB/s, to 64 MB (1 x 4640 x 7680: 18.7 -> 11.8 us; 4 x 9024 x 6656: 21.9 -> 16.3; 3 x 5200 x 13312: 22.0 -> 22.5), to 44 where the
+// swapped family fills the SMs (3 x 9656 x 4096: 15.3 -> 14.7; 5 x 14768 x 3072: 14.5 -> 14.6).  With two tiles of rows the multiply itself shows: to 24 MB, and with fewer blocks than
 // SMs 12288 of K, else 7168 (16 x 5712 x 3584: 13.9 -> 10.5; 9 x 2864 x 13824: 17.5 -> 22.7; 16 x 2592 x 9216: 13.3 -> 14.8); with four to 8 MB and 4096
 // (28 x 1352 x 3584: 12.3 -> 8.7; 32 x 2112 x 7168: 12.3 -> 12.9; 30 x 528 x 9728: 12.1 -> 14.3).
 static bool prefer_skinny(const dg_desc* d) {
@@ -361,7 +361,7 @@ static bool prefer_skinny(const dg_desc* d) {
     const uint32_t sms = d->num_sms ? d->num_sms : 148;
     const double mb = static_cast<double>(d->n) * d->k * 1e-6;
     const bool one_wave = ceil_div(d->n, dg::kSkinnyCols) <= sms;
-    const bool few = d->m <= 8    ? mb <= (2 * ceil_div(d->n, 128) >= sms ? 48.0 : 64.0)
+    const bool few = d->m <= 8    ? mb <= (2 * ceil_div(d->n, 128) >= sms ? 44.0 : 64.0)
                      : d->m <= 16 ? mb <= 24.0 && d->k <= (one_wave ? 12288u : 7168u)
                                   : d->m <= 32 && mb <= 8.0 && d->k <= 4096;
     if (!few || knob_signature() == 0) return few;
