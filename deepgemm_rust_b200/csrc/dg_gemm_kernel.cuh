@@ -216,6 +216,14 @@ struct Scheduler {
     }
 };
 
+// A duty cycle below 100 %: idles for the share that goes with the tensor time of the UMMAs just done, `columns` of a tile times 128-byte
+// slabs of K, at 2 * 128 * 128 / 8192 = 4 cycles each (the reference's figure; 8-bit operands take half of it).  Every kernel counts the
+// same way, so that a problem is paced alike whichever tiles it gets.
+DG_DEVICE void duty_cycle_pause(uint32_t util, uint32_t columns) {
+    const long long busy = 4ll * columns, idle = (100ll - util) * busy / util, t0 = clock64();
+    while (clock64() - t0 < idle) {}
+}
+
 // How often a scale word must be (re)loaded and how many words one k-block needs.
 //   block_k_elems = 128 (e4m3) or 256 (e2m1 pairs).  A word covers 4*gran elements.
 struct SfPlan {
@@ -548,10 +556,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                         __syncwarp();
                         if (!mbar_wait_warp(bar_tc, tc_phase, abort_flag, p.status, 0x480)) { ok = false; break; }
                         tc_phase ^= 1;
-                        const long long busy = 4ll * n_tile * halves;      // 2 * 128 * N * (128 * halves) / 8192 cycles per k-block and SM
-                        const long long idle = (100ll - p.tc_util) * busy / p.tc_util;
-                        const long long t0 = clock64();
-                        while (clock64() - t0 < idle) {}
+                        duty_cycle_pause(p.tc_util, n_tile * halves);
                         __syncwarp();
                     }
                     DG_PROF_ADD(3, t_issue);

@@ -505,10 +505,7 @@ dg_gemm_swap_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                         __syncwarp();
                         if (!mbar_wait_warp(bar_tc, tc_phase, abort_flag, p.status, 0x480)) { ok = false; break; }
                         tc_phase ^= 1;
-                        const long long busy = 4ll * t.n * kHalves;
-                        const long long idle = (100ll - p.tc_util) * busy / p.tc_util;
-                        const long long t0 = clock64();
-                        while (clock64() - t0 < idle) {}
+                        duty_cycle_pause(p.tc_util, t.n * kHalves);
                         __syncwarp();
                     }
                     if (need_sf && ++slot == kSwapSfSlots) slot = 0;

@@ -264,8 +264,7 @@ dg_gemm_wide_kernel(const __grid_constant__ GemmParams p, const __grid_constant_
                         __syncwarp();
                         if (!mbar_wait_warp(bar_tc, tc_phase, abort_flag, p.status, 0x480)) { ok = false; break; }
                         tc_phase ^= 1;
-                        const long long busy = 2ll * (n[0] + n[1]), idle = (100ll - p.tc_util) * busy / p.tc_util, t0 = clock64();
-                        while (clock64() - t0 < idle) {}
+                        duty_cycle_pause(p.tc_util, n[0] + n[1]);
                         __syncwarp();
                     }
                     if (++stage == num_stages) { stage = 0; phase ^= 1; }

@@ -24,19 +24,25 @@ def operand(ctx, rows, k, bits, seed, groups=1, gran=128, rows_per_group=None):
     return dg.LpOperand(data, sf, rows_per_group or rows, k, ld, 8, gran)
 
 
-def both(ctx, monkeypatch, run):
-    """What run(out) leaves with the wide tiles and with 224-column tiles of a CTA pair."""
+def each(monkeypatch, run):
+    """run() with the wide tiles and with 224-column tiles of a CTA pair."""
     monkeypatch.setenv("DG_WIDE_TILE", "1")
     wide = run()
-    ctx.sync()
     monkeypatch.setenv("DG_WIDE_TILE", "0")
     monkeypatch.setenv("DG_SWAP", "0")
     monkeypatch.setenv("DG_BLOCK_N", "224")
     monkeypatch.setenv("DG_CTAS", "2")
     monkeypatch.setenv("DG_SPLITS", "1")
-    narrow = run()
-    ctx.sync()
-    assert torch.equal(wide, narrow)
+    return wide, run()
+
+
+def both(ctx, monkeypatch, run):
+    """Both leave the same."""
+    def done():
+        d = run()
+        ctx.sync()
+        return d
+    assert torch.equal(*each(monkeypatch, done))
 
 
 # units of work: fewer than pairs of CTAs; whole tiles, then at most one half each, then at most two; an odd number of halves across, and a last
@@ -70,6 +76,28 @@ def test_outputs_and_scales(ctx, monkeypatch, epilogue, f32, gran_a, gran_b):
         dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d, n) if f32 else dg.Sm100Out.Bf16(d, n), dg.Sm100Epilogue(**epilogue))
         return d
     both(ctx, monkeypatch, run)
+
+
+@pytest.mark.gpu
+def test_duty_cycle_paces_them_like_the_other_tiles(ctx, monkeypatch):
+    # 37 x 896: one wide tile per pair of CTAs, or two of 224 columns: the same columns and slabs of K, so the same pauses, four times what the
+    # tensor cores take for bf16 operands and eight times for these, in which the tiles' own differences drown
+    m, n, k = 37 * 256, 896, 4096
+    a, b = operand(ctx, m, k, 8, 8), operand(ctx, n, k, 8, 9)
+    d = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda")
+
+    def run():
+        times = []
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.Bf16(d, n), dg.Sm100Epilogue(tc_util=20))
+            e1.record()
+            ctx.sync()
+            times.append(e0.elapsed_time(e1))
+        return sorted(times)[2]
+    wide, narrow = each(monkeypatch, run)
+    assert 0.85 * narrow < wide < 1.15 * narrow
 
 
 @pytest.mark.gpu
