@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kerne
         #pragma unroll
         for (uint32_t v = 0; v < 4; ++v) sums[warp][i * 8 + 2 * t + v % 2][g + 8 * (v / 2)] = acc[i][v];
     __syncthreads();
-    // a thread per output, its sums added in the order of the warps
+    // A thread per output, its sums added in the order of the warps.  Accumulation adds in memory, as the first family's TMA reduction does:
+    // calls on two streams may add into one output.
     for (uint32_t o = threadIdx.x; o < kTiles * 8 * kSkinnyCols; o += kWarps * 32) {
         const uint32_t row = o / kSkinnyCols, col = o % kSkinnyCols;
         float s = 0.0f;
@@ -133,11 +134,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kerne
         const size_t at = static_cast<size_t>(row) * p.out_ld + n0 + col;
         if constexpr (kF32) {
             float* d = static_cast<float*>(p.out) + at;
-            *d = p.accumulate ? *d + s : s;
+            if (p.accumulate) red_add_f32(d, s);
+            else *d = s;
         } else {
             uint16_t* d = static_cast<uint16_t*>(p.out) + at;
-            const uint32_t y = pack_bf16x2(s, 0.0f);
-            *d = static_cast<uint16_t>(p.accumulate ? add_bf16x2(y, *d) : y);
+            const uint16_t y = static_cast<uint16_t>(pack_bf16x2(s, 0.0f));
+            if (p.accumulate) red_add_bf16(d, y);
+            else *d = y;
         }
     }
 }

@@ -441,6 +441,9 @@ DG_DEVICE uint32_t pack_bf16x2(float lo, float hi) {
 DG_DEVICE uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     return pack_bf16x2(__uint_as_float(a << 16) + __uint_as_float(b << 16), __uint_as_float(a & 0xFFFF0000u) + __uint_as_float(b & 0xFFFF0000u));
 }
+// Additions into global memory that no other thread's can get lost beside.
+DG_DEVICE void red_add_f32(float* to, float x) { asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(to), "f"(x) : "memory"); }
+DG_DEVICE void red_add_bf16(uint16_t* to, uint16_t x) { asm volatile("red.relaxed.gpu.global.add.noftz.bf16 [%0], %1;" ::"l"(to), "h"(x) : "memory"); }
 DG_DEVICE uint32_t cvt_e4m3x2(float lo, float hi) {
     uint16_t r;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));

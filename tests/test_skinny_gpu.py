@@ -83,6 +83,32 @@ def test_epilogue(ctx, m, f32):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("f32", [True, False])
+def test_calls_on_two_streams_add_into_one_output(f32):
+    # the first column of both operands is 1, the rest 0: every call adds 1, exact in bf16 up to 256
+    m, n, k, calls = 8, 2112, 1024, 100
+    assert is_skinny(m, n, k)
+    ops = []
+    for rows in (m, n):
+        data = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
+        data[:, 0] = 0x38
+        words = dg.sf_packed_cols(k, 128) * dg.sf_aligned_rows(rows)
+        ops.append(dg.LpOperand(data, torch.full((words,), 0x7F7F7F7F, dtype=torch.int32, device="cuda"), rows, k, k, 8, 128))
+    d = torch.zeros((m, n), dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+    out = dg.Sm100Out.F32(d, n) if f32 else dg.Sm100Out.Bf16(d, n)
+    torch.cuda.synchronize()
+    contexts = [dg.DgContext(0, own_stream=True) for _ in range(2)]
+    for _ in range(calls):
+        for c in contexts:
+            dg.fp8_fp4_gemm_dev(c, *ops, out, dg.Sm100Epilogue(accumulate=True))
+    for c in contexts:
+        c.sync()
+    assert bool((d == 2 * calls).all())
+    for c in contexts:
+        c.close()
+
+
+@pytest.mark.gpu
 def test_scales_and_codes_at_the_ends_of_their_range(ctx, monkeypatch):
     # exponents far apart whose product is ordinary, scales of 2^-127, NaN scales and NaN codes: as the block-scaled tensor core has them
     m, n, k = 5, 64, 512
