@@ -348,22 +348,31 @@ static bool prefer_swapped(const dg_desc* d) {
            ((d->m <= 32 && (2 * blocks >= sms || short_k)) || (d->m <= 64 && 5 * blocks >= 4 * sms));
 }
 
-// Is the kernel for a handful of activation rows (dg_gemm_skinny.cuh) the one for this problem?  Measured behind the activation quantiser
-// over 300 problems (m 1-32, n 512-24576, k 1024-16384): it takes 8.5 us (what the host needs for the two calls) wherever the weights
-// are below 15 MB, where the first family's K ranges with their second launch take 12.4 and the swapped family's blocks 10.  Up to 8 rows
-// that lasts, at 4 TB/s, to 64 MB (1 x 4640 x 7680: 18.7 -> 11.8 us; 4 x 9024 x 6656: 21.9 -> 16.3; 3 x 5200 x 13312: 22.0 -> 22.5), to 44 where the
-// swapped family fills the SMs (3 x 9656 x 4096: 15.3 -> 14.7; 5 x 14768 x 3072: 14.5 -> 14.6).  With two tiles of rows the multiply itself shows: to 24 MB, and with fewer blocks than
-// SMs 12288 of K, else 7168 (16 x 5712 x 3584: 13.9 -> 10.5; 9 x 2864 x 13824: 17.5 -> 22.7; 16 x 2592 x 9216: 13.3 -> 14.8); with four to 8 MB and 4096
-// (28 x 1352 x 3584: 12.3 -> 8.7; 32 x 2112 x 7168: 12.3 -> 12.9; 30 x 528 x 9728: 12.1 -> 14.3).
+// Is the kernel for a handful of activation rows (dg_gemm_skinny.cuh) the one for this problem?  Measured against the other kernels over 1263
+// problems (m 1-32, n 16-343744, k 128-62464), the GEMM alone, in a loop and in a graph of 24, weights from DRAM.  What bounds it is the latency of plain
+// loads: a warp's rounds of K blocks, times the waves of blocks (four of four warps fit an SM).  Inside the lines below it takes 0.72 of the
+// others' time on average and 1.03 at most; the figures are of the graphs.
+//   Up to 8 rows it wins to 64 MB (5 x 4472 x 13312: 17.4 -> 14.4 us; 1 x 6144 x 9728: 17.3 -> 17.3), to 44 where the swapped family
+//     fills the SMs (8 x 16384 x 2560: 11.6 -> 11.0), and to 16384 of K (8 x 256 x 16384: 8.7 -> 8.2, x 32768: 10.5 -> 14.8), 24576 where blocks of 16 warps
+//     take more than half of the SMs (8 x 1280 x 24576: 13.0 -> 12.7; 8 x 1024 x 28672: 13.2 -> 13.7).
+//   9-16 rows: while the blocks fit at once to 24 MB (16 x 9472 x 2304: 9.9 -> 8.7) and 7168 of K (16 x 2400 x 6656: 10.6 -> 10.6), with 16 warps
+//     12288 (16 x 1024 x 12288: 9.8 -> 9.7), or 10240 with so few blocks that K ranges occupy more SMs (16 x 512 x 10240: 8.6 -> 8.6, x 12288: 8.7 -> 9.6);
+//     in two waves two rounds of K (16 x 18432 x 1024: 8.8 -> 8.1, x 1152: 9.5 -> 9.9), in more one (16 x 28672 x 512: 8.6 -> 7.6, x 640: 9.3 -> 10.8).
+//   17-32 rows, whose K blocks are not prefetched: to 8 MB and 4096 of K (32 x 3072 x 2560: 9.5 -> 8.5), with four warps to 896
+//     (32 x 4800 x 896: 6.4 -> 6.2, x 1024: 6.4 -> 6.7), in two waves one round (32 x 12288 x 512: 6.7 -> 6.7, x 640: 7.3 -> 9.7).
+//   More short blocks than 14 (7) per SM: 8 x 65536 x 128 9.0 -> 9.2, 8 x 343744 x 128 30.7 -> 42.4, 32 x 32768 x 128 6.8 -> 10.2.
 static bool prefer_skinny(const dg_desc* d) {
     if (d->gemm_type != DG_GEMM_NORMAL || d->k % 128 != 0 || (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32)) return false;
     if (d->a_bits != 8 || d->b_bits != 8 || d->gran_a != 128 || d->gran_b != 128 || d->major_a_mn || d->major_b_mn) return false;
     const uint32_t sms = d->num_sms ? d->num_sms : 148;
     const double mb = static_cast<double>(d->n) * d->k * 1e-6;
-    const bool one_wave = ceil_div(d->n, dg::kSkinnyCols) <= sms;
-    const bool few = d->m <= 8    ? mb <= (2 * ceil_div(d->n, 128) >= sms ? 44.0 : 64.0)
-                     : d->m <= 16 ? mb <= 24.0 && d->k <= (one_wave ? 12288u : 7168u)
-                                  : d->m <= 32 && mb <= 8.0 && d->k <= 4096;
+    const uint32_t blocks = ceil_div(d->n, dg::kSkinnyCols);
+    bool few = false;
+    if (d->m <= 8) few = blocks <= 14 * sms && mb <= (2 * ceil_div(d->n, 128) >= sms ? 44.0 : 64.0) && d->k <= (blocks <= sms && 2 * blocks > sms ? 24576u : 16384u);
+    else if (d->m <= 16 && blocks <= 4 * sms) few = mb <= 24.0 && d->k <= (blocks > sms ? 7168u : (blocks >= 64 ? 12288u : 10240u));
+    else if (d->m <= 16) few = blocks <= 14 * sms && d->k <= (blocks <= 8 * sms ? 1024u : 512u);
+    else if (d->m <= 32 && blocks <= 4 * sms) few = mb <= 8.0 && d->k <= (blocks <= 2 * sms ? 4096u : 896u);
+    else if (d->m <= 32) few = blocks <= 7 * sms && mb <= 6.3 && d->k <= 512;
     if (!few || knob_signature() == 0) return few;
     // DG_SKINNY=0 turns it off, and so does a knob that asks for something of another kernel
     for (const char* knob : {"DG_SWAP", "DG_BLOCK_N", "DG_CTAS", "DG_STAGES", "DG_SPLITS", "DG_K_SLABS"})

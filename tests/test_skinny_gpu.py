@@ -31,8 +31,14 @@ def is_skinny(m, n, k):
 
 @pytest.mark.parametrize("m,n,k,skinny", [
     (8, 2112, 7168, True), (1, 4096, 15616, True), (8, 4096, 15744, False), (8, 9344, 5248, True), (8, 9352, 5248, False), (16, 5856, 4096, True),
-    (16, 5864, 4096, False), (9, 512, 12288, True), (9, 512, 12416, False), (9, 2376, 7168, True), (9, 2376, 7296, False), (32, 1952, 4096, True),
+    (16, 5864, 4096, False), (9, 1016, 12288, True), (9, 1016, 12416, False), (9, 2376, 7168, True), (9, 2376, 7296, False), (32, 1952, 4096, True),
     (17, 1960, 4096, False), (17, 512, 4224, False), (33, 512, 1024, False),
+    # K that few blocks share among 16 warps; blocks in one, two and more waves; more of them than those of a few warps are worth
+    (8, 1184, 16384, True), (8, 1184, 16512, False), (8, 1192, 24576, True), (8, 2368, 24704, False), (8, 2376, 16512, False),
+    (9, 1008, 10240, True), (9, 1008, 10368, False), (8, 33152, 128, True), (8, 33160, 128, False), (8, 343744, 128, False),
+    (16, 9472, 2432, True), (16, 9480, 1024, True), (16, 9480, 1152, False), (16, 18944, 1024, True), (16, 18952, 640, False), (16, 33152, 512, True),
+    (16, 33160, 128, False), (17, 4736, 1664, True), (17, 4744, 896, True), (17, 4744, 1024, False), (17, 9472, 768, True), (17, 9480, 512, True),
+    (17, 9480, 640, False), (17, 16576, 256, True), (17, 16584, 128, False),
     (8, 2112, 7200, False),
 ])
 def test_which_problems_get_it(m, n, k, skinny):
@@ -43,7 +49,7 @@ def test_which_problems_get_it(m, n, k, skinny):
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n,k", [
     (8, 128), (16, 256), (24, 2048),              # one block, a block and a part; fewer K blocks than warps, and as many
-    (2368, 2176), (2376, 384), (4736, 640), (4744, 1152),      # either side of the lines between 16, 8 and 4 warps; odd numbers of K blocks per warp
+    (2368, 2176), (2376, 384), (4736, 640), (4744, 896),      # either side of the lines between 16, 8 and 4 warps; odd numbers of K blocks per warp
 ])
 @pytest.mark.parametrize("f32", [True, False])
 def test_product(ctx, m, n, k, f32):
