@@ -377,8 +377,8 @@ static bool prefer_skinny(const dg_desc* d) {
     // DG_SKINNY=0 turns it off, and so does a knob that asks for something of another kernel
     for (const char* knob : {"DG_SWAP", "DG_BLOCK_N", "DG_CTAS", "DG_STAGES", "DG_SPLITS", "DG_K_SLABS"})
         if (getenv(knob)) return false;
-    const char* skinny = getenv("DG_SKINNY");
-    return !(skinny && atoi(skinny) == 0);
+    const char *skinny = getenv("DG_SKINNY"), *wide = getenv("DG_WIDE_TILE");
+    return !(skinny && atoi(skinny) == 0) && !(wide && atoi(wide) != 0);
 }
 const char* dg_kernel_name(const dg_desc* d) {
     if (d == nullptr) return nullptr;

@@ -27,6 +27,8 @@ def operand(ctx, rows, k, bits, seed, groups=1, gran=128, rows_per_group=None):
 def each(monkeypatch, run):
     """run() with the wide tiles and with 224-column tiles of a CTA pair."""
     monkeypatch.setenv("DG_WIDE_TILE", "1")
+    for rows in (1, 4096):
+        assert dg.kernel_name(dg.Sm100Desc(dg.GemmType.Normal, rows, 392, 128)) == "dg_gemm_wide_kernel"
     wide = run()
     monkeypatch.setenv("DG_WIDE_TILE", "0")
     monkeypatch.setenv("DG_SWAP", "0")
