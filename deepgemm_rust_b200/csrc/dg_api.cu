@@ -239,10 +239,11 @@ struct KernelPlan {
     uint32_t epi_bufs;         // staging buffers of an epilogue warp (first tile family)
     uint32_t block_n2;         // wide tiles: columns of the second half (0: not a wide tile)
     uint32_t table_groups;     // groups whose rows and tiles are kept in shared memory (swapped family)
+    uint32_t skinny_warps;     // the kernel for a handful of rows: warps of its blocks (0: another kernel)
 };
 // What a call rules out that its description does not tell: K ranges (the caller adds into the output: their sum is written, not added), wide
-// tiles (no bf16 operands).
-constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2;
+// tiles (no bf16 operands), the kernel for a handful of rows (neither bf16 operands nor a duty cycle).
+constexpr uint32_t kNoKRanges = 1, kNoWideTiles = 2, kNoSkinny = 4;
 static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, KernelPlan* plan);
 int dg_best_config(const dg_desc* d, dg_config* out) {
     KernelPlan plan;
@@ -380,20 +381,37 @@ static bool prefer_skinny(const dg_desc* d) {
     const char *skinny = getenv("DG_SKINNY"), *wide = getenv("DG_WIDE_TILE");
     return !(skinny && atoi(skinny) == 0) && !(wide && atoi(wide) != 0);
 }
-const char* dg_kernel_name(const dg_desc* d) {
-    if (d == nullptr) return nullptr;
-    if (prefer_skinny(d)) return "dg_gemm_skinny_kernel";
-    dg_config cfg;
-    KernelPlan plan;
-    if (search_config(d, 0, &cfg, &plan)) return nullptr;
-    return plan.swap ? "dg_gemm_swap_kernel" : (plan.block_n2 != 0 ? "dg_gemm_wide_kernel" : "dg_gemm_kernel");
-}
 // Warps of its blocks.  Blocks of 16 columns that all fit at once share K among as many warps as there are; with more blocks it is
 // several of them per SM that keep loads in flight (8 x 2112 x 7168 with 4 / 8 / 16 warps: 9.5 / 8.1 / 8.0 us; 1 x 4096 x 7168: 12.7 / 10.7 / 11.6;
 // 16 x 7168 x 2048: 8.4 / 9.4 / 11.5).
 static uint32_t skinny_warps(uint32_t n, uint32_t sms) {
     const uint32_t blocks = ceil_div(n, dg::kSkinnyCols);
     return blocks <= sms ? 16 : (blocks <= 2 * sms ? 8 : 4);
+}
+static uint32_t skinny_row_tiles(uint32_t m) { return m <= 8 ? 1 : (m <= 16 ? 2 : 4); }      // of 8 activation rows
+static void skinny_config(const dg_desc* d, dg_config* out, KernelPlan* plan) {
+    memset(plan, 0, sizeof(*plan));
+    plan->skinny_warps = skinny_warps(d->n, d->num_sms ? d->num_sms : 148);
+    plan->splits = 1;
+    plan->tiles = ceil_div(d->n, dg::kSkinnyCols);
+    const uint32_t row_tiles = skinny_row_tiles(d->m);
+    out->swap_ab = 0;
+    out->block_m = 8 * row_tiles;
+    out->block_n = dg::kSkinnyCols;
+    out->block_k = 128;
+    out->cluster_m = out->cluster_n = 1;
+    out->num_stages = row_tiles <= 2 ? 2 : 1;      // K blocks that a warp has in registers
+    out->num_accum_stages = 1;
+    out->smem_size = plan->smem = dg::skinny_smem_bytes(row_tiles, plan->skinny_warps);
+    out->num_tiles = plan->tiles;
+    out->num_splits = 1;
+}
+const char* dg_kernel_name(const dg_desc* d) {
+    dg_config cfg;
+    KernelPlan plan;
+    if (search_config(d, 0, &cfg, &plan)) return nullptr;
+    if (plan.skinny_warps != 0) return "dg_gemm_skinny_kernel";
+    return plan.swap ? "dg_gemm_swap_kernel" : (plan.block_n2 != 0 ? "dg_gemm_wide_kernel" : "dg_gemm_kernel");
 }
 
 // How a dense problem's tiles of two halves are dealt out to the CTA pairs.
@@ -462,7 +480,7 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, bool force
         best = cost;
         plan->swap = false;
         plan->ctas = 2; plan->umma_n = bn; plan->block_n2 = bn2; plan->halves = 1; plan->stages = stages; plan->accum = 1;
-        plan->splits = 1; plan->tiles = tiles; plan->epi_bufs = epi_bufs; plan->table_groups = 0;
+        plan->splits = 1; plan->tiles = tiles; plan->epi_bufs = epi_bufs; plan->table_groups = plan->skinny_warps = 0;
         plan->smem = smem();
         out->swap_ab = 0;
         out->block_m = 256;
@@ -559,7 +577,7 @@ static bool search_swapped(const dg_desc* d, uint32_t sms, dg_config* out, Kerne
                     // the group table takes what the stages leave of the shared memory
                     const uint32_t room = !dense && dg::swap_has_table(ctas, halves) ? (kSmemCapacity - plan->smem) / 16 : 0;
                     plan->table_groups = groups < room ? groups : room;
-                    plan->block_n2 = 0;
+                    plan->block_n2 = plan->skinny_warps = 0;
                     plan->smem += plan->table_groups * 16;
                     out->swap_ab = 1;
                     out->block_m = bn;            // activation rows per tile (an upper bound: a tile's UMMA N follows its rows)
@@ -583,6 +601,10 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
     if (d == nullptr || out == nullptr) return fail(DG_ERR_SHAPE, "null argument");
     if ((d->a_bits != 8 && d->a_bits != 4) || (d->b_bits != 8 && d->b_bits != 4)) return fail(DG_ERR_SHAPE, "operand bits must be 8 or 4");
     if ((d->major_a_mn && d->a_bits == 4) || (d->major_b_mn && d->b_bits == 4)) return fail(DG_ERR_SHAPE, "FP4 operands must be K-major");
+    if (!(limits & kNoSkinny) && prefer_skinny(d)) {
+        skinny_config(d, out, plan);
+        return DG_OK;
+    }
     // two packed e2m1 operands run on kind::mxf4 (256 elements per 128-byte slab); an e4m3 x e2m1 pair runs on
     // kind::mxf8f6f4 with the e2m1 side expanded to one code per byte by the TMA load (128 elements per slab)
     const bool mxf4 = d->a_bits == 4 && d->b_bits == 4;
@@ -734,7 +756,7 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
         if (!forbidden && search_wide(d, sms, best_cost, forced, out, plan)) return DG_OK;
     }
     const uint32_t stages = best_stages;
-    plan->block_n2 = 0;
+    plan->block_n2 = plan->skinny_warps = 0;
     plan->swap = false;
     plan->ctas = best_ctas; plan->umma_n = best_n; plan->halves = best_halves; plan->stages = best_stages; plan->accum = best_accum;
     plan->splits = best_splits; plan->tiles = best_tiles; plan->table_groups = 0;
@@ -996,8 +1018,8 @@ int reserve(dg_ctx* ctx, ScratchBuffer* buf, size_t bytes, bool zeroed = false) 
     return DG_OK;
 }
 
-int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue& e, const Problem& pr) {
-    const uint32_t tiles = pr.m <= 8 ? 1 : (pr.m <= 16 ? 2 : 4);      // of 8 activation rows
+int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, const dg_out* out, const dg_epilogue& e, const Problem& pr, uint32_t warps) {
+    const uint32_t tiles = skinny_row_tiles(pr.m);
     // what the tensor maps of the other kernels ask for
     if (reinterpret_cast<uintptr_t>(a->data) % 16 != 0 || reinterpret_cast<uintptr_t>(b->data) % 16 != 0 || reinterpret_cast<uintptr_t>(a->sf) % 16 != 0 ||
         reinterpret_cast<uintptr_t>(b->sf) % 16 != 0 || reinterpret_cast<uintptr_t>(out->buf) % 16 != 0)
@@ -1014,7 +1036,6 @@ int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, c
         if (tiles == 1) return f32 ? run(dg::dg_gemm_skinny_kernel<1, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<1, kWarps, false>, kWarps);
         return f32 ? run(dg::dg_gemm_skinny_kernel<2, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<2, kWarps, false>, kWarps);
     };
-    const uint32_t warps = skinny_warps(pr.n, static_cast<uint32_t>(ctx->num_sms));
     if (print_configs()) fprintf(stderr, "[dgb200] few rows: m=%u n=%u k=%u -> block=%ux%u warps=%u\n", pr.m, pr.n, pr.k, 8 * tiles, dg::kSkinnyCols, warps);
     const cudaError_t ce = warps == 4 ? with_warps(std::integral_constant<uint32_t, 4>()) : (warps == 8 ? with_warps(std::integral_constant<uint32_t, 8>()) : with_warps(std::integral_constant<uint32_t, 16>()));
     if (ce != cudaSuccess) return fail(DG_ERR_DRIVER, "kernel launch failed: %s", cudaGetErrorString(ce));
@@ -1066,11 +1087,11 @@ int launch_gemm(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, con
                     static_cast<uint32_t>(out->kind), static_cast<uint32_t>(ctx->num_sms), (!pr.bf16 && a->major_mn) ? 1u : 0u,
                     (!pr.bf16 && b->major_mn) ? 1u : 0u};
     const uint32_t tc_util = (e.tc_util == 0 || e.tc_util > 100) ? 100 : e.tc_util;      // 0 means "unset", as in ops_sm100.rs:518-522
-    if (!pr.bf16 && tc_util == 100 && prefer_skinny(&desc)) return launch_skinny(ctx, a, b, out, e, pr);
     dg_config cfg;
     KernelPlan plan;
-    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles : 0u), &cfg, &plan);
+    rc = choose_config(&desc, (e.accumulate ? kNoKRanges : 0u) | (pr.bf16 ? kNoWideTiles : 0u) | (pr.bf16 || tc_util < 100 ? kNoSkinny : 0u), &cfg, &plan);
     if (rc) return rc;
+    if (plan.skinny_warps != 0) return launch_skinny(ctx, a, b, out, e, pr, plan.skinny_warps);
     const bool swap = plan.swap;
     // the swapped family's kernel takes the operands with their roles exchanged: its operand A (UMMA M side) is the weights
     const dg_lp_operand* ka = swap ? b : a;

@@ -29,6 +29,9 @@ struct SkinnyParams {
     float alpha;
 };
 
+// Shared memory of a block, in the kernel's static array (host side).
+constexpr uint32_t skinny_smem_bytes(uint32_t row_tiles, uint32_t warps) { return warps * row_tiles * 8 * (kSkinnyCols + 1) * 4; }
+
 DG_DEVICE void mma_16x8x32_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])

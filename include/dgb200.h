@@ -312,11 +312,11 @@ typedef struct {
     uint32_t num_tiles;          /* expected tiles (from expected_m for grouped layouts) */
     uint32_t num_splits;         /* dense GEMMs with few tiles: K ranges computed by different CTAs and summed in f32 */
 } dg_config;
-/* heuristics_sm100.rs:455 (best_config) */
+/* heuristics_sm100.rs:455 (best_config): what an e4m3 / e2m1 call of this description launches if it neither accumulates (no K ranges
+ * then) nor sets a duty cycle (then not the kernel for a handful of dense rows).  That kernel's blocks hold block_m activation rows by block_n columns, all
+ * of K; its stages are the K blocks that a warp has in registers, its shared memory is static. */
 int dg_best_config(const dg_desc* desc, dg_config* out);
-/* The kernel that an e4m3 / e2m1 call of this description launches (without accumulation and duty cycle); null if none fits.  Where it is
- * dg_gemm_skinny_kernel, the one for a handful of dense activation rows, which has no tiles of this kind, dg_best_config describes what the
- * problem gets with DG_SKINNY=0. */
+/* The kernel of that call; null if none fits. */
 const char* dg_kernel_name(const dg_desc* desc);
 
 #ifdef __cplusplus

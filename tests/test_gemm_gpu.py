@@ -738,8 +738,9 @@ def test_swapped_masked_fp8_output_is_the_requantised_accumulator(ctx):
 
 
 @pytest.mark.parametrize("m,n", [(1, 9480), (17, 9480), (32, 18936), (64, 18936)])
-def test_rule_picks_the_swapped_family_for_few_dense_rows(ctx, m, n):
+def test_rule_picks_the_swapped_family_for_few_dense_rows(ctx, m, n, monkeypatch):
     k = 1280          # 75 and 148 weight blocks, the last one ragged; ten k-blocks
+    monkeypatch.setenv("DG_SKINNY", "0")
     assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).swap_ab
     _, aq, asf = fp8_operand_1d(m, k, 321)
     _, bq, bsf = fp8_operand_1d(n, k, 322)
@@ -760,8 +761,9 @@ def test_rule_picks_the_swapped_family_for_few_dense_rows(ctx, m, n):
 
 
 @pytest.mark.parametrize("m,n,k,picked", [(1, 3080, 1920, True), (32, 3080, 1920, True), (31, 9344, 4480, True), (5, 3080, 2048, False), (5, 3072, 1920, False)])
-def test_rule_picks_the_swapped_family_for_few_weight_blocks_with_short_k(ctx, m, n, k, picked):
+def test_rule_picks_the_swapped_family_for_few_weight_blocks_with_short_k(ctx, m, n, k, picked, monkeypatch):
     # 25 weight blocks are the fewest and 15 K slabs the most for them; 24 blocks or 16 slabs keep the K ranges
+    monkeypatch.setenv("DG_SKINNY", "0")
     assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).swap_ab == picked
     _, aq, asf = fp8_operand_1d(m, k, 331)
     _, bq, bsf = fp8_operand_1d(n, k, 332)
@@ -774,10 +776,11 @@ def test_rule_picks_the_swapped_family_for_few_weight_blocks_with_short_k(ctx, m
     assert not np.isnan(got).any()
 
 
-def test_a_failed_call_does_not_fail_the_next_one(ctx):
+def test_a_failed_call_does_not_fail_the_next_one(ctx, monkeypatch):
     # the allocation of 2^50 bytes is refused by the host and leaves its error with the runtime; the calls after it launch well and
     # have to say so (K ranges: two launches; quantiser: one; group table: a memset and two)
     m, n, k = 8, 2112, 7168
+    monkeypatch.setenv("DG_SKINNY", "0")
     assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).num_splits > 1
     x = torch.randn((m, k), device="cuda").bfloat16()
     calls = [lambda: run_dense(ctx, m, n, k), lambda: dg.cast_bf16_to_fp8_sf_dev(ctx, x, k, m, k, 128),

@@ -45,7 +45,7 @@ def contiguous(ctx, m, n, k):
 CASES = {
     "f32 scales, K ranges": (f32scale, (64, 1024, 2048), (64, 4096, 7168), {}),
     "f32 scales by their exponents": (f32scale, (64, 1024, 2048), (64, 4096, 7168), {"DG_F32_SCALES": "exponent"}),
-    "dense, K ranges": (dense, (8, 2112, 7168), (128, 7168, 16384), {}),
+    "dense, K ranges": (dense, (8, 2112, 7168), (128, 7168, 16384), {"DG_SKINNY": "0"}),
     "dense, swapped family, K ranges": (dense, (8, 1024, 4096), (128, 2048, 8192), {"DG_SWAP": "1", "DG_SPLITS": "3"}),
     "contiguous groups": (contiguous, (512, 256, 512), (8 * 128, 256, 512), {}),
 }
@@ -56,6 +56,10 @@ def test_scratch_of_a_captured_call(case, stream, monkeypatch):
     make, small, large, env = CASES[case]
     for name, value in env.items():
         monkeypatch.setenv(name, value)
+    if make is dense:
+        for size in (small, large):
+            choice = dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, *size))
+            assert choice.num_splits > 1 and choice.swap_ab == ("DG_SWAP" in env)
     warm = dg.DgContext(0)
     call, big_call = make(warm, *small), make(warm, *large)
     outs = [torch.zeros(size[:2], dtype=torch.bfloat16, device="cuda") for size in (small, small, small, large, large)]

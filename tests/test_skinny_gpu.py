@@ -45,6 +45,31 @@ def test_which_problems_get_it(m, n, k, skinny):
     assert is_skinny(m, n, k) == skinny
 
 
+@pytest.mark.parametrize("m,n,k,stages,smem", [(8, 2112, 7168, 2, 16 * 8 * 17 * 4), (16, 4736, 4096, 2, 8 * 16 * 17 * 4), (17, 4744, 896, 1, 4 * 32 * 17 * 4)])
+def test_tile_choice_describes_it(m, n, k, stages, smem, monkeypatch):
+    # 16, 8 and 4 warps: what the query reports is what a call launches
+    c = dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k))
+    assert (c.swap_ab, c.block_m, c.block_n, c.block_k, c.cluster_m, c.cluster_n) == (False, -(-m // 8) * 8 if m <= 16 else 32, 16, 128, 1, 1)
+    assert (c.num_stages, c.num_accum_stages, c.smem_size, c.num_tiles, c.num_splits) == (stages, 1, smem, -(-n // 16), 1)
+    monkeypatch.setenv("DG_SKINNY", "0")
+    assert dg.best_config(dg.Sm100Desc(dg.GemmType.Normal, m, n, k)).block_n > 16
+
+
+@pytest.mark.gpu
+def test_a_duty_cycle_goes_to_the_tiles_that_have_one(ctx):
+    # the order of the sums tells the kernels apart
+    m, n, k = 8, 2112, 7168
+    (a, _), (b, _) = operand(m, k, k, 8), operand(n, k, k, 9)
+    d = [torch.zeros((m, n), dtype=torch.float32, device="cuda") for _ in range(3)]
+    dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d[0], n), dg.Sm100Epilogue(tc_util=99))
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setenv("DG_SKINNY", "0")
+        dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d[1], n))
+    dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d[2], n))
+    ctx.sync()
+    assert torch.equal(d[0], d[1]) and not torch.equal(d[0], d[2])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n,k", [
