@@ -1340,10 +1340,14 @@ struct F32Plan {
     uint32_t ctas, block_n;          // a pair of CTAs with 256 x 256 tiles, or single CTAs with 128 x 128 tiles
     uint32_t splits, kb_per_split;   // K ranges (dense problems with few tiles), in k-blocks of 128
 };
-// Costs in microseconds, fitted on B200 over 22 problems (m 68-6900, n 560-8096, k 1152-8064): a K block takes 0.36 of a 128 x 128
-// tile and 0.45 of a 256 x 256 one (a quarter as many tiles, half the SM pairs), so the pair wins wherever its waves are fewer than
-// 0.8 of the others.  (Over the 40 problems that went over to the pair when its 0.56 became 0.45, it takes 0.93 of the other's time,
-// 0.87 to 1.01: 1315 x 4000 x 5376 54.1 -> 47.8 us, 6432 x 1344 x 2432 37.5 -> 38.0.)  K ranges pay 3.5 plus their planes for the second launch, and never more than one wave.
+// Costs in microseconds.  A K block takes 0.36 of a 128 x 128 tile; that, and the 3.5 that K ranges pay for the second launch beside their planes, were
+// fitted on B200 over 22 dense problems (m 68-6900, n 560-8096, k 1152-8064).  K ranges never make more than one wave.  A 256 x 256 tile (a quarter
+// as many tiles, half the SM pairs) counts with
+//   0.45 in dense problems: the pair wins wherever its waves are fewer than 0.8 of the others.  It took 0.56 before its loop became shorter; over 25
+//     problems between the two lines (m 1046-7787, n 736-4976, k 1024-5760) it takes 0.94 of the single tiles' time, 0.88 to 1.01;
+//   0.56 in contiguous groups, of which an arena says only how many rows they may have: over 50 problems between the two lines (2-96 groups) the pair takes 0.93
+//     of the time where more than three quarters of the arena are live, 1.04 with 0.4 and 1.27 with 0.1 of it (16 groups of 75 rows in 8192, 1120 x 2816:
+//     20.5 -> 35.3 us), 1.09 on average.
 F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint32_t groups, uint32_t sms) {
     const uint32_t kbs = k / 128;
     const bool dense = type == DG_GEMM_NORMAL;
@@ -1358,7 +1362,7 @@ F32Plan choose_f32scale(uint32_t type, uint32_t m, uint32_t n, uint32_t k, uint3
     auto waves = [](double t, uint32_t workers) { return static_cast<double>(static_cast<uint64_t>(t / workers + 0.999)); };
     F32Plan best = {1, 128, 1, kbs};
     double best_cost = waves(tiles, sms) * (kbs * 0.36 + 0.6);
-    const double pair_cost = sms >= 2 ? waves(pair_tiles, sms / 2) * (kbs * 0.45 + 1.2) : best_cost;
+    const double pair_cost = sms >= 2 ? waves(pair_tiles, sms / 2) * (kbs * (dense ? 0.45 : 0.56) + 1.2) : best_cost;
     // (a masked group's rows are known to the device only and usually fewer than its slot: small tiles)
     if (type != DG_GEMM_M_GROUPED_MASKED && pair_cost < best_cost) {
         best = {2, 256, 1, kbs};

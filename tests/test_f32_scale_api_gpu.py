@@ -232,11 +232,12 @@ def test_one_context_on_two_streams(ctx):
 
 def test_small_contiguous_groups_get_small_tiles():
     # arenas of 128 rows per group: a group fits one tile of 128 rows and all tiles one wave of the SMs; the arena's padding must not
-    # be taken for rows that make a second wave of them
+    # be taken for rows that make a second wave of them.  16 groups of at most 512: pairs are faster by a little if the arena is full and slower
+    # by up to 1.7 if it is not, which only the device knows.
     code = """
 import torch, deepgemm_rust_b200 as dg
 ctx = dg.DgContext(0)
-for groups, rows, n, k in ((12, 128, 1152, 3456), (18, 128, 1024, 512)):
+for groups, rows, n, k in ((12, 128, 1152, 3456), (18, 128, 1024, 512), (16, 512, 1152, 2816)):
     m = groups * rows
     a, b = (dg.Fp8Tensor(torch.zeros((r, k), dtype=torch.uint8, device="cuda"), r, k, k) for r in (m, groups * n))
     sfa_t = dg.transform_sf_dev(ctx, torch.ones((m, k // 128), device="cuda"), m, k // 128)
@@ -249,7 +250,7 @@ ctx.sync()
                          env={**os.environ, "DG_PRINT_CONFIGS": "1"})
     assert run.returncode == 0, run.stderr
     lines = [line for line in run.stderr.splitlines() if "f32 scales" in line]
-    assert len(lines) == 2 and all("block=128x128 ctas=1" in line for line in lines), lines
+    assert len(lines) == 3 and all("block=128x128 ctas=1" in line for line in lines), lines
 
 
 @pytest.mark.parametrize("k_blocks", [1, 2, 3, 6])
