@@ -433,13 +433,17 @@ static WideWaves wide_waves(uint32_t m, uint32_t n, uint32_t block_n, uint32_t p
 }
 
 // Wide tiles (dg_gemm_wide.cuh) for a problem that costs `other` in the first family's other tiles; false if those are the better ones (or
-// the only ones), unless `forced`.
-// Measured under the power cap that long runs settle at, both in turn.  Contiguous groups of 450-6500 rows, from three waves of tiles on
-// (27 problems, k 1024-6656, n 1024-6848): 0.96 of the other tiles' time on average, 0.92 to 1.02; with fewer waves up to 1.14.  Dense problems, from two and
-// a half waves on (50 of them, k 1024-16384): the constants below are fitted to those, and with them the 33 that are chosen take
+// the only ones, of width `other_n`), unless `forced`.
+// Contiguous groups of 450 rows on, where the first 256 rows of each alone make three and a half waves of tiles: an arena may be sized for far more rows than it
+// holds, and what the device finds is what decides.  Both tiles measured in three ways: under the power cap (bursts of 0.5 s a side, balanced), and single passes
+// in turn after a 256 MB fill and after 20 ms of idling.  18 problems inside the lines (k 2048-7168, n 2112-7168, 22-64 groups) take 0.96, 0.99 and
+// 0.99 of the other tiles' time with a full arena, up to 1.00, 1.03 and 1.03; 0.98, 0.99 and 0.97 with 3 % of it live, up to 1.03, 1.05 and 1.07.  With fewer tiles (17
+// problems) 0.96, 0.97 and 0.98 full, but 1.05, 1.09 and 1.08 with 3 % live, up to 1.32 (8 groups of 47 rows in 13696, 1600 x 7168: 28.5 -> 35.2 us).  K of less
+// than 16 slabs, and tiles that cover more columns than the others do, lose too (23 groups of 4211 rows, 1152 x 1024, single passes: 1.01; of 1052: 1.14).
+// Dense problems, from two and a half waves on (50 of them, k 1024-16384): the constants below are fitted to those, and with them the 33 that are chosen take
 // 0.98 of the time, 0.90 to 1.05.  Halves of 160 columns were slower than both (5841 x 3720 x 11776 mxfp4: 114 -> 124 us).  Masked and batched problems, and
 // e4m3 operands with per-32 scales, were not measured and keep the other tiles.
-static bool search_wide(const dg_desc* d, uint32_t sms, double other, bool forced, dg_config* out, KernelPlan* plan) {
+static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t other_n, bool forced, dg_config* out, KernelPlan* plan) {
     if (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32) return false;
     if (d->major_a_mn || d->major_b_mn || sms < 2 || d->gemm_type == DG_GEMM_BATCHED) return false;
     if (!forced && (d->gemm_type == DG_GEMM_M_GROUPED_MASKED || (d->a_bits == 8 && d->gran_a != 128) || (d->b_bits == 8 && d->gran_b != 128))) return false;
@@ -474,7 +478,9 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, bool force
         while (stages > 3 && smem() > kSmemCapacity) --stages;
         if (smem() > kSmemCapacity) continue;
         const double cost = halves * (total_kb * (2.0 * bn + 130.0) + 1500.0 + (d->cd_dtype == DG_OUT_F32 ? 1000.0 : 0.0)) + 8000.0;
-        if (!forced && (dense ? halves < 5 || cost >= other : halves < 6 || group_rows(d) < 450.0)) continue;
+        const uint32_t across = ceil_div(d->n, bn + bn2);
+        const bool wider = across * (bn + bn2) > 1.02 * (ceil_div(d->n, other_n) * other_n);
+        if (!forced && (dense ? halves < 5 || cost >= other : 2 * groups * across < 7 * pairs || group_rows(d) < 450.0 || total_kb < 16 || wider)) continue;
         if (found && cost >= best) continue;
         found = true;
         best = cost;
@@ -753,7 +759,7 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
     {
         const char* wide = getenv("DG_WIDE_TILE");       // 0: never, 1: wherever they apply
         const bool forced = wide && atoi(wide) != 0, forbidden = (wide && atoi(wide) == 0) || (limits & kNoWideTiles) || pinned;
-        if (!forbidden && search_wide(d, sms, best_cost, forced, out, plan)) return DG_OK;
+        if (!forbidden && search_wide(d, sms, best_cost, best_n, forced, out, plan)) return DG_OK;
     }
     const uint32_t stages = best_stages;
     plan->block_n2 = plan->skinny_warps = 0;

@@ -148,7 +148,9 @@ CONTIGUOUS = dg.GemmType.MGroupedContiguous
     ((dg.GemmType.Normal, 4096, 7168, 16384), dict(gran_a=32), False), ((dg.GemmType.Normal, 4096, 7168, 16384), dict(cd_dtype=2), False),
     ((dg.GemmType.Normal, 1024, 4096, 7168), {}, False),                                       # one wave
     ((CONTIGUOUS, 32 * 2112, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 520, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 512, 4096, 7168, 32), {}, False),
-    ((CONTIGUOUS, 4 * 1024, 2048, 7168, 4), {}, False),                                        # less than three waves
+    # groups whose first 256 rows make three and a half waves of tiles, whatever the arena holds; 16 slabs of K; no more columns than the other tiles have
+    ((CONTIGUOUS, 26 * 2048, 4096, 7168, 26), {}, True), ((CONTIGUOUS, 25 * 2048, 4096, 7168, 25), {}, False), ((CONTIGUOUS, 13696, 1600, 7168, 8), {}, False),
+    ((CONTIGUOUS, 32 * 2112, 4096, 2048, 32), {}, True), ((CONTIGUOUS, 32 * 2112, 4096, 1920, 32), {}, False), ((CONTIGUOUS, 32 * 2112, 5568, 7168, 32), {}, False),
     ((dg.GemmType.MGroupedMasked, 2048, 4096, 7168, 32, 2048), {}, False), ((dg.GemmType.Batched, 2048, 4096, 7168, 16), {}, False),
 ])
 def test_which_problems_get_them(sizes, kw, wide):
