@@ -433,17 +433,23 @@ static WideWaves wide_waves(uint32_t m, uint32_t n, uint32_t block_n, uint32_t p
 }
 
 // Wide tiles (dg_gemm_wide.cuh) for a problem that costs `other` in the first family's other tiles; false if those are the better ones (or
-// the only ones, of width `other_n`), unless `forced`.
+// the only ones, of width `other_n`, `other_columns` of them for each CTA or pair), unless `forced`.
 // Contiguous groups of 450 rows on, where the first 256 rows of each alone make three and a half waves of tiles: an arena may be sized for far more rows than it
 // holds, and what the device finds is what decides.  Both tiles measured in three ways: under the power cap (bursts of 0.5 s a side, balanced), and single passes
 // in turn after a 256 MB fill and after 20 ms of idling.  18 problems inside the lines (k 2048-7168, n 2112-7168, 22-64 groups) take 0.96, 0.99 and
 // 0.99 of the other tiles' time with a full arena, up to 1.00, 1.03 and 1.03; 0.98, 0.99 and 0.97 with 3 % of it live, up to 1.03, 1.05 and 1.07.  With fewer tiles (17
 // problems) 0.96, 0.97 and 0.98 full, but 1.05, 1.09 and 1.08 with 3 % live, up to 1.32 (8 groups of 47 rows in 13696, 1600 x 7168: 28.5 -> 35.2 us).  K of less
 // than 16 slabs, and tiles that cover more columns than the others do, lose too (23 groups of 4211 rows, 1152 x 1024, single passes: 1.01; of 1052: 1.14).
-// Dense problems, from two and a half waves on (50 of them, k 1024-16384): the constants below are fitted to those, and with them the 33 that are chosen take
-// 0.98 of the time, 0.90 to 1.05.  Halves of 160 columns were slower than both (5841 x 3720 x 11776 mxfp4: 114 -> 124 us).  Masked and batched problems, and
-// e4m3 operands with per-32 scales, were not measured and keep the other tiles.
-static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t other_n, bool forced, dg_config* out, KernelPlan* plan) {
+// Dense problems by cost, within lines.  Of 180 that the cost alone picks (m 200-8192, n 512-16384, k 1024-16384) the 75 inside take 0.96, 0.97 and 0.98 of
+// the other tiles' time, measured in the same ways, up to 1.00, 1.01 and 1.02; the others 0.99, 1.03 and 1.03, up to 1.09, 1.16 and 1.13:
+//   f32 outputs of two e2m1 operands (22 of them: 1.02, 1.06 and 1.06), whose stores take longer than the UMMAs of their K;
+//   short K, by the drain of two accumulators per tile: below 32 slabs with an e4m3 operand (23: 1.00, 1.03, 1.04), 16 with two of e2m1 (22: 0.96, 1.04, 0.98);
+//   an even number of halves per pair, which ends in two single halves on one accumulator (8 or 10 of them, e4m3: 1.00, 1.01, 1.02), unless there are
+//     many, or two e2m1 operands have a long K;
+//   more columns for a pair to work through than `other_columns` (2607 x 6624 x 10240, e4m3 x e2m1: 1.01, 1.03, 1.05).
+// Halves of 160 columns were slower than both (5841 x 3720 x 11776 mxfp4: 114 -> 124 us).  Masked and batched problems, and e4m3 operands with per-32
+// scales, were not measured and keep the other tiles.
+static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t other_n, uint32_t other_columns, bool forced, dg_config* out, KernelPlan* plan) {
     if (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32) return false;
     if (d->major_a_mn || d->major_b_mn || sms < 2 || d->gemm_type == DG_GEMM_BATCHED) return false;
     if (!forced && (d->gemm_type == DG_GEMM_M_GROUPED_MASKED || (d->a_bits == 8 && d->gran_a != 128) || (d->b_bits == 8 && d->gran_b != 128))) return false;
@@ -451,7 +457,7 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t o
     const uint32_t sfa_words = 4 * d->gran_a >= block_k ? 1 : block_k / (4 * d->gran_a), sfb_words = 4 * d->gran_b >= block_k ? 1 : block_k / (4 * d->gran_b);
     const uint32_t total_kb = ceil_div(d->k, block_k);
     const bool dense = d->gemm_type == DG_GEMM_NORMAL;
-    bool found = false;
+    bool found = false, chosen = false;
     double best = 0;
     for (uint32_t most = 224; most >= 192; most -= 32) {
         uint32_t bn = most, bn2 = most, tiles;
@@ -480,10 +486,15 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t o
         const double cost = halves * (total_kb * (2.0 * bn + 130.0) + 1500.0 + (d->cd_dtype == DG_OUT_F32 ? 1000.0 : 0.0)) + 8000.0;
         const uint32_t across = ceil_div(d->n, bn + bn2);
         const bool wider = across * (bn + bn2) > 1.02 * (ceil_div(d->n, other_n) * other_n);
-        if (!forced && (dense ? halves < 5 || cost >= other : 2 * groups * across < 7 * pairs || group_rows(d) < 450.0 || total_kb < 16 || wider)) continue;
+        const bool odd = static_cast<uint32_t>(halves) % 2 != 0;
+        bool inside;
+        if (!dense) inside = 2 * groups * across >= 7 * pairs && group_rows(d) >= 450.0 && total_kb >= 16 && !wider;
+        else if (block_k == 256) inside = d->cd_dtype == DG_OUT_BF16 && total_kb >= 16 && (odd || (total_kb >= 24 && halves >= 8));
+        else inside = total_kb >= 32 && (halves >= 11 || (odd && total_kb >= 48));
         if (found && cost >= best) continue;
         found = true;
         best = cost;
+        chosen = forced || (inside && !(dense && (halves < 5 || cost >= other || halves * bn > 1.05 * other_columns)));
         plan->swap = false;
         plan->ctas = 2; plan->umma_n = bn; plan->block_n2 = bn2; plan->halves = 1; plan->stages = stages; plan->accum = 1;
         plan->splits = 1; plan->tiles = tiles; plan->epi_bufs = epi_bufs; plan->table_groups = plan->skinny_warps = 0;
@@ -500,7 +511,7 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t o
         out->num_tiles = tiles;
         out->num_splits = 1;
     }
-    return found;
+    return chosen;
 }
 
 // Tile choice of the swapped family; false if nothing fits (or the DG_* knobs leave nothing).
@@ -759,7 +770,7 @@ static int search_config(const dg_desc* d, uint32_t limits, dg_config* out, Kern
     {
         const char* wide = getenv("DG_WIDE_TILE");       // 0: never, 1: wherever they apply
         const bool forced = wide && atoi(wide) != 0, forbidden = (wide && atoi(wide) == 0) || (limits & kNoWideTiles) || pinned;
-        if (!forbidden && search_wide(d, sms, best_cost, best_n, forced, out, plan)) return DG_OK;
+        if (!forbidden && search_wide(d, sms, best_cost, best_n, ceil_div(best_tiles, sms / best_ctas) * best_n, forced, out, plan)) return DG_OK;
     }
     const uint32_t stages = best_stages;
     plan->block_n2 = plan->skinny_warps = 0;

@@ -141,12 +141,20 @@ def test_grouped(ctx, monkeypatch, alignment, n, f32):
 
 
 CONTIGUOUS = dg.GemmType.MGroupedContiguous
+E2M1 = dict(a_bits=4, b_bits=4, gran_a=32, gran_b=32)
+MIXED = dict(b_bits=4, gran_b=32)
 
 
 @pytest.mark.parametrize("sizes,kw,wide", [
     ((dg.GemmType.Normal, 4096, 7168, 16384), {}, True), ((dg.GemmType.Normal, 4096, 7168, 7168), dict(a_bits=4, b_bits=4, gran_a=32, gran_b=32), True),
     ((dg.GemmType.Normal, 4096, 7168, 16384), dict(gran_a=32), False), ((dg.GemmType.Normal, 4096, 7168, 16384), dict(cd_dtype=2), False),
     ((dg.GemmType.Normal, 1024, 4096, 7168), {}, False),                                       # one wave
+    ((dg.GemmType.Normal, 4096, 7168, 7168), dict(**E2M1, cd_dtype=1), False),
+    # K of 32 slabs with many halves per pair, of 16 and 24 with two e2m1 operands; few and even numbers of halves; more columns
+    ((dg.GemmType.Normal, 8192, 8192, 4096), {}, True), ((dg.GemmType.Normal, 8192, 8192, 3968), {}, False), ((dg.GemmType.Normal, 5604, 3400, 8192), {}, True),
+    ((dg.GemmType.Normal, 5604, 3400, 6016), {}, False), ((dg.GemmType.Normal, 6516, 4616, 9216), {}, False), ((dg.GemmType.Normal, 2607, 6624, 10240), MIXED, False),
+    ((dg.GemmType.Normal, 4096, 7168, 4096), E2M1, True), ((dg.GemmType.Normal, 4096, 7168, 3840), E2M1, False),
+    ((dg.GemmType.Normal, 7300, 4216, 6144), E2M1, True), ((dg.GemmType.Normal, 7300, 4216, 4096), E2M1, False),
     ((CONTIGUOUS, 32 * 2112, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 520, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 512, 4096, 7168, 32), {}, False),
     # groups whose first 256 rows make three and a half waves of tiles, whatever the arena holds; 16 slabs of K; no more columns than the other tiles have
     ((CONTIGUOUS, 26 * 2048, 4096, 7168, 26), {}, True), ((CONTIGUOUS, 25 * 2048, 4096, 7168, 25), {}, False), ((CONTIGUOUS, 13696, 1600, 7168, 8), {}, False),
