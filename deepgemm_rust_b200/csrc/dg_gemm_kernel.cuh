@@ -156,8 +156,10 @@ struct Scheduler {
         }
     }
 
-    DG_DEVICE bool next(Tile& t) {
-        uint32_t idx = worker + (iter++) * num_workers;
+    DG_DEVICE bool next(Tile& t) { return tile(worker + (iter++) * num_workers, t); }
+
+    // The tile of that number; grouped layouts: numbers may not go back from call to call.
+    DG_DEVICE bool tile(uint32_t idx, Tile& t) {
         const uint32_t total_kb = (p.k + p.block_k_elems - 1) / p.block_k_elems;
         t.kb0 = 0;
         t.kb1 = total_kb;

@@ -104,7 +104,8 @@ def test_duty_cycle_paces_them_like_the_other_tiles(ctx, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("alignment", [16, 128])
-@pytest.mark.parametrize("n", [456, 1096])
+# 24 and 36 tiles, all as single halves; 72 whole ones; 74 whole ones and 10 as halves, some of which have no columns
+@pytest.mark.parametrize("n", [456, 1096, 2600, 2704])
 @pytest.mark.parametrize("f32", [True, False])
 def test_grouped(ctx, monkeypatch, alignment, n, f32):
     # groups of nothing, of one row, of just a tile, of a tile and a row: boxes that cross a group's end, tiles that run into the next group
@@ -156,9 +157,10 @@ MIXED = dict(b_bits=4, gran_b=32)
     ((dg.GemmType.Normal, 4096, 7168, 4096), E2M1, True), ((dg.GemmType.Normal, 4096, 7168, 3840), E2M1, False),
     ((dg.GemmType.Normal, 7300, 4216, 6144), E2M1, True), ((dg.GemmType.Normal, 7300, 4216, 4096), E2M1, False),
     ((CONTIGUOUS, 32 * 2112, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 520, 4096, 7168, 32), {}, True), ((CONTIGUOUS, 32 * 512, 4096, 7168, 32), {}, False),
-    # groups whose first 256 rows make three and a half waves of tiles, whatever the arena holds; 16 slabs of K; no more columns than the other tiles have
-    ((CONTIGUOUS, 26 * 2048, 4096, 7168, 26), {}, True), ((CONTIGUOUS, 25 * 2048, 4096, 7168, 25), {}, False), ((CONTIGUOUS, 13696, 1600, 7168, 8), {}, False),
-    ((CONTIGUOUS, 32 * 2112, 4096, 2048, 32), {}, True), ((CONTIGUOUS, 32 * 2112, 4096, 1920, 32), {}, False), ((CONTIGUOUS, 32 * 2112, 5568, 7168, 32), {}, False),
+    # groups whose first 256 rows make 1.3 waves of tiles, whatever the arena holds, with K below 20 slabs three and a half; no more columns than the other tiles have
+    ((CONTIGUOUS, 10 * 2048, 4096, 2560, 10), {}, True), ((CONTIGUOUS, 9 * 2048, 4096, 7168, 9), {}, False), ((CONTIGUOUS, 13696, 1600, 7168, 8), {}, False),
+    ((CONTIGUOUS, 26 * 2048, 4096, 2048, 26), {}, True), ((CONTIGUOUS, 25 * 2048, 4096, 2048, 25), {}, False), ((CONTIGUOUS, 25 * 2048, 4096, 2560, 25), {}, True),
+    ((CONTIGUOUS, 32 * 2112, 4096, 1920, 32), {}, False), ((CONTIGUOUS, 32 * 2112, 5568, 7168, 32), {}, False),
     ((dg.GemmType.MGroupedMasked, 2048, 4096, 7168, 32, 2048), {}, False), ((dg.GemmType.Batched, 2048, 4096, 7168, 16), {}, False),
 ])
 def test_which_problems_get_them(sizes, kw, wide):
