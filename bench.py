@@ -230,6 +230,21 @@ def gemm_kernel(dg, *sizes, **kw):
     return dg.kernel_name(dg.Sm100Desc(*sizes, **kw))
 
 
+def traffic_entry(table, launch, kernel):
+    """The entry of profiles/traffic.json that was captured from this launch by this kernel, or None."""
+    def matches(key, entry):
+        if not launch.startswith(key) or entry["kernel"] != kernel:
+            return False
+        # an entry measured (or scaled) for a given number of routed rows only describes launches within 5 % of it
+        want = entry.get("routed_rows")
+        if not want or "routed rows" not in launch:
+            return True
+        have = int(launch.split(" routed rows")[0].split(", ")[-1])
+        return abs(have - want) <= 0.05 * want
+    keys = [key for key, entry in table.items() if matches(key, entry)]
+    return table[max(keys, key=len)] if keys else None
+
+
 class DenseWork:
     """The ten dense FP8 GEMMs; operands quantised once by the library's own kernels and kept resident."""
 
@@ -1240,15 +1255,7 @@ def main():
             us, name, fl, nbytes, kernel = cand
             row = launch_bound(fl, nbytes, us * 1e-6, peaks, 2)
 
-            def rows_match(entry):
-                # an entry measured (or scaled) for a given number of routed rows only describes launches within 5 % of it
-                want = entry.get("routed_rows")
-                if not want or "routed rows" not in name:
-                    return True
-                have = int(name.split(" routed rows")[0].split(", ")[-1])
-                return abs(have - want) <= 0.05 * want
-            keys = [key for key in traffic_table if name.startswith(key) and rows_match(traffic_table[key])]
-            tr = traffic_table[max(keys, key=len)] if keys else None
+            tr = traffic_entry(traffic_table, name, kernel.split("<")[0])
             entry = {"bound": row["bound"], "kernel": kernel, "launch": name, "us_in_step": round(us, 1),
                      "share_of_step": round(us * 1e-3 / ms_per_step, 3), "sm_mhz_median": sm_mhz,
                      "traffic": tr["dram_bytes_per_launch"] if tr else None, "traffic_source": tr["source"] if tr else None,
