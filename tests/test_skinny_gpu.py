@@ -78,6 +78,20 @@ def test_a_duty_cycle_goes_to_the_tiles_that_have_one(ctx):
 ])
 @pytest.mark.parametrize("f32", [True, False])
 def test_product(ctx, m, n, k, f32):
+    check_product(ctx, m, n, k, f32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [
+    (8, 2112, 7168), (8, 1280, 24576), (1, 4096, 15616), (8, 9344, 5248),      # the longest K of 16, 8 and 4 warps
+    (9, 1024, 12288), (16, 3344, 7168), (16, 9472, 2432), (32, 1920, 4096), (17, 9472, 768),
+])
+@pytest.mark.parametrize("f32", [True, False])
+def test_product_of_the_longest_k(ctx, m, n, k, f32):
+    check_product(ctx, m, n, k, f32)
+
+
+def check_product(ctx, m, n, k, f32):
     assert is_skinny(m, n, k)
     (a, fa), (b, fb) = operand(m, k, k + 16, 1), operand(n, k, k + 32, 2)
     ld = n + 8
@@ -85,8 +99,8 @@ def test_product(ctx, m, n, k, f32):
     dg.fp8_fp4_gemm_dev(ctx, a, b, dg.Sm100Out.F32(d, ld) if f32 else dg.Sm100Out.Bf16(d, ld))
     ctx.sync()
     want, size = fa @ fb.T, fa.abs() @ fb.abs().T
-    # f32 sums: fewer than 128 roundings of 2^-24 of the terms' magnitudes (8 instructions per K block, 17 blocks at most, 16 warps); a bf16 result
-    # is rounded once more, 8 significant bits
+    # f32 sums: fewer than 128 roundings of 2^-24 of the terms' magnitudes (four instructions and a sum for each of a warp's K blocks, 16 at most, then the
+    # warps', 16 at most); a bf16 result is rounded once more, 8 significant bits
     bound = 128 * 2.0 ** -24 * size + (0.0 if f32 else 2.0 ** -8) * want.abs()
     assert bool(((d[:, :n].double() - want).abs() <= bound).all())
     assert bool((d[:, n:] == 7.0).all())
