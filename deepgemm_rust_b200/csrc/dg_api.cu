@@ -351,16 +351,18 @@ static bool prefer_swapped(const dg_desc* d) {
 
 // Is the kernel for a handful of activation rows (dg_gemm_skinny.cuh) the one for this problem?  Measured against the other kernels over 1263
 // problems (m 1-32, n 16-343744, k 128-62464), the GEMM alone, in a loop and in a graph of 24, weights from DRAM.  What bounds it is the latency of plain
-// loads: a warp's rounds of K blocks, times the waves of blocks (four of four warps fit an SM).  Inside the lines below it takes 0.72 of the
-// others' time on average and 1.03 at most; the figures are of the graphs.
+// loads: a warp's rounds of K blocks, times the waves of blocks (four of four warps fit an SM).  Inside the lines below it takes 0.73 of the
+// others' time on average and 1.10 at most (16 x 512 x 12288); behind the activation quantiser, where its shorter start-up shows, 0.93 and 1.03 at most over the
+// 69 problems nearest to the lines, 0.88 at most with weights in L2.  The figures are of the graphs, or of both launches where it says so.
 //   Up to 8 rows it wins to 64 MB (5 x 4472 x 13312: 17.4 -> 14.4 us; 1 x 6144 x 9728: 17.3 -> 17.3), to 44 where the swapped family
 //     fills the SMs (8 x 16384 x 2560: 11.6 -> 11.0), and to 16384 of K (8 x 256 x 16384: 8.7 -> 8.2, x 32768: 10.5 -> 14.8), 24576 where blocks of 16 warps
 //     take more than half of the SMs (8 x 1280 x 24576: 13.0 -> 12.7; 8 x 1024 x 28672: 13.2 -> 13.7).
 //   9-16 rows: while the blocks fit at once to 24 MB (16 x 9472 x 2304: 9.9 -> 8.7) and 7168 of K (16 x 2400 x 6656: 10.6 -> 10.6), with 16 warps
-//     12288 (16 x 1024 x 12288: 9.8 -> 9.7), or 10240 with so few blocks that K ranges occupy more SMs (16 x 512 x 10240: 8.6 -> 8.6, x 12288: 8.7 -> 9.6);
-//     in two waves two rounds of K (16 x 18432 x 1024: 8.8 -> 8.1, x 1152: 9.5 -> 9.9), in more one (16 x 28672 x 512: 8.6 -> 7.6, x 640: 9.3 -> 10.8).
-//   17-32 rows, whose K blocks are not prefetched: to 8 MB and 4096 of K (32 x 3072 x 2560: 9.5 -> 8.5), with four warps to 896
-//     (32 x 4800 x 896: 6.4 -> 6.2, x 1024: 6.4 -> 6.7), in two waves one round (32 x 12288 x 512: 6.7 -> 6.7, x 640: 7.3 -> 9.7).
+//     12288 (16 x 1024 x 12288: 9.8 -> 9.7; 16 x 512: 8.7 -> 9.6, with the quantiser 12.5 -> 12.1), or 10240 with so few blocks that K ranges occupy more SMs (16 x 16 x
+//     10240: 7.2 -> 7.1, x 12288: 7.2 -> 8.1); in two waves two rounds of K (16 x 18432 x 1024: 8.8 -> 8.1, x 1152: 9.5 -> 9.9), in more one, or two full ones
+//     (16 x 28672 x 512: 8.6 -> 7.6, x 640: 9.3 -> 10.8; 16 x 22528 x 1024: 9.9 -> 9.9, with the quantiser 12.6 -> 12.5, x 896: 9.3 -> 9.6).
+//   17-32 rows, whose K blocks are not prefetched: to 8 MB and 4096 of K (32 x 3072 x 2560: 9.5 -> 8.5), with four warps two rounds
+//     of K (32 x 6144 x 1024: 6.7 -> 6.8, with the quantiser 10.3 -> 9.0, x 1280: 7.5 -> 8.3), in two waves one round (32 x 12288 x 512: 6.7 -> 6.7, x 640: 7.3 -> 9.7).
 //   More short blocks than 14 (7) per SM: 8 x 65536 x 128 9.0 -> 9.2, 8 x 343744 x 128 30.7 -> 42.4, 32 x 32768 x 128 6.8 -> 10.2.
 static bool prefer_skinny(const dg_desc* d) {
     if (d->gemm_type != DG_GEMM_NORMAL || d->k % 128 != 0 || (d->cd_dtype != DG_OUT_BF16 && d->cd_dtype != DG_OUT_F32)) return false;
@@ -370,9 +372,9 @@ static bool prefer_skinny(const dg_desc* d) {
     const uint32_t blocks = ceil_div(d->n, dg::kSkinnyCols);
     bool few = false;
     if (d->m <= 8) few = blocks <= 14 * sms && mb <= (2 * ceil_div(d->n, 128) >= sms ? 44.0 : 64.0) && d->k <= (blocks <= sms && 2 * blocks > sms ? 24576u : 16384u);
-    else if (d->m <= 16 && blocks <= 4 * sms) few = mb <= 24.0 && d->k <= (blocks > sms ? 7168u : (blocks >= 64 ? 12288u : 10240u));
-    else if (d->m <= 16) few = blocks <= 14 * sms && d->k <= (blocks <= 8 * sms ? 1024u : 512u);
-    else if (d->m <= 32 && blocks <= 4 * sms) few = mb <= 8.0 && d->k <= (blocks <= 2 * sms ? 4096u : 896u);
+    else if (d->m <= 16 && blocks <= 4 * sms) few = mb <= 24.0 && d->k <= (blocks > sms ? 7168u : (blocks >= 32 ? 12288u : 10240u));
+    else if (d->m <= 16) few = blocks <= 14 * sms && mb <= 24.0 && (d->k <= 512 || (d->k <= 1024 && (blocks <= 8 * sms || d->k % 512 == 0)));
+    else if (d->m <= 32 && blocks <= 4 * sms) few = mb <= 8.0 && d->k <= (blocks <= 2 * sms ? 4096u : 1024u);
     else if (d->m <= 32) few = blocks <= 7 * sms && mb <= 6.3 && d->k <= 512;
     if (!few || knob_signature() == 0) return few;
     // DG_SKINNY=0 turns it off, and so does a knob that asks for something of another kernel

@@ -35,9 +35,10 @@ def is_skinny(m, n, k):
     (17, 1960, 4096, False), (17, 512, 4224, False), (33, 512, 1024, False),
     # K that few blocks share among 16 warps; blocks in one, two and more waves; more of them than those of a few warps are worth
     (8, 1184, 16384, True), (8, 1184, 16512, False), (8, 1192, 24576, True), (8, 2368, 24704, False), (8, 2376, 16512, False),
-    (9, 1008, 10240, True), (9, 1008, 10368, False), (8, 33152, 128, True), (8, 33160, 128, False), (8, 343744, 128, False),
-    (16, 9472, 2432, True), (16, 9480, 1024, True), (16, 9480, 1152, False), (16, 18944, 1024, True), (16, 18952, 640, False), (16, 33152, 512, True),
-    (16, 33160, 128, False), (17, 4736, 1664, True), (17, 4744, 896, True), (17, 4744, 1024, False), (17, 9472, 768, True), (17, 9480, 512, True),
+    (9, 496, 10240, True), (9, 496, 10368, False), (9, 504, 12288, True), (9, 504, 12416, False), (8, 33152, 128, True), (8, 33160, 128, False), (8, 343744, 128, False),
+    (16, 9472, 2432, True), (16, 9480, 1024, True), (16, 9480, 1152, False), (16, 18944, 896, True), (16, 18952, 896, False),
+    (16, 18952, 1024, True), (16, 23440, 1024, False), (16, 33152, 512, True),
+    (16, 33160, 128, False), (17, 4736, 1664, True), (17, 4744, 1024, True), (17, 4744, 1152, False), (17, 9472, 768, True), (17, 9480, 512, True),
     (17, 9480, 640, False), (17, 16576, 256, True), (17, 16584, 128, False),
     (8, 2112, 7200, False),
 ])
