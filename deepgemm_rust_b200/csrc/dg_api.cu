@@ -441,8 +441,10 @@ static WideWaves wide_waves(uint32_t m, uint32_t n, uint32_t block_n, uint32_t p
 // balanced), and single passes in turn after a 256 MB fill and after 20 ms of idling.  24 problems below 3.5 waves (k 2560-7168, n 1152-7104, 8-50 groups) take 0.96,
 // 0.95 and 0.96 of the other tiles' time with a full arena, 0.98, 1.01 and 1.00 with 3 % of it live, up to 1.07, 1.08 and 1.19 (14 groups of 48 rows, 3200 x 3584: 48.7 ->
 // 52.1 us); 18 above (k 2048-7168, 22-64 groups) 0.96, 0.99 and 0.99 full, 0.98, 0.99 and 0.97 with 3 %.  With fewer tiles it was up to 1.32 (8 groups of 47
-// rows in 13696, 1600 x 7168: 28.5 -> 35.2 us).  K below 16 slabs, and tiles that cover more columns than the others do, lose too (23 groups of
-// 4211 rows, 1152 x 1024, single passes: 1.01; of 1052: 1.14).
+// rows in 13696, 1600 x 7168: 28.5 -> 35.2 us).  K below 16 slabs loses too (23 groups of 4211 rows, 1152 x 1024, single
+// passes: 1.01; of 1052: 1.14), and so do tiles that cover more columns than the others do, unless K is long: 1.03 to 1.05 times as
+// many, full and 3 % live, take 0.99 and 1.02 under load, 1.03 and 1.06 after a fill at 20 slabs of K, 0.98, 0.99, 1.00 and 1.01 at 24-32 (12 problems), 0.95,
+// 0.99, 0.94 and 1.01 from 40 on.
 // Dense problems by cost, within lines.  Of 180 that the cost alone picks (m 200-8192, n 512-16384, k 1024-16384) the 75 inside take 0.96, 0.97 and 0.98 of
 // the other tiles' time, measured in the same ways, up to 1.00, 1.01 and 1.02; the others 0.99, 1.03 and 1.03, up to 1.09, 1.16 and 1.13:
 //   f32 outputs of two e2m1 operands (22 of them: 1.02, 1.06 and 1.06), whose stores take longer than the UMMAs of their K;
@@ -488,7 +490,7 @@ static bool search_wide(const dg_desc* d, uint32_t sms, double other, uint32_t o
         if (smem() > kSmemCapacity) continue;
         const double cost = halves * (total_kb * (2.0 * bn + 130.0) + 1500.0 + (d->cd_dtype == DG_OUT_F32 ? 1000.0 : 0.0)) + 8000.0;
         const uint32_t across = ceil_div(d->n, bn + bn2);
-        const bool wider = across * (bn + bn2) > 1.02 * (ceil_div(d->n, other_n) * other_n);
+        const bool wider = across * (bn + bn2) > (total_kb >= 40 ? 1.06 : (total_kb >= 24 ? 1.04 : 1.02)) * (ceil_div(d->n, other_n) * other_n);
         const bool odd = static_cast<uint32_t>(halves) % 2 != 0;
         bool inside;
         if (!dense) inside = (total_kb >= 20 ? 10 * groups * across >= 13 * pairs : total_kb >= 16 && 2 * groups * across >= 7 * pairs) && group_rows(d) >= 450.0 && !wider;

@@ -160,7 +160,9 @@ MIXED = dict(b_bits=4, gran_b=32)
     # groups whose first 256 rows make 1.3 waves of tiles, whatever the arena holds, with K below 20 slabs three and a half; no more columns than the other tiles have
     ((CONTIGUOUS, 10 * 2048, 4096, 2560, 10), {}, True), ((CONTIGUOUS, 9 * 2048, 4096, 7168, 9), {}, False), ((CONTIGUOUS, 13696, 1600, 7168, 8), {}, False),
     ((CONTIGUOUS, 26 * 2048, 4096, 2048, 26), {}, True), ((CONTIGUOUS, 25 * 2048, 4096, 2048, 25), {}, False), ((CONTIGUOUS, 25 * 2048, 4096, 2560, 25), {}, True),
-    ((CONTIGUOUS, 32 * 2112, 4096, 1920, 32), {}, False), ((CONTIGUOUS, 32 * 2112, 5568, 7168, 32), {}, False),
+    ((CONTIGUOUS, 32 * 2112, 4096, 1920, 32), {}, False), ((CONTIGUOUS, 32 * 2112, 5568, 7168, 32), {}, True),
+    ((CONTIGUOUS, 32 * 2112, 5568, 3072, 32), {}, True), ((CONTIGUOUS, 32 * 2112, 5568, 2944, 32), {}, False), ((CONTIGUOUS, 17 * 1414, 3840, 5120, 17), {}, True),
+    ((CONTIGUOUS, 17 * 1414, 3840, 4992, 17), {}, False),
     ((dg.GemmType.MGroupedMasked, 2048, 4096, 7168, 32, 2048), {}, False), ((dg.GemmType.Batched, 2048, 4096, 7168, 16), {}, False),
 ])
 def test_which_problems_get_them(sizes, kw, wide):
