@@ -1047,20 +1047,16 @@ int launch_skinny(dg_ctx* ctx, const dg_lp_operand* a, const dg_lp_operand* b, c
         reinterpret_cast<uintptr_t>(b->sf) % 16 != 0 || reinterpret_cast<uintptr_t>(out->buf) % 16 != 0)
         return fail(DG_ERR_SHAPE, "operands, scales and output must be 16-byte aligned");
     dg::SkinnyParams p = {static_cast<const uint8_t*>(a->data), static_cast<const uint8_t*>(b->data), a->sf, b->sf, out->buf, pr.m, pr.n, pr.k / 128,
-                          a->ld, b->ld, align4(pr.m), align4(pr.n), out->ld, e.has_alpha ? 1u : 0u, e.alpha};
+                          a->ld, b->ld, align4(pr.m), align4(pr.n), out->ld, e.has_alpha ? 1u : 0u, e.accumulate ? 1u : 0u, e.alpha};
     DG_CUDA(cudaSetDevice(ctx->ordinal));
     const bool f32 = out->kind == DG_OUT_F32;
     const dim3 grid(ceil_div(pr.n, dg::kSkinnyCols));
-    auto run = [&](auto kernel) { return launch(kernel, grid, warps * 32, 0, ctx->stream, p); };
-    auto with_output = [&](auto rows, auto count, auto add) {
-        constexpr uint32_t kTiles = decltype(rows)::value, kWarps = decltype(count)::value;
-        return f32 ? run(dg::dg_gemm_skinny_kernel<kTiles, kWarps, true, decltype(add)::value>) : run(dg::dg_gemm_skinny_kernel<kTiles, kWarps, false, decltype(add)::value>);
-    };
-    auto with_tiles = [&](auto rows, auto count) { return e.accumulate ? with_output(rows, count, std::true_type()) : with_output(rows, count, std::false_type()); };
+    auto run = [&](auto kernel, uint32_t warps) { return launch(kernel, grid, warps * 32, 0, ctx->stream, p); };
     auto with_warps = [&](auto count) {
-        if (tiles == 4) return with_tiles(std::integral_constant<uint32_t, 4>(), count);
-        if (tiles == 1) return with_tiles(std::integral_constant<uint32_t, 1>(), count);
-        return with_tiles(std::integral_constant<uint32_t, 2>(), count);
+        constexpr uint32_t kWarps = decltype(count)::value;
+        if (tiles == 4) return f32 ? run(dg::dg_gemm_skinny_kernel<4, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<4, kWarps, false>, kWarps);
+        if (tiles == 1) return f32 ? run(dg::dg_gemm_skinny_kernel<1, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<1, kWarps, false>, kWarps);
+        return f32 ? run(dg::dg_gemm_skinny_kernel<2, kWarps, true>, kWarps) : run(dg::dg_gemm_skinny_kernel<2, kWarps, false>, kWarps);
     };
     if (print_configs()) fprintf(stderr, "[dgb200] few rows: m=%u n=%u k=%u -> block=%ux%u warps=%u\n", pr.m, pr.n, pr.k, 8 * tiles, dg::kSkinnyCols, warps);
     const cudaError_t ce = warps == 4 ? with_warps(std::integral_constant<uint32_t, 4>()) : (warps == 8 ? with_warps(std::integral_constant<uint32_t, 8>()) : with_warps(std::integral_constant<uint32_t, 16>()));

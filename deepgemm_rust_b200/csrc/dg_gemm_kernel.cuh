@@ -485,7 +485,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                     DG_PROF_T(t_issue);
                     tc_fence_after();
                     // One single-lane region per stage holds the scale copies, every UMMA of the stage and the commits; all operands
-                    // are computed before it by the whole warp (warp-uniform values).  Measured on 4096 x 7168 x 16384 (a size that gets the wide tiles since): with one region
+                    // are computed before it by the whole warp (warp-uniform values).  Measured on 4096 x 7168 x 16384: with one region
                     // per K slab plus one each for the copies and the commits this warp spent 435 cycles per 128 bytes of K issuing
                     // (the tensor pipe needs 512 / 448 at N = 256 / 224 and was starved by the rest of the loop); with one region 283.
                     const uint32_t sfa_addr = smem_u32(smem_sfa + stage * sfa_bytes), sfb_addr = smem_u32(smem_sfb + stage * sfb_bytes);
@@ -515,7 +515,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                     if (leader_lane) {
                         // straight-line code: with run-time trip counts a copy cost this warp ~50 cycles more (beside running UMMAs the
                         // copies themselves are free).  256 x 7168 x 7168 e4m3 x e2m1 19.9 -> 18.5 us, 128 x 7168 x 16384 e4m3 29.5 -> 28.9,
-                        // 4096 x 7168 x 16384 e4m3 347 -> 340 (now with the wide tiles)
+                        // 4096 x 7168 x 16384 e4m3 347 -> 340
                         if (need_a) {
                             #pragma unroll
                             for (uint32_t c = 0; c < kMaxWords; ++c)
@@ -592,7 +592,7 @@ dg_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                     const uint32_t chunks_b = need_b ? plan_b.words * (sf_block_n / 128) : 0u;
                     // Six chunks at a time, their loads all on the way before the first store: one by one (~100 cycles each, a shared-memory
                     // round trip) the 12 chunks of a packed e2m1 stage took longer than its UMMAs, and every stage with new words waited.
-                    // 4096 x 7168 x 7168 mxfp4 78.5 -> 71.6 us (now with the wide tiles, which re-order alike); with fewer chunks per stage nothing changes.
+                    // 4096 x 7168 x 7168 mxfp4 78.5 -> 71.6 us; with fewer chunks per stage nothing changes.
                     constexpr uint32_t kBatch = 6;
                     for (uint32_t c0 = 0; c0 < chunks_a + chunks_b; c0 += kBatch) {
                         uint32_t w[kBatch][4];

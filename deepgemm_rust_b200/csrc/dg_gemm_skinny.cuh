@@ -25,7 +25,7 @@ struct SkinnyParams {
     const uint32_t* sfb;
     void* out;                 // (m, out_ld) bf16 or f32
     uint32_t m, n, k_blocks, a_ld, b_ld, sfa_stride, sfb_stride, out_ld;
-    uint32_t has_alpha;
+    uint32_t has_alpha, accumulate;
     float alpha;
 };
 
@@ -44,8 +44,8 @@ DG_DEVICE float scale_by_exponents(float x, uint32_t ea, uint32_t eb) {
     return ea == 255 || eb == 255 ? __uint_as_float(0x7FC00000u) : y;      // 255 is NaN
 }
 
-// kTiles: activation rows in tiles of 8.  kWarps of a block share K.  kAdd: the product is added to the output.
-template <uint32_t kTiles, uint32_t kWarps, bool kF32, bool kAdd>
+// kTiles: activation rows in tiles of 8.  kWarps of a block share K.
+template <uint32_t kTiles, uint32_t kWarps, bool kF32>
 __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kernel(const __grid_constant__ SkinnyParams p) {
     __shared__ float sums[kWarps][kTiles * 8][kSkinnyCols + 1];
     griddep_wait();
@@ -126,8 +126,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kerne
         for (uint32_t v = 0; v < 4; ++v) sums[warp][i * 8 + 2 * t + v % 2][g + 8 * (v / 2)] = acc[i][v];
     __syncthreads();
     // A thread per output, its sums added in the order of the warps.  Accumulation adds in memory, as the first family's TMA reduction does:
-    // calls on two streams may add into one output.  (In a kernel of its own: beside the plain store, with or without a branch, 15 x 19328 x 1024 took 7.76
-    // instead of 7.58 us.)
+    // calls on two streams may add into one output.
     for (uint32_t o = threadIdx.x; o < kTiles * 8 * kSkinnyCols; o += kWarps * 32) {
         const uint32_t row = o / kSkinnyCols, col = o % kSkinnyCols;
         float s = 0.0f;
@@ -138,12 +137,12 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kerne
         const size_t at = static_cast<size_t>(row) * p.out_ld + n0 + col;
         if constexpr (kF32) {
             float* d = static_cast<float*>(p.out) + at;
-            if constexpr (kAdd) red_add_f32(d, s);
+            if (p.accumulate) red_add_f32(d, s);
             else *d = s;
         } else {
             uint16_t* d = static_cast<uint16_t*>(p.out) + at;
             const uint16_t y = static_cast<uint16_t>(pack_bf16x2(s, 0.0f));
-            if constexpr (kAdd) red_add_bf16(d, y);
+            if (p.accumulate) red_add_bf16(d, y);
             else *d = y;
         }
     }
