@@ -125,23 +125,32 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dg_gemm_skinny_kerne
         #pragma unroll
         for (uint32_t v = 0; v < 4; ++v) sums[warp][i * 8 + 2 * t + v % 2][g + 8 * (v / 2)] = acc[i][v];
     __syncthreads();
-    // A thread per output, its sums added in the order of the warps.  Accumulation adds in memory, as the first family's TMA reduction does:
-    // calls on two streams may add into one output.
-    for (uint32_t o = threadIdx.x; o < kTiles * 8 * kSkinnyCols; o += kWarps * 32) {
-        const uint32_t row = o / kSkinnyCols, col = o % kSkinnyCols;
-        float s = 0.0f;
+    // A thread per output, its sums added in the order of the warps; all of a thread's outputs before the first is stored.  Accumulation adds in memory, as the
+    // first family's TMA reduction does: calls on two streams may add into one output.
+    constexpr uint32_t kOutputs = kTiles * 8 * kSkinnyCols, kEach = (kOutputs + kWarps * 32 - 1) / (kWarps * 32);
+    static_assert(kEach == 1 || kOutputs % (kWarps * 32) == 0, "a thread has all of its outputs or none");
+    float out[kEach];
+    #pragma unroll
+    for (uint32_t i = 0; i < kEach; ++i) {
+        const uint32_t o = threadIdx.x + i * kWarps * 32, row = o / kSkinnyCols, col = o % kSkinnyCols;
+        if (o >= kOutputs) return;
+        out[i] = 0.0f;
         #pragma unroll
-        for (uint32_t w = 0; w < kWarps; ++w) s += sums[w][row][col];
+        for (uint32_t w = 0; w < kWarps; ++w) out[i] += sums[w][row][col];
+        if (p.has_alpha) out[i] *= p.alpha;
+    }
+    #pragma unroll
+    for (uint32_t i = 0; i < kEach; ++i) {
+        const uint32_t o = threadIdx.x + i * kWarps * 32, row = o / kSkinnyCols, col = o % kSkinnyCols;
         if (row >= p.m || n0 + col >= p.n) continue;
-        if (p.has_alpha) s *= p.alpha;
         const size_t at = static_cast<size_t>(row) * p.out_ld + n0 + col;
         if constexpr (kF32) {
             float* d = static_cast<float*>(p.out) + at;
-            if (p.accumulate) red_add_f32(d, s);
-            else *d = s;
+            if (p.accumulate) red_add_f32(d, out[i]);
+            else *d = out[i];
         } else {
             uint16_t* d = static_cast<uint16_t*>(p.out) + at;
-            const uint16_t y = static_cast<uint16_t>(pack_bf16x2(s, 0.0f));
+            const uint16_t y = static_cast<uint16_t>(pack_bf16x2(out[i], 0.0f));
             if (p.accumulate) red_add_bf16(d, y);
             else *d = y;
         }
