@@ -618,7 +618,7 @@ def _desc(desc: Sm100Desc) -> _Desc:
 
 
 def kernel_name(desc: Sm100Desc) -> Optional[str]:
-    """The kernel that a call of this description launches."""
+    """The kernel that a call of this description launches, unless it accumulates or sets a duty cycle."""
     name = _kernel_name(C.byref(_desc(desc)))
     return name.decode() if name else None
 
